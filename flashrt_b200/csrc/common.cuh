@@ -39,8 +39,12 @@ __device__ __forceinline__ void unpack_bf16x2(uint32_t w, float& lo, float& hi) 
 __device__ __forceinline__ uint32_t f32_to_bf16_bits(float f) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(f));
 }
+// both halves in one conversion: two scalar ones and an or go through the slow transcendental pipe (one instruction per
+// value there in the LayerNorm kernel's profile)
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    return f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
 // ---------------------------------------------------------------- fp8 e4m3
@@ -53,6 +57,8 @@ __device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float lo, float hi) {
     // low byte = lo, high byte = hi
     return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
 }
+// clamp448 in front of the conversion, in one instruction: the conversion itself saturates, and fmaxf maps NaN to -448
+__device__ __forceinline__ float clamp448_lo(float v) { return fmaxf(v, -448.0f); }
 __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, float d) {
     return f32x2_to_e4m3x2(a, b) | (f32x2_to_e4m3x2(c, d) << 16);
 }
@@ -124,6 +130,41 @@ __device__ __forceinline__ float warp_max_butterfly(float v) {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
     return v;
+}
+
+// One warp per row: the same sum as "butterfly per 256-column warp slice, then the slices in order" (the tree of the
+// one-CTA-per-row kernels and of the C oracle), for a row whose slices all live in ONE warp -- part[w] is this lane's
+// partial of slice w.  The butterflies of all slices run together: at every exchange distance a lane keeps half of the
+// slices it still holds and hands its partner the other half, so NS slices cost about NS + 5 shuffles instead of 5 * NS
+// (every addition keeps its two operands, and an IEEE addition commutes: same bits).  Slices from `n` on do not enter the
+// total.
+template <int NS>
+__device__ __forceinline__ float warp_row_total(const float (&part)[NS], int n) {
+    constexpr int P = NS <= 1 ? 1 : NS <= 2 ? 2 : NS <= 4 ? 4 : NS <= 8 ? 8 : NS <= 16 ? 16 : 32;
+    static_assert(NS <= 32, "at most 32 slices of 256 columns");
+    const int lane = threadIdx.x & 31;
+    float v[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) v[i] = i < NS ? part[i] : 0.0f;
+    int d = 16;
+#pragma unroll
+    for (int h = P / 2; h >= 1; h >>= 1, d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, d));
+        }
+    }
+#pragma unroll
+    for (; d >= 1; d >>= 1) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], d));
+    float tot = __shfl_sync(0xffffffffu, v[0], 0);
+#pragma unroll
+    for (int w = 1; w < NS; ++w) {
+        const float x = __shfl_sync(0xffffffffu, v[0], w * (32 / P));
+        if (w < n) tot = __fadd_rn(tot, x);
+    }
+    return tot;
 }
 
 // Element of every bf16 GEMM epilogue: alpha * acc, or alpha * acc + bias with ONE rounding.  Written out so that every

@@ -161,15 +161,16 @@ norm_row_kernel(NormArgs a) {
         constexpr int FAM = OUT == OUT_NVFP4_A ? 0 : 1;
         float amax = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = __bfloat162float(__float2bfloat16_rn(v[i]));
-            amax = fmaxf(amax, fabsf(v[i]));
+        for (int i = 0; i < 8; i += 2) {
+            unpack_bf16x2(pack_bf16x2(v[i], v[i + 1]), v[i], v[i + 1]);
+            amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[i + 1])));
         }
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        float inv;
-        const uint32_t sb = nvfp4::block_scale<FAM>(amax, inv);
+        float s;
+        const uint32_t sb = nvfp4::block_scale<FAM>(amax, s);
+        const float2 inv = nvfp4::inv_off_ties<FAM>(nvfp4::inverse<FAM>(s), s);
         if (active) {
-            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(a.out) + (roff >> 1)) = nvfp4::pack8<FAM>(v, inv);
+            *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(a.out) + (roff >> 1)) = nvfp4::pack8_bf16<FAM>(v, s, inv);
             if ((tid & 1) == 0) a.sf_out[nvfp4::sf_offset(row, col >> 4, (a.dim + 63) >> 6)] = (uint8_t)sb;
             if (HAS_STYLE && a.gate_out) st_global_v4(a.gate_out + roff, gt);
         }
@@ -193,10 +194,148 @@ norm_row_kernel(NormArgs a) {
     if (HAS_STYLE && a.gate_out) st_global_v4(a.gate_out + roff, gt);
 }
 
+// Many rows: one WARP per row, the row in registers (NS slices of 256 columns, 16 bytes per lane and slice, bf16 bits).
+// The one-CTA-per-row kernel above is bound by its latency chain -- one load, one block barrier and a serial sum of warp
+// totals per 6 KB row, with five CTAs of 384 threads on an SM.  Here every lane has NS loads in flight, there is no barrier,
+// and 16-24 rows share an SM.  Same sums in the same order (warp_row_total), same bits.  RMSNorm -> FP8: 8192 x 3072 27.2 ->
+// 18.2 us, 20480 x 3072 63.7 -> 36.9 us (5.1 TB/s); -> NVFP4: 20480 x 3072 85.7 -> 59.9 us (bound by its instructions).
+template <int OUT, int NS>
+__global__ void __launch_bounds__(128)
+norm_warp_kernel(NormArgs a) {
+    constexpr bool OUT_FP8 = OUT == OUT_E4M3;
+    constexpr bool OUT_FP4 = OUT == OUT_NVFP4_A || OUT == OUT_NVFP4_B;
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    float inv_scale = 1.0f;
+    if (OUT_FP8) inv_scale = __fdiv_rn(1.0f, *a.d_scale);
+    if (row >= a.rows) return;
+    const int n = (a.dim + 255) >> 8;                       // slices of this row, n <= NS
+    const size_t rbase = (size_t)row * a.dim + lane * 8;
+    const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
+    uint8_t* sf = nullptr;                                  // scale byte of this lane's block: + 4 atoms per slice
+    const bool sf_words = OUT_FP4 && (a.dim & 63) == 0;
+    if (OUT_FP4) sf = a.sf_out + nvfp4::sf_offset(row, (lane >> 3) * 4, (a.dim + 63) >> 6);
+    pdl_wait();
+    uint4 rv[NS];
+    float ssq[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        rv[w] = make_uint4(0, 0, 0, 0);
+        if (w * 256 < left) rv[w] = ld_stream_v4(a.residual + rbase + w * 256);
+    }
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float r0, r1;
+            unpack_bf16x2(rw[i], r0, r1);
+            s = __fmaf_rn(r0, r0, s);
+            s = __fmaf_rn(r1, r1, s);
+        }
+        ssq[w] = s;
+    }
+    const float tot = warp_row_total<NS>(ssq, n);
+    const float var = __fadd_rn(__fdiv_rn(tot, (float)a.dim), a.eps);
+    const float rms = __fdiv_rn(1.0f, __fsqrt_rn(var));
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const bool on = w * 256 < left;
+        uint4 wv = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+        if (on && a.weight) wv = ld_global_v4(a.weight + lane * 8 + w * 256);
+        const uint32_t* rw = &rv[w].x;
+        const uint32_t* ww = &wv.x;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float r0, r1, w0, w1;
+            unpack_bf16x2(rw[i], r0, r1);
+            unpack_bf16x2(ww[i], w0, w1);
+            v[2 * i] = __fmul_rn(__fmul_rn(r0, rms), w0);
+            v[2 * i + 1] = __fmul_rn(__fmul_rn(r1, rms), w1);
+        }
+        const size_t roff = rbase + w * 256;
+        if (OUT_FP4) {
+            constexpr int FAM = OUT == OUT_NVFP4_A ? 0 : 1;
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                unpack_bf16x2(pack_bf16x2(v[i], v[i + 1]), v[i], v[i + 1]);
+                amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[i + 1])));
+            }
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            float s;
+            uint32_t sb = nvfp4::block_scale<FAM>(amax, s);
+            const float2 inv = nvfp4::inv_off_ties<FAM>(nvfp4::inverse<FAM>(s), s);
+            const uint32_t pk = nvfp4::pack8_bf16<FAM>(v, s, inv);
+            if (on) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(a.out) + (roff >> 1)) = pk;
+            // the scale bytes of four neighbouring blocks (eight lanes) are one aligned word of the scale layout
+            if (sf_words) {
+                sb |= __shfl_down_sync(0xffffffffu, sb, 2) << 8;
+                sb |= __shfl_down_sync(0xffffffffu, sb, 4) << 16;
+                if (on && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf + w * 2048) = sb;
+            } else if (on && (lane & 1) == 0) {
+                sf[w * 2048 + ((lane >> 1) & 3)] = (uint8_t)sb;
+            }
+        } else if (OUT_FP8) {
+            uint2 o;
+            o.x = f32x4_to_e4m3x4(clamp448_lo(__fmul_rn(v[0], inv_scale)), clamp448_lo(__fmul_rn(v[1], inv_scale)),
+                                  clamp448_lo(__fmul_rn(v[2], inv_scale)), clamp448_lo(__fmul_rn(v[3], inv_scale)));
+            o.y = f32x4_to_e4m3x4(clamp448_lo(__fmul_rn(v[4], inv_scale)), clamp448_lo(__fmul_rn(v[5], inv_scale)),
+                                  clamp448_lo(__fmul_rn(v[6], inv_scale)), clamp448_lo(__fmul_rn(v[7], inv_scale)));
+            if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + roff, o);
+        } else {
+            uint4 o;
+            o.x = pack_bf16x2(v[0], v[1]);
+            o.y = pack_bf16x2(v[2], v[3]);
+            o.z = pack_bf16x2(v[4], v[5]);
+            o.w = pack_bf16x2(v[6], v[7]);
+            if (on) st_global_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + roff, o);
+        }
+    }
+}
+
+template <int OUT, int NS>
+static int launch_norm_warp(const NormArgs& a, cudaStream_t stream, bool pdl) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((a.rows + 3) / 4));
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, norm_warp_kernel<OUT, NS>, a);
+    return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
+}
+
+// Rows from which the warp-per-row kernel wins (graph of back-to-back launches, dim 1024 .. 4096): below, the rows of the
+// CTA kernel are all on the chip at once and its chain is shorter.  The NVFP4 result needs twice the instructions per
+// value, so more rows have to share an SM before the load latency is what counts.  The residual form stays with the CTA
+// kernel at every size (it already streams 5.6 TB/s; two register-held rows per lane were slower).
+template <int OUT>
+static constexpr int norm_warp_rows() { return OUT == OUT_BF16 || OUT == OUT_E4M3 ? 1536 : 3072; }
+
 template <bool HAS_X, bool HAS_GATE, bool HAS_STYLE, int OUT>
 static int launch_norm(const NormArgs& a, cudaStream_t stream, bool pdl) {
     if (a.rows < 0 || a.dim <= 0 || (a.dim & 7) || a.dim > 8192) return FRT_ERR_UNSUPPORTED;
     if (a.rows == 0) return FRT_OK;
+    if (!HAS_X && !HAS_STYLE && a.rows >= norm_warp_rows<OUT>() && a.dim > 512 &&
+        (reinterpret_cast<uintptr_t>(a.sf_out) & 3) == 0) {
+        switch ((a.dim + 511) / 512) {
+            case 2: return launch_norm_warp<OUT, 4>(a, stream, pdl);
+            case 3: return launch_norm_warp<OUT, 6>(a, stream, pdl);
+            case 4: return launch_norm_warp<OUT, 8>(a, stream, pdl);
+            case 5: return launch_norm_warp<OUT, 10>(a, stream, pdl);
+            case 6: return launch_norm_warp<OUT, 12>(a, stream, pdl);
+            case 7: return launch_norm_warp<OUT, 14>(a, stream, pdl);
+            case 8: return launch_norm_warp<OUT, 16>(a, stream, pdl);
+            default: break;                                  // wider rows: the CTA kernel
+        }
+    }
     int threads = ((a.dim / 8 + 31) / 32) * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.rows);

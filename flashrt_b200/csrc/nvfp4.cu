@@ -48,11 +48,18 @@ quantize_nvfp4_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict_
             if (has_g) v[i] = __fmul_rn(v[i], inv_g);
             amax = fmaxf(amax, fabsf(v[i]));
         }
-        float inv;
-        const uint32_t sb = nvfp4::block_scale<FAMILY>(amax, inv);
+        float s;
+        const uint32_t sb = nvfp4::block_scale<FAMILY>(amax, s);
+        const float inv = nvfp4::inverse<FAMILY>(s);
         uint2 o;
-        o.x = nvfp4::pack8<FAMILY>(v, inv);
-        o.y = nvfp4::pack8<FAMILY>(v + 8, inv);
+        if (has_g) {
+            o.x = nvfp4::pack8<FAMILY>(v, inv);
+            o.y = nvfp4::pack8<FAMILY>(v + 8, inv);
+        } else {
+            const float2 inv2 = nvfp4::inv_off_ties<FAMILY>(inv, s);
+            o.x = nvfp4::pack8_bf16<FAMILY>(v, s, inv2);
+            o.y = nvfp4::pack8_bf16<FAMILY>(v + 8, s, inv2);
+        }
         st_global_v2(packed + row * (D >> 1) + blk * 8, o);
         sf[nvfp4::sf_offset(row, blk, katoms)] = (uint8_t)sb;
     }
@@ -87,8 +94,9 @@ geglu_nvfp4_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict
             v[2 * i + 1] = __fmul_rn(det_gelu_tanh(gb), ub);
             amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
         }
-        float inv;
-        const uint32_t sb = nvfp4::block_scale<FAMILY>(amax, inv);
+        float s;
+        const uint32_t sb = nvfp4::block_scale<FAMILY>(amax, s);
+        const float inv = nvfp4::inverse<FAMILY>(s);
         uint2 o;
         o.x = nvfp4::pack8<FAMILY>(v, inv);
         o.y = nvfp4::pack8<FAMILY>(v + 8, inv);
