@@ -141,6 +141,174 @@ layer_norm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
     }
 }
 
+// Many rows: one warp per row, the row in registers as bf16 bits (NS slices of 256 columns).  The one-CTA-per-row kernel
+// above needs four block barriers and two serial sums of warp totals per 6 KB row; this one has NS loads of a row in flight
+// per lane, no barrier and the same sums in the same order (warp_row_total): 20480 x 3072 -> FP8 125 -> 54 us.
+// With `x` the residual update in front of the norm is part of the pass (one read and one write of the stream saved):
+//   res_out = bf16(res + x * gate)   (gate NULL: res + x),  y = LayerNorm of the rounded value.
+struct ResNormArgs {
+    const __nv_bfloat16* res;      // (rows, dim)
+    const __nv_bfloat16* x;        // (rows, dim) or null
+    const __nv_bfloat16* gate;     // rows at + (r / mod_rows) * mod_stride, or null
+    __nv_bfloat16* res_out;        // (rows, dim), may be res; unused without x
+    const __nv_bfloat16* weight;
+    const __nv_bfloat16* bias;
+    const __nv_bfloat16* scale;    // rows at + (r / mod_rows) * mod_stride
+    const __nv_bfloat16* shift;
+    long long mod_stride, mod_rows;
+    void* out;                     // null: residual update only
+    const float* d_scale;
+    long long rows;
+    int dim;
+    float eps;
+};
+
+// AFFINE / MOD: weight, bias / scale, shift given (both, neither: any combination)
+template <bool OUT_FP8, int NS, bool AFFINE, bool MOD>
+__global__ void __launch_bounds__(128, NS <= 12 ? 5 : NS <= 16 ? 4 : 2)
+layer_norm_warp_kernel(ResNormArgs a) {
+    const int lane = threadIdx.x & 31;
+    const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    float inv_a = 1.0f;
+    if (OUT_FP8 && a.out) inv_a = __fdiv_rn(1.0f, *a.d_scale);
+    if (row >= a.rows) return;
+    const int n = (a.dim + 255) >> 8;                       // n <= NS
+    const size_t rbase = (size_t)row * a.dim + lane * 8;
+    const size_t mbase = (size_t)(row / a.mod_rows) * a.mod_stride + lane * 8;
+    const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
+    pdl_wait();
+    uint4 rv[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        rv[w] = make_uint4(0, 0, 0, 0);
+        if (w * 256 < left) rv[w] = ld_stream_v4(a.res + rbase + w * 256);
+    }
+    if (a.x) {
+        constexpr int B = 4;                                // slices of x in flight
+#pragma unroll
+        for (int w0 = 0; w0 < NS; w0 += B) {
+            uint4 xv[B], gv[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                xv[j] = make_uint4(0, 0, 0, 0);
+                gv[j] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);   // no gate: x * 1 + r rounds once, as the add
+                if (w0 + j < NS && (w0 + j) * 256 < left) {
+                    xv[j] = ld_stream_v4(a.x + rbase + (w0 + j) * 256);
+                    if (a.gate) gv[j] = ld_global_v4(a.gate + mbase + (w0 + j) * 256);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < B && w0 + j < NS; ++j) {
+                const int w = w0 + j;
+                uint32_t* rw = &rv[w].x;
+                const uint32_t* xw = &xv[j].x;
+                const uint32_t* gw = &gv[j].x;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float r0, r1, x0, x1, g0, g1;
+                    unpack_bf16x2(rw[i], r0, r1);
+                    unpack_bf16x2(xw[i], x0, x1);
+                    unpack_bf16x2(gw[i], g0, g1);
+                    rw[i] = pack_bf16x2(__fmaf_rn(x0, g0, r0), __fmaf_rn(x1, g1, r1));
+                }
+                if (w * 256 < left) st_global_v4(a.res_out + rbase + w * 256, rv[w]);
+            }
+        }
+    }
+    pdl_launch_dependents();
+    if (!a.out) return;
+    float part[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            s = __fadd_rn(s, v0);
+            s = __fadd_rn(s, v1);
+        }
+        part[w] = s;
+    }
+    const float mean = __fdiv_rn(warp_row_total<NS>(part, n), (float)a.dim);
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float q = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            v0 = __fsub_rn(v0, mean);
+            v1 = __fsub_rn(v1, mean);
+            q = __fmaf_rn(v0, v0, q);
+            q = __fmaf_rn(v1, v1, q);
+        }
+        part[w] = w * 256 < left ? q : 0.0f;
+    }
+    const float var = __fadd_rn(__fdiv_rn(warp_row_total<NS>(part, n), (float)a.dim), a.eps);
+    const float inv_std = __fdiv_rn(1.0f, __fsqrt_rn(var));
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const bool on = w * 256 < left;
+        uint4 wv = make_uint4(0, 0, 0, 0), bv = wv, sc = wv, sh = wv;
+        if (on) {
+            if (AFFINE) {
+                wv = ld_global_v4(a.weight + lane * 8 + w * 256);
+                if (a.bias) bv = ld_global_v4(a.bias + lane * 8 + w * 256);
+            }
+            if (MOD) {
+                sc = ld_global_v4(a.scale + mbase + w * 256);
+                sh = ld_global_v4(a.shift + mbase + w * 256);
+            }
+        }
+        const uint32_t* rw = &rv[w].x;
+        const uint32_t* ww = &wv.x;
+        const uint32_t* bw = &bv.x;
+        const uint32_t* scw = &sc.x;
+        const uint32_t* shw = &sh.x;
+        uint4 o16;
+        uint32_t* ow = &o16.x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            float n0 = __fmul_rn(__fsub_rn(v0, mean), inv_std), n1 = __fmul_rn(__fsub_rn(v1, mean), inv_std);
+            if (AFFINE) {
+                float w0, w1, b0, b1;
+                unpack_bf16x2(ww[i], w0, w1);
+                unpack_bf16x2(bw[i], b0, b1);
+                n0 = __fmaf_rn(n0, w0, b0);
+                n1 = __fmaf_rn(n1, w1, b1);
+            }
+            if (MOD) {
+                float s0, s1, h0, h1;
+                unpack_bf16x2(scw[i], s0, s1);
+                unpack_bf16x2(shw[i], h0, h1);
+                n0 = __fmaf_rn(n0, __fadd_rn(1.0f, s0), h0);
+                n1 = __fmaf_rn(n1, __fadd_rn(1.0f, s1), h1);
+            }
+            ow[i] = pack_bf16x2(n0, n1);
+        }
+        if (!OUT_FP8) {
+            if (on) st_global_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + rbase + w * 256, o16);
+        } else {
+            float r[8];                                      // quantise the bf16-rounded value
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                unpack_bf16x2(ow[i], r[2 * i], r[2 * i + 1]);
+                r[2 * i] = clamp448_lo(__fmul_rn(r[2 * i], inv_a));
+                r[2 * i + 1] = clamp448_lo(__fmul_rn(r[2 * i + 1], inv_a));
+            }
+            uint2 o8;
+            o8.x = f32x4_to_e4m3x4(r[0], r[1], r[2], r[3]);
+            o8.y = f32x4_to_e4m3x4(r[4], r[5], r[6], r[7]);
+            if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + rbase + w * 256, o8);
+        }
+    }
+}
+
 // ------------------------------------------------------------------ QKV split + q/k RMSNorm + 3-D RoPE
 // packed (rows, 3*dim) bf16 = [q | k | v]; q_out / k_out (rows, dim); row = b * L + t
 __global__ void __launch_bounds__(1024)
@@ -223,6 +391,95 @@ qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_
     }
     st_global_v4(q_out + (size_t)row * dim + col, oq);
     st_global_v4(k_out + (size_t)row * dim + col, ok);
+}
+
+// Many rows: one warp per (row, q or k); see layer_norm_warp_kernel.  20480 x 3 x 3072: 163 -> 82 us (6.2 TB/s).
+template <int NS>
+__global__ void __launch_bounds__(128)
+qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_bfloat16* __restrict__ wq,
+                                const __nv_bfloat16* __restrict__ wk, const float* __restrict__ fre,
+                                const float* __restrict__ fim, __nv_bfloat16* __restrict__ q_out,
+                                __nv_bfloat16* __restrict__ k_out, int L, int dim, int D_h, int seq_len, float eps,
+                                const float* __restrict__ ext_ssq_q, const float* __restrict__ ext_ssq_k, int full_dim,
+                                int rows) {
+    const int lane = threadIdx.x & 31;
+    const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int row = item >> 1;
+    const bool is_k = item & 1;
+    if (row >= rows) return;
+    const int n = (dim + 255) >> 8;
+    const int t = row % L;
+    const bool rope = t < seq_len;
+    const __nv_bfloat16* w_ = (is_k ? wk : wq) + lane * 8;
+    const __nv_bfloat16* src = packed + (size_t)row * 3 * dim + (is_k ? dim : 0) + lane * 8;
+    __nv_bfloat16* dst = (is_k ? k_out : q_out) + (size_t)row * dim + lane * 8;
+    const int left = dim - lane * 8;                        // slice w of this lane exists while w * 256 < left
+    pdl_wait();
+    uint4 xv[NS];
+    float part[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        xv[w] = make_uint4(0, 0, 0, 0);
+        if (w * 256 < left) xv[w] = ld_stream_v4(src + w * 256);
+    }
+    pdl_launch_dependents();
+    const float* ext = is_k ? ext_ssq_k : ext_ssq_q;
+    float tot;
+    if (ext) {
+        tot = ext[row];
+    } else {
+#pragma unroll
+        for (int w = 0; w < NS; ++w) {
+            const uint32_t* xw = &xv[w].x;
+            float s = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float a, b;
+                unpack_bf16x2(xw[i], a, b);
+                s = __fmaf_rn(a, a, s);
+                s = __fmaf_rn(b, b, s);
+            }
+            part[w] = s;
+        }
+        tot = warp_row_total<NS>(part, n);
+    }
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, (float)full_dim), eps)));
+    // a head of 8, 16, ..., 256 columns (a power of two): this lane sits at the same place of a head in every slice
+    const bool same_place = (D_h & (D_h - 1)) == 0 && D_h <= 256;
+    float4 fr = make_float4(1.f, 1.f, 1.f, 1.f), fi = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* fre_t = fre + (size_t)t * (D_h >> 1);
+    const float* fim_t = fim + (size_t)t * (D_h >> 1);
+    if (rope && same_place && left > 0) {
+        fr = *reinterpret_cast<const float4*>(fre_t + ((lane * 8) & (D_h - 1)) / 2);
+        fi = *reinterpret_cast<const float4*>(fim_t + ((lane * 8) & (D_h - 1)) / 2);
+    }
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const bool on = w * 256 < left;
+        uint4 wv = make_uint4(0, 0, 0, 0);
+        if (on) wv = ld_global_v4(w_ + w * 256);
+        if (on && rope && !same_place) {
+            const int cp = ((w * 256 + lane * 8) % D_h) >> 1;   // first complex pair of this vector inside its head
+            fr = *reinterpret_cast<const float4*>(fre_t + cp);
+            fi = *reinterpret_cast<const float4*>(fim_t + cp);
+        }
+        const float f_re[4] = {fr.x, fr.y, fr.z, fr.w}, f_im[4] = {fi.x, fi.y, fi.z, fi.w};
+        const uint32_t* xw = &xv[w].x;
+        const uint32_t* ww = &wv.x;
+        uint4 o;
+        uint32_t* ow = &o.x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float x0, x1, a0, a1;
+            unpack_bf16x2(xw[i], x0, x1);
+            unpack_bf16x2(ww[i], a0, a1);
+            const float re = __fmul_rn(__fmul_rn(x0, inv), a0), im = __fmul_rn(__fmul_rn(x1, inv), a1);
+            ow[i] = rope ? pack_bf16x2(__fmaf_rn(re, f_re[i], -__fmul_rn(im, f_im[i])),
+                                       __fmaf_rn(re, f_im[i], __fmul_rn(im, f_re[i])))
+                         : pack_bf16x2(re, im);
+        }
+        if (on) st_global_v4(dst + w * 256, o);
+    }
 }
 
 // ------------------------------------------------------------------ bias + GELU(tanh) -> FP8
@@ -402,6 +659,26 @@ static inline unsigned cap_grid(long long items, int threads) {
     return (unsigned)(need < 1 ? 1 : (need < cap ? need : cap));
 }
 
+// Rows from which the warp-per-row kernels win over one CTA per row (graph of back-to-back launches, dim 1024 .. 4096).
+enum { LN_WARP_ROWS = 1024, ROPE_WARP_ROWS = 512 };
+
+template <bool OUT_FP8, bool AFFINE, bool MOD>
+static int launch_layer_norm_warp(const ResNormArgs& a, bool pdl, cudaStream_t s) {
+    const unsigned grid = (unsigned)((a.rows + 3) / 4);
+    if (a.dim <= 1024) return launch_k(layer_norm_warp_kernel<OUT_FP8, 4, AFFINE, MOD>, grid, 128, s, pdl, a);
+    if (a.dim <= 2048) return launch_k(layer_norm_warp_kernel<OUT_FP8, 8, AFFINE, MOD>, grid, 128, s, pdl, a);
+    if (a.dim <= 3072) return launch_k(layer_norm_warp_kernel<OUT_FP8, 12, AFFINE, MOD>, grid, 128, s, pdl, a);
+    if (a.dim <= 4096) return launch_k(layer_norm_warp_kernel<OUT_FP8, 16, AFFINE, MOD>, grid, 128, s, pdl, a);
+    return launch_k(layer_norm_warp_kernel<OUT_FP8, 32, AFFINE, MOD>, grid, 128, s, pdl, a);
+}
+template <bool OUT_FP8>
+static int dispatch_layer_norm_warp(const ResNormArgs& a, bool pdl, cudaStream_t s) {
+    if (a.weight) return a.scale ? launch_layer_norm_warp<OUT_FP8, true, true>(a, pdl, s)
+                                 : launch_layer_norm_warp<OUT_FP8, true, false>(a, pdl, s);
+    return a.scale ? launch_layer_norm_warp<OUT_FP8, false, true>(a, pdl, s)
+                   : launch_layer_norm_warp<OUT_FP8, false, false>(a, pdl, s);
+}
+
 }  // namespace frt
 
 using namespace frt;
@@ -422,6 +699,23 @@ int frt_b200_layer_norm(const void* x, const void* weight, const void* bias, con
         mis(out_fp8, 8))
         return FRT_ERR_INVALID;
     if (rows == 0) return FRT_OK;
+    if (rows >= LN_WARP_ROWS) {
+        ResNormArgs a = {};
+        a.res = (const __nv_bfloat16*)x;
+        a.weight = (const __nv_bfloat16*)weight;
+        a.bias = (const __nv_bfloat16*)bias;
+        a.scale = (const __nv_bfloat16*)scale;
+        a.shift = (const __nv_bfloat16*)shift;
+        a.mod_stride = mod_stride;
+        a.mod_rows = 1;
+        a.out = out_fp8 ? out_fp8 : out_bf16;
+        a.d_scale = d_scale;
+        a.rows = rows;
+        a.dim = dim;
+        a.eps = eps;
+        return out_fp8 ? dispatch_layer_norm_warp<true>(a, flags & 1, (cudaStream_t)stream)
+                       : dispatch_layer_norm_warp<false>(a, flags & 1, (cudaStream_t)stream);
+    }
     const unsigned threads = ((dim / 8 + 31) / 32) * 32;
     auto X = (const __nv_bfloat16*)x;
     auto W = (const __nv_bfloat16*)weight;
@@ -433,6 +727,30 @@ int frt_b200_layer_norm(const void* x, const void* weight, const void* bias, con
                         mod_stride, out_fp8, d_scale, dim, eps);
     return launch_k(layer_norm_row_kernel<false>, rows, threads, (cudaStream_t)stream, flags & 1, X, W, B, SC, SH,
                     mod_stride, out_bf16, d_scale, dim, eps);
+}
+
+// Residual update and the LayerNorm behind it in one pass (bias_gate_mul_residual / residual_add, then ada_layer_norm_fp8
+// or layer_norm -> FP8; the same bits as the two calls):
+//   res_out = bf16(res + x * gate)  (gate NULL: res + x; x NULL: no update),
+//   out_fp8 = e4m3(clamp(bf16(LN(res_out) [* weight + bias] [* (1 + scale) + shift]) * (1 / *d_scale))), NULL: update only.
+// gate / scale / shift rows at + (r / mod_rows) * mod_stride: one row per batch element of mod_rows tokens.
+int frt_b200_residual_layer_norm_fp8(const void* res, const void* x, const void* gate, void* res_out, const void* weight,
+                                     const void* bias, const void* scale, const void* shift, long long mod_stride,
+                                     long long mod_rows, void* out_fp8, const float* d_scale, long long rows, int dim,
+                                     float eps, int flags, void* stream) {
+    if (!res || rows < 0 || dim <= 0 || mod_rows <= 0 || (!x && !out_fp8)) return FRT_ERR_INVALID;
+    if ((x && !res_out) || (gate && !x) || (out_fp8 && !d_scale)) return FRT_ERR_INVALID;
+    if ((scale == nullptr) != (shift == nullptr) || (bias && !weight)) return FRT_ERR_INVALID;
+    if ((dim & 7) || dim > 8192 || (mod_stride & 7)) return FRT_ERR_UNSUPPORTED;
+    if (mis(res, 16) || mis(x, 16) || mis(gate, 16) || mis(res_out, 16) || mis(weight, 16) || mis(bias, 16) ||
+        mis(scale, 16) || mis(shift, 16) || mis(out_fp8, 8))
+        return FRT_ERR_INVALID;
+    if (rows == 0) return FRT_OK;
+    ResNormArgs a = {(const __nv_bfloat16*)res, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gate,
+                     (__nv_bfloat16*)res_out, (const __nv_bfloat16*)weight, (const __nv_bfloat16*)bias,
+                     (const __nv_bfloat16*)scale, (const __nv_bfloat16*)shift, mod_stride, mod_rows, out_fp8, d_scale,
+                     rows, dim, eps};
+    return dispatch_layer_norm_warp<true>(a, flags & 1, (cudaStream_t)stream);
 }
 
 // packed_qkv (B*L, 3*dim) bf16, dim = N * D_h; q_out / k_out (B*L, dim); freqs (seq_len.., D_h/2) fp32.
@@ -448,6 +766,21 @@ int frt_b200_qkv_split_norm_rope(const void* packed_qkv, const void* norm_q_w, c
         mis(q_out, 16) || mis(k_out, 16))
         return FRT_ERR_INVALID;
     if (B == 0) return FRT_OK;
+    const bool ext = ext_ssq_q && ext_ssq_k;
+    const long long rows = (long long)B * L;
+    if (rows >= ROPE_WARP_ROWS && rows < (1LL << 30) && dim <= 4096) {
+        auto go = [&](auto kern) {
+            return launch_k(kern, (unsigned)((rows * 2 + 3) / 4), 128, (cudaStream_t)stream, flags & 1,
+                            (const __nv_bfloat16*)packed_qkv, (const __nv_bfloat16*)norm_q_w,
+                            (const __nv_bfloat16*)norm_k_w, freqs_re, freqs_im, (__nv_bfloat16*)q_out,
+                            (__nv_bfloat16*)k_out, L, (int)dim, D_h, seq_len, eps, ext ? ext_ssq_q : (const float*)nullptr,
+                            ext ? ext_ssq_k : (const float*)nullptr, ext && full_dim > 0 ? full_dim : (int)dim, (int)rows);
+        };
+        if (dim <= 1024) return go(qkv_split_norm_rope_warp_kernel<4>);
+        if (dim <= 2048) return go(qkv_split_norm_rope_warp_kernel<8>);
+        if (dim <= 3072) return go(qkv_split_norm_rope_warp_kernel<12>);
+        return go(qkv_split_norm_rope_warp_kernel<16>);
+    }
     const unsigned threads = (unsigned)(((dim / 8 + 31) / 32) * 32);
     return launch_k(qkv_split_norm_rope_kernel, (unsigned)(B * L), threads, (cudaStream_t)stream, flags & 1,
                     (const __nv_bfloat16*)packed_qkv, (const __nv_bfloat16*)norm_q_w, (const __nv_bfloat16*)norm_k_w,

@@ -185,6 +185,15 @@ def ada_layer_norm_fp8(x_bf16, scale_bf16, shift_bf16, out_fp8, act_scale, seq_l
          seq_len, dim, eps, _f(pdl), stream)
 
 
+def residual_layer_norm_fp8(res, x, gate, res_out, out_fp8, act_scale, rows, dim, eps=1e-6, stream=0, *, weight=0, bias=0,
+                            scale=0, shift=0, mod_stride=0, mod_rows=1, pdl=False):
+    """``bias_gate_mul_residual_bf16`` (gate 0: ``residual_add``; x 0: no update) and the LayerNorm -> FP8 behind it in one
+    pass.  gate / scale / shift: one row of ``mod_stride`` elements per ``mod_rows`` rows.  out_fp8 0: update only."""
+    call("frt_b200_residual_layer_norm_fp8", res, x or None, gate or None, res_out or None, weight or None, bias or None,
+         scale or None, shift or None, mod_stride, mod_rows, out_fp8 or None, act_scale or None, rows, dim, eps, _f(pdl),
+         stream)
+
+
 def qkv_split_norm_rope_bf16(packed_qkv, norm_q_w, norm_k_w, freqs_re, freqs_im, q_rope_out, k_rope_out, B, L_v, N,
                              D_h, seq_len, eps=1e-6, stream=0, *, pdl=False, ext_ssq_q=0, ext_ssq_k=0, full_dim=0):
     call("frt_b200_qkv_split_norm_rope", packed_qkv, norm_q_w, norm_k_w, freqs_re, freqs_im, q_rope_out, k_rope_out,

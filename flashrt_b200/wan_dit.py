@@ -189,7 +189,7 @@ class WanDiTB200:
         self.cq, self.cqn = z(M, dl), z(M, dl)
         self.f1, self.f8 = z(M, fl), z(M, fl, dtype=torch.uint8)
         self.ssq = z(2, M, dtype=torch.float32)
-        self.e = z(6, self.B, D)
+        self.e2 = z(2, 6, self.B, D)                       # modulation tensors, alternating between blocks
         self.ctx_k = self.ctx_v = None
         self.scales = torch.ones(len(self.blocks), len(SITES), dtype=torch.float32, device=dev)
         self.scratch = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -215,7 +215,6 @@ class WanDiTB200:
             Ml = self.Mb * self.C
             self.xl, self.ol = z(Ml, D), z(Ml, D)
             self.h8l = z(Ml, D, dtype=torch.uint8)
-            self.e2 = z(2, 6, self.B, D)
         self.calibrated = False
         self.launches_per_step = 0
 
@@ -464,11 +463,10 @@ class WanDiTB200:
                      out_fp8=out8.data_ptr() if scale_ptr else 0, out_scale=scale_ptr or 0)
         self.launches_per_step += 1
 
-    def _quant(self, src, dst8, i, site, st, calibrate):
-        """FP8 quantisation of a bf16 activation with the site's scale (calibration: measure it first)."""
-        if calibrate:
-            fvk.quantize_fp8_device(src.data_ptr(), dst8.data_ptr(), self.scratch.data_ptr(), src.numel(), st)
-            fvk.fp8_accumulate_scale_max(self.scratch.data_ptr(), self._sp(i, site), st)
+    def _quant_measured(self, src, dst8, i, site, st):
+        """FP8 quantisation of a bf16 activation with the site's scale, measured first."""
+        fvk.quantize_fp8_device(src.data_ptr(), dst8.data_ptr(), self.scratch.data_ptr(), src.numel(), st)
+        fvk.fp8_accumulate_scale_max(self.scratch.data_ptr(), self._sp(i, site), st)
         fvk.quantize_fp8_static(src.data_ptr(), dst8.data_ptr(), self._sp(i, site), src.numel(), st)
 
     # ---- text context: projected once per prompt -------------------------------
@@ -500,78 +498,81 @@ class WanDiTB200:
 
     # ---- one denoise step -----------------------------------------------------------
     def step(self, x: torch.Tensor, time_proj: torch.Tensor, calibrate: bool = False) -> torch.Tensor:
-        """x (B, L, D) latent tokens, time_proj (B, 6, D) fp32 -> updated tokens (B, L, D) bf16 (all 30 blocks)."""
-        st = torch.cuda.current_stream().cuda_stream
-        B, L, M, D, dl, fl, hl, hd = self.B, self.L, self.M, self.dim, self.dl, self.fl, self.hl, self.hd
+        """x (B, L, D) latent tokens, time_proj (B, 6, D) fp32 -> updated tokens (B, L, D) bf16 (all blocks)."""
         self.launches_per_step = 0
-        tp_dev = time_proj.to(self.device, torch.float32).reshape(B, 1, 6, D).contiguous()
-        if self.sp and not calibrate:
-            return self._step_sequence_parallel(x.to(self.device, BF16), tp_dev)
-        self.x.copy_(x.reshape(M, D))
-        e_out = [self.e[j] for j in range(6)]
-        kstr_self = (L * 3 * dl, 3 * dl, hd)
+        tp_dev = time_proj.to(self.device, torch.float32).reshape(self.B, 1, 6, self.dim).contiguous()
+        x = x.to(self.device, BF16)
+        if calibrate:
+            return self._step_calibrate(x, tp_dev)
+        return self._step_sequence_parallel(x, tp_dev) if self.sp else self._step_replicated(x, tp_dev)
+
+    def _modulation(self, i, tp_dev, st):
+        """Six (B, D) modulation tensors of block i; two sets alternate (the FFN gate of block i is read by the launch that
+        also normalises for block i + 1)."""
+        e = self.e2[i & 1]
+        fvk.adaln_modulation6_bf16(tp_dev.data_ptr(), self.blocks[i]["modulation"].data_ptr(),
+                                   *[e[j].data_ptr() for j in range(6)], self.B, 1, self.dim, st)
+        return e
+
+    def _self_attention_inputs(self, b, st):
+        """Full-width q / k RMSNorm and 3-D RoPE of the packed QKV rows."""
+        B, L, M, dl = self.B, self.L, self.M, self.dl
+        ext = {}
+        if self.tp > 1:
+            fvk.row_sumsq(self.qkv.data_ptr(), 3 * dl, 0, dl, self.ssq[0].data_ptr(), M, st)
+            fvk.row_sumsq(self.qkv.data_ptr(), 3 * dl, dl, dl, self.ssq[1].data_ptr(), M, st)
+            self._allreduce(self.ssq)
+            ext = dict(ext_ssq_q=self.ssq[0].data_ptr(), ext_ssq_k=self.ssq[1].data_ptr(), full_dim=self.dim)
+        fvk.qkv_split_norm_rope_bf16(self.qkv.data_ptr(), b["norm_q"].data_ptr(), b["norm_k"].data_ptr(),
+                                     self.fre.data_ptr(), self.fim.data_ptr(), self.q.data_ptr(), self.k.data_ptr(), B, L,
+                                     self.hl, self.hd, L, 1e-6, st, **ext)
+
+    def _cross_query_norm(self, b, st):
+        """Full-width RMSNorm of the cross-attention queries (one pass when this rank holds all heads)."""
+        M, D, dl = self.M, self.dim, self.dl
+        if self.tp == 1:
+            fvk.rms_norm(self.cq.data_ptr(), b["norm_cq"].data_ptr(), self.cqn.data_ptr(), M, D, 1e-6, st)
+            return
+        fvk.row_sumsq(self.cq.data_ptr(), dl, 0, dl, self.ssq[0].data_ptr(), M, st)
+        self._allreduce(self.ssq[0])
+        fvk.rms_norm_ext(self.cq.data_ptr(), dl, b["norm_cq"].data_ptr(), self.ssq[0].data_ptr(), self.cqn.data_ptr(), dl,
+                         M, dl, D, 1e-6, st)
+
+    def _step_replicated(self, x, tp_dev):
+        """The residual stream in one piece on every rank.  A residual update and the LayerNorm behind it are one launch
+        over all batch elements; the stream is read from the caller's ``x`` until its first update and its last update
+        goes straight into the returned tensor."""
+        st = torch.cuda.current_stream().cuda_stream
+        L, M, D, dl, fl = self.L, self.M, self.dim, self.dl, self.fl
+        ks, kv, kc = (L * dl, dl, self.hd), (L * 3 * dl, 3 * dl, self.hd), (self.T * dl, dl, self.hd)
+        v_view = self.qkv[:, 2 * dl:]
+        xin = x.reshape(M, D).contiguous()
+        out = torch.empty(M, D, dtype=BF16, device=self.device)
+        e = self._modulation(0, tp_dev, st)
+        fvk.residual_layer_norm_fp8(xin.data_ptr(), 0, 0, 0, self.h8.data_ptr(), self._sp(0, "qkv"), M, D, 1e-6, st,
+                                    scale=e[1].data_ptr(), shift=e[0].data_ptr(), mod_stride=D, mod_rows=L)
+        res, cur = xin.data_ptr(), self.x.data_ptr()
+        last = len(self.blocks) - 1
         for i, b in enumerate(self.blocks):
-            # six modulation rows per batch element
-            fvk.adaln_modulation6_bf16(tp_dev.data_ptr(), b["modulation"].data_ptr(), *[t.data_ptr() for t in e_out],
-                                       B, 1, D, st)
             # ---- self-attention
-            self._adaln(i, "qkv", e_out[1], e_out[0], st, calibrate)
             self._gemm(self.h8, b["qkv8"], b["qkv_s"], self.qkv, M, 3 * dl, D, self._sp(i, "qkv"), st, bias=b["qkv_b"])
-            if self.tp > 1:
-                fvk.row_sumsq(self.qkv.data_ptr(), 3 * dl, 0, dl, self.ssq[0].data_ptr(), M, st)
-                fvk.row_sumsq(self.qkv.data_ptr(), 3 * dl, dl, dl, self.ssq[1].data_ptr(), M, st)
-                self._allreduce(self.ssq)
-                fvk.qkv_split_norm_rope_bf16(self.qkv.data_ptr(), b["norm_q"].data_ptr(), b["norm_k"].data_ptr(),
-                                             self.fre.data_ptr(), self.fim.data_ptr(), self.q.data_ptr(),
-                                             self.k.data_ptr(), B, L, hl, hd, L, 1e-6, st,
-                                             ext_ssq_q=self.ssq[0].data_ptr(), ext_ssq_k=self.ssq[1].data_ptr(),
-                                             full_dim=D)
-            else:
-                fvk.qkv_split_norm_rope_bf16(self.qkv.data_ptr(), b["norm_q"].data_ptr(), b["norm_k"].data_ptr(),
-                                             self.fre.data_ptr(), self.fim.data_ptr(), self.q.data_ptr(),
-                                             self.k.data_ptr(), B, L, hl, hd, L, 1e-6, st)
-            v_view = self.qkv[:, 2 * dl:]
-            ks = (L * dl, dl, hd)
-            if calibrate:
-                self._attn(self.q, self.k, v_view, self.a, self.a8, 0, L, L, ks, kstr_self, st)
-                self._quant(self.a, self.a8, i, "o", st, True)
-            else:
-                self._attn(self.q, self.k, v_view, self.a, self.a8, self._sp(i, "o"), L, L, ks, kstr_self, st)
+            self._self_attention_inputs(b, st)
+            self._attn(self.q, self.k, v_view, self.a, self.a8, self._sp(i, "o"), L, L, ks, kv, st)
             self._gemm_allreduce(self.a8, b["o8"], b["o_s"], self.o, M, D, dl, self._sp(i, "o"), st, bias=b["o_b"])
-            self._gated_residual(self.o, e_out[2], st)
             # ---- cross-attention to the text tokens
-            if calibrate:
-                fvk.layer_norm(self.x.data_ptr(), b["norm3_w"].data_ptr(), b["norm3_b"].data_ptr(), self.hb.data_ptr(),
-                               M, D, 1e-6, st)
-                self._quant(self.hb, self.h8, i, "cq", st, True)
-            else:
-                fvk.call("frt_b200_layer_norm", self.x.data_ptr(), b["norm3_w"].data_ptr(), b["norm3_b"].data_ptr(),
-                         None, None, 0, self.h8.data_ptr(), None, self._sp(i, "cq"), M, D, 1e-6, 0, st)
+            fvk.residual_layer_norm_fp8(res, self.o.data_ptr(), e[2].data_ptr(), cur, self.h8.data_ptr(), self._sp(i, "cq"),
+                                        M, D, 1e-6, st, weight=b["norm3_w"].data_ptr(), bias=b["norm3_b"].data_ptr(),
+                                        mod_stride=D, mod_rows=L)
+            res = cur
             self._gemm(self.h8, b["cq8"], b["cq_s"], self.cq, M, dl, D, self._sp(i, "cq"), st, bias=b["cq_b"])
-            fvk.row_sumsq(self.cq.data_ptr(), dl, 0, dl, self.ssq[0].data_ptr(), M, st)
-            self._allreduce(self.ssq[0])
-            fvk.rms_norm_ext(self.cq.data_ptr(), dl, b["norm_cq"].data_ptr(), self.ssq[0].data_ptr(),
-                             self.cqn.data_ptr(), dl, M, dl, D, 1e-6, st)
-            kc = (self.T * dl, dl, hd)
-            if calibrate:
-                self._attn(self.cqn, self.ctx_k[i], self.ctx_v[i], self.a, self.a8, 0, L, self.T, kc, kc, st)
-                self._quant(self.a, self.a8, i, "co", st, True)
-            else:
-                self._attn(self.cqn, self.ctx_k[i], self.ctx_v[i], self.a, self.a8, self._sp(i, "co"), L, self.T, kc,
-                           kc, st)
-            self._gemm_allreduce(self.a8, b["co8"], b["co_s"], self.o, M, D, dl, self._sp(i, "co"), st,
-                                 bias=b["co_b"])
-            fvk.residual_add(self.x.data_ptr(), self.o.data_ptr(), M * D, st)
+            self._cross_query_norm(b, st)
+            self._attn(self.cqn, self.ctx_k[i], self.ctx_v[i], self.a, self.a8, self._sp(i, "co"), L, self.T, kc, kc, st)
+            self._gemm_allreduce(self.a8, b["co8"], b["co_s"], self.o, M, D, dl, self._sp(i, "co"), st, bias=b["co_b"])
             # ---- FFN
-            self._adaln(i, "f1", e_out[4], e_out[3], st, calibrate)
-            if calibrate or not self.fuse_epilogues or M <= 256 or fl < 128:
+            fvk.residual_layer_norm_fp8(cur, self.o.data_ptr(), 0, cur, self.h8.data_ptr(), self._sp(i, "f1"), M, D, 1e-6,
+                                        st, scale=e[4].data_ptr(), shift=e[3].data_ptr(), mod_stride=D, mod_rows=L)
+            if not self.fuse_epilogues or M <= 256 or fl < 128:
                 self._gemm(self.h8, b["f18"], b["f1_s"], self.f1, M, fl, D, self._sp(i, "f1"), st)
-                if calibrate:
-                    # scale of the GELU output, measured on a bf16 copy (calibration only; host-side torch math)
-                    tmp = self.f1.clone()
-                    fvk.add_bias_bf16(tmp.data_ptr(), b["f1_b"].data_ptr(), M, fl, st)
-                    act = torch.nn.functional.gelu(tmp.float(), approximate="tanh").to(BF16)
-                    self._quant(act, self.f8, i, "f2", st, True)
                 fvk.bias_gelu_quantize_fp8_static_bf16(self.f1.data_ptr(), b["f1_b"].data_ptr(), self.f8.data_ptr(),
                                                        self._sp(i, "f2"), M, fl, st)
             else:
@@ -581,22 +582,62 @@ class WanDiTB200:
                                                    self._sp(i, "f2"), st, fast_gelu=self.fast_gelu)
                 self.launches_per_step += 1
             self._gemm_allreduce(self.f8, b["f28"], b["f2_s"], self.o, M, D, fl, self._sp(i, "f2"), st, bias=b["f2_b"])
-            self._gated_residual(self.o, e_out[5], st)
-        return self.x.reshape(B, L, D).clone()
+            gate = e[5].data_ptr()
+            if i == last:
+                fvk.residual_layer_norm_fp8(cur, self.o.data_ptr(), gate, out.data_ptr(), 0, 0, M, D, 1e-6, st,
+                                            mod_stride=D, mod_rows=L)
+            else:
+                e = self._modulation(i + 1, tp_dev, st)
+                fvk.residual_layer_norm_fp8(cur, self.o.data_ptr(), gate, cur, self.h8.data_ptr(), self._sp(i + 1, "qkv"),
+                                            M, D, 1e-6, st, scale=e[1].data_ptr(), shift=e[0].data_ptr(), mod_stride=D,
+                                            mod_rows=L)
+        return out.reshape(self.B, L, D)
 
-    def _adaln(self, i, site, scale_rows, shift_rows, st, calibrate):
-        """adaLN of every batch element with its own (D,) scale / shift row -> FP8 activations of ``site``."""
+    def _step_calibrate(self, x, tp_dev):
+        """The step with every FP8 input produced in bf16 first and its scale measured."""
+        st = torch.cuda.current_stream().cuda_stream
+        L, M, D, dl, fl = self.L, self.M, self.dim, self.dl, self.fl
+        ks, kv, kc = (L * dl, dl, self.hd), (L * 3 * dl, 3 * dl, self.hd), (self.T * dl, dl, self.hd)
+        self.x.copy_(x.reshape(M, D))
+        for i, b in enumerate(self.blocks):
+            e_out = self._modulation(i, tp_dev, st)
+            self._adaln_measured(i, "qkv", e_out[1], e_out[0], st)
+            self._gemm(self.h8, b["qkv8"], b["qkv_s"], self.qkv, M, 3 * dl, D, self._sp(i, "qkv"), st, bias=b["qkv_b"])
+            self._self_attention_inputs(b, st)
+            self._attn(self.q, self.k, self.qkv[:, 2 * dl:], self.a, self.a8, 0, L, L, ks, kv, st)
+            self._quant_measured(self.a, self.a8, i, "o", st)
+            self._gemm_allreduce(self.a8, b["o8"], b["o_s"], self.o, M, D, dl, self._sp(i, "o"), st, bias=b["o_b"])
+            self._gated_residual(self.o, e_out[2], st)
+            fvk.layer_norm(self.x.data_ptr(), b["norm3_w"].data_ptr(), b["norm3_b"].data_ptr(), self.hb.data_ptr(), M, D,
+                           1e-6, st)
+            self._quant_measured(self.hb, self.h8, i, "cq", st)
+            self._gemm(self.h8, b["cq8"], b["cq_s"], self.cq, M, dl, D, self._sp(i, "cq"), st, bias=b["cq_b"])
+            self._cross_query_norm(b, st)
+            self._attn(self.cqn, self.ctx_k[i], self.ctx_v[i], self.a, self.a8, 0, L, self.T, kc, kc, st)
+            self._quant_measured(self.a, self.a8, i, "co", st)
+            self._gemm_allreduce(self.a8, b["co8"], b["co_s"], self.o, M, D, dl, self._sp(i, "co"), st, bias=b["co_b"])
+            fvk.residual_add(self.x.data_ptr(), self.o.data_ptr(), M * D, st)
+            self._adaln_measured(i, "f1", e_out[4], e_out[3], st)
+            self._gemm(self.h8, b["f18"], b["f1_s"], self.f1, M, fl, D, self._sp(i, "f1"), st)
+            # scale of the GELU output, measured on a bf16 copy (host-side torch math)
+            tmp = self.f1.clone()
+            fvk.add_bias_bf16(tmp.data_ptr(), b["f1_b"].data_ptr(), M, fl, st)
+            act = torch.nn.functional.gelu(tmp.float(), approximate="tanh").to(BF16)
+            self._quant_measured(act, self.f8, i, "f2", st)
+            fvk.bias_gelu_quantize_fp8_static_bf16(self.f1.data_ptr(), b["f1_b"].data_ptr(), self.f8.data_ptr(),
+                                                   self._sp(i, "f2"), M, fl, st)
+            self._gemm_allreduce(self.f8, b["f28"], b["f2_s"], self.o, M, D, fl, self._sp(i, "f2"), st, bias=b["f2_b"])
+            self._gated_residual(self.o, e_out[5], st)
+        return self.x.reshape(self.B, L, D).clone()
+
+    def _adaln_measured(self, i, site, scale_rows, shift_rows, st):
+        """adaLN of every batch element with its own (D,) scale / shift row, measured and quantised for ``site``."""
         L, D = self.L, self.dim
         for bi in range(self.B):
-            xs = self.x[bi * L:(bi + 1) * L]
-            if calibrate:
-                fvk.ada_layer_norm_bf16(xs.data_ptr(), scale_rows[bi].data_ptr(), shift_rows[bi].data_ptr(),
-                                        self.hb[bi * L:(bi + 1) * L].data_ptr(), L, D, 1e-6, st)
-            else:
-                fvk.ada_layer_norm_fp8(xs.data_ptr(), scale_rows[bi].data_ptr(), shift_rows[bi].data_ptr(),
-                                       self.h8[bi * L:(bi + 1) * L].data_ptr(), self._sp(i, site), L, D, 1e-6, st)
-        if calibrate:
-            self._quant(self.hb, self.h8, i, site, st, True)
+            rows = slice(bi * L, (bi + 1) * L)
+            fvk.ada_layer_norm_bf16(self.x[rows].data_ptr(), scale_rows[bi].data_ptr(), shift_rows[bi].data_ptr(),
+                                    self.hb[rows].data_ptr(), L, D, 1e-6, st)
+        self._quant_measured(self.hb, self.h8, i, site, st)
 
     def _gated_residual(self, y, gate_rows, st):
         L, D = self.L, self.dim

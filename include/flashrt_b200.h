@@ -216,6 +216,14 @@ int frt_b200_status_words_async(int* out3, int reset, int flags, void* stream);
  * reset != 0 restarts the launch slots and clears the stamps after copying them out.  Synchronises the device. */
 int frt_b200_phase_stamps_read(unsigned long long* gemm_host, unsigned long long* attn_host, int reset);
 
+/* Residual update and the LayerNorm behind it in one pass, same bits as the two calls: res_out = bf16(res + x * gate)
+ * (gate NULL: + x; x NULL: none); out_fp8 = e4m3 of the (affine, modulated) LayerNorm of the result, NULL: update only.
+ * gate / scale / shift rows at + (r / mod_rows) * mod_stride. */
+int frt_b200_residual_layer_norm_fp8(const void* res, const void* x, const void* gate, void* res_out, const void* weight,
+                                     const void* bias, const void* scale, const void* shift, long long mod_stride,
+                                     long long mod_rows, void* out_fp8, const float* d_scale, long long rows, int dim,
+                                     float eps, int flags, void* stream);
+
 /* ---------------------------------------------------------------- video-DiT (Wan-shape) fused producers
  * ada_layer_norm_fp8                 csrc/bindings.cpp:3482-3495 -> csrc/quantize/ada_layer_norm_fp8.cu:58-147
  * ada_layer_norm_bf16[_per_token]    csrc/bindings.cpp:2802-2816 -> csrc/kernels/dit_bf16.cu:151-278

@@ -1,0 +1,108 @@
+"""The warp-per-row kernels (many rows) against the one-CTA-per-row kernels on the same rows in smaller calls: the same
+bits, at partial slices, partial CTAs and both sides of the row threshold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STEP = 384      # rows per small call: below every threshold, whole scale-factor atoms
+
+
+def _dev(a):
+    from gpu_util import Dev
+    return Dev(a)
+
+
+def _rows(seed, rows, dim):
+    from gpu_util import rand_bf16
+    x = rand_bf16(np.random.default_rng(seed), (rows, dim))
+    x[3, : dim // 2] = 0
+    x[5] = 0x8000                                            # a row of -0
+    x[7, 16:32] = 0x4300
+    return x
+
+
+@pytest.mark.parametrize("rows,dim", [(1536, 1024), (3075, 776), (3073, 2064), (3072, 4096), (1539, 3072)])
+@pytest.mark.parametrize("kind", ["fp8", "bf16", "nvfp4_0", "nvfp4_1"])
+def test_norm_rows(rows, dim, kind):
+    from flashrt_b200 import _lib
+    from gpu_util import f32, rand_bf16, zeros
+    if kind.startswith("nvfp4"):
+        rows, dim = max(rows, 3072), dim // 16 * 16
+    x = _rows(rows + dim, rows, dim)
+    w = _dev(rand_bf16(np.random.default_rng(1), (dim,)))
+    sc, got = f32(0.011), []
+    katoms = (dim + 63) // 64
+    for step in (rows, STEP):
+        d_x, d_o = _dev(x), zeros((rows, dim * (2 if kind == "bf16" else 1)), np.uint8)
+        d_sf = zeros(((rows + 127) // 128 * katoms * 512,), np.uint8)
+        for r in range(0, rows, step):
+            n = min(step, rows - r)
+            xp = d_x.ptr + r * dim * 2
+            if kind == "fp8":
+                _lib.call("frt_b200_norm_fp8", xp, None, None, 0, w.ptr, None, 0, d_o.ptr + r * dim, None, n, dim, 1e-6, sc.ptr, 0, 0)
+            elif kind == "bf16":
+                _lib.call("frt_b200_norm_bf16", xp, None, None, 0, None, None, 0, d_o.ptr + r * dim * 2, None, n, dim, 1e-6, 0, 0)
+            else:
+                _lib.call("frt_b200_norm_nvfp4", xp, None, None, 0, w.ptr, None, 0, d_o.ptr + r * dim // 2,
+                          d_sf.ptr + r // 128 * katoms * 512, None, n, dim, 1e-6, int(kind[-1]), 0, 0)
+        got.append((d_o.get(), d_sf.get()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("rows,dim", [(1024, 3072), (1027, 520), (1025, 4104)])
+@pytest.mark.parametrize("mod", ["affine", "modulated", "plain"])
+def test_layer_norm_rows_and_residual_form(rows, dim, mod):
+    """Also the residual update in the same pass against bias_gate_mul_residual / residual_add, then layer_norm."""
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import f32, rand_bf16, zeros
+    rng = np.random.default_rng(rows + dim)
+    x, y = _rows(2, rows, dim), rand_bf16(rng, (rows, dim))
+    w, b, sc, sh, gate = (_dev(rand_bf16(rng, (2, dim))) for _ in range(5))
+    aff = (w.ptr, b.ptr) if mod == "affine" else (None, None)
+    md = (sc.ptr, sh.ptr) if mod == "modulated" else (None, None)
+    s8, outs = f32(0.013), []
+    for step in (rows, STEP):
+        d_x, d_o = _dev(x), zeros((rows, dim), np.uint8)
+        for r in range(0, rows, step):
+            _lib.call("frt_b200_layer_norm", d_x.ptr + r * dim * 2, *aff, *md, 0, d_o.ptr + r * dim, None, s8.ptr,
+                      min(step, rows - r), dim, 1e-6, 0, 0)
+        outs.append(d_o.get())
+    assert np.array_equal(outs[0], outs[1])
+    # two modulation rows, the second from row `half` on
+    half = rows // 2 + 1
+    for g in (gate.ptr, 0):
+        d_x, d_y, d_o = _dev(x), _dev(y), zeros((rows, dim), np.uint8)
+        d_r, d_o2 = zeros((rows, dim), np.uint16), zeros((rows, dim), np.uint8)
+        fvk.residual_layer_norm_fp8(d_x.ptr, d_y.ptr, g, d_r.ptr, d_o2.ptr, s8.ptr, rows, dim, 1e-6, 0, weight=aff[0] or 0,
+                                    bias=aff[1] or 0, scale=md[0] or 0, shift=md[1] or 0, mod_stride=dim, mod_rows=half)
+        for i, (r, n) in enumerate(((0, half), (half, rows - half))):
+            o = r * dim * 2
+            if g:
+                fvk.bias_gate_mul_residual_bf16(d_x.ptr + o, d_y.ptr + o, 0, g + i * dim * 2, n, dim, 0, gate_stride=0)
+            else:
+                fvk.residual_add(d_x.ptr + o, d_y.ptr + o, n * dim, 0)
+            _lib.call("frt_b200_layer_norm", d_x.ptr + o, *aff, *(p + i * dim * 2 if p else None for p in md), 0,
+                      d_o.ptr + r * dim, None, s8.ptr, n, dim, 1e-6, 0, 0)
+        assert np.array_equal(d_r.get() & 0x7fff, d_x.get() & 0x7fff)          # up to the sign of zeros
+        assert np.array_equal(d_o.get(), d_o2.get())
+
+
+@pytest.mark.parametrize("L,heads,hd,seq", [(512, 24, 128, 512), (515, 3, 40, 400), (513, 5, 256, 513)])
+def test_qkv_split_norm_rope_rows(L, heads, hd, seq):
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import rand_bf16, zeros
+    rng = np.random.default_rng(L)
+    dim = heads * hd
+    qkv, wq, wk = _dev(rand_bf16(rng, (L, 3 * dim))), _dev(rand_bf16(rng, (dim,))), _dev(rand_bf16(rng, (dim,)))
+    fr, fi = (_dev(rng.standard_normal((L, hd // 2)).astype(np.float32)) for _ in range(2))
+    outs = []
+    for step in (L, 256):
+        q, k = zeros((L, dim), np.uint16), zeros((L, dim), np.uint16)
+        for r in range(0, L, step):
+            n = min(step, L - r)
+            o = r * hd // 2 * 4
+            fvk.qkv_split_norm_rope_bf16(qkv.ptr + r * 3 * dim * 2, wq.ptr, wk.ptr, fr.ptr + o, fi.ptr + o, q.ptr + r * dim * 2,
+                                         k.ptr + r * dim * 2, 1, n, heads, hd, max(0, min(n, seq - r)), 1e-6, 0)
+        outs.append((q.get(), k.get()))
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
