@@ -47,6 +47,13 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return r;
 }
 
+// v rounded to bf16, as fp32: the upper half of a packed conversion whose lower half is zero IS the fp32 value
+__device__ __forceinline__ float bf16_round(float v) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v), "f"(0.0f));
+    return __uint_as_float(r);
+}
+
 // ---------------------------------------------------------------- fp8 e4m3
 // clamp to +-448 (fmaxf/fminf return the non-NaN operand, so NaN -> -448),
 // then round-to-nearest-even, saturating-finite.

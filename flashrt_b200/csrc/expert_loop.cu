@@ -89,7 +89,7 @@ __device__ __forceinline__ float ex2(float x) {
     asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float bf16r(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
+__device__ __forceinline__ float bf16r(float f) { return bf16_round(f); }
 __device__ __forceinline__ void work_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // unit of GEMM phase `ph` (0 QKV, 1 O, 2 gate|up, 3 down) of global layer `gl` that CTA `cta` owns, or -1

@@ -479,8 +479,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
                         unpack_bf16x2(rw[k], r0, r1);
                         unpack_bf16x2(gw[k], g0, g1);
                         // the GEMM result is rounded to bf16 as the separate kernel stores it, then x += o * gate
-                        const float o0 = __bfloat162float(__float2bfloat16_rn(a[2 * k] * alpha));
-                        const float o1 = __bfloat162float(__float2bfloat16_rn(a[2 * k + 1] * alpha));
+                        const float o0 = bf16_round(a[2 * k] * alpha);
+                        const float o1 = bf16_round(a[2 * k + 1] * alpha);
                         r0 = __fmaf_rn(o0, g0, r0);
                         r1 = __fmaf_rn(o1, g1, r1);
                         ssq = __fmaf_rn(r0, r0, ssq);
@@ -647,7 +647,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
                     if (n >= p.N) continue;
                     float v[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(a[j] * alpha));
+                    for (int j = 0; j < 8; ++j) v[j] = bf16_round(a[j] * alpha);
                     const bool is_q = n < p.q_dim;
                     const bool is_k = !is_q && n < p.q_dim + p.k_dim;
                     const int nr = is_q ? n : (is_k ? n - p.q_dim : n - p.q_dim - p.k_dim);
@@ -680,8 +680,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
                     float q[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float gt = __bfloat162float(__float2bfloat16_rn(a[j] * alpha));
-                        const float up = __bfloat162float(__float2bfloat16_rn(b[j] * alpha));
+                        const float gt = bf16_round(a[j] * alpha);
+                        const float up = bf16_round(b[j] * alpha);
                         q[j] = clamp448(__fmul_rn(__fmul_rn(det_gelu_tanh(gt), up), inv_os));
                     }
                     uint2 o8;

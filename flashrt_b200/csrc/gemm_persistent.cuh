@@ -307,7 +307,7 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                                 const bool hb = p.bias != nullptr;
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) {
-                                    float x = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j + e]) * alpha));
+                                    float x = bf16_round(__uint_as_float(v[j + e]) * alpha);
                                     if (hb) x = __fadd_rn(x, bj[e]);
                                     g[e] = clamp448(__fmul_rn(EPI == EPI_P_BIAS_GELU_FAST_FP8 ? fast_gelu_tanh(x) : gelu_tanh_form_rn(x),
                                                               inv_os));

@@ -617,10 +617,10 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         const float rs = s_rms[t];
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
-                            v[j] = __bfloat162float(__float2bfloat16_rn(__fadd_rn(__fmul_rn(a[j] * alpha, rs), cc[j])));
+                            v[j] = bf16_round(__fadd_rn(__fmul_rn(a[j] * alpha, rs), cc[j]));
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(a[j] * alpha));
+                        for (int j = 0; j < 8; ++j) v[j] = bf16_round(a[j] * alpha);
                     }
                     const bool is_q = n < p.q_dim;
                     const bool is_k = !is_q && n < p.q_dim + p.k_dim;
@@ -681,8 +681,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float gt = __bfloat162float(__float2bfloat16_rn(a[j]));
-                        const float up = __bfloat162float(__float2bfloat16_rn(b[j]));
+                        const float gt = bf16_round(a[j]);
+                        const float up = bf16_round(b[j]);
                         const float act = ACT == 2 ? fast_gelu_tanh(gt) : ACT == 1 ? det_silu(gt) : det_gelu_tanh(gt);
                         q[j] = clamp448(__fmul_rn(__fmul_rn(act, up), inv_os));
                     }
@@ -714,8 +714,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         float r0, r1, g0, g1;
                         unpack_bf16x2(rw[k], r0, r1);
                         unpack_bf16x2(gw[k], g0, g1);
-                        const float o0 = __bfloat162float(__float2bfloat16_rn(a[2 * k] * alpha));
-                        const float o1 = __bfloat162float(__float2bfloat16_rn(a[2 * k + 1] * alpha));
+                        const float o0 = bf16_round(a[2 * k] * alpha);
+                        const float o1 = bf16_round(a[2 * k + 1] * alpha);
                         r0 = __fmaf_rn(o0, g0, r0);
                         r1 = __fmaf_rn(o1, g1, r1);
                         ssq = __fmaf_rn(r0, r0, ssq);

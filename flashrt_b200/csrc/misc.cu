@@ -40,7 +40,7 @@ small_gemm_bf16_kernel(const void* __restrict__ Av, const __nv_bfloat16* __restr
             const int r = i / kc, k = i - r * kc;
             const size_t ai = (size_t)(m0 + r) * K + k0 + k;
             // an fp32 operand is rounded to bf16 first: the projection multiplies bf16 by bf16
-            a_s[r][k] = (m0 + r < M) ? (A_F32 ? __bfloat162float(__float2bfloat16_rn(Af[ai])) : __bfloat162float(A[ai]))
+            a_s[r][k] = (m0 + r < M) ? (A_F32 ? bf16_round(Af[ai]) : __bfloat162float(A[ai]))
                                      : 0.0f;
         }
         __syncthreads();
@@ -146,8 +146,8 @@ step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, c
             unpack_bf16x2(shw[i], h0, h1);
             const float n0 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i], rms), 1.0f), __fadd_rn(1.0f, s0), h0);
             const float n1 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i + 1], rms), 1.0f), __fadd_rn(1.0f, s1), h1);
-            a_s[col + 2 * i] = __bfloat162float(__float2bfloat16_rn(n0));
-            a_s[col + 2 * i + 1] = __bfloat162float(__float2bfloat16_rn(n1));
+            a_s[col + 2 * i] = bf16_round(n0);
+            a_s[col + 2 * i + 1] = bf16_round(n1);
         }
         __syncthreads();
         // out-projection: column n, K-slices ks = k mod 16; thread (n, g) forms the slices g, g + groups, ...
@@ -178,7 +178,7 @@ step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, c
     {
         float a[SB_ACTION];
 #pragma unroll
-        for (int k = 0; k < SB_ACTION; ++k) a[k] = __bfloat162float(__float2bfloat16_rn(nz[k]));
+        for (int k = 0; k < SB_ACTION; ++k) a[k] = bf16_round(nz[k]);
         const uint4 bv = b_in ? ld_global_v4(b_in + col) : make_uint4(0, 0, 0, 0);
         const uint32_t* bw = &bv.x;
         uint4 ov;
@@ -194,7 +194,7 @@ step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, c
                 s += acc;
             }
             if (b_in) s += bf16_bits_to_f32((bw[j >> 1] >> ((j & 1) * 16)) & 0xffffu);
-            xb[j] = __bfloat162float(__float2bfloat16_rn(s));
+            xb[j] = bf16_round(s);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
