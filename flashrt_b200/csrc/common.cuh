@@ -55,17 +55,13 @@ __device__ __forceinline__ float bf16_round(float v) {
 }
 
 // ---------------------------------------------------------------- fp8 e4m3
-// clamp to +-448 (fmaxf/fminf return the non-NaN operand, so NaN -> -448),
-// then round-to-nearest-even, saturating-finite.
-__device__ __forceinline__ float clamp448(float v) {
-    return fminf(fmaxf(v, -448.0f), 448.0f);
-}
+// clamp to +-448 (NaN -> -448, as fminf(fmaxf(v, -448), 448) gives) in front of a saturating E4M3 conversion: the
+// conversion itself does the upper bound, so one instruction remains
+__device__ __forceinline__ float clamp448(float v) { return fmaxf(v, -448.0f); }
 __device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float lo, float hi) {
     // low byte = lo, high byte = hi
     return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(lo, hi), __NV_SATFINITE, __NV_E4M3);
 }
-// clamp448 in front of the conversion, in one instruction: the conversion itself saturates, and fmaxf maps NaN to -448
-__device__ __forceinline__ float clamp448_lo(float v) { return fmaxf(v, -448.0f); }
 __device__ __forceinline__ uint32_t f32x4_to_e4m3x4(float a, float b, float c, float d) {
     return f32x2_to_e4m3x2(a, b) | (f32x2_to_e4m3x2(c, d) << 16);
 }

@@ -96,7 +96,6 @@ struct GemmParams {
     uint8_t* out8;             // EPI_GEGLU_FP8: (M, half) e4m3 codes
     const float* out_scale;    //   device scalar: quantisation scale of the GeGLU result
     int half;                  //   hidden width; weight rows [0, half) = gate, [half, 2 half) = up
-    int fast_act;              // bias + GELU + FP8 epilogue: GELU through the hardware tanh instead of the exact form
     // NVFP4 kernels: unsigned-E4M3 block scales of both operands in 512-byte atoms (128 rows x 4 blocks)
     const uint8_t* sf_lane;
     const uint8_t* sf_col;
@@ -110,6 +109,7 @@ struct GemmParams {
     const __nv_bfloat16* style;
     float eps;
     int w_kn;                  // large-M persistent kernel: weights stored (K, N) row-major
+    int tile_gm;               // large-M kernels: m-tiles per group of the tile order
 };
 
 enum { EPI_BF16 = 0, EPI_ROPE_SPLIT = 1, EPI_GEGLU_FP8 = 2, EPI_GATE_RES_NORM_FP8 = 3 };
@@ -905,6 +905,43 @@ static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, in
     return launch_gemm<256, true, EPI, true>(A, W, p, K, sp, pdl, s);
 }
 
+// ------------------------------------------------------------------ choice among the large-M FP8 kernels
+enum { LARGE_128 = 0, LARGE_256 = 1, LARGE_PAIR = 2, LARGE_PAIR_128 = 3 };
+
+// Microseconds of a launch: a fixed part, then whole waves of tiles, each as long as its k-blocks of 128.  The constants are
+// fitted to a sweep of graph-launched products on one B200 (M 130 .. 8192, N 1024 .. 32768, K 1024 .. 16384; the choice was
+// within 3 % of the best kernel on all but a few of its points):
+//   128 x 128 tile per CTA 3.6 + 0.32 per k-block, 128 x 256 per CTA 4.5 + 0.40, 256 x 256 per CTA pair 5.6 + 0.34,
+//   256 x 128 per CTA pair 4.6 + 0.225.
+// The pair of 256 x 256 moves the fewest operand bytes per flop and wins wherever its tile list is long; the others win
+// where a short list of large tiles would leave the last wave nearly empty, or rows of a half-empty 256-row tile.
+static double large_cost(int kind, int M, int N, int K) {
+    static const struct { int tm, tn, pair; double fixed, per_kb; } c[4] = {
+        {128, 128, 0, 3.6, 0.32}, {128, 256, 0, 4.5, 0.40}, {256, 256, 1, 5.6, 0.34}, {256, 128, 1, 4.6, 0.225}};
+    const int workers = device_sm_count() / (c[kind].pair ? 2 : 1);
+    const long long tiles = (long long)((M + c[kind].tm - 1) / c[kind].tm) * ((N + c[kind].tn - 1) / c[kind].tn);
+    return c[kind].fixed + (double)((tiles + workers - 1) / workers) * ((K + 127) / 128) * c[kind].per_kb;
+}
+static int pick_large(int M, int N, int K, bool no_pair, double* cost = nullptr) {
+    int best = LARGE_128;
+    double t = large_cost(LARGE_128, M, N, K);
+    for (int k = LARGE_256; k <= LARGE_PAIR_128 && N >= 256; ++k) {
+        if (k >= LARGE_PAIR && no_pair) break;
+        const double tk = large_cost(k, M, N, K);
+        if (tk < t) { t = tk; best = k; }
+    }
+    if (cost) *cost = t;
+    return best;
+}
+
+template <int EPI>
+static int launch_large(int kind, const void* A, const void* W, const GemmParams& p, int K, bool pdl, cudaStream_t s) {
+    if (kind == LARGE_PAIR) return launch_gemm_pair<256, EPI>(A, W, p, K, pdl, s);
+    if (kind == LARGE_PAIR_128) return launch_gemm_pair<128, EPI>(A, W, p, K, pdl, s);
+    if (kind == LARGE_256) return launch_gemm_persistent<256, EPI>(A, W, p, K, pdl, s);
+    return launch_gemm_persistent<128, EPI>(A, W, p, K, pdl, s);
+}
+
 }  // namespace frt
 
 using namespace frt;
@@ -949,7 +986,22 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     p.kb_total = (K + 127) / 128;
     cudaStream_t s = (cudaStream_t)stream;
     bool pdl = flags & 1;
-    if (tok_eligible(M, N, K, flags, splits)) {
+    // M <= 256 without a hint: the kernels below it stream the weights through clusters that split K, which wins while the
+    // product is small or K is long; from about 8 MB of weights (M <= 128), or for most of 129 .. 256, the persistent kernels
+    // of the large products do.  Microseconds again: token-major 5 + 0.3 per MB of weights (5.2 + 0.45 above 64 rows),
+    // swapped 13 + 0.115 per k-block (e.g. 256 x 4096 x 1024: swapped 14.3, persistent 6.4; 50 x 14336 x 3072: token-major
+    // 15.9, persistent 12.7).
+    const bool hinted = splits > 0 || (flags & (16 | 0x300));
+    if (M <= 256 && M > 16 && !hinted && !(flags & 2) && N >= 128) {
+        double t_large = 0.0;
+        const int kind = pick_large(M, N, K, M <= 128 || (flags & 32) != 0, &t_large);
+        const double mb = (double)N * K / 1048576.0;
+        const double t_small = M > 128 ? 13.0 + 0.115 * p.kb_total : M > 64 ? 5.2 + 0.45 * mb : 5.0 + 0.3 * mb;
+        if (t_large + 0.3 < t_small) return launch_large<EPI_P_BF16>(kind, A, W, p, K, pdl, s);
+    }
+    // the swapped kernel's splits keep up with a long K better than the token-major kernel's exchange
+    const bool long_k = !hinted && (M > 64 ? p.kb_total >= 96 : p.kb_total >= 128);
+    if (!long_k && tok_eligible(M, N, K, flags, splits)) {
         TokParams t = {};
         t.M = M; t.N = N; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = alpha_host;
         t.out = (__nv_bfloat16*)D; t.bias = (const __nv_bfloat16*)bias;
@@ -958,20 +1010,9 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     }
     if (M <= 256) return dispatch_small_m<EPI_BF16>(A, W, p, K, M, (N + 127) / 128, splits, pdl, s);
     int sp = splits > 0 ? pick_splits(1, p.kb_total, splits > 8 ? 8 : splits) : 1;
-    // One 256 x 256 tile per CTA pair (cta_group::2): measured 3-10 % faster than the one-CTA persistent kernel once
-    // the tile list fills at least two waves of pairs and K >= 2048 (e.g. 20480 x 14336 x 3072: 698 vs 744 us), a few
-    // percent slower on short lists and at K = 1024.  flags bit 3 forces it, flags bit 5 keeps the one-CTA kernel.
-    const long long tiles256 = (long long)((M + 255) / 256) * ((N + 255) / 256);
-    const bool pair_pays = tiles256 >= 148 && K >= 2048 && !(flags & 32) && !(flags & 2);
-    if (sp == 1 && ((flags & 8) || pair_pays) && N >= 256) return launch_gemm_pair(A, W, p, K, pdl, s);
-    if (sp == 1 && !(flags & 2)) {      // flags bit1 keeps the one-tile-per-CTA kernel (for comparison runs)
-        // 128-column tiles only where the 256-column tile list leaves more than half of the SMs idle (2048 x 1024: 64
-        // wide tiles for 148 SMs: 9.6 -> 8.6 us); from one wave on the wide tile wins (2048 x 3072 x 3072: 24.9 us wide,
-        // 32.4 us narrow)
-        const long long wide_tiles = (long long)((M + 127) / 128) * ((N + 255) / 256);
-        const bool narrow = N > 64 && wide_tiles * 2 <= device_sm_count();
-        if (N >= 256 && !narrow) return launch_gemm_persistent<256, EPI_P_BF16>(A, W, p, K, pdl, s);
-        if (N > 64) return launch_gemm_persistent<128, EPI_P_BF16>(A, W, p, K, pdl, s);
+    if (sp == 1 && !(flags & 2) && N > 64) {      // flags bit 1 keeps the one-tile-per-CTA kernel (for comparison runs)
+        const int kind = (flags & 8) && N >= 256 ? LARGE_PAIR : pick_large(M, N, K, (flags & 32) != 0);
+        return launch_large<EPI_P_BF16>(kind, A, W, p, K, pdl, s);
     }
     if (N >= 256) return launch_gemm<256, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
@@ -1212,14 +1253,9 @@ int frt_b200_gemm_fp8_nt_bias_gelu_fp8(const void* A, const void* W, void* out8,
     p.kb_total = (K + 127) / 128;
     p.out8 = (uint8_t*)out8;
     p.out_scale = d_out_scale;
-    p.fast_act = (flags & 128) ? 1 : 0;
-    if (p.fast_act) {
-        if (N >= 256)
-            return launch_gemm_persistent<256, EPI_P_BIAS_GELU_FAST_FP8>(A, W, p, K, flags & 1, (cudaStream_t)stream);
-        return launch_gemm_persistent<128, EPI_P_BIAS_GELU_FAST_FP8>(A, W, p, K, flags & 1, (cudaStream_t)stream);
-    }
-    if (N >= 256) return launch_gemm_persistent<256, EPI_P_BIAS_GELU_FP8>(A, W, p, K, flags & 1, (cudaStream_t)stream);
-    return launch_gemm_persistent<128, EPI_P_BIAS_GELU_FP8>(A, W, p, K, flags & 1, (cudaStream_t)stream);
+    const int kind = pick_large(M, N, K, false);
+    if (flags & 128) return launch_large<EPI_P_BIAS_GELU_FAST_FP8>(kind, A, W, p, K, flags & 1, (cudaStream_t)stream);
+    return launch_large<EPI_P_BIAS_GELU_FP8>(kind, A, W, p, K, flags & 1, (cudaStream_t)stream);
 }
 
 // Row-parallel projection with the gated residual update fused (M <= 128, N % 64 == 0, K % 128 == 0):

@@ -295,9 +295,9 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 tc::tma_load_2d(tiles + i * STAGE_BYTES, &tmA, &full[i], (kb0 + i) * 128, m0);
         }
         *issued = pre;
+        int s = 0;                                    // ring position: i = pre = STG here
+        uint32_t ph = 0;
         for (int i = pre; i < nkb; ++i) {
-            const int s = i % STG;
-            const uint32_t ph = ((i / STG) - 1) & 1;
             if (!tc::mbar_wait_until(&empty[s], ph, deadline, abort_flag)) {
                 *abort_flag = 1;
                 atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
@@ -307,6 +307,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             load_w(s, kb0 + i);
             if (PRO == TOK_PRO_TMA) tc::tma_load_2d(tiles + s * STAGE_BYTES, &tmA, &full[s], (kb0 + i) * 128, m0);
             *issued = i + 1;
+            if (++s == STG) { s = 0; ph ^= 1; }
         }
     }
 
@@ -418,9 +419,9 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                     : tc::make_desc_kmajor_sw128(tc::smem_u32(tiles + A_BYTES));
         // one K = 32 step: 32 bytes along a K-major row, or 32 rows of 128 bytes of an MN-major tile
         const uint64_t wstep = p.w_kn ? (uint64_t)((32 * 128) >> 4) : 2u;
+        int s = 0;
+        uint32_t ph = 0;
         for (int i = 0; i < nkb && !failed; ++i) {
-            const int s = i % STG;
-            const uint32_t ph = (i / STG) & 1;
             if (!tc::mbar_wait_until(&full[s], ph, deadline, abort_flag)) {
                 *abort_flag = 1;
                 atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
@@ -437,6 +438,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 tc::mma_f8(tmem_d, dA0 + so + 2 * k, dW0 + so + wstep * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
             tc::mma_commit(&empty[s]);
             *consumed = i + 1;
+            if (++s == STG) { s = 0; ph ^= 1; }
         }
         if (!failed) tc::mma_commit(accum_bar);
 #ifdef FRT_PHASE_STAMPS

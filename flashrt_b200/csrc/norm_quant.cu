@@ -281,10 +281,10 @@ norm_warp_kernel(NormArgs a) {
             }
         } else if (OUT_FP8) {
             uint2 o;
-            o.x = f32x4_to_e4m3x4(clamp448_lo(__fmul_rn(v[0], inv_scale)), clamp448_lo(__fmul_rn(v[1], inv_scale)),
-                                  clamp448_lo(__fmul_rn(v[2], inv_scale)), clamp448_lo(__fmul_rn(v[3], inv_scale)));
-            o.y = f32x4_to_e4m3x4(clamp448_lo(__fmul_rn(v[4], inv_scale)), clamp448_lo(__fmul_rn(v[5], inv_scale)),
-                                  clamp448_lo(__fmul_rn(v[6], inv_scale)), clamp448_lo(__fmul_rn(v[7], inv_scale)));
+            o.x = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[0], inv_scale)), clamp448(__fmul_rn(v[1], inv_scale)),
+                                  clamp448(__fmul_rn(v[2], inv_scale)), clamp448(__fmul_rn(v[3], inv_scale)));
+            o.y = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[4], inv_scale)), clamp448(__fmul_rn(v[5], inv_scale)),
+                                  clamp448(__fmul_rn(v[6], inv_scale)), clamp448(__fmul_rn(v[7], inv_scale)));
             if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + roff, o);
         } else {
             uint4 o;

@@ -77,7 +77,56 @@ __device__ __forceinline__ bool mbar_wait_until(uint64_t* bar, uint32_t parity, 
     }
 }
 
+// The same by shared-memory address, for the loops that feed and issue MMAs: a k-block of 128 x 128 x 128 is 256 cycles of
+// tensor time, and a completed wait costs its thread about 70, so the loops look at the NEXT barrier (mbar_test, which never
+// suspends) before they issue the current k-block and only wait where that look failed.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_until(uint32_t bar, uint32_t parity, uint64_t deadline_ns,
+                                                volatile int* abort_flag) {
+    for (uint32_t i = 0;; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, P;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if ((i & 3) == 3 && global_timer_ns() > deadline_ns) return false;
+    }
+}
+// Whole warp: true on every lane once the phase has completed, false on every lane when a wait gave up.  The loops that
+// issue TMA copies and MMAs run on all 32 lanes with only the instructions themselves behind elect_one(): a loop inside
+// `if (lane == 0)` keeps its descriptors and addresses in per-thread registers and moves them to uniform registers for every
+// single instruction (a k-block of four 128 x 128 x 32 MMAs then takes 525 cycles to issue instead of the 256 of its math).
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, bool ready, uint64_t deadline_ns,
+                                          volatile int* abort_flag) {
+    const bool ok = ready || mbar_wait_until(bar, parity, deadline_ns, abort_flag);
+    return __all_sync(0xffffffffu, ok) != 0;
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
 // ---------------------------------------------------------------- TMA (tiled, 2D / 3D loads)
+__device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_dst), "l"(m), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
@@ -107,6 +156,12 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
         ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+        ::"r"(smem_dst), "l"(gsrc), "r"(bytes), "r"(bar)
         : "memory");
 }
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
@@ -286,6 +341,10 @@ __device__ __forceinline__ void mma_nvfp4(uint32_t tmem_d, uint64_t adesc, uint6
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // ---------------------------------------------------------------- cluster / DSMEM

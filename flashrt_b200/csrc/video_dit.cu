@@ -298,8 +298,8 @@ layer_norm_warp_kernel(ResNormArgs a) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 unpack_bf16x2(ow[i], r[2 * i], r[2 * i + 1]);
-                r[2 * i] = clamp448_lo(__fmul_rn(r[2 * i], inv_a));
-                r[2 * i + 1] = clamp448_lo(__fmul_rn(r[2 * i + 1], inv_a));
+                r[2 * i] = clamp448(__fmul_rn(r[2 * i], inv_a));
+                r[2 * i + 1] = clamp448(__fmul_rn(r[2 * i + 1], inv_a));
             }
             uint2 o8;
             o8.x = f32x4_to_e4m3x4(r[0], r[1], r[2], r[3]);
