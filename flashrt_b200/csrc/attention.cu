@@ -152,6 +152,18 @@ enum { AERR_PRODUCER = 0x11, AERR_MMA = 0x12, AERR_SOFTMAX = 0x13 };
         }                                                                                \
     } while (0)
 
+// The same for a whole warp whose lanes stay together (the TMA and MMA roles, see tc::warp_wait): false on every lane when the
+// wait gave up.
+__device__ __forceinline__ bool attn_warp_wait(uint64_t* bar, uint32_t parity, int code, uint64_t deadline,
+                                               volatile int* abort_flag) {
+    const bool ok = tc::warp_wait(tc::smem_u32(bar), parity, false, deadline, abort_flag);
+    if (!ok) {
+        if ((threadIdx.x & 31) == 0 && !*abort_flag) atomicCAS(&g_attn_status, 0, code | (blockIdx.x << 8));
+        *abort_flag = 1;
+    }
+    return ok;
+}
+
 template <int D, int BKV>
 __global__ void __launch_bounds__(192, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

@@ -159,17 +159,19 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
 
     pdl_launch_dependents();
 
-    if (warp == 4 && lane == 0) {
-        // ---------------- TMA producer
+    if (warp == 4) {
+        // ---------------- TMA producer (whole warp)
         auto load_kv = [&](int j) {
             const int st = j & 1;
             const int key0 = (c_begin + j) * BKV;
-            tc::mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
-            for (int db = 0; db < 4; ++db)
-                tc::tma_load_4d(sK + st * Cfg::KV_BYTES + db * (BKV * 128), &tmK, &k_full[st], db * 64, hk, key0, b);
-            tc::mbar_arrive_expect_tx(&v_full[st], V_BYTES);
-            for (int db = 0; db < DV / 64; ++db)
-                tc::tma_load_4d(sV + st * V_BYTES + db * (BKV * 128), &tmV, &v_full[st], dq * DV + db * 64, hk, key0, b);
+            if (tc::elect_one()) {
+                tc::mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
+                for (int db = 0; db < 4; ++db)
+                    tc::tma_load_4d(sK + st * Cfg::KV_BYTES + db * (BKV * 128), &tmK, &k_full[st], db * 64, hk, key0, b);
+                tc::mbar_arrive_expect_tx(&v_full[st], V_BYTES);
+                for (int db = 0; db < DV / 64; ++db)
+                    tc::tma_load_4d(sV + st * V_BYTES + db * (BKV * 128), &tmV, &v_full[st], dq * DV + db * 64, hk, key0, b);
+            }
         };
         // chunks that lie inside the rows the previous kernel does not write may be fetched while it still runs
         int early = 0;
@@ -178,72 +180,84 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
             ++early;
         }
         pdl_wait();
-        ATT_STAMP_ANY(1);
+#ifdef FRT_PHASE_STAMPS
+        if (lane == 0) ATT_STAMP_ANY(1);
+#endif
         // Q arrives as four 64-column blocks, each on its own barrier: the first chunk's Q.K^T starts on the first block
         // while the others are still in flight
-        for (int db = 0; db < 4; ++db) {
-            uint64_t* qb = db == 0 ? q_full : &q_part[db - 1];
-            tc::mbar_arrive_expect_tx(qb, Cfg::Q_BYTES / 4);
-            tc::tma_load_5d(sQ + db * (128 * 128), &tmQ, qb, db * 64, 0, hk, tok0, b);
+        if (tc::elect_one()) {
+            for (int db = 0; db < 4; ++db) {
+                uint64_t* qb = db == 0 ? q_full : &q_part[db - 1];
+                tc::mbar_arrive_expect_tx(qb, Cfg::Q_BYTES / 4);
+                tc::tma_load_5d(sQ + db * (128 * 128), &tmQ, qb, db * 64, 0, hk, tok0, b);
+            }
         }
-        for (int j = early; j < nchunks && !*abort_flag; ++j) {
-            if (j >= 2) ATTN_WAIT(&kv_empty[j & 1], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER);
-            if (*abort_flag) break;
+        for (int j = early; j < nchunks; ++j) {
+            if (j >= 2 && !attn_warp_wait(&kv_empty[j & 1], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER, deadline, abort_flag)) break;
             load_kv(j);
         }
-    } else if (warp == 5 && lane == 0) {
-        // ---------------- MMA issuer
+    } else if (warp == 5) {
+        // ---------------- MMA issuer (whole warp)
         constexpr uint32_t idesc_s = tc::make_idesc(1, 1, 0, 0, 128, BKV);
         const uint32_t idesc_o = tc::make_idesc(1, 1, 0, 1, 128, (uint32_t)DV);    // A = P from TMEM, B = V MN-major
         const uint64_t dq_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sQ));
         const uint64_t dk_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sK));
         const uint64_t dv_base = tc::make_desc_mnmajor_sw128(tc::smem_u32(sV), BKV * 128);
-        auto qk = [&](int j) {
-            const uint64_t dk = dk_base + (uint64_t)((j & 1) * (Cfg::KV_BYTES >> 4));
+        const uint32_t s_full_a = tc::smem_u32(s_full), kv_empty_a = tc::smem_u32(kv_empty), o_full_a = tc::smem_u32(o_full);
+        // the 64-column block `blk` of Q . K^T(j)
+        auto qk_block = [&](int j, int blk) {
+            const uint64_t dk = dk_base + (uint64_t)((j & 1) * (Cfg::KV_BYTES >> 4) + blk * ((BKV * 128) >> 4));
+            const uint64_t dqb = dq_base + (uint64_t)(blk * ((128 * 128) >> 4));
             const uint32_t d_tm = tmem + Cfg::S_COL + (j & 1) * 64;
+            if (tc::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
-                if (j == 0 && k > 0 && (k % 4) == 0) {          // next 64-column block of Q (first chunk only)
-                    ATTN_WAIT(&q_part[k / 4 - 1], 0u, AERR_MMA);
-                    if (*abort_flag) return;
-                    tc::tc_fence_after_sync();
-                }
-                tc::mma_f16(d_tm, dq_base + (uint64_t)((k / 4) * ((128 * 128) >> 4) + 2 * (k % 4)),
-                            dk + (uint64_t)((k / 4) * ((BKV * 128) >> 4) + 2 * (k % 4)), idesc_s, k > 0 ? 1u : 0u);
+                for (int k = 0; k < 4; ++k)
+                    tc::mma_f16(d_tm, dqb + 2 * k, dk + 2 * k, idesc_s, (blk > 0 || k > 0) ? 1u : 0u);
+                if (blk == 3) tc::mma_commit(s_full_a + 8 * (j & 1));
             }
-            tc::mma_commit(&s_full[j & 1]);
         };
-        ATTN_WAIT(q_full, 0u, AERR_MMA);
-        ATT_STAMP_ANY(2);
-        if (nchunks > 0 && !*abort_flag) {
-            ATTN_WAIT(&k_full[0], 0u, AERR_MMA);
-            if (!*abort_flag) {
-                tc::tc_fence_after_sync();
-                qk(0);
+        bool ok = attn_warp_wait(q_full, 0u, AERR_MMA, deadline, abort_flag);
+#ifdef FRT_PHASE_STAMPS
+        if (lane == 0) ATT_STAMP_ANY(2);
+#endif
+        if (ok && nchunks > 0) {
+            ok = attn_warp_wait(&k_full[0], 0u, AERR_MMA, deadline, abort_flag);
+#pragma unroll
+            for (int blk = 0; blk < 4; ++blk) {              // the first chunk follows the blocks of Q as they land
+                if (ok && blk > 0) ok = attn_warp_wait(&q_part[blk - 1], 0u, AERR_MMA, deadline, abort_flag);
+                if (ok) {
+                    tc::tc_fence_after_sync();
+                    qk_block(0, blk);
+                }
             }
         }
-        for (int j = 0; j < nchunks && !*abort_flag; ++j) {
+        for (int j = 0; ok && j < nchunks; ++j) {
             if (j + 1 < nchunks) {      // S of the next chunk goes to the other buffer while the softmax works on this one
-                ATTN_WAIT(&k_full[(j + 1) & 1], (uint32_t)(((j + 1) >> 1) & 1), AERR_MMA);
-                if (*abort_flag) break;
+                ok = attn_warp_wait(&k_full[(j + 1) & 1], (uint32_t)(((j + 1) >> 1) & 1), AERR_MMA, deadline, abort_flag);
+                if (!ok) break;
                 tc::tc_fence_after_sync();
-                qk(j + 1);
+#pragma unroll
+                for (int blk = 0; blk < 4; ++blk) qk_block(j + 1, blk);
             }
-            ATTN_WAIT(&p_ready[j & 1], (uint32_t)((j >> 1) & 1), AERR_MMA);
-            ATTN_WAIT(&v_full[j & 1], (uint32_t)((j >> 1) & 1), AERR_MMA);
-            if (*abort_flag) break;
+            ok = attn_warp_wait(&v_full[j & 1], (uint32_t)((j >> 1) & 1), AERR_MMA, deadline, abort_flag) &&
+                 attn_warp_wait(&p_ready[j & 1], (uint32_t)((j >> 1) & 1), AERR_MMA, deadline, abort_flag);
+            if (!ok) break;
             tc::tc_fence_after_sync();
             const uint64_t dv = dv_base + (uint64_t)((j & 1) * (V_BYTES >> 4));
             const uint32_t a_tm = tmem + Cfg::S_COL + (j & 1) * 64;
+            if (tc::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BKV / 16; ++k)
-                tc::mma_f16_ts(tmem + Cfg::O_COL, a_tm + 8 * k, dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o,
-                               (j > 0 || k > 0) ? 1u : 0u);
-            tc::mma_commit(&kv_empty[j & 1]);
-            tc::mma_commit(o_full);
+                for (int k = 0; k < BKV / 16; ++k)
+                    tc::mma_f16_ts(tmem + Cfg::O_COL, a_tm + 8 * k, dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o,
+                                   (j > 0 || k > 0) ? 1u : 0u);
+                tc::mma_commit(kv_empty_a + 8 * (j & 1));
+                tc::mma_commit(o_full_a);
+            }
         }
-        if (!*abort_flag) tc::mma_commit(o_done);
-        ATT_STAMP_ANY(3);
+        if (ok && tc::elect_one()) tc::mma_commit(o_done);
+#ifdef FRT_PHASE_STAMPS
+        if (lane == 0) ATT_STAMP_ANY(3);
+#endif
     } else if (warp < 4) {
         // ---------------- softmax: thread = row
         pdl_wait();

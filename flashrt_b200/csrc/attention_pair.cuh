@@ -86,85 +86,93 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     pdl_launch_dependents();
 
-    if (warp == 8 && lane == 0) {
-        // ---------------- TMA producer
+    if (warp == 8) {
+        // ---------------- TMA producer (whole warp)
         pdl_wait();
-        tc::mbar_arrive_expect_tx(q_full, 2 * Cfg::Q_BYTES);
-        for (int t = 0; t < 2; ++t)
-            for (int db = 0; db < 2; ++db)
-                tc::tma_load_5d(sQ + t * Cfg::Q_BYTES + db * (128 * 128), &tmQ, q_full, db * 64, 0, hk,
-                                tok0 + t * tok_per_tile, b);
-        for (int j = 0; j < nchunks && !*abort_flag; ++j) {
-            const int st = j & 1;
-            if (j >= 2) ATTN_WAIT(&kv_empty[st], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER);
-            if (*abort_flag) break;
-            const int key0 = j * BKV;
-            tc::mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
-            for (int db = 0; db < 2; ++db)
-                tc::tma_load_4d(sK + st * Cfg::KV_BYTES + db * (BKV * 128), &tmK, &k_full[st], db * 64, hk, key0, b);
-            tc::mbar_arrive_expect_tx(&v_full[st], Cfg::KV_BYTES);
-            for (int db = 0; db < 2; ++db)
-                tc::tma_load_4d(sV + st * Cfg::KV_BYTES + db * (BKV * 128), &tmV, &v_full[st], db * 64, hk, key0, b);
+        if (tc::elect_one()) {
+            tc::mbar_arrive_expect_tx(q_full, 2 * Cfg::Q_BYTES);
+            for (int t = 0; t < 2; ++t)
+                for (int db = 0; db < 2; ++db)
+                    tc::tma_load_5d(sQ + t * Cfg::Q_BYTES + db * (128 * 128), &tmQ, q_full, db * 64, 0, hk,
+                                    tok0 + t * tok_per_tile, b);
         }
-    } else if (warp == 9 && lane == 0) {
-        // ---------------- MMA issuer
+        for (int j = 0; j < nchunks; ++j) {
+            const int st = j & 1;
+            if (j >= 2 && !attn_warp_wait(&kv_empty[st], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER, deadline, abort_flag)) break;
+            if (tc::elect_one()) {
+                const int key0 = j * BKV;
+                tc::mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
+                for (int db = 0; db < 2; ++db)
+                    tc::tma_load_4d(sK + st * Cfg::KV_BYTES + db * (BKV * 128), &tmK, &k_full[st], db * 64, hk, key0, b);
+                tc::mbar_arrive_expect_tx(&v_full[st], Cfg::KV_BYTES);
+                for (int db = 0; db < 2; ++db)
+                    tc::tma_load_4d(sV + st * Cfg::KV_BYTES + db * (BKV * 128), &tmV, &v_full[st], db * 64, hk, key0, b);
+            }
+        }
+    } else if (warp == 9) {
+        // ---------------- MMA issuer (whole warp)
         constexpr uint32_t idesc_s = tc::make_idesc(1, 1, 0, 0, 128, BKV);   // bf16 x bf16, both K-major
         constexpr uint32_t idesc_o = tc::make_idesc(1, 1, 0, 1, 128, D);     // A = P from TMEM, B = V MN-major
         // descriptors differ only in their start-address field (units of 16 bytes): build the bases once
         const uint64_t dq_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sQ));
         const uint64_t dk_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sK));
         const uint64_t dv_base = tc::make_desc_mnmajor_sw128(tc::smem_u32(sV), BKV * 128);
+        const uint32_t s_full_a = tc::smem_u32(s_full), kv_empty_a = tc::smem_u32(kv_empty);
         auto qk = [&](int t, int j) {
             const uint64_t dq = dq_base + (uint64_t)(t * (Cfg::Q_BYTES >> 4));
             const uint64_t dk = dk_base + (uint64_t)((j & 1) * (Cfg::KV_BYTES >> 4));
             const uint32_t d_tm = tmem + t * 128;
+            if (tc::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
-                // 64-element block k / 4 (16 KB apart), 32 bytes per K = 16 step inside the 128-byte row
-                const uint64_t off = (uint64_t)((k / 4) * ((128 * 128) >> 4) + 2 * (k % 4));
-                tc::mma_f16(d_tm, dq + off, dk + off, idesc_s, k > 0 ? 1u : 0u);
+                for (int k = 0; k < D / 16; ++k) {
+                    // 64-element block k / 4 (16 KB apart), 32 bytes per K = 16 step inside the 128-byte row
+                    const uint64_t off = (uint64_t)((k / 4) * ((128 * 128) >> 4) + 2 * (k % 4));
+                    tc::mma_f16(d_tm, dq + off, dk + off, idesc_s, k > 0 ? 1u : 0u);
+                }
+                tc::mma_commit(s_full_a + 8 * t);
             }
-            tc::mma_commit(&s_full[t]);
         };
-        auto pv = [&](int t, int j) {
+        auto pv = [&](int t, int j, bool release) {
             const uint64_t dv = dv_base + (uint64_t)((j & 1) * (Cfg::KV_BYTES >> 4));
             const uint32_t d_tm = tmem + 256 + t * 128, a_tm = tmem + t * 128;
+            if (tc::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BKV / 16; ++k)       // 16 keys = 16 rows of 128 bytes further on
-                tc::mma_f16_ts(d_tm, a_tm + 8 * k, dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o,
-                               (j > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < BKV / 16; ++k)       // 16 keys = 16 rows of 128 bytes further on
+                    tc::mma_f16_ts(d_tm, a_tm + 8 * k, dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o,
+                                   (j > 0 || k > 0) ? 1u : 0u);
+                if (release) tc::mma_commit(kv_empty_a + 8 * (j & 1));
+            }
         };
-        ATTN_WAIT(q_full, 0u, AERR_MMA);
-        if (nchunks > 0 && !*abort_flag) {
-            ATTN_WAIT(&k_full[0], 0u, AERR_MMA);
-            if (!*abort_flag) {
+        bool ok = attn_warp_wait(q_full, 0u, AERR_MMA, deadline, abort_flag);
+        if (ok && nchunks > 0) {
+            ok = attn_warp_wait(&k_full[0], 0u, AERR_MMA, deadline, abort_flag);
+            if (ok) {
                 tc::tc_fence_after_sync();
                 qk(0, 0);
                 qk(1, 0);
             }
         }
-        for (int j = 0; j < nchunks && !*abort_flag; ++j) {
+        for (int j = 0; ok && j < nchunks; ++j) {
             const int st = j & 1;
             const uint32_t ph = (uint32_t)(j & 1);
-            ATTN_WAIT(&p_ready[0], ph, AERR_MMA);
-            ATTN_WAIT(&v_full[st], (uint32_t)((j >> 1) & 1), AERR_MMA);
-            if (*abort_flag) break;
+            ok = attn_warp_wait(&v_full[st], (uint32_t)((j >> 1) & 1), AERR_MMA, deadline, abort_flag) &&
+                 attn_warp_wait(&p_ready[0], ph, AERR_MMA, deadline, abort_flag);
+            if (!ok) break;
             tc::tc_fence_after_sync();
-            pv(0, j);
+            pv(0, j, false);
             if (j + 1 < nchunks) {
-                ATTN_WAIT(&k_full[(j + 1) & 1], (uint32_t)(((j + 1) >> 1) & 1), AERR_MMA);
-                if (*abort_flag) break;
+                ok = attn_warp_wait(&k_full[(j + 1) & 1], (uint32_t)(((j + 1) >> 1) & 1), AERR_MMA, deadline, abort_flag);
+                if (!ok) break;
                 tc::tc_fence_after_sync();
                 qk(0, j + 1);
             }
-            ATTN_WAIT(&p_ready[1], ph, AERR_MMA);
-            if (*abort_flag) break;
+            ok = attn_warp_wait(&p_ready[1], ph, AERR_MMA, deadline, abort_flag);
+            if (!ok) break;
             tc::tc_fence_after_sync();
-            pv(1, j);
-            tc::mma_commit(&kv_empty[st]);
+            pv(1, j, true);
             if (j + 1 < nchunks) qk(1, j + 1);
         }
-        if (!*abort_flag) tc::mma_commit(o_done);
+        if (ok && tc::elect_one()) tc::mma_commit(o_done);
     } else if (warp < 8) {
         // ---------------- softmax: tile t, thread = row
         pdl_wait();

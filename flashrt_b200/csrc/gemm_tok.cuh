@@ -2,9 +2,8 @@
 //
 // Included by gemm_fp8.cu inside namespace frt (tensor-map cache, status word, arithmetic helpers).
 //
-// Why this orientation for M <= 128 activation rows: a tcgen05.mma (kind::f8f6f4, K = 32) costs the issuing
-// thread about 160 cycles whatever its shape (measured: 128 x 256, 128 x 64 and 64 x 8 all take the same time), so
-// the launch-latency-bound GEMMs of the denoise loop want as many weight bytes per instruction as possible and as
+// Why this orientation for M <= 128 activation rows: an M = 128 tcgen05.mma takes N / 2 cycles but not less than about 50,
+// so the launch-latency-bound GEMMs of the denoise loop want as many weight bytes per instruction as possible and as
 // few instructions per CTA as possible:
 //   * weights on N: up to 256 weight rows x 32 K-bytes = 8 KB per instruction (the swapped kernel moves 4 KB);
 //   * split-K over a thread-block cluster (1 x 1 x S, S <= 8): a CTA owns BN weight rows x K / S, i.e. 2-4 k-blocks
@@ -264,49 +263,57 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
     pdl_launch_dependents();
 
-    if (warp == 0 && lane == 0) {
-        // ---------------- TMA producer: the weights do not depend on the producer grid and start streaming now
+    if (warp == 0) {
+        // ---------------- TMA producer (whole warp, see warp_wait): the weights do not depend on the producer grid and start
+        // streaming now
         const uint32_t tx = (PRO == TOK_PRO_TMA) ? STAGE_BYTES : Cfg::W_BYTES;
+        const uint32_t ring = tc::smem_u32(tiles), full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty);
         auto load_w = [&](int stage, int kb) {
-            uint8_t* dst = tiles + stage * STAGE_BYTES + A_BYTES;
+            const uint32_t dst = ring + stage * STAGE_BYTES + A_BYTES, bar = full_a + 8 * stage;
             if (p.w_kn) {
                 // (K, N) weights: boxes of 128 K-rows x 128 N-bytes, one per 128 output features; the tile is then an
                 // MN-major operand (128-byte rows along N, 8 K-rows per swizzle atom, 16 KB between the chunks)
 #pragma unroll
                 for (int j = 0; j < (BN >= 128 ? BN / 128 : 1); ++j) {
                     const int nj = (EPI == TOK_EPI_GEGLU && j == 1) ? p.half + n0 : n0 + j * 128;
-                    tc::tma_load_2d(dst + j * 16384, &tmW, &full[stage], nj, kb * 128);
+                    tc::tma_load_2d(dst + j * 16384, &tmW, bar, nj, kb * 128);
                 }
             } else if (EPI == TOK_EPI_GEGLU) {      // tmW has a box of BN / 2 rows here
-                tc::tma_load_2d(dst, &tmW, &full[stage], kb * 128, n0);
-                tc::tma_load_2d(dst + (BN / 2) * 128, &tmW, &full[stage], kb * 128, p.half + n0);
+                tc::tma_load_2d(dst, &tmW, bar, kb * 128, n0);
+                tc::tma_load_2d(dst + (BN / 2) * 128, &tmW, bar, kb * 128, p.half + n0);
             } else {
-                tc::tma_load_2d(dst, &tmW, &full[stage], kb * 128, n0);
+                tc::tma_load_2d(dst, &tmW, bar, kb * 128, n0);
             }
         };
         const int pre = nkb < STG ? nkb : STG;
-        for (int i = 0; i < pre; ++i) {
-            tc::mbar_arrive_expect_tx(&full[i], tx);
-            load_w(i, kb0 + i);
+        if (tc::elect_one()) {
+            for (int i = 0; i < pre; ++i) {
+                tc::mbar_arrive_expect_tx(full_a + 8 * i, tx);
+                load_w(i, kb0 + i);
+            }
         }
         pdl_wait();
-        if (PRO == TOK_PRO_TMA) {
-            for (int i = 0; i < pre; ++i)
-                tc::tma_load_2d(tiles + i * STAGE_BYTES, &tmA, &full[i], (kb0 + i) * 128, m0);
+        if (tc::elect_one()) {
+            if (PRO == TOK_PRO_TMA) {
+                for (int i = 0; i < pre; ++i)
+                    tc::tma_load_2d(ring + i * STAGE_BYTES, &tmA, full_a + 8 * i, (kb0 + i) * 128, m0);
+            }
+            *issued = pre;
         }
-        *issued = pre;
         int s = 0;                                    // ring position: i = pre = STG here
         uint32_t ph = 0;
         for (int i = pre; i < nkb; ++i) {
-            if (!tc::mbar_wait_until(&empty[s], ph, deadline, abort_flag)) {
+            if (!tc::warp_wait(empty_a + 8 * s, ph, false, deadline, abort_flag)) {
                 *abort_flag = 1;
-                atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
+                if (lane == 0) atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
                 break;
             }
-            tc::mbar_arrive_expect_tx(&full[s], tx);
-            load_w(s, kb0 + i);
-            if (PRO == TOK_PRO_TMA) tc::tma_load_2d(tiles + s * STAGE_BYTES, &tmA, &full[s], (kb0 + i) * 128, m0);
-            *issued = i + 1;
+            if (tc::elect_one()) {
+                tc::mbar_arrive_expect_tx(full_a + 8 * s, tx);
+                load_w(s, kb0 + i);
+                if (PRO == TOK_PRO_TMA) tc::tma_load_2d(ring + s * STAGE_BYTES, &tmA, full_a + 8 * s, (kb0 + i) * 128, m0);
+                *issued = i + 1;
+            }
             if (++s == STG) { s = 0; ph ^= 1; }
         }
     }
@@ -403,17 +410,12 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         TOK_STAMP(12);
     }
 
-    if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer
+    if (warp == 1) {
+        // ---------------- MMA issuer (whole warp)
         const uint32_t idesc = tc::make_idesc(0, 0, 0, 0, m64 ? 64 : 128, BN) | (p.w_kn ? (1u << 16) : 0u);   // bit 16: B MN-major
         bool failed = false;
-        if (PRO == TOK_PRO_NORM) {
-            if (!tc::mbar_wait_until(a_ready, 0, deadline, abort_flag)) {
-                *abort_flag = 1;
-                atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
-                failed = true;
-            }
-        }
+        if (PRO == TOK_PRO_NORM) failed = !tc::warp_wait(tc::smem_u32(a_ready), 0, false, deadline, abort_flag);
+        const uint32_t full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty), accum_a = tc::smem_u32(accum_bar);
         const uint64_t dA0 = tc::make_desc_kmajor_sw128(tc::smem_u32(tiles));
         const uint64_t dW0 = p.w_kn ? tc::make_desc_mnmajor_sw128(tc::smem_u32(tiles + A_BYTES), 16384)
                                     : tc::make_desc_kmajor_sw128(tc::smem_u32(tiles + A_BYTES));
@@ -421,28 +423,35 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const uint64_t wstep = p.w_kn ? (uint64_t)((32 * 128) >> 4) : 2u;
         int s = 0;
         uint32_t ph = 0;
+        bool ready = false;
         for (int i = 0; i < nkb && !failed; ++i) {
-            if (!tc::mbar_wait_until(&full[s], ph, deadline, abort_flag)) {
-                *abort_flag = 1;
-                atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
+            if (!tc::warp_wait(full_a + 8 * s, ph, ready, deadline, abort_flag)) {
                 failed = true;
                 break;
             }
             tc::tc_fence_after_sync();
 #ifdef FRT_PHASE_STAMPS
-            if (i == 0) g_tok_trace[p.trace_slot][(blockIdx.z * gridDim.x + blockIdx.x) % 160][10] = tc::global_timer_ns();
+            if (i == 0 && lane == 0) g_tok_trace[p.trace_slot][(blockIdx.z * gridDim.x + blockIdx.x) % 160][10] = tc::global_timer_ns();
 #endif
             const uint64_t so = (uint64_t)((s * STAGE_BYTES) >> 4);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)   // 4 x (K = 32) per 128-byte k-block; +32 bytes = +2 in the address field
-                tc::mma_f8(tmem_d, dA0 + so + 2 * k, dW0 + so + wstep * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-            tc::mma_commit(&empty[s]);
-            *consumed = i + 1;
+            const uint32_t done = empty_a + 8 * s;
             if (++s == STG) { s = 0; ph ^= 1; }
+            ready = tc::mbar_test(full_a + 8 * s, ph);
+            if (tc::elect_one()) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)   // 4 x (K = 32) per 128-byte k-block; +32 bytes = +2 in the address field
+                    tc::mma_f8(tmem_d, dA0 + so + 2 * k, dW0 + so + wstep * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                if (i + STG < nkb) tc::mma_commit(done);         // a slot that is filled again
+                if (i == nkb - 1) tc::mma_commit(accum_a);
+                *consumed = i + 1;
+            }
         }
-        if (!failed) tc::mma_commit(accum_bar);
+        if (failed) {
+            *abort_flag = 1;
+            if (lane == 0) atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
+        }
 #ifdef FRT_PHASE_STAMPS
-        g_tok_trace[p.trace_slot][(blockIdx.z * gridDim.x + blockIdx.x) % 160][11] = tc::global_timer_ns();
+        if (lane == 0) g_tok_trace[p.trace_slot][(blockIdx.z * gridDim.x + blockIdx.x) % 160][11] = tc::global_timer_ns();
 #endif
     }
     __syncwarp();
