@@ -679,11 +679,10 @@ static int launch_attn(const void* Q, const void* K, const void* V, AttnParams p
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = p.o_accum ? 1 : splits;
     ++na;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    if (!pdl) p.kv_static_rows = 0;                     // nothing is fetched before the kernel in front has finished
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
     cfg.attrs = attr;
     cfg.numAttrs = na;
     if (p.o_accum && splits > 1) {
@@ -763,7 +762,12 @@ int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, voi
         // through the caller's scratch, or there is nothing to combine; flags bit 1 keeps the single-tile kernel
         if (!(flags & 2)) {
             const int chunks64 = (seqlen_k + 63) / 64;
-            int sp64 = kv_splits > 0 ? kv_splits : (tiles >= 74 ? 1 : (chunks64 < 8 ? chunks64 : 8));
+            // Without scratch one split of this kernel (about 5 + 1.1 us per chunk) against the single-tile kernel's cluster
+            // of splits (about 15 us while all clusters fit one wave): one split when the chain is short or the tiles alone
+            // cover the device (768 x 768 x 8 heads, 48 tiles: 58 us as clusters of four in two waves, MEASURED_ENC as one
+            // split each).
+            const bool one = p.o_accum ? tiles >= 74 : (tiles > 18 || chunks64 <= 9);
+            int sp64 = kv_splits > 0 ? kv_splits : (one ? 1 : (chunks64 < 8 ? chunks64 : 8));
             if (sp64 > 8) sp64 = 8;
             if (p.o_accum || sp64 == 1)
                 return launch_attn_d256(Q, K, V, p, q_strides, k_strides, v_strides, p.o_accum ? sp64 : 1, pdl, s);
@@ -780,7 +784,7 @@ int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, voi
     if (sp > 8) sp = 8;
     // one split and at least two row tiles: the two-tile ping-pong kernel (softmax overlapped with the MMAs)
     if (sp == 1 && (seqlen_q * G + 127) / 128 >= 2)
-        return launch_attn_pair(Q, K, V, p, q_strides, k_strides, v_strides, pdl, s);
+        return launch_attn_pair(Q, K, V, p, q_strides, k_strides, v_strides, s);
     return launch_attn<128, BKV>(Q, K, V, p, q_strides, k_strides, v_strides, sp, pdl, s);
 }
 

@@ -892,11 +892,10 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    if (!pdl) p.kv_static_rows = 0;                     // nothing is fetched before the kernel in front has finished
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
     if (xc) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = 1;

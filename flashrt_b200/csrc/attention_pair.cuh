@@ -312,7 +312,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnParams p, const long long* qs,
-                            const long long* ks, const long long* vs, bool pdl, cudaStream_t stream) {
+                            const long long* ks, const long long* vs, cudaStream_t stream) {
     using Cfg = PairCfg;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
@@ -352,7 +352,7 @@ static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnPar
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;                                  // nothing global is read before the wait
     cudaError_t e = cudaLaunchKernelEx(&cfg, attn_pair_kernel, tmQ, tmK, tmV, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

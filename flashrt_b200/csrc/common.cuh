@@ -202,8 +202,12 @@ __device__ __forceinline__ void st_global_v2(void* p, uint2 v) {
     *reinterpret_cast<uint2*>(p) = v;
 }
 
-// programmatic dependent launch: wait for the producer grid's memory, and
-// let the dependent grid start its prologue early.
+// Programmatic dependent launch: wait for the producer grid's memory, and let the dependent grid start its prologue early.
+// Every kernel that waits before its first global access is launched with the programmatic attribute, whether or not the
+// caller passed the PDL flag: its CTAs are then set up (barriers, tensor memory, descriptors) while the kernel in front
+// drains, about 1 us per launch.  Behind a kernel that never calls launch_dependents the attribute changes nothing.  The
+// caller's flag says more: weights, styles and scales do not come from the kernel in front and may be read before the wait
+// (`early`).
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

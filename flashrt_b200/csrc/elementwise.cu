@@ -34,7 +34,7 @@ static inline unsigned grid_for(long long work_items, int threads, int ctas_per_
 }
 
 template <typename K, typename... Args>
-static int launch(K kernel, unsigned grid, unsigned block, cudaStream_t stream, bool pdl, Args... args) {
+static int launch(K kernel, unsigned grid, unsigned block, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -43,7 +43,7 @@ static int launch(K kernel, unsigned grid, unsigned block, cudaStream_t stream, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;                    // every kernel launched here waits before its first global access
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
@@ -54,8 +54,9 @@ template <int ACT>
 __global__ void __launch_bounds__(256)
 geglu_fp8_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict__ out, int rows, int H,
                  const float* __restrict__ d_scale) {
-    const float inv_scale = __fdiv_rn(1.0f, *d_scale);
+    pdl_launch_dependents();
     pdl_wait();
+    const float inv_scale = __fdiv_rn(1.0f, *d_scale);
     const int vec_per_row = H >> 3;
     const long long total = (long long)rows * vec_per_row;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -81,13 +82,13 @@ geglu_fp8_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict__
         ov.y = f32x4_to_e4m3x4(o[4], o[5], o[6], o[7]);
         st_global_v2(out + row * H + col, ov);
     }
-    pdl_launch_dependents();
 }
 
 // merged -> bf16 (non-quantised sibling, reference gate_geglu_merged)
 template <int ACT>
 __global__ void __launch_bounds__(256)
 geglu_bf16_kernel(const __nv_bfloat16* __restrict__ merged, __nv_bfloat16* __restrict__ out, int rows, int H) {
+    pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = H >> 3;
     const long long total = (long long)rows * vec_per_row;
@@ -111,15 +112,15 @@ geglu_bf16_kernel(const __nv_bfloat16* __restrict__ merged, __nv_bfloat16* __res
         }
         st_global_v4(out + row * H + col, ov);
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ bf16 -> FP8, given scale
 __global__ void __launch_bounds__(256)
 quantize_fp8_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict__ out, long long n,
                     const float* __restrict__ d_scale) {
-    const float inv_scale = __fdiv_rn(1.0f, *d_scale);
+    pdl_launch_dependents();
     pdl_wait();
+    const float inv_scale = __fdiv_rn(1.0f, *d_scale);
     const long long nvec = n >> 3;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
          i += (long long)gridDim.x * blockDim.x) {
@@ -144,7 +145,6 @@ quantize_fp8_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict__ 
             out[j] = (uint8_t)(f32x2_to_e4m3x2(f, 0.0f) & 0xff);
         }
     }
-    pdl_launch_dependents();
 }
 
 // absmax into *d_amax (float, non-negative: ordered as int)
@@ -185,6 +185,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256)
 add_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
            const __nv_bfloat16* __restrict__ aux, long long aux_stride, long long rows, int dim) {
+    pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = dim >> 3;
     const long long total = rows * vec_per_row;
@@ -222,7 +223,6 @@ add_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
         }
         st_global_v4(res + i * 8, ov);
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ RoPE + QKV split + KV append
@@ -235,8 +235,9 @@ qkv_split_rope_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16
                       __nv_bfloat16* __restrict__ Q, __nv_bfloat16* __restrict__ K,
                       __nv_bfloat16* __restrict__ V, const int* __restrict__ devpos, int seq, int q_dim,
                       int k_dim, int v_dim, int head_dim) {
-    const int pos = devpos ? *devpos : 0;
+    pdl_launch_dependents();
     pdl_wait();
+    const int pos = devpos ? *devpos : 0;
     const int row_w = q_dim + k_dim + v_dim;
     const int vec_per_row = row_w >> 3;
     const long long total = (long long)seq * vec_per_row;
@@ -269,7 +270,6 @@ qkv_split_rope_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16
         if (is_q) st_global_v4(Q + (long long)row * q_dim + c, o);
         else st_global_v4(K + (long long)(pos + row) * k_dim + c, o);
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ classifier-free guidance combine
@@ -278,6 +278,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 cfg_combine_kernel(T* __restrict__ residual, const T* __restrict__ v_cond, const T* __restrict__ v_uncond,
                    float beta, long long n) {
+    pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float r, vc, vu;
@@ -289,11 +290,11 @@ cfg_combine_kernel(T* __restrict__ residual, const T* __restrict__ v_cond, const
         const float out = __fadd_rn(r, __fmaf_rn(beta, __fsub_rn(vc, vu), vu));
         if constexpr (sizeof(T) == 4) residual[i] = out; else residual[i] = __float2bfloat16_rn(out);
     }
-    pdl_launch_dependents();
 }
 
 // the three status words of the tensor-core kernels into one array (and optionally cleared), in stream order
 __global__ void status_gather_kernel(int* gemm, int* attn, int* loop, int* out, int reset) {
+    pdl_launch_dependents();
     pdl_wait();
     if (threadIdx.x == 0) {
         out[0] = *gemm;
@@ -317,9 +318,9 @@ int frt_b200_geglu_fp8(const void* merged, void* out_fp8, int rows, int half_dim
     if (rows == 0) return FRT_OK;
     long long items = (long long)rows * (half_dim >> 3);
     if (flags & 2)      // SiLU gate (SwiGLU)
-        return launch(geglu_fp8_kernel<1>, grid_for(items, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+        return launch(geglu_fp8_kernel<1>, grid_for(items, 256, 8), 256, (cudaStream_t)stream,
                       (const __nv_bfloat16*)merged, (uint8_t*)out_fp8, rows, half_dim, d_scale);
-    return launch(geglu_fp8_kernel<0>, grid_for(items, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(geglu_fp8_kernel<0>, grid_for(items, 256, 8), 256, (cudaStream_t)stream,
                   (const __nv_bfloat16*)merged, (uint8_t*)out_fp8, rows, half_dim, d_scale);
 }
 
@@ -329,9 +330,9 @@ int frt_b200_geglu_bf16(const void* merged, void* out_bf16, int rows, int half_d
     if (rows == 0) return FRT_OK;
     long long items = (long long)rows * (half_dim >> 3);
     if (flags & 2)
-        return launch(geglu_bf16_kernel<1>, grid_for(items, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+        return launch(geglu_bf16_kernel<1>, grid_for(items, 256, 8), 256, (cudaStream_t)stream,
                       (const __nv_bfloat16*)merged, (__nv_bfloat16*)out_bf16, rows, half_dim);
-    return launch(geglu_bf16_kernel<0>, grid_for(items, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(geglu_bf16_kernel<0>, grid_for(items, 256, 8), 256, (cudaStream_t)stream,
                   (const __nv_bfloat16*)merged, (__nv_bfloat16*)out_bf16, rows, half_dim);
 }
 
@@ -340,7 +341,7 @@ int frt_b200_quantize_fp8_static(const void* in_bf16, void* out_fp8, const float
     if (!in_bf16 || !out_fp8 || !d_scale || n < 0) return FRT_ERR_INVALID;
     if (mis16(in_bf16) || (reinterpret_cast<uintptr_t>(out_fp8) & 7)) return FRT_ERR_UNSUPPORTED;
     if (n == 0) return FRT_OK;
-    return launch(quantize_fp8_kernel, grid_for((n + 7) >> 3, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(quantize_fp8_kernel, grid_for((n + 7) >> 3, 256, 8), 256, (cudaStream_t)stream,
                   (const __nv_bfloat16*)in_bf16, (uint8_t*)out_fp8, n, d_scale);
 }
 
@@ -372,7 +373,7 @@ int frt_b200_residual_add(void* residual, const void* x, long long n, int flags,
     if (!residual || !x || n < 0) return FRT_ERR_INVALID;
     if ((n & 7) || mis16(residual) || mis16(x)) return FRT_ERR_UNSUPPORTED;
     if (n == 0) return FRT_OK;
-    return launch(add_kernel<0>, grid_for(n >> 3, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(add_kernel<0>, grid_for(n >> 3, 256, 8), 256, (cudaStream_t)stream,
                   (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)nullptr, 0LL,
                   (long long)1, (int)n);
 }
@@ -383,7 +384,7 @@ int frt_b200_bias_residual(void* residual, const void* x, const void* bias, int 
     if ((dim & 7) || mis16(residual) || mis16(x) || mis16(bias)) return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
     return launch(add_kernel<1>, grid_for((long long)rows * (dim >> 3), 256, 8), 256, (cudaStream_t)stream,
-                  flags & 1, (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)bias, 0LL,
+                  (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)bias, 0LL,
                   (long long)rows, dim);
 }
 
@@ -393,7 +394,7 @@ int frt_b200_gate_mul_residual(void* residual, const void* x, const void* gate, 
     if ((dim & 7) || (gate_stride & 7) || mis16(residual) || mis16(x) || mis16(gate)) return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
     return launch(add_kernel<2>, grid_for((long long)rows * (dim >> 3), 256, 8), 256, (cudaStream_t)stream,
-                  flags & 1, (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gate,
+                  (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gate,
                   gate_stride, (long long)rows, dim);
 }
 
@@ -406,7 +407,7 @@ int frt_b200_qkv_split_rope(const void* qkv, const void* rope, void* Q, void* K,
     if (mis16(qkv) || mis16(rope) || mis16(Q) || mis16(K) || mis16(V)) return FRT_ERR_UNSUPPORTED;
     if (seq == 0) return FRT_OK;
     long long items = (long long)seq * ((q_dim + k_dim + v_dim) >> 3);
-    return launch(qkv_split_rope_kernel, grid_for(items, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(qkv_split_rope_kernel, grid_for(items, 256, 8), 256, (cudaStream_t)stream,
                   (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)rope, (__nv_bfloat16*)Q, (__nv_bfloat16*)K,
                   (__nv_bfloat16*)V, devpos, seq, q_dim, k_dim, v_dim, head_dim);
 }
@@ -419,9 +420,9 @@ int frt_b200_cfg_combine_into_residual(void* residual, const void* v_cond, const
     if (n & 1) return FRT_ERR_UNSUPPORTED;
     if (n == 0) return FRT_OK;
     if (f32)
-        return launch(cfg_combine_kernel<float>, grid_for(n, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+        return launch(cfg_combine_kernel<float>, grid_for(n, 256, 8), 256, (cudaStream_t)stream,
                       (float*)residual, (const float*)v_cond, (const float*)v_uncond, beta, n);
-    return launch(cfg_combine_kernel<__nv_bfloat16>, grid_for(n, 256, 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch(cfg_combine_kernel<__nv_bfloat16>, grid_for(n, 256, 8), 256, (cudaStream_t)stream,
                   (__nv_bfloat16*)residual, (const __nv_bfloat16*)v_cond, (const __nv_bfloat16*)v_uncond, beta, n);
 }
 
@@ -442,7 +443,7 @@ int frt_b200_status_words_async(int* out3, int reset, int flags, void* stream) {
         if (!a || !b || !c) return FRT_ERR_INVALID;
         ptrs[dev][0] = a; ptrs[dev][1] = b; ptrs[dev][2] = c;
     }
-    return launch(status_gather_kernel, 1, 32, (cudaStream_t)stream, flags & 1, ptrs[dev][0], ptrs[dev][1], ptrs[dev][2],
+    return launch(status_gather_kernel, 1, 32, (cudaStream_t)stream, ptrs[dev][0], ptrs[dev][1], ptrs[dev][2],
                   out3, reset);
 }
 

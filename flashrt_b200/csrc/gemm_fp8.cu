@@ -110,6 +110,7 @@ struct GemmParams {
     float eps;
     int w_kn;                  // large-M persistent kernel: weights stored (K, N) row-major
     int tile_gm;               // large-M kernels: m-tiles per group of the tile order
+    int early;                 // the weights may be read before the kernel in front has finished
 };
 
 enum { EPI_BF16 = 0, EPI_ROPE_SPLIT = 1, EPI_GEGLU_FP8 = 2, EPI_GATE_RES_NORM_FP8 = 3 };
@@ -228,8 +229,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
 
     pdl_launch_dependents();
 
-    if (warp == 0 && lane == 0) {
-        // ---------------- TMA producer
+    if (warp == 0) {
+        // ---------------- TMA producer (whole warp, see tc::warp_wait)
         const CUtensorMap* tmW = p.w_is_lane ? &tmL : &tmC;
         const CUtensorMap* tmX = p.w_is_lane ? &tmC : &tmL;
         const int w_off = p.w_is_lane ? 0 : Cfg::L_BYTES;
@@ -237,15 +238,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
         const int w_row = p.w_is_lane ? lane0 : col0;
         const int x_row = p.w_is_lane ? col0 : lane0;
         const int pre = nkb < STAGES ? nkb : STAGES;
+        const uint32_t ring = tc::smem_u32(stage_base), full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty);
         // weights do not depend on the producer grid: start streaming them now
         auto load_w = [&](int stage, int kb) {
-            uint8_t* dst = stage_base + stage * Cfg::STAGE_BYTES + w_off;
-            if (EPI == EPI_GEGLU_FP8) {   // tmL has a 64-row box here
-                tc::tma_load_2d(dst, tmW, &full[stage], kb * 128, w_row);
-                tc::tma_load_2d(dst + 64 * 128, tmW, &full[stage], kb * 128, p.half + w_row);
-            } else {
-                tc::tma_load_2d(dst, tmW, &full[stage], kb * 128, w_row);
-            }
+            const uint32_t dst = ring + stage * Cfg::STAGE_BYTES + w_off, bar = full_a + 8 * stage;
+            tc::tma_load_2d(dst, tmW, bar, kb * 128, w_row);
+            if (EPI == EPI_GEGLU_FP8)     // tmL has a 64-row box here
+                tc::tma_load_2d(dst + 64 * 128, tmW, bar, kb * 128, p.half + w_row);
         };
         // NVFP4: the scale atoms of a k-block (4 K-steps) are 2048 contiguous bytes per 128-row group
         int c_atoms = Cfg::CB;
@@ -255,92 +254,106 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
         }
         const uint32_t stage_tx = Cfg::STAGE_BYTES - (FP4 ? (Cfg::CB - c_atoms) * 2048 : 0);
         auto load_sf_lane = [&](int stage, int kb) {
-            uint8_t* dst = stage_base + stage * Cfg::STAGE_BYTES + Cfg::L_BYTES + Cfg::C_BYTES;
-            tc::bulk_load(dst, p.sf_lane + ((size_t)(lane0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512, 2048,
-                          &full[stage]);
+            tc::bulk_load(ring + stage * Cfg::STAGE_BYTES + Cfg::L_BYTES + Cfg::C_BYTES,
+                          p.sf_lane + ((size_t)(lane0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512, 2048, full_a + 8 * stage);
         };
         auto load_sf_col = [&](int stage, int kb) {
-            uint8_t* dst = stage_base + stage * Cfg::STAGE_BYTES + Cfg::L_BYTES + Cfg::C_BYTES + Cfg::SFL_BYTES;
+            const uint32_t dst = ring + stage * Cfg::STAGE_BYTES + Cfg::L_BYTES + Cfg::C_BYTES + Cfg::SFL_BYTES;
             for (int j = 0; j < c_atoms; ++j)
                 tc::bulk_load(dst + j * 2048,
                               p.sf_col + ((size_t)(col0 / 128 + j) * p.sf_katoms + (size_t)kb * 4) * 512, 2048,
-                              &full[stage]);
+                              full_a + 8 * stage);
         };
-        for (int i = 0; i < pre; ++i) {
-            tc::mbar_arrive_expect_tx(&full[i], stage_tx);
-            load_w(i, kb_begin + i);
-            if (FP4) { if (p.w_is_lane) load_sf_lane(i, kb_begin + i); else load_sf_col(i, kb_begin + i); }
+        if (!p.early) pdl_wait();
+        if (tc::elect_one()) {
+            for (int i = 0; i < pre; ++i) {
+                tc::mbar_arrive_expect_tx(full_a + 8 * i, stage_tx);
+                load_w(i, kb_begin + i);
+                if (FP4) { if (p.w_is_lane) load_sf_lane(i, kb_begin + i); else load_sf_col(i, kb_begin + i); }
+            }
         }
         pdl_wait();
-        for (int i = 0; i < pre; ++i) {
-            tc::tma_load_2d(stage_base + i * Cfg::STAGE_BYTES + x_off, tmX, &full[i], (kb_begin + i) * 128, x_row);
-            if (FP4) { if (p.w_is_lane) load_sf_col(i, kb_begin + i); else load_sf_lane(i, kb_begin + i); }
+        if (tc::elect_one()) {
+            for (int i = 0; i < pre; ++i) {
+                tc::tma_load_2d(ring + i * Cfg::STAGE_BYTES + x_off, tmX, full_a + 8 * i, (kb_begin + i) * 128, x_row);
+                if (FP4) { if (p.w_is_lane) load_sf_col(i, kb_begin + i); else load_sf_lane(i, kb_begin + i); }
+            }
+            *issued = pre;
         }
-        *issued = pre;
+        int s = 0;
+        uint32_t ph = 0;
+        bool ready = false;
         for (int i = pre; i < nkb; ++i) {
-            const int s = i % STAGES;
-            const uint32_t ph = ((i / STAGES) - 1) & 1;
-            const bool ok = tc::mbar_wait_until(&empty[s], ph, deadline, abort_flag);
-            if (!ok) {
+            if (!tc::warp_wait(empty_a + 8 * s, ph, ready, deadline, abort_flag)) {
                 *abort_flag = 1;
-                atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
+                if (lane == 0) atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
                 break;
             }
-            tc::mbar_arrive_expect_tx(&full[s], stage_tx);
-            load_w(s, kb_begin + i);
-            tc::tma_load_2d(stage_base + s * Cfg::STAGE_BYTES + x_off, tmX, &full[s], (kb_begin + i) * 128, x_row);
-            if (FP4) {
-                load_sf_lane(s, kb_begin + i);
-                load_sf_col(s, kb_begin + i);
+            const int at = s;
+            if (++s == STAGES) { s = 0; ph ^= 1; }
+            ready = tc::mbar_test(empty_a + 8 * s, ph);
+            if (tc::elect_one()) {
+                tc::mbar_arrive_expect_tx(full_a + 8 * at, stage_tx);
+                load_w(at, kb_begin + i);
+                tc::tma_load_2d(ring + at * Cfg::STAGE_BYTES + x_off, tmX, full_a + 8 * at, (kb_begin + i) * 128, x_row);
+                if (FP4) {
+                    load_sf_lane(at, kb_begin + i);
+                    load_sf_col(at, kb_begin + i);
+                }
+                *issued = i + 1;
             }
-            *issued = i + 1;
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (whole warp)
         constexpr uint32_t idesc = FP4 ? tc::make_idesc_nvfp4(128, BN) : tc::make_idesc(0, 0, 0, 0, 128, BN);
         // NVFP4 scale factors in tensor memory, behind the accumulator: 4 columns per (operand atom, K-step)
         const uint32_t tmem_sfl = tmem_d + Cfg::ACC_COLS;
         const uint32_t tmem_sfc = tmem_sfl + 16;
         const uint32_t sfc_off = BN < 128 ? (uint32_t)((col0 & 127) >> 5) : 0u;   // 32-row group of this column tile
-        bool failed = false;
+        const uint32_t ring = tc::smem_u32(stage_base), full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty);
+        const uint32_t accum_a = tc::smem_u32(accum_bar);
+        const uint64_t dL0 = tc::make_desc_kmajor_sw128(ring), dC0 = tc::make_desc_kmajor_sw128(ring + Cfg::L_BYTES);
+        bool failed = false, ready = false;
+        int s = 0;
+        uint32_t ph = 0;
         for (int i = 0; i < nkb; ++i) {
-            const int s = i % STAGES;
-            const uint32_t ph = (i / STAGES) & 1;
-            const bool ok = tc::mbar_wait_until(&full[s], ph, deadline, abort_flag);
-            if (!ok) {
-                *abort_flag = 1;
-                atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
+            if (!tc::warp_wait(full_a + 8 * s, ph, ready, deadline, abort_flag)) {
                 failed = true;
                 break;
             }
             tc::tc_fence_after_sync();
-            const uint32_t sL = tc::smem_u32(stage_base + s * Cfg::STAGE_BYTES);
-            const uint32_t sC = sL + Cfg::L_BYTES;
-            const uint64_t dL = tc::make_desc_kmajor_sw128(sL);
-            const uint64_t dC = tc::make_desc_kmajor_sw128(sC);
-            if (FP4) {
-                const uint32_t sSFL = sC + Cfg::C_BYTES;
-                const uint32_t sSFC = sSFL + Cfg::SFL_BYTES;
+            const uint64_t so = (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
+            const uint32_t sf = ring + s * Cfg::STAGE_BYTES + Cfg::L_BYTES + Cfg::C_BYTES, done = empty_a + 8 * s;
+            if (++s == STAGES) { s = 0; ph ^= 1; }
+            ready = tc::mbar_test(full_a + 8 * s, ph);
+            if (tc::elect_one()) {
+                if (FP4) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    tc::tmem_cp_sf_atom(tmem_sfl + 4 * k, sSFL + 512 * k);
+                    for (int k = 0; k < 4; ++k) {
+                        tc::tmem_cp_sf_atom(tmem_sfl + 4 * k, sf + 512 * k);
 #pragma unroll
-                    for (int j = 0; j < Cfg::CB; ++j)
-                        tc::tmem_cp_sf_atom(tmem_sfc + k * 4 * Cfg::CB + 4 * j, sSFC + j * 2048 + 512 * k);
+                        for (int j = 0; j < Cfg::CB; ++j)
+                            tc::tmem_cp_sf_atom(tmem_sfc + k * 4 * Cfg::CB + 4 * j,
+                                                sf + Cfg::SFL_BYTES + j * 2048 + 512 * k);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)   // 4 x (K = 64 e2m1 = 32 bytes) per 128-byte k-block
+                        tc::mma_nvfp4(tmem_d, dL0 + so + 2 * k, dC0 + so + 2 * k, idesc, tmem_sfl + 4 * k,
+                                      tmem_sfc + k * 4 * Cfg::CB + sfc_off, (i > 0 || k > 0) ? 1u : 0u);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)   // 4 x (K = 32) per 128-byte k-block; +32 bytes = +2 in the address field
+                        tc::mma_f8(tmem_d, dL0 + so + 2 * k, dC0 + so + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
                 }
-#pragma unroll
-                for (int k = 0; k < 4; ++k)   // 4 x (K = 64 e2m1 = 32 bytes) per 128-byte k-block
-                    tc::mma_nvfp4(tmem_d, dL + 2 * k, dC + 2 * k, idesc, tmem_sfl + 4 * k,
-                                  tmem_sfc + k * 4 * Cfg::CB + sfc_off, (i > 0 || k > 0) ? 1u : 0u);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)   // 4 x (K = 32) per 128-byte k-block; +32 bytes = +2 in the address field
-                    tc::mma_f8(tmem_d, dL + 2 * k, dC + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                if (i + STAGES < nkb) tc::mma_commit(done);      // a slot that is filled again
+                if (i == nkb - 1) tc::mma_commit(accum_a);
+                *consumed = i + 1;
             }
-            tc::mma_commit(&empty[s]);
-            *consumed = i + 1;
         }
-        if (!failed) tc::mma_commit(accum_bar);
+        if (failed) {
+            *abort_flag = 1;
+            if (lane == 0) atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
+        }
     }
     __syncwarp();
 
@@ -809,11 +822,10 @@ static int launch_gemm(const void* A, const void* W, GemmParams p, int K, int sp
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = splits;
     ++na;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+    p.early = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<BN, SWAP, EPI, FP4>, tmL, tmC, p);
@@ -869,11 +881,10 @@ static int launch_gemm_gate_res_norm(const void* A, const void* W, GemmParams p,
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = splits;
     ++na;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+    p.early = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmL, tmC, p);
@@ -935,11 +946,11 @@ static int pick_large(int M, int N, int K, bool no_pair, double* cost = nullptr)
 }
 
 template <int EPI>
-static int launch_large(int kind, const void* A, const void* W, const GemmParams& p, int K, bool pdl, cudaStream_t s) {
-    if (kind == LARGE_PAIR) return launch_gemm_pair<256, EPI>(A, W, p, K, pdl, s);
-    if (kind == LARGE_PAIR_128) return launch_gemm_pair<128, EPI>(A, W, p, K, pdl, s);
-    if (kind == LARGE_256) return launch_gemm_persistent<256, EPI>(A, W, p, K, pdl, s);
-    return launch_gemm_persistent<128, EPI>(A, W, p, K, pdl, s);
+static int launch_large(int kind, const void* A, const void* W, const GemmParams& p, int K, cudaStream_t s) {
+    if (kind == LARGE_PAIR) return launch_gemm_pair<256, EPI>(A, W, p, K, s);
+    if (kind == LARGE_PAIR_128) return launch_gemm_pair<128, EPI>(A, W, p, K, s);
+    if (kind == LARGE_256) return launch_gemm_persistent<256, EPI>(A, W, p, K, s);
+    return launch_gemm_persistent<128, EPI>(A, W, p, K, s);
 }
 
 }  // namespace frt
@@ -997,7 +1008,7 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
         const int kind = pick_large(M, N, K, M <= 128 || (flags & 32) != 0, &t_large);
         const double mb = (double)N * K / 1048576.0;
         const double t_small = M > 128 ? 13.0 + 0.115 * p.kb_total : M > 64 ? 5.2 + 0.45 * mb : 5.0 + 0.3 * mb;
-        if (t_large + 0.3 < t_small) return launch_large<EPI_P_BF16>(kind, A, W, p, K, pdl, s);
+        if (t_large + 0.3 < t_small) return launch_large<EPI_P_BF16>(kind, A, W, p, K, s);
     }
     // the swapped kernel's splits keep up with a long K better than the token-major kernel's exchange
     const bool long_k = !hinted && (M > 64 ? p.kb_total >= 96 : p.kb_total >= 128);
@@ -1012,7 +1023,7 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     int sp = splits > 0 ? pick_splits(1, p.kb_total, splits > 8 ? 8 : splits) : 1;
     if (sp == 1 && !(flags & 2) && N > 64) {      // flags bit 1 keeps the one-tile-per-CTA kernel (for comparison runs)
         const int kind = (flags & 8) && N >= 256 ? LARGE_PAIR : pick_large(M, N, K, (flags & 32) != 0);
-        return launch_large<EPI_P_BF16>(kind, A, W, p, K, pdl, s);
+        return launch_large<EPI_P_BF16>(kind, A, W, p, K, s);
     }
     if (N >= 256) return launch_gemm<256, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
@@ -1049,8 +1060,8 @@ int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, in
     p.N = N;
     p.kb_total = K / 128;
     p.w_kn = 1;
-    if (N >= 256) return launch_gemm_persistent<256, EPI_P_BF16>(A, B, p, K, pdl, s);
-    return launch_gemm_persistent<128, EPI_P_BF16>(A, B, p, K, pdl, s);
+    if (N >= 256) return launch_gemm_persistent<256, EPI_P_BF16>(A, B, p, K, s);
+    return launch_gemm_persistent<128, EPI_P_BF16>(A, B, p, K, s);
 }
 
 // QKV projection with the RoPE + split + KV-append epilogue fused (M <= 256):
@@ -1159,7 +1170,7 @@ int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const 
     // Persistent kernel with two 128-column accumulators: measured faster than the 128 x 256 one-tile kernel while
     // the per-tile prologue / epilogue dominates (K < 3072); at larger K the wider tile's lower operand traffic wins.
     if (sp == 1 && N > 64 && !(flags & 2) && (K < 3072 || N < 256 || (flags & 4)))
-        return launch_gemm_persistent<128, EPI_P_BF16, true>(A, W, p, K, pdl, s);
+        return launch_gemm_persistent<128, EPI_P_BF16, true>(A, W, p, K, s);
     if (N >= 256) return launch_gemm<256, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     return launch_gemm<64, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
@@ -1254,8 +1265,8 @@ int frt_b200_gemm_fp8_nt_bias_gelu_fp8(const void* A, const void* W, void* out8,
     p.out8 = (uint8_t*)out8;
     p.out_scale = d_out_scale;
     const int kind = pick_large(M, N, K, false);
-    if (flags & 128) return launch_large<EPI_P_BIAS_GELU_FAST_FP8>(kind, A, W, p, K, flags & 1, (cudaStream_t)stream);
-    return launch_large<EPI_P_BIAS_GELU_FP8>(kind, A, W, p, K, flags & 1, (cudaStream_t)stream);
+    if (flags & 128) return launch_large<EPI_P_BIAS_GELU_FAST_FP8>(kind, A, W, p, K, (cudaStream_t)stream);
+    return launch_large<EPI_P_BIAS_GELU_FP8>(kind, A, W, p, K, (cudaStream_t)stream);
 }
 
 // Row-parallel projection with the gated residual update fused (M <= 128, N % 64 == 0, K % 128 == 0):

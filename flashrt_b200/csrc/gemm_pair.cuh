@@ -234,7 +234,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 }
 
 template <int BN, int EPI>
-static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, bool pdl, cudaStream_t stream) {
+static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, cudaStream_t stream) {
     using Cfg = GemmPairCfg<BN>;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
@@ -265,11 +265,9 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, b
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = 1;
     ++na;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;    // nothing global is read before the wait
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI>, tmA, tmW, p);

@@ -438,7 +438,7 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
 }
 
 template <int BN, int EPI, bool FP4 = false>
-static int launch_gemm_persistent(const void* A, const void* W, GemmParams p, int K, bool pdl, cudaStream_t stream) {
+static int launch_gemm_persistent(const void* A, const void* W, GemmParams p, int K, cudaStream_t stream) {
     using Cfg = PGemmCfg<BN, FP4>;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
@@ -468,7 +468,7 @@ static int launch_gemm_persistent(const void* A, const void* W, GemmParams p, in
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;                   // nothing global is read before the wait
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_persistent_kernel<BN, EPI, FP4>, tmA, tmW, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

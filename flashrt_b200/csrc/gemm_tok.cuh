@@ -97,6 +97,7 @@ struct TokParams {
     const __nv_bfloat16* style;
     float eps;
     int w_kn;                  // weights stored (K, N) row-major (the MN-major B operand) instead of (N, K)
+    int early;                 // weights and style may be read before the kernel in front has finished
     // Deferred row scale (TOK_PRO_TMA with TOK_EPI_ROPE / TOK_EPI_GEGLU, active when stats_in != NULL): the A operand
     // holds e4m3(x * (1 + scale)) WITHOUT the 1 / rms factor; the finish applies it per token and adds the column
     // term:  y[m][n] = bf16(alpha * acc[m][n] * rms[m] + col_term[n]),  rms from stats_in / n_stat / K / eps as above,
@@ -262,6 +263,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     TOK_STAMP(1);
 
     pdl_launch_dependents();
+    if (!p.early) pdl_wait();
 
     if (warp == 0) {
         // ---------------- TMA producer (whole warp, see warp_wait): the weights do not depend on the producer grid and start
@@ -889,11 +891,10 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = pl.S;
     ++na;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+    p.early = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, p);

@@ -245,7 +245,7 @@ int frt_b200_gemm_bf16_nn_small(const void* A, const void* B, void* D, const voi
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (flags & 1) ? 1 : 0;
+    cfg.numAttrs = 1;
     const __nv_bfloat16* Bp = (const __nv_bfloat16*)B;
     const __nv_bfloat16* bp = (const __nv_bfloat16*)bias;
     cudaError_t e;

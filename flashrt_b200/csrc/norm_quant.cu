@@ -45,6 +45,7 @@ struct NormArgs {
     int rows;
     int dim;
     float eps;
+    int early;                     // weight, style and scale may be read before the kernel in front has finished
 };
 
 template <bool HAS_X, bool HAS_GATE, bool HAS_STYLE, int OUT>
@@ -68,6 +69,7 @@ norm_row_kernel(NormArgs a) {
     // The next kernel in the stream may start its own input-independent prologue right away (it still waits for
     // this grid to finish before it touches anything this grid writes).
     pdl_launch_dependents();
+    if (!a.early) pdl_wait();
     // Everything that does not depend on the producer kernel is fetched first.
     if (active) {
         if (a.weight) wv = ld_global_v4(a.weight + col);
@@ -207,6 +209,7 @@ norm_warp_kernel(NormArgs a) {
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
     pdl_launch_dependents();
+    pdl_wait();
     float inv_scale = 1.0f;
     if (OUT_FP8) inv_scale = __fdiv_rn(1.0f, *a.d_scale);
     if (row >= a.rows) return;
@@ -216,7 +219,6 @@ norm_warp_kernel(NormArgs a) {
     uint8_t* sf = nullptr;                                  // scale byte of this lane's block: + 4 atoms per slice
     const bool sf_words = OUT_FP4 && (a.dim & 63) == 0;
     if (OUT_FP4) sf = a.sf_out + nvfp4::sf_offset(row, (lane >> 3) * 4, (a.dim + 63) >> 6);
-    pdl_wait();
     uint4 rv[NS];
     float ssq[NS];
 #pragma unroll
@@ -298,7 +300,7 @@ norm_warp_kernel(NormArgs a) {
 }
 
 template <int OUT, int NS>
-static int launch_norm_warp(const NormArgs& a, cudaStream_t stream, bool pdl) {
+static int launch_norm_warp(const NormArgs& a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((a.rows + 3) / 4));
     cfg.blockDim = dim3(128);
@@ -307,7 +309,7 @@ static int launch_norm_warp(const NormArgs& a, cudaStream_t stream, bool pdl) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, norm_warp_kernel<OUT, NS>, a);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
@@ -320,19 +322,20 @@ template <int OUT>
 static constexpr int norm_warp_rows() { return OUT == OUT_BF16 || OUT == OUT_E4M3 ? 1536 : 3072; }
 
 template <bool HAS_X, bool HAS_GATE, bool HAS_STYLE, int OUT>
-static int launch_norm(const NormArgs& a, cudaStream_t stream, bool pdl) {
+static int launch_norm(NormArgs a, cudaStream_t stream, bool pdl) {
+    a.early = pdl ? 1 : 0;
     if (a.rows < 0 || a.dim <= 0 || (a.dim & 7) || a.dim > 8192) return FRT_ERR_UNSUPPORTED;
     if (a.rows == 0) return FRT_OK;
     if (!HAS_X && !HAS_STYLE && a.rows >= norm_warp_rows<OUT>() && a.dim > 512 &&
         (reinterpret_cast<uintptr_t>(a.sf_out) & 3) == 0) {
         switch ((a.dim + 511) / 512) {
-            case 2: return launch_norm_warp<OUT, 4>(a, stream, pdl);
-            case 3: return launch_norm_warp<OUT, 6>(a, stream, pdl);
-            case 4: return launch_norm_warp<OUT, 8>(a, stream, pdl);
-            case 5: return launch_norm_warp<OUT, 10>(a, stream, pdl);
-            case 6: return launch_norm_warp<OUT, 12>(a, stream, pdl);
-            case 7: return launch_norm_warp<OUT, 14>(a, stream, pdl);
-            case 8: return launch_norm_warp<OUT, 16>(a, stream, pdl);
+            case 2: return launch_norm_warp<OUT, 4>(a, stream);
+            case 3: return launch_norm_warp<OUT, 6>(a, stream);
+            case 4: return launch_norm_warp<OUT, 8>(a, stream);
+            case 5: return launch_norm_warp<OUT, 10>(a, stream);
+            case 6: return launch_norm_warp<OUT, 12>(a, stream);
+            case 7: return launch_norm_warp<OUT, 14>(a, stream);
+            case 8: return launch_norm_warp<OUT, 16>(a, stream);
             default: break;                                  // wider rows: the CTA kernel
         }
     }
@@ -346,7 +349,7 @@ static int launch_norm(const NormArgs& a, cudaStream_t stream, bool pdl) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, norm_row_kernel<HAS_X, HAS_GATE, HAS_STYLE, OUT>, a);
     if (e != cudaSuccess) return FRT_CUDA_ERR(e);
     return FRT_OK;

@@ -22,11 +22,11 @@ quantize_nvfp4_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict_
     const int nblk = D >> 4;
     const int katoms = (D + 63) >> 6;
     const long long total = rows * nblk;
+    pdl_launch_dependents();
+    pdl_wait();
     float inv_g = 1.0f;
     const bool has_g = d_global != nullptr;
     if (has_g) inv_g = __fdiv_rn(1.0f, *d_global);
-    pdl_launch_dependents();
-    pdl_wait();
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const long long row = idx / nblk;
@@ -106,7 +106,7 @@ geglu_nvfp4_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict
 }
 
 template <typename K, typename... Args>
-static int launch_1d(K kernel, long long work, bool pdl, cudaStream_t stream, Args... args) {
+static int launch_1d(K kernel, long long work, cudaStream_t stream, Args... args) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -121,7 +121,7 @@ static int launch_1d(K kernel, long long work, bool pdl, cudaStream_t stream, Ar
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
@@ -152,9 +152,9 @@ int frt_b200_quantize_nvfp4(const void* in, void* packed, void* sf, long long ro
     if (rows == 0) return FRT_OK;
     const long long work = rows * (D / 16);
     if (family == 0)
-        return launch_1d(quantize_nvfp4_kernel<0>, work, flags & 1, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+        return launch_1d(quantize_nvfp4_kernel<0>, work, (cudaStream_t)stream, (const __nv_bfloat16*)in,
                          (uint8_t*)packed, (uint8_t*)sf, rows, D, d_global_scale);
-    return launch_1d(quantize_nvfp4_kernel<1>, work, flags & 1, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+    return launch_1d(quantize_nvfp4_kernel<1>, work, (cudaStream_t)stream, (const __nv_bfloat16*)in,
                      (uint8_t*)packed, (uint8_t*)sf, rows, D, d_global_scale);
 }
 
@@ -168,9 +168,9 @@ int frt_b200_geglu_nvfp4(const void* merged, void* packed, void* sf, int rows, i
     if (rows == 0) return FRT_OK;
     const long long work = (long long)rows * (H / 16);
     if (family == 0)
-        return launch_1d(geglu_nvfp4_kernel<0>, work, flags & 1, (cudaStream_t)stream, (const __nv_bfloat16*)merged,
+        return launch_1d(geglu_nvfp4_kernel<0>, work, (cudaStream_t)stream, (const __nv_bfloat16*)merged,
                          (uint8_t*)packed, (uint8_t*)sf, rows, H);
-    return launch_1d(geglu_nvfp4_kernel<1>, work, flags & 1, (cudaStream_t)stream, (const __nv_bfloat16*)merged,
+    return launch_1d(geglu_nvfp4_kernel<1>, work, (cudaStream_t)stream, (const __nv_bfloat16*)merged,
                      (uint8_t*)packed, (uint8_t*)sf, rows, H);
 }
 

@@ -52,6 +52,8 @@ layer_norm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
                       const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ scale,
                       const __nv_bfloat16* __restrict__ shift, long long mod_stride, void* __restrict__ out,
                       const float* __restrict__ d_scale, int dim, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float warp_tot[32];
     const int row = blockIdx.x;
     const int col = threadIdx.x * 8;
@@ -66,7 +68,6 @@ layer_norm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
     }
     float inv_a = 1.0f;
     if (OUT_FP8) inv_a = __fdiv_rn(1.0f, *d_scale);
-    pdl_wait();
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = 0.0f;
@@ -81,7 +82,6 @@ layer_norm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
             s = __fadd_rn(s, v[2 * i + 1]);
         }
     }
-    pdl_launch_dependents();
     const float mean = __fdiv_rn(block_sum_fixed(s, warp_tot), (float)dim);
     float q = 0.0f;
     if (active) {
@@ -167,6 +167,8 @@ struct ResNormArgs {
 template <bool OUT_FP8, int NS, bool AFFINE, bool MOD>
 __global__ void __launch_bounds__(128, NS <= 12 ? 5 : NS <= 16 ? 4 : 2)
 layer_norm_warp_kernel(ResNormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     float inv_a = 1.0f;
@@ -176,7 +178,6 @@ layer_norm_warp_kernel(ResNormArgs a) {
     const size_t rbase = (size_t)row * a.dim + lane * 8;
     const size_t mbase = (size_t)(row / a.mod_rows) * a.mod_stride + lane * 8;
     const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
-    pdl_wait();
     uint4 rv[NS];
 #pragma unroll
     for (int w = 0; w < NS; ++w) {
@@ -215,7 +216,6 @@ layer_norm_warp_kernel(ResNormArgs a) {
             }
         }
     }
-    pdl_launch_dependents();
     if (!a.out) return;
     float part[NS];
 #pragma unroll
@@ -317,6 +317,8 @@ qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_
                            const float* __restrict__ fim, __nv_bfloat16* __restrict__ q_out,
                            __nv_bfloat16* __restrict__ k_out, int L, int dim, int D_h, int seq_len, float eps,
                            const float* __restrict__ ext_ssq_q, const float* __restrict__ ext_ssq_k, int full_dim) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float warp_tot[32];
     const int row = blockIdx.x;
     const int t = row % L;
@@ -336,7 +338,6 @@ qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_
             fi[0] = b.x; fi[1] = b.y; fi[2] = b.z; fi[3] = b.w;
         }
     }
-    pdl_wait();
     float q[8], k[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) q[i] = k[i] = 0.0f;
@@ -356,7 +357,6 @@ qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_
             sk = __fmaf_rn(k[2 * i + 1], k[2 * i + 1], sk);
         }
     }
-    pdl_launch_dependents();
     // tensor-parallel use: this CTA only sees its heads' slice of the row; the sums over the full width come in
     float tq, tk;
     if (ext_ssq_q) {
@@ -402,6 +402,8 @@ qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const 
                                 __nv_bfloat16* __restrict__ k_out, int L, int dim, int D_h, int seq_len, float eps,
                                 const float* __restrict__ ext_ssq_q, const float* __restrict__ ext_ssq_k, int full_dim,
                                 int rows) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int row = item >> 1;
@@ -414,7 +416,6 @@ qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const 
     const __nv_bfloat16* src = packed + (size_t)row * 3 * dim + (is_k ? dim : 0) + lane * 8;
     __nv_bfloat16* dst = (is_k ? k_out : q_out) + (size_t)row * dim + lane * 8;
     const int left = dim - lane * 8;                        // slice w of this lane exists while w * 256 < left
-    pdl_wait();
     uint4 xv[NS];
     float part[NS];
 #pragma unroll
@@ -422,7 +423,6 @@ qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const 
         xv[w] = make_uint4(0, 0, 0, 0);
         if (w * 256 < left) xv[w] = ld_stream_v4(src + w * 256);
     }
-    pdl_launch_dependents();
     const float* ext = is_k ? ext_ssq_k : ext_ssq_q;
     float tot;
     if (ext) {
@@ -486,8 +486,9 @@ qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const 
 __global__ void __launch_bounds__(256)
 bias_gelu_fp8_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ bias,
                      uint8_t* __restrict__ out, const float* __restrict__ d_scale, long long rows, int N) {
-    const float inv_s = __fdiv_rn(1.0f, *d_scale);
+    pdl_launch_dependents();
     pdl_wait();
+    const float inv_s = __fdiv_rn(1.0f, *d_scale);
     const int vec_per_row = N >> 3;
     const long long total = rows * vec_per_row;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -512,7 +513,6 @@ bias_gelu_fp8_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* 
         ov.y = f32x4_to_e4m3x4(o[4], o[5], o[6], o[7]);
         st_global_v2(out + i * 8, ov);
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ residual <- residual + (x + bias) * gate   (gate per row or shared)
@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(256)
 bias_gate_res_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
                      const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ gate,
                      long long gate_stride, long long rows, int dim) {
+    pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = dim >> 3;
     const long long total = rows * vec_per_row;
@@ -560,7 +561,6 @@ bias_gate_res_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __res
         }
         st_global_v4(res + i * 8, ov);
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ six modulation tensors
@@ -569,6 +569,7 @@ __global__ void __launch_bounds__(256)
 modulation6_kernel(const float* __restrict__ params, const float* __restrict__ layer_mod,
                    __nv_bfloat16* o0, __nv_bfloat16* o1, __nv_bfloat16* o2, __nv_bfloat16* o3, __nv_bfloat16* o4,
                    __nv_bfloat16* o5, int D, long long n) {
+    pdl_launch_dependents();
     pdl_wait();
     __nv_bfloat16* outs[6] = {o0, o1, o2, o3, o4, o5};
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
@@ -579,7 +580,6 @@ modulation6_kernel(const float* __restrict__ params, const float* __restrict__ l
         for (int j = 0; j < 6; ++j)
             outs[j][idx] = __float2bfloat16_rn(__fadd_rn(params[base + (long long)j * D], layer_mod[(long long)j * D + d]));
     }
-    pdl_launch_dependents();
 }
 
 // ------------------------------------------------------------------ tensor-parallel helpers for full-width norms
@@ -587,6 +587,7 @@ modulation6_kernel(const float* __restrict__ params, const float* __restrict__ l
 __global__ void __launch_bounds__(256)
 row_sumsq_kernel(const __nv_bfloat16* __restrict__ x, long long row_stride, int col0, int ncols,
                  float* __restrict__ out, long long rows) {
+    pdl_launch_dependents();
     pdl_wait();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -613,6 +614,7 @@ __global__ void __launch_bounds__(256)
 rms_norm_ext_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ w,
                     const float* __restrict__ ssq, __nv_bfloat16* __restrict__ out, long long out_stride,
                     long long rows, int dim, int full_dim, float eps) {
+    pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = dim >> 3;
     const long long total = rows * vec_per_row;
@@ -639,7 +641,7 @@ rms_norm_ext_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, con
 }
 
 template <typename K, typename... Args>
-static int launch_k(K kernel, unsigned grid, unsigned block, cudaStream_t stream, bool pdl, Args... args) {
+static int launch_k(K kernel, unsigned grid, unsigned block, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -648,7 +650,7 @@ static int launch_k(K kernel, unsigned grid, unsigned block, cudaStream_t stream
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;                    // every kernel launched here waits before its first global access
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
@@ -663,20 +665,20 @@ static inline unsigned cap_grid(long long items, int threads) {
 enum { LN_WARP_ROWS = 1024, ROPE_WARP_ROWS = 512 };
 
 template <bool OUT_FP8, bool AFFINE, bool MOD>
-static int launch_layer_norm_warp(const ResNormArgs& a, bool pdl, cudaStream_t s) {
+static int launch_layer_norm_warp(const ResNormArgs& a, cudaStream_t s) {
     const unsigned grid = (unsigned)((a.rows + 3) / 4);
-    if (a.dim <= 1024) return launch_k(layer_norm_warp_kernel<OUT_FP8, 4, AFFINE, MOD>, grid, 128, s, pdl, a);
-    if (a.dim <= 2048) return launch_k(layer_norm_warp_kernel<OUT_FP8, 8, AFFINE, MOD>, grid, 128, s, pdl, a);
-    if (a.dim <= 3072) return launch_k(layer_norm_warp_kernel<OUT_FP8, 12, AFFINE, MOD>, grid, 128, s, pdl, a);
-    if (a.dim <= 4096) return launch_k(layer_norm_warp_kernel<OUT_FP8, 16, AFFINE, MOD>, grid, 128, s, pdl, a);
-    return launch_k(layer_norm_warp_kernel<OUT_FP8, 32, AFFINE, MOD>, grid, 128, s, pdl, a);
+    if (a.dim <= 1024) return launch_k(layer_norm_warp_kernel<OUT_FP8, 4, AFFINE, MOD>, grid, 128, s, a);
+    if (a.dim <= 2048) return launch_k(layer_norm_warp_kernel<OUT_FP8, 8, AFFINE, MOD>, grid, 128, s, a);
+    if (a.dim <= 3072) return launch_k(layer_norm_warp_kernel<OUT_FP8, 12, AFFINE, MOD>, grid, 128, s, a);
+    if (a.dim <= 4096) return launch_k(layer_norm_warp_kernel<OUT_FP8, 16, AFFINE, MOD>, grid, 128, s, a);
+    return launch_k(layer_norm_warp_kernel<OUT_FP8, 32, AFFINE, MOD>, grid, 128, s, a);
 }
 template <bool OUT_FP8>
-static int dispatch_layer_norm_warp(const ResNormArgs& a, bool pdl, cudaStream_t s) {
-    if (a.weight) return a.scale ? launch_layer_norm_warp<OUT_FP8, true, true>(a, pdl, s)
-                                 : launch_layer_norm_warp<OUT_FP8, true, false>(a, pdl, s);
-    return a.scale ? launch_layer_norm_warp<OUT_FP8, false, true>(a, pdl, s)
-                   : launch_layer_norm_warp<OUT_FP8, false, false>(a, pdl, s);
+static int dispatch_layer_norm_warp(const ResNormArgs& a, cudaStream_t s) {
+    if (a.weight) return a.scale ? launch_layer_norm_warp<OUT_FP8, true, true>(a, s)
+                                 : launch_layer_norm_warp<OUT_FP8, true, false>(a, s);
+    return a.scale ? launch_layer_norm_warp<OUT_FP8, false, true>(a, s)
+                   : launch_layer_norm_warp<OUT_FP8, false, false>(a, s);
 }
 
 }  // namespace frt
@@ -713,8 +715,8 @@ int frt_b200_layer_norm(const void* x, const void* weight, const void* bias, con
         a.rows = rows;
         a.dim = dim;
         a.eps = eps;
-        return out_fp8 ? dispatch_layer_norm_warp<true>(a, flags & 1, (cudaStream_t)stream)
-                       : dispatch_layer_norm_warp<false>(a, flags & 1, (cudaStream_t)stream);
+        return out_fp8 ? dispatch_layer_norm_warp<true>(a, (cudaStream_t)stream)
+                       : dispatch_layer_norm_warp<false>(a, (cudaStream_t)stream);
     }
     const unsigned threads = ((dim / 8 + 31) / 32) * 32;
     auto X = (const __nv_bfloat16*)x;
@@ -723,9 +725,9 @@ int frt_b200_layer_norm(const void* x, const void* weight, const void* bias, con
     auto SC = (const __nv_bfloat16*)scale;
     auto SH = (const __nv_bfloat16*)shift;
     if (out_fp8)
-        return launch_k(layer_norm_row_kernel<true>, rows, threads, (cudaStream_t)stream, flags & 1, X, W, B, SC, SH,
+        return launch_k(layer_norm_row_kernel<true>, rows, threads, (cudaStream_t)stream, X, W, B, SC, SH,
                         mod_stride, out_fp8, d_scale, dim, eps);
-    return launch_k(layer_norm_row_kernel<false>, rows, threads, (cudaStream_t)stream, flags & 1, X, W, B, SC, SH,
+    return launch_k(layer_norm_row_kernel<false>, rows, threads, (cudaStream_t)stream, X, W, B, SC, SH,
                     mod_stride, out_bf16, d_scale, dim, eps);
 }
 
@@ -750,7 +752,7 @@ int frt_b200_residual_layer_norm_fp8(const void* res, const void* x, const void*
                      (__nv_bfloat16*)res_out, (const __nv_bfloat16*)weight, (const __nv_bfloat16*)bias,
                      (const __nv_bfloat16*)scale, (const __nv_bfloat16*)shift, mod_stride, mod_rows, out_fp8, d_scale,
                      rows, dim, eps};
-    return dispatch_layer_norm_warp<true>(a, flags & 1, (cudaStream_t)stream);
+    return dispatch_layer_norm_warp<true>(a, (cudaStream_t)stream);
 }
 
 // packed_qkv (B*L, 3*dim) bf16, dim = N * D_h; q_out / k_out (B*L, dim); freqs (seq_len.., D_h/2) fp32.
@@ -770,7 +772,7 @@ int frt_b200_qkv_split_norm_rope(const void* packed_qkv, const void* norm_q_w, c
     const long long rows = (long long)B * L;
     if (rows >= ROPE_WARP_ROWS && rows < (1LL << 30) && dim <= 4096) {
         auto go = [&](auto kern) {
-            return launch_k(kern, (unsigned)((rows * 2 + 3) / 4), 128, (cudaStream_t)stream, flags & 1,
+            return launch_k(kern, (unsigned)((rows * 2 + 3) / 4), 128, (cudaStream_t)stream,
                             (const __nv_bfloat16*)packed_qkv, (const __nv_bfloat16*)norm_q_w,
                             (const __nv_bfloat16*)norm_k_w, freqs_re, freqs_im, (__nv_bfloat16*)q_out,
                             (__nv_bfloat16*)k_out, L, (int)dim, D_h, seq_len, eps, ext ? ext_ssq_q : (const float*)nullptr,
@@ -782,7 +784,7 @@ int frt_b200_qkv_split_norm_rope(const void* packed_qkv, const void* norm_q_w, c
         return go(qkv_split_norm_rope_warp_kernel<16>);
     }
     const unsigned threads = (unsigned)(((dim / 8 + 31) / 32) * 32);
-    return launch_k(qkv_split_norm_rope_kernel, (unsigned)(B * L), threads, (cudaStream_t)stream, flags & 1,
+    return launch_k(qkv_split_norm_rope_kernel, (unsigned)(B * L), threads, (cudaStream_t)stream,
                     (const __nv_bfloat16*)packed_qkv, (const __nv_bfloat16*)norm_q_w, (const __nv_bfloat16*)norm_k_w,
                     freqs_re, freqs_im, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_out, L, (int)dim, D_h, seq_len, eps,
                     (ext_ssq_q && ext_ssq_k) ? ext_ssq_q : (const float*)nullptr,
@@ -796,7 +798,7 @@ int frt_b200_row_sumsq(const void* x, long long row_stride, int col0, int ncols,
     if (!x || !out || rows < 0 || ncols <= 0 || col0 < 0) return FRT_ERR_INVALID;
     if ((ncols & 7) || (col0 & 7) || (row_stride & 7) || mis(x, 16)) return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
-    return launch_k(row_sumsq_kernel, (unsigned)((rows + 7) / 8), 256, (cudaStream_t)stream, flags & 1,
+    return launch_k(row_sumsq_kernel, (unsigned)((rows + 7) / 8), 256, (cudaStream_t)stream,
                     (const __nv_bfloat16*)x, row_stride, col0, ncols, out, rows);
 }
 
@@ -808,7 +810,7 @@ int frt_b200_rms_norm_ext(const void* x, long long x_stride, const void* weight,
     if ((dim & 7) || (x_stride & 7) || (out_stride & 7) || mis(x, 16) || mis(weight, 16) || mis(out, 16))
         return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
-    return launch_k(rms_norm_ext_kernel, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream, flags & 1,
+    return launch_k(rms_norm_ext_kernel, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream,
                     (const __nv_bfloat16*)x, x_stride, (const __nv_bfloat16*)weight, ssq, (__nv_bfloat16*)out,
                     out_stride, rows, dim, full_dim, eps);
 }
@@ -819,7 +821,7 @@ int frt_b200_bias_gelu_quantize_fp8(const void* in_bf16, const void* bias, void*
     if (!in_bf16 || !out_fp8 || !d_scale || M < 0 || N <= 0) return FRT_ERR_INVALID;
     if ((N & 7) || mis(in_bf16, 16) || mis(bias, 16) || mis(out_fp8, 8)) return FRT_ERR_UNSUPPORTED;
     if (M == 0) return FRT_OK;
-    return launch_k(bias_gelu_fp8_kernel, cap_grid(M * (N >> 3), 256), 256, (cudaStream_t)stream, flags & 1,
+    return launch_k(bias_gelu_fp8_kernel, cap_grid(M * (N >> 3), 256), 256, (cudaStream_t)stream,
                     (const __nv_bfloat16*)in_bf16, (const __nv_bfloat16*)bias, (uint8_t*)out_fp8, d_scale, M, N);
 }
 
@@ -830,7 +832,7 @@ int frt_b200_bias_gate_mul_residual(void* residual, const void* x, const void* b
     if ((dim & 7) || (gate_stride & 7) || mis(residual, 16) || mis(x, 16) || mis(bias, 16) || mis(gate, 16))
         return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
-    return launch_k(bias_gate_res_kernel<0>, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream, flags & 1,
+    return launch_k(bias_gate_res_kernel<0>, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream,
                     (__nv_bfloat16*)residual, (const __nv_bfloat16*)x, (const __nv_bfloat16*)bias,
                     (const __nv_bfloat16*)gate, gate_stride, rows, dim);
 }
@@ -840,7 +842,7 @@ int frt_b200_add_bias(void* x, const void* bias, long long rows, int dim, int fl
     if (!x || !bias || rows < 0 || dim <= 0) return FRT_ERR_INVALID;
     if ((dim & 7) || mis(x, 16) || mis(bias, 16)) return FRT_ERR_UNSUPPORTED;
     if (rows == 0) return FRT_OK;
-    return launch_k(bias_gate_res_kernel<1>, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream, flags & 1,
+    return launch_k(bias_gate_res_kernel<1>, cap_grid(rows * (dim >> 3), 256), 256, (cudaStream_t)stream,
                     (__nv_bfloat16*)x, (const __nv_bfloat16*)nullptr, (const __nv_bfloat16*)bias,
                     (const __nv_bfloat16*)nullptr, 0LL, rows, dim);
 }
@@ -853,7 +855,7 @@ int frt_b200_adaln_modulation6(const float* adaln_params, const float* layer_mod
     if (B < 0 || S < 0 || D <= 0) return FRT_ERR_INVALID;
     const long long n = (long long)B * S * D;
     if (n == 0) return FRT_OK;
-    return launch_k(modulation6_kernel, cap_grid(n, 256), 256, (cudaStream_t)stream, flags & 1, adaln_params,
+    return launch_k(modulation6_kernel, cap_grid(n, 256), 256, (cudaStream_t)stream, adaln_params,
                     layer_modulation, (__nv_bfloat16*)out0, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2,
                     (__nv_bfloat16*)out3, (__nv_bfloat16*)out4, (__nv_bfloat16*)out5, D, n);
 }
