@@ -60,7 +60,7 @@ struct D256Cfg {
 // out of tensor memory -- the longest single step of the scratch path: 3 us for 128 x 256 fp32 -- shrinks by DQ and
 // the grid covers 4 x more SMs.
 //
-// XC (with DQ = 4): the C kv splits of a (row tile, head-dim part) are the CTAs of one thread-block cluster (1 x 1 x C)
+// XC (with DQ = 4 or 2): the C kv splits of a (row tile, head-dim part) are the CTAs of one thread-block cluster (1 x 1 x C)
 // and exchange their partials through distributed shared memory instead of the global scratch: the thread of a row
 // pushes, straight from registers with st.async, the 64 / C columns that split s finishes (normalised, bf16) and the
 // row's log-sum-exp into split s's receive slot, the bytes counted on s's mbarrier; it then waits for its own slot to
@@ -806,6 +806,9 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
         e = cudaFuncSetAttribute(attn_d256_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg::smem_bytes(4, true));
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        e = cudaFuncSetAttribute(attn_d256_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Cfg::smem_bytes(2, true));
+        if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         e = cudaFuncSetAttribute(attn_d256_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg::ragged_smem_bytes());
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
@@ -835,55 +838,86 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
     g_attn_trace_slot = (g_attn_trace_slot + 1) % 8;
 #endif
     p.chunks_total = (p.Skv + Cfg::BKV - 1) / Cfg::BKV;
+    const int bound = splits;
     if (splits > p.chunks_total) splits = p.chunks_total;
     if (splits < 1) splits = 1;
     while (splits & (splits - 1)) --splits;            // power of two: each split finishes D / splits columns
     if (splits == 1) p.o_accum = nullptr;
     const int tiles = (p.Sq * p.G + 127) / 128;
+    const int groups = p.Hkv * p.B;
     int dq = 1;
-    if (p.o_accum) {
-        const long long ctas = (long long)tiles * p.Hkv * p.B * splits;
-        if (ctas > sms) return FRT_ERR_UNSUPPORTED;    // the CTAs of a tile wait for one another
-        // four head-dim parts per (tile, split) while the whole grid still fits one wave and a slice keeps 8 columns
-        if (ctas * 4 <= sms && 64 / splits >= 8 && !(p.flags & 4)) dq = 4;
-    }
-    // with four head-dim parts the kv splits of a (tile, part) exchange their partials as one cluster (flags bit 3
-    // keeps the global scratch) -- when the device can hold all those clusters at once: CTAs of this size run one per
-    // SM and how many clusters of them fit depends on the part's enabled SMs.  Otherwise the last tile in two parts, if
-    // that fits; otherwise the scratch.
-    bool xc = dq == 4 && !(p.flags & 8);
-    bool ragged = false;
-    if (xc) {
-        int lg = 0;
-        while ((1 << lg) < splits) ++lg;                     // splits is 2, 4 or 8 here
-        static int max_clusters[64][4][2];                   // [device][log2 splits][ragged], 0 = not asked yet
-        auto fits = [&](bool rg, int need) {
-            int& m = max_clusters[dev][lg][rg ? 1 : 0];
+    bool xc = false, ragged = false;
+    // Cluster exchange (flags bit 3 keeps the global scratch): the C kv splits of a (row tile, head-dim part) are one
+    // cluster, and the device has to hold all of them at once: CTAs of this size run one per SM and how many clusters of
+    // them fit depends on the part's enabled SMs.
+    if (p.o_accum && !(p.flags & 12)) {
+        static int max_clusters[64][4][3];                       // [device][log2 C][parts 2, 4, ragged], 0 = not asked yet
+        auto fits = [&](int c, int parts, bool rg) {
+            int lg = 0;
+            while ((1 << lg) < c) ++lg;
+            int& m = max_clusters[dev][lg][rg ? 2 : parts / 2 - 1];
+            const int need = (rg ? 4 * (tiles - 1) + 2 : tiles * parts) * groups;
+            if ((long long)need * c > sms) return false;
             if (m == 0) {
                 cudaLaunchConfig_t q = {};
-                q.gridDim = dim3(rg ? 4 * (tiles - 1) + 2 : tiles * 4, p.Hkv * p.B, splits);
+                q.gridDim = dim3(rg ? 4 * (tiles - 1) + 2 : tiles * parts, groups, c);
                 q.blockDim = dim3(192);
-                q.dynamicSmemBytes = rg ? Cfg::ragged_smem_bytes() : Cfg::smem_bytes(4, true);
+                q.dynamicSmemBytes = rg ? Cfg::ragged_smem_bytes() : Cfg::smem_bytes(parts, true);
                 cudaLaunchAttribute qa[1];
                 qa[0].id = cudaLaunchAttributeClusterDimension;
                 qa[0].val.clusterDim.x = 1;
                 qa[0].val.clusterDim.y = 1;
-                qa[0].val.clusterDim.z = (unsigned)splits;
+                qa[0].val.clusterDim.z = (unsigned)c;
                 q.attrs = qa;
                 q.numAttrs = 1;
                 int n = 0;
-                cudaError_t qe = rg ? cudaOccupancyMaxActiveClusters(&n, attn_d256_ragged_kernel, &q)
-                                    : cudaOccupancyMaxActiveClusters(&n, attn_d256_kernel<4, true>, &q);
+                cudaError_t qe = rg           ? cudaOccupancyMaxActiveClusters(&n, attn_d256_ragged_kernel, &q)
+                                 : parts == 4 ? cudaOccupancyMaxActiveClusters(&n, attn_d256_kernel<4, true>, &q)
+                                              : cudaOccupancyMaxActiveClusters(&n, attn_d256_kernel<2, true>, &q);
                 m = (qe == cudaSuccess && n > 0) ? n : -1;
                 if (qe != cudaSuccess) cudaGetLastError();
             }
             return need <= m;
         };
-        if (!fits(false, tiles * 4 * p.Hkv * p.B)) {
-            const int tail_rows = p.Sq * p.G - 128 * (tiles - 1);
-            if (tail_rows <= Cfg::RAGGED_ROWS && fits(true, (4 * (tiles - 1) + 2) * p.Hkv * p.B)) ragged = true;
-            else xc = false;
+        const bool tail = p.Sq * p.G - 128 * (tiles - 1) <= Cfg::RAGGED_ROWS;
+        auto place = [&](int c, int parts) {
+            if (fits(c, parts, false)) { xc = true; ragged = false; }
+            else if (parts == 4 && tail && fits(c, 4, true)) { xc = true; ragged = true; }
+            else return false;
+            dq = parts;
+            splits = c;
+            return true;
+        };
+        if (!(p.flags & 16)) {
+            place(splits, 4);
+        } else {
+            // kv_splits is a bound: the cheapest split that fits, by the times of the captured action-expert loop (10-64
+            // queries x 8 heads, 100-1088 keys, batch 1-4; units of 0.1 us): 1.6 us per chunk of a split's chain, 1.7
+            // more when a CTA moves out 128 columns of O instead of 64, and for the combine through the scratch
+            // 2.3 more in four parts, 6.0 in one.  (2 x 50 x 768 + 50 keys: 4 splits of 4 parts 12.3 -> 9.8 us.)
+            const long long one = (long long)tiles * groups * splits;
+            int best = 16 * ((p.chunks_total + splits - 1) / splits) + (one * 4 <= sms && splits <= 8 ? 23 : 60);
+            if (one > sms) best = 1 << 30;                  // does not fit as scratch
+            int bc = 0, bp = 0;
+            for (int c = 8; c >= 2; c >>= 1) {
+                if (c > bound || c / 2 >= p.chunks_total) continue;
+                for (int parts = 4; parts >= 2; parts -= 2) {
+                    const int cost = 16 * ((p.chunks_total + c - 1) / c) + (parts == 2 ? 17 : 0);
+                    if (cost < best && (fits(c, parts, false) || (parts == 4 && tail && fits(c, 4, true)))) {
+                        best = cost;
+                        bc = c;
+                        bp = parts;
+                    }
+                }
+            }
+            if (bc) place(bc, bp);
         }
+    }
+    if (p.o_accum && !xc) {
+        const long long ctas = (long long)tiles * groups * splits;
+        if (ctas > sms) return FRT_ERR_UNSUPPORTED;    // the CTAs of a tile wait for one another
+        // four head-dim parts per (tile, split) while the whole grid still fits one wave and a slice keeps 8 columns
+        if (ctas * 4 <= sms && 64 / splits >= 8 && !(p.flags & 4)) dq = 4;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ragged ? 4 * (tiles - 1) + 2 : tiles * dq, p.Hkv * p.B, splits);
@@ -906,6 +940,7 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = ragged    ? cudaLaunchKernelEx(&cfg, attn_d256_ragged_kernel, tmQ, tmK, tmV, p)
+                    : xc && dq == 2 ? cudaLaunchKernelEx(&cfg, attn_d256_kernel<2, true>, tmQ, tmK, tmV, p)
                     : xc      ? cudaLaunchKernelEx(&cfg, attn_d256_kernel<4, true>, tmQ, tmK, tmV, p)
                     : dq == 4 ? cudaLaunchKernelEx(&cfg, attn_d256_kernel<4, false>, tmQ, tmK, tmV, p)
                               : cudaLaunchKernelEx(&cfg, attn_d256_kernel<1, false>, tmQ, tmK, tmV, p);

@@ -1269,9 +1269,9 @@ int frt_b200_gemm_fp8_nt_bias_gelu_fp8(const void* A, const void* W, void* out8,
     return launch_large<EPI_P_BIAS_GELU_FP8>(kind, A, W, p, K, (cudaStream_t)stream);
 }
 
-// Row-parallel projection with the gated residual update fused (M <= 128, N % 64 == 0, K % 128 == 0):
+// Row-parallel projection with the gated residual update fused (M <= 256, N % 64 == 0, K % 128 == 0):
 //   o = bf16(sa * sb * A . W^T);  residual(M, N) <- bf16(residual + o * gate),  gate (N,) shared by all rows;
-//   stats_out[tile][m] (row pitch 128 floats, N / tile_width rows; may be NULL) = sum over the tile's features of the
+//   stats_out[tile][m] (row pitch 128 floats, 256 for M > 128; N / tile_width rows; may be NULL) = sum over the tile's features of the
 //   squares of the UNROUNDED updated residual -- the first pass of gate_residual_ada_norm_fp8
 //   (csrc/kernels/fusion.cu:41-47); frt_b200_norm_gemm_fp8_nt_* finishes the norm inside the next projection.
 // *stat_tiles (host int, may be NULL) receives the number of statistics rows written.
@@ -1290,7 +1290,8 @@ int frt_b200_gemm_fp8_nt_gate_residual_q8(const void* A, const void* W, int M, i
                                           const float* d_q8_scale, int splits, int flags, void* stream) {
     if (!A || !W || !residual || !gate || M < 0 || N <= 0 || K <= 0) return FRT_ERR_INVALID;
     if (q8_out && (!next_scale || !d_q8_scale)) return FRT_ERR_INVALID;
-    if ((K % 128) || M > 128 || (N % 64)) return FRT_ERR_UNSUPPORTED;
+    // statistics without the next operand: the form whose callers hold rows of 128 floats
+    if ((K % 128) || M > (q8_out || !stats_out ? 256 : 128) || (N % 64)) return FRT_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(residual) & 15) || (reinterpret_cast<uintptr_t>(gate) & 15)) return FRT_ERR_INVALID;
     if (q8_out && ((reinterpret_cast<uintptr_t>(q8_out) & 7) || (reinterpret_cast<uintptr_t>(next_scale) & 15)))
         return FRT_ERR_INVALID;
@@ -1301,7 +1302,8 @@ int frt_b200_gemm_fp8_nt_gate_residual_q8(const void* A, const void* W, int M, i
     TokPlan pl;
     int bn = tok_bn_hint(flags);
     if (bn == 0 && (N % 128)) bn = 64;
-    if (!tok_plan(N, K, 1, M < 128 ? (M > 0 ? M : 1) : 128, TOK_EPI_RESID, TOK_PRO_TMA, tok_sm_count(), bn,
+    const int mts = tok_m_tiles(M, flags & 1024);
+    if (!tok_plan(N, K, mts, M > 0 ? (M + mts - 1) / mts : 1, TOK_EPI_RESID, TOK_PRO_TMA, tok_sm_count(), bn,
                   tok_split_hint(splits), &pl))
         return FRT_ERR_UNSUPPORTED;
     if (stat_tiles) *stat_tiles = N / pl.BN;
@@ -1319,6 +1321,34 @@ int frt_b200_gemm_fp8_nt_gate_residual(const void* A, const void* W, int M, int 
                                                  stat_tiles, nullptr, nullptr, nullptr, splits, flags, stream);
 }
 
+// QKV projection of a batch (M <= 256 rows = elements of rows_per_batch tokens; 0: one element), K % 128 == 0: with stats_in
+// as the row-scaled form below, without (stats_in NULL) the plain product; rope row and cache row of token m are
+// m % rows_per_batch, the K / V caches of the elements lie kv_batch_stride elements apart.  One launch instead of a GEMM and
+// one frt_b200_qkv_split_rope per element.
+int frt_b200_gemm_fp8_nt_rope_split_batched(const void* A, const void* W, int M, int K, const float* d_scale_a,
+                                            const float* d_scale_b, const float* stats_in, int n_stat, float eps,
+                                            const float* col_term, const void* rope, void* Q, void* Kout, void* Vout,
+                                            const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim,
+                                            int rows_per_batch, long long kv_batch_stride, int splits, int flags,
+                                            void* stream) {
+    if (!A || !W || !rope || !Q || !Kout || !Vout || M < 0 || K <= 0 || rows_per_batch < 0) return FRT_ERR_INVALID;
+    if (stats_in && (!col_term || n_stat <= 0)) return FRT_ERR_INVALID;
+    if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
+    if ((K % 128) || M > 256 || (head_dim % 8) || (q_dim % head_dim) || (k_dim % head_dim) || (v_dim % 8))
+        return FRT_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(col_term) & 15) || (kv_batch_stride & 7)) return FRT_ERR_INVALID;
+    if (M == 0) return FRT_OK;
+    TokParams t = {};
+    t.M = M; t.N = q_dim + k_dim + v_dim; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = 1.0f;
+    t.rope = (const __nv_bfloat16*)rope; t.outQ = (__nv_bfloat16*)Q; t.outK = (__nv_bfloat16*)Kout;
+    t.outV = (__nv_bfloat16*)Vout; t.devpos = devpos;
+    t.q_dim = q_dim; t.k_dim = k_dim; t.v_dim = v_dim; t.head_dim = head_dim;
+    t.rows_per_batch = rows_per_batch; t.kv_batch_stride = kv_batch_stride;
+    t.stats_in = stats_in; t.n_stat = n_stat; t.eps = eps; t.col_term = col_term;
+    return dispatch_gemm_tok<TOK_PRO_TMA, TOK_EPI_ROPE>(A, W, t, K, tok_bn_hint(flags), tok_split_hint(splits),
+                                                       flags & 1, (cudaStream_t)stream, flags & 1024);
+}
+
 // QKV projection of an operand written by frt_b200_gemm_fp8_nt_gate_residual_q8 (M <= 128, K % 128 == 0):
 //   row[m][n] = bf16(sa * sb * (A . W^T)[m][n] * rms[m] + col_term[n]),
 //   rms[m] = 1 / sqrt(sum_t stats_in[t][m] / K + eps)   (stats_in: n_stat rows of 128 floats, summed in order),
@@ -1329,33 +1359,23 @@ int frt_b200_gemm_fp8_nt_rope_split_rowscale(const void* A, const void* W, int M
                                              const float* col_term, const void* rope, void* Q, void* Kout, void* Vout,
                                              const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim,
                                              int splits, int flags, void* stream) {
-    if (!A || !W || !stats_in || !col_term || !rope || !Q || !Kout || !Vout || M < 0 || K <= 0 || n_stat <= 0)
-        return FRT_ERR_INVALID;
-    if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
-    if ((K % 128) || M > 128 || (head_dim % 8) || (q_dim % head_dim) || (k_dim % head_dim) || (v_dim % 8))
-        return FRT_ERR_UNSUPPORTED;
-    if (reinterpret_cast<uintptr_t>(col_term) & 15) return FRT_ERR_INVALID;
-    if (M == 0) return FRT_OK;
-    TokParams t = {};
-    t.M = M; t.N = q_dim + k_dim + v_dim; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = 1.0f;
-    t.rope = (const __nv_bfloat16*)rope; t.outQ = (__nv_bfloat16*)Q; t.outK = (__nv_bfloat16*)Kout;
-    t.outV = (__nv_bfloat16*)Vout; t.devpos = devpos;
-    t.q_dim = q_dim; t.k_dim = k_dim; t.v_dim = v_dim; t.head_dim = head_dim;
-    t.stats_in = stats_in; t.n_stat = n_stat; t.eps = eps; t.col_term = col_term;
-    return dispatch_gemm_tok<TOK_PRO_TMA, TOK_EPI_ROPE>(A, W, t, K, tok_bn_hint(flags), tok_split_hint(splits),
-                                                       flags & 1, (cudaStream_t)stream);
+    if (!stats_in || !col_term || n_stat <= 0) return FRT_ERR_INVALID;
+    if (M > 128) return FRT_ERR_UNSUPPORTED;
+    return frt_b200_gemm_fp8_nt_rope_split_batched(A, W, M, K, d_scale_a, d_scale_b, stats_in, n_stat, eps, col_term, rope,
+                                                   Q, Kout, Vout, devpos, q_dim, k_dim, v_dim, head_dim, 0, 0, splits, flags,
+                                                   stream);
 }
 
 // gate|up projection of such an operand: gate / up values = bf16(sa * sb * acc * rms[m] + col_term[n]) (col_term has
 // 2 * half entries, gate rows first), then the GeGLU -> FP8 epilogue of frt_b200_gemm_fp8_nt_geglu_fp8
-// (M <= 128, half % 64 == 0, K % 128 == 0).
+// (M <= 256, half % 64 == 0, K % 128 == 0).
 int frt_b200_gemm_fp8_nt_geglu_fp8_rowscale(const void* A, const void* W, void* out8, int M, int half, int K,
                                             const float* d_scale_a, const float* d_scale_b, const float* stats_in,
                                             int n_stat, float eps, const float* col_term, const float* d_out_scale,
                                             int splits, int flags, void* stream) {
     if (!A || !W || !out8 || !stats_in || !col_term || !d_out_scale || M < 0 || half <= 0 || K <= 0 || n_stat <= 0)
         return FRT_ERR_INVALID;
-    if ((K % 128) || M > 128 || (half % 64)) return FRT_ERR_UNSUPPORTED;
+    if ((K % 128) || M > 256 || (half % 64)) return FRT_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(col_term) & 15) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     TokParams t = {};
@@ -1363,7 +1383,7 @@ int frt_b200_gemm_fp8_nt_geglu_fp8_rowscale(const void* A, const void* W, void* 
     t.out8 = (uint8_t*)out8; t.out_scale = d_out_scale; t.half = half; t.gate_act = (flags & 128) ? 2 : 0;
     t.stats_in = stats_in; t.n_stat = n_stat; t.eps = eps; t.col_term = col_term;
     return dispatch_gemm_tok<TOK_PRO_TMA, TOK_EPI_GEGLU>(A, W, t, K, tok_bn_hint(flags), tok_split_hint(splits),
-                                                        flags & 1, (cudaStream_t)stream);
+                                                        flags & 1, (cudaStream_t)stream, flags & 1024);
 }
 
 // QKV projection whose FP8 input is produced inside the kernel from the residual stream (M <= 128, K = 128, 256, 512

@@ -53,7 +53,8 @@ enum { TOK_EPI_BF16 = 0, TOK_EPI_ROPE = 1, TOK_EPI_GEGLU = 2, TOK_EPI_RESID = 3 
 // load instead of 4); four floats of padding rotate them apart.
 constexpr int TOK_ROW_PAD = 4;
 enum { TOK_PRO_TMA = 0, TOK_PRO_NORM = 1 };
-enum { TOK_STAT_STRIDE = 128 };          // floats between the per-tile rows of a statistics buffer
+// floats between the per-tile rows of a statistics buffer
+static inline int tok_stat_stride(int M) { return M <= 128 ? 128 : 256; }
 
 struct TokParams {
     int M, N;                  // activation rows (all m-tiles), output features
@@ -65,7 +66,9 @@ struct TokParams {
     int per_magic;             // ceil(65536 / per): row / per == (row * per_magic) >> 16 for row < 128 (no division on the
                                // path between the last MMA and the first pushed row)
     int ring_bytes;            // bytes of the operand ring / staging area in front of the receive slots
-    int m64;                   // one m-tile of at most 64 tokens: M = 64 MMAs over a 64-row A tile (8 KB per k-block), token
+    int m_rows;                // tokens of an m-tile (the last one may have fewer)
+    int stat_stride;           // tok_stat_stride(M)
+    int m64;                   // m-tiles of at most 64 tokens: M = 64 MMAs over a 64-row A tile (8 KB per k-block), token
                                // 16 i + j on tensor-memory lane 32 i + j; a CTA then leaves room for a neighbour's CTA
     const float* sa;           // device scalars (may be null = 1): activation / weight scale
     const float* sb;
@@ -80,16 +83,18 @@ struct TokParams {
     __nv_bfloat16* outV;
     const int* devpos;
     int q_dim, k_dim, v_dim, head_dim;
+    int rows_per_batch;        // tokens of a batch element (>= M: one element): rope row and cache row are m % rows_per_batch,
+    long long kv_batch_stride; // the caches of the elements lie kv_batch_stride elements apart
     // TOK_EPI_GEGLU
     uint8_t* out8;
     const float* out_scale;
     int half;
     int gate_act;              // 0 = GELU(tanh) gate (GeGLU), 1 = SiLU gate (SwiGLU), 2 = GELU(tanh) with the hardware tanh
-    // TOK_EPI_RESID: residual (M, N) bf16 in/out, gate (N,), stats_out [tile][TOK_STAT_STRIDE] (may be null)
+    // TOK_EPI_RESID: residual (M, N) bf16 in/out, gate (N,), stats_out [tile][stat_stride] (may be null)
     __nv_bfloat16* resid;
     const __nv_bfloat16* gate;
     float* stats_out;
-    // TOK_PRO_NORM: x (M, K) bf16, stats_in [n_stat][TOK_STAT_STRIDE], style = [scale (K) | shift (K)] one row
+    // TOK_PRO_NORM: x (M, K) bf16, stats_in [n_stat][stat_stride], style = [scale (K) | shift (K)] one row
     const __nv_bfloat16* x;
     const float* stats_in;
     int n_stat;
@@ -147,6 +152,13 @@ __device__ __forceinline__ void cluster_wait_acquire() {
 // column inside a head: a mask for the usual power-of-two head sizes, a division otherwise
 __device__ __forceinline__ int rope_col(int n, int head_dim) {
     return (head_dim & (head_dim - 1)) == 0 ? (n & (head_dim - 1)) : n % head_dim;
+}
+
+// (batch element, token inside it) of row m
+__device__ __forceinline__ int2 tok_batch_row(int m, const TokParams& p) {
+    if (p.rows_per_batch >= p.M) return make_int2(0, m);
+    const int b = m / p.rows_per_batch;
+    return make_int2(b, m - b * p.rows_per_batch);
 }
 
 // Sum over the S slots (fixed order) of the 8 received fp32 values of (token t of this rank, columns c8*8 .. +7).
@@ -218,8 +230,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int tile = blockIdx.x;
     // first weight row of the tile; with GeGLU a tile is BN / 2 gate rows + the BN / 2 matching up rows
     const int n0 = (EPI == TOK_EPI_GEGLU) ? tile * (BN / 2) : tile * BN;
-    const int m0 = blockIdx.y * 128;
-    const int Mt = (p.M - m0) < 128 ? (p.M - m0) : 128;         // tokens of this m-tile
+    const int m0 = blockIdx.y * p.m_rows;
+    const int Mt = (p.M - m0) < p.m_rows ? (p.M - m0) : p.m_rows;   // tokens of this m-tile
     const int S = (int)tc::cluster_nctarank();
     const int rank = (int)tc::cluster_ctarank();
     const int nkb = p.nkb;
@@ -369,7 +381,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
                         for (int t = 0; t < 16; ++t)
                             v[t] = (t0 + t < p.n_stat)
-                                       ? __ldcg(p.stats_in + (t0 + t) * TOK_STAT_STRIDE + m0 + threadIdx.x) : 0.0f;
+                                       ? __ldcg(p.stats_in + (t0 + t) * p.stat_stride + m0 + threadIdx.x) : 0.0f;
 #pragma unroll
                         for (int t = 0; t < 16; ++t)
                             if (t0 + t < p.n_stat) tot = __fadd_rn(tot, v[t]);
@@ -485,7 +497,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             float v[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t)
-                v[t] = (t0 + t < p.n_stat) ? __ldcg(p.stats_in + (t0 + t) * TOK_STAT_STRIDE + m) : 0.0f;
+                v[t] = (t0 + t < p.n_stat) ? __ldcg(p.stats_in + (t0 + t) * p.stat_stride + m) : 0.0f;
 #pragma unroll
             for (int t = 0; t < 16; ++t)
                 if (t0 + t < p.n_stat) tot = __fadd_rn(tot, v[t]);
@@ -516,7 +528,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 if (emit_q8) pre2 = ld_global_v4(p.q8_mod + n);
             } else if (EPI == TOK_EPI_ROPE && n < p.q_dim + p.k_dim) {
                 const int nr = n < p.q_dim ? n : n - p.q_dim;
-                pre0 = ld_global_v4(p.rope + (size_t)m * p.head_dim + rope_col(nr, p.head_dim));
+                pre0 = ld_global_v4(p.rope + (size_t)tok_batch_row(m, p).y * p.head_dim + rope_col(nr, p.head_dim));
             } else if (EPI == TOK_EPI_BF16 && p.bias && n + 8 <= p.N &&
                        (reinterpret_cast<uintptr_t>(p.bias + n) & 15) == 0) {
                 pre0 = ld_global_v4(p.bias + n);
@@ -638,10 +650,11 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     const bool is_q = n < p.q_dim;
                     const bool is_k = !is_q && n < p.q_dim + p.k_dim;
                     const int nr = is_q ? n : (is_k ? n - p.q_dim : n - p.q_dim - p.k_dim);
+                    const int2 br = tok_batch_row(m, p);
                     uint4 o;
                     if (is_q || is_k) {
                         uint4 tq = pre0;
-                        if (!first) tq = ld_global_v4(p.rope + (size_t)m * p.head_dim + rope_col(nr, p.head_dim));
+                        if (!first) tq = ld_global_v4(p.rope + (size_t)br.y * p.head_dim + rope_col(nr, p.head_dim));
                         const uint32_t* tw = &tq.x;
                         uint32_t* ow = &o.x;
 #pragma unroll
@@ -658,8 +671,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         o.w = pack_bf16x2(v[6], v[7]);
                     }
                     __nv_bfloat16* dst = is_q ? p.outQ + (size_t)m * p.q_dim + nr
-                                              : (is_k ? p.outK + (size_t)(pos + m) * p.k_dim + nr
-                                                      : p.outV + (size_t)(pos + m) * p.v_dim + nr);
+                                              : (is_k ? p.outK + br.x * p.kv_batch_stride + (size_t)(pos + br.y) * p.k_dim + nr
+                                                      : p.outV + br.x * p.kv_batch_stride + (size_t)(pos + br.y) * p.v_dim + nr);
                     st_global_v4(dst, o);
                 }
             } else if (EPI == TOK_EPI_GEGLU) {
@@ -754,7 +767,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 // the G lanes of a token are neighbours (G divides 32): butterfly inside the group, fixed order
 #pragma unroll
                 for (int off = G / 2; off >= 1; off >>= 1) ssq = __fadd_rn(ssq, __shfl_xor_sync(0xffffffffu, ssq, off));
-                if (act && g == 0 && p.stats_out) p.stats_out[tile * TOK_STAT_STRIDE + m] = ssq;
+                if (act && g == 0 && p.stats_out) p.stats_out[tile * p.stat_stride + m] = ssq;
             }
         }
     }
@@ -779,7 +792,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 }
 
 // ------------------------------------------------------------------ host side
-struct TokPlan { int BN, S, nkb, stages; };
+struct TokPlan { int BN, S, nkb, stages, m_tiles; };
 
 // Tile width and split-K factor for (M, N, K) from a serial cost model in microseconds, fitted to device-timer
 // traces of the four decoder projections at 50 tokens: 0.33 per resident k-block (four MMA issues), 0.06 per KB a
@@ -802,7 +815,7 @@ static bool tok_plan(int N, int K, int m_tiles, int mt, int epi, int pro, int sm
         if (w_kn && (BN == 64 || (epi == TOK_EPI_GEGLU && BN != 256))) continue;   // 128-feature boxes of (K, N) weights
         const int tiles = (epi == TOK_EPI_GEGLU ? (N / 2 + BN / 2 - 1) / (BN / 2) : (N + BN - 1) / BN) * m_tiles;
         const int max_st = BN == 256 ? 4 : BN == 128 ? 6 : 8;
-        const int stage_bytes = (m_tiles == 1 && mt <= 64 ? 8192 : 16384) + BN * 128;
+        const int stage_bytes = (mt <= 64 ? 8192 : 16384) + BN * 128;
         for (int S = 1; S <= 8; S *= 2) {
             if (want_s > 0 && S != want_s) continue;
             if (kbt % S) continue;
@@ -823,7 +836,7 @@ static bool tok_plan(int N, int K, int m_tiles, int mt, int epi, int pro, int sm
             else if (ctas > sms) cost += 1.0 * (ctas - sms) / sms;   // SMs that carry two CTAs run both slower
             if (cost < best) {
                 best = cost;
-                out->BN = BN; out->S = S; out->nkb = nkb; out->stages = stages;
+                out->BN = BN; out->S = S; out->nkb = nkb; out->stages = stages; out->m_tiles = m_tiles;
                 found = true;
             }
         }
@@ -831,18 +844,24 @@ static bool tok_plan(int N, int K, int m_tiles, int mt, int epi, int pro, int sm
     return found;
 }
 
+// m-tiles of at most 128 tokens, or (half) of at most 64: M = 64 MMAs over 8 KB operand tiles, two CTAs to an SM
+static inline int tok_m_tiles(int M, bool half) { return M <= 0 ? 1 : half ? (M + 63) / 64 : (M + 127) / 128; }
+
 template <int BN, int PRO, int EPI, int ACT = 0>
 static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, const TokPlan& pl, bool pdl,
                            cudaStream_t stream) {
     using Cfg = TokCfg<BN>;
     auto kern = gemm_tok_kernel<BN, PRO, EPI, ACT>;
-    const int m_tiles = (p.M + 127) / 128;
-    const int mt = p.M < 128 ? p.M : 128;
+    const int m_tiles = pl.m_tiles;
+    const int mt = (p.M + m_tiles - 1) / m_tiles;             // rows spread evenly over the m-tiles
+    p.m_rows = mt;
+    p.stat_stride = tok_stat_stride(p.M);
+    if (p.rows_per_batch <= 0) p.rows_per_batch = p.M;
     p.nkb = pl.nkb;
     p.stages = pl.stages;
     p.per = (mt + pl.S - 1) / pl.S;
     p.per_magic = (65536 + p.per - 1) / p.per;
-    p.m64 = (m_tiles == 1 && mt <= 64) ? 1 : 0;
+    p.m64 = mt <= 64 ? 1 : 0;
     const bool m64 = p.m64 != 0;
     // padded receive rows unless even a two-stage ring would not fit beside them
     const int need_stages = PRO == TOK_PRO_NORM ? pl.nkb : (p.stages < 2 ? p.stages : 2);   // the ring's lower bound
@@ -912,9 +931,10 @@ static int tok_sm_count() {
 
 template <int PRO, int EPI>
 static int dispatch_gemm_tok(const void* A, const void* W, TokParams p, int K, int want_bn, int want_s, bool pdl,
-                             cudaStream_t s) {
+                             cudaStream_t s, bool half_tiles = false) {
     TokPlan pl;
-    if (!tok_plan(EPI == TOK_EPI_GEGLU ? 2 * p.half : p.N, K, (p.M + 127) / 128, p.M < 128 ? p.M : 128, EPI, PRO,
+    const int mts = tok_m_tiles(p.M, half_tiles);
+    if (!tok_plan(EPI == TOK_EPI_GEGLU ? 2 * p.half : p.N, K, mts, (p.M + mts - 1) / mts, EPI, PRO,
                   tok_sm_count(), want_bn, want_s, &pl, p.w_kn != 0))
         return FRT_ERR_UNSUPPORTED;
     if constexpr (EPI == TOK_EPI_GEGLU) {

@@ -274,9 +274,10 @@ class GemmRunner:
 
     # -- the decoder's projections with the norm kernel between them folded in ------------------------------
     def fp8_nt_dev_gate_residual(self, A, B, M, N, K, d_scale_a, d_scale_b, residual, gate, stats_out, stream=0, *,
-                                 pdl=False, splits=0, tile_n=0, next_scale=0, q8_out=0, d_scale_q8=0) -> int:
+                                 pdl=False, splits=0, tile_n=0, next_scale=0, q8_out=0, d_scale_q8=0,
+                                 half_tiles=False) -> int:
         """``fp8_nt_dev`` + the first pass of ``gate_residual_ada_norm_fp8``: residual <- residual + o * gate and
-        the per-tile row sums of squares into ``stats_out`` (rows of 128 floats).  Returns the number of rows
+        the per-tile row sums of squares into ``stats_out`` (rows of 128 floats, 256 for M > 128).  Returns the number of rows
         written, which the consuming ``norm_fp8_nt_dev_*`` / ``fp8_nt_dev_*_rowscale`` call takes as ``n_stat``.
         With ``q8_out``: also the next projection's FP8 operand e4m3(residual * (1 + next_scale) / *d_scale_q8),
         i.e. the norm's output without its per-row 1 / rms, which ``fp8_nt_dev_*_rowscale`` applies afterwards."""
@@ -284,7 +285,7 @@ class GemmRunner:
         n = ctypes.c_int(0)
         call("frt_b200_gemm_fp8_nt_gate_residual_q8", A, B, M, N, K, d_scale_a, d_scale_b, residual, gate,
              stats_out or None, ctypes.addressof(n), next_scale or None, q8_out or None, d_scale_q8 or None, splits,
-             _f(pdl) | _tile_hint(tile_n), stream)
+             _f(pdl) | _tile_hint(tile_n) | (1024 if half_tiles else 0), stream)
         return n.value
 
     def fp8_nt_dev_rope_split_rowscale(self, A, B, M, K, d_scale_a, d_scale_b, stats, n_stat, col_term, rope_weights,
@@ -296,12 +297,24 @@ class GemmRunner:
              col_term, rope_weights, Q, Kc, Vc, devpos or None, q_dim, k_dim, v_dim, head_dim, splits,
              _f(pdl) | _tile_hint(tile_n), stream)
 
+    def fp8_nt_dev_rope_split_batched(self, A, B, M, K, d_scale_a, d_scale_b, stats, n_stat, col_term, rope_weights, Q, Kc, Vc,
+                                      q_dim, k_dim, v_dim, head_dim, rows_per_batch, kv_batch_stride, stream=0, *, eps=1e-6,
+                                      devpos=0, pdl=False, splits=0, tile_n=0, half_tiles=False):
+        """The QKV projection of a batch in one launch: ``fp8_nt_dev_rope_split_rowscale`` (``stats`` 0: the plain
+        projection) with the rope row and cache row of token m at m % rows_per_batch and the elements' K / V caches
+        ``kv_batch_stride`` elements apart.  ``half_tiles``: m-tiles of at most 64 tokens."""
+        call("frt_b200_gemm_fp8_nt_rope_split_batched", A, B, M, K, d_scale_a, d_scale_b, stats or None, n_stat, eps,
+             col_term or None, rope_weights, Q, Kc, Vc, devpos or None, q_dim, k_dim, v_dim, head_dim, rows_per_batch,
+             kv_batch_stride, splits, _f(pdl) | _tile_hint(tile_n) | (1024 if half_tiles else 0), stream)
+
     def fp8_nt_dev_geglu_fp8_rowscale(self, A, B, out, M, half_dim, K, d_scale_a, d_scale_b, stats, n_stat, col_term,
-                                      d_scale_out, stream=0, *, eps=1e-6, pdl=False, splits=0, tile_n=0, fast_gelu=False):
+                                      d_scale_out, stream=0, *, eps=1e-6, pdl=False, splits=0, tile_n=0, fast_gelu=False,
+                                      half_tiles=False):
         """gate|up projection of such an operand, ``gate_geglu_merged_fp8`` behind it (``fast_gelu``: the GELU through
         the hardware tanh)."""
         call("frt_b200_gemm_fp8_nt_geglu_fp8_rowscale", A, B, out, M, half_dim, K, d_scale_a, d_scale_b, stats, n_stat,
-             eps, col_term, d_scale_out, splits, _f(pdl) | (128 if fast_gelu else 0) | _tile_hint(tile_n), stream)
+             eps, col_term, d_scale_out, splits,
+             _f(pdl) | (128 if fast_gelu else 0) | _tile_hint(tile_n) | (1024 if half_tiles else 0), stream)
 
     def norm_fp8_nt_dev_rope_split(self, x, stats, n_stat, style, B, M, K, d_scale_a, d_scale_b, rope_weights, Q, Kc,
                                    Vc, q_dim, k_dim, v_dim, head_dim, stream=0, *, eps=1e-6, devpos=0, pdl=False,

@@ -173,6 +173,19 @@ def rope_table(start: int, count: int) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------ kernel composition
+def projection_tiles(rows: int):
+    """Tile width / split-K of the four projections (QKV, attention-out, gate|up, FFN-down) of the folded loop, from timings
+    of the whole captured loop.  Up to 64 rows one m-tile does; up to 128 rows two tiles of 64 beat one of 128 (the narrow
+    N = 1024 / 2560 products leave the chip idle: 100 rows 7.00 ms per loop against 7.09-7.9); above, the MMA's fixed cost per
+    128-row weight tile makes two tiles of up to 128 better than four of 64 (200 rows 8.45 against 9.3), except for the
+    QKV product, where both do the same."""
+    if rows <= 64:
+        return (dict(splits=4, tile_n=64), dict(splits=8, tile_n=64), dict(splits=2, tile_n=128), dict(splits=8, tile_n=64))
+    half = rows <= 128
+    return (dict(splits=2, tile_n=64, half_tiles=True), dict(splits=4, tile_n=64),
+            dict(splits=1, tile_n=128, half_tiles=half), dict(splits=4, tile_n=64, half_tiles=half))
+
+
 SITES = ("qkv", "o", "gu", "d")
 
 
@@ -245,7 +258,7 @@ class StepIO:
         qs = (S * DEC_NH * DEC_HD, DEC_NH * DEC_HD, DEC_HD)
         ks = (fe.kv_rows * DEC_NKV * DEC_HD, DEC_NKV * DEC_HD, DEC_HD)
         kw = dict(pdl=pdl, out_fp8=out_fp8, out_scale=out_scale, kv_splits=self.attn_splits,
-                  counters=self.attn_counters.data_ptr())
+                  counters=self.attn_counters.data_ptr(), flags=self.attn_flags)
         common = (fe.batch, S, T, DEC_NH, DEC_NKV, DEC_HD, qs, ks, ks, qs, 1.0 / math.sqrt(DEC_HD), fe.sm_count, stream)
         q, k, v, o = (self.q.data_ptr(), fe.k_cache[layer].data_ptr(), fe.v_cache[layer].data_ptr(),
                       self.attn.data_ptr())
@@ -291,13 +304,14 @@ class Pi05DecoderPipeline(StepIO):
         self.ones = torch.ones(DEC_D, dtype=BF16, device=dev)
         # split-KV scratch of the attention kernel (the reference's FA2 o_accum / softmax_lse_accum buffers)
         self.attn_splits = fe.attn_splits
+        self.attn_flags = 16                           # attn_splits is a bound, the split is chosen by size
         self.o_accum = z(self.attn_splits, S, DEC_NH, DEC_HD, dtype=torch.float32)
         self.lse_accum = z(self.attn_splits, DEC_NH, S, dtype=torch.float32)
         self.attn_counters = z(2 * fe.batch * ((fe.chunk_size * DEC_NH + 127) // 128), dtype=torch.int32)
         # activation scales: one per GEMM input site, per layer, per denoise step (pipeline_rtx.py:649-660)
         self.act_scale = torch.ones(N, L, len(SITES), dtype=torch.float32, device=dev)
         # per-tile row sums of squares handed from a row-parallel projection to the next column-parallel one
-        self.row_stats = torch.zeros(16, 128, dtype=torch.float32, device=dev)
+        self.row_stats = torch.zeros(16, 256, dtype=torch.float32, device=dev)
         # deferred row scale: scales of the un-normalised operands x * (1 + scale) ([..., 0]: QKV input of the layer,
         # [..., 1]: gate|up input) and the column terms W . shift of both projections, per step and layer
         self.raw_scale = torch.ones(N, L, 2, dtype=torch.float32, device=dev)
@@ -493,7 +507,8 @@ class Pi05DecoderPipeline(StepIO):
 
     def _folds_norms(self) -> bool:
         fe = self.fe
-        return fe.fold_norms and fe.batch == 1 and self.M <= 128
+        # several elements: the row-scaled forms only (the in-kernel norm producer takes one element of up to 128 tokens)
+        return fe.fold_norms and (self.M <= 256 if fe.defer_norm else fe.batch == 1 and self.M <= 128)
 
     def _folded_layers(self, step, stream, pdl, attention: bool = True, first_norm: bool = True) -> None:
         """The 18 blocks of one Euler step with five launches each: QKV (RoPE + split + KV append behind), attention
@@ -510,21 +525,21 @@ class Pi05DecoderPipeline(StepIO):
         qd, kd = DEC_NH * DEC_HD, DEC_NKV * DEC_HD
         gate_off = 2 * DEC_D * 2
         n_stat = 0
-        # tile width / split-K of the four projections at <= 64 tokens, from per-launch timings of the captured chain
-        # (QKV 64 x 4, attention-out 64 x 8, gate|up 64 + 64 x 2, FFN-down 64 x 8); larger row counts use the
-        # library's own choice
-        tuned = S <= 64
         defer = fe.defer_norm
-        t_qkv = dict(splits=4, tile_n=64) if tuned else {}
-        t_o = dict(splits=8, tile_n=64) if tuned else {}
-        t_gu = dict(splits=2, tile_n=128) if tuned else {}
-        t_d = dict(splits=8, tile_n=64) if tuned else {}
+        t_qkv, t_o, t_gu, t_d = (dict(t) for t in projection_tiles(S))
         t_gu["fast_gelu"] = fe.fast_gelu
         for i in range(L):
             kp, vp, dp = self._kv_dst(i, 0)
-            if i == 0:
-                if attention and first_norm:
-                    self._norm(None, None, "attn", step, 0, "qkv", stream, pdl, False)
+            if i == 0 and attention and first_norm:
+                self._norm(None, None, "attn", step, 0, "qkv", stream, pdl, False)
+            if fe.batch > 1:
+                a_scale, rs = ((self._scale_ptr(step, i, "qkv"), (0, 0, 0)) if i == 0 else
+                               (self._raw_ptr(step, i, 0), (stats, n_stat, self.col_qkv[step, i].data_ptr())))
+                g.fp8_nt_dev_rope_split_batched(self.act8.data_ptr(), fe.w_qkv[i].data_ptr(), S, DEC_D, a_scale,
+                                                fe.ws_qkv_t[i].data_ptr(), *rs, fe.rope.data_ptr(), self.q.data_ptr(), kp,
+                                                vp, qd, kd, kd, DEC_HD, fe.chunk_size, fe.kv_rows * kd, stream, devpos=dp,
+                                                pdl=pdl, **t_qkv)
+            elif i == 0:
                 g.fp8_nt_dev_rope_split(self.act8.data_ptr(), fe.w_qkv[i].data_ptr(), S, DEC_D,
                                         self._scale_ptr(step, i, "qkv"), fe.ws_qkv_t[i].data_ptr(),
                                         fe.rope.data_ptr(), self.q.data_ptr(), kp, vp, qd, kd, kd, DEC_HD, stream,
@@ -562,8 +577,8 @@ class Pi05DecoderPipeline(StepIO):
                        d_scale_q8=self._raw_ptr(step, i + 1, 0)) if defer and i < L - 1 else {})
             n_stat = g.fp8_nt_dev_gate_residual(self.hid8.data_ptr(), fe.w_d[i].data_ptr(), S, DEC_D, DEC_H,
                                                 self._scale_ptr(step, i, "d"), fe.ws_d_t[i].data_ptr(), x,
-                                                self._style("ffn", step, i) + gate_off, stats, stream, pdl=pdl,
-                                                **t_d, **q8)
+                                                self._style("ffn", step, i) + gate_off,
+                                                stats if i < L - 1 else 0, stream, pdl=pdl, **t_d, **q8)
 
     def launches_per_layer(self) -> float:
         """Average over the layers (the last layer keeps its separate residual kernel when the norms are fused)."""

@@ -70,6 +70,7 @@ class Pi05DecoderNvfp4Pipeline(StepIO):
         self.hid4, self.hid4_sf = z(M, DEC_H // 2, dtype=torch.uint8), sfb(DEC_H)
         self.ones = torch.ones(DEC_D, dtype=BF16, device=dev)
         self.attn_splits = fe.attn_splits
+        self.attn_flags = 0                            # the same split at every batch size: a batch gives the bits of single runs
         self.o_accum = z(self.attn_splits, B, S, DEC_NH, DEC_HD, dtype=torch.float32)
         self.lse_accum = z(self.attn_splits, B, DEC_NH, S, dtype=torch.float32)
         self.attn_counters = z(2 * B * ((S * DEC_NH + 127) // 128), dtype=torch.int32)

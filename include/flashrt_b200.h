@@ -178,7 +178,8 @@ int frt_b200_gemm_status(int reset);
  *   device; with a last tile of at most 32 rows that tile may run in two parts instead to make them fit), else
  *   (b) through the scratch, published with an arrival counter per tile.  (a) and (b) give the same bits.
  *   flags: bit 0 = programmatic dependent launch; bit 1 = keep the single-tile kernel; head_dim 256 with scratch:
- *   bit 2 = one CTA per (tile, split) instead of four head-dim parts, bit 3 = always (b). */
+ *   bit 2 = one CTA per (tile, split) instead of four head-dim parts, bit 3 = always (b), bit 4 = kv_splits (> 0) is an upper
+ *   bound: the number of splits (2, 4 or 8, one of them possibly without keys) and of parts (4 or 2) is chosen by size. */
 int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, void* O, void* O_fp8,
                                 const float* out_scale, float* lse, const int* seqused_k, int batch, int seqlen_q,
                                 int seqlen_k, int num_heads_q, int num_heads_kv, int head_dim,
@@ -216,9 +217,9 @@ int frt_b200_status_words_async(int* out3, int reset, int flags, void* stream);
  * reset != 0 restarts the launch slots and clears the stamps after copying them out.  Synchronises the device. */
 int frt_b200_phase_stamps_read(unsigned long long* gemm_host, unsigned long long* attn_host, int reset);
 
-/* Residual update and the LayerNorm behind it in one pass, same bits as the two calls: res_out = bf16(res + x * gate)
- * (gate NULL: + x; x NULL: none); out_fp8 = e4m3 of the (affine, modulated) LayerNorm of the result, NULL: update only.
- * gate / scale / shift rows at + (r / mod_rows) * mod_stride. */
+/* Residual update and the LayerNorm behind it in one pass, same bits as the two calls (no counterpart in the reference as
+ * one launch): res_out = bf16(res + x * gate) (gate NULL: + x; x NULL: none); out_fp8 = e4m3 of the (affine, modulated)
+ * LayerNorm of the result, NULL: update only.  gate / scale / shift rows at + (r / mod_rows) * mod_stride. */
 int frt_b200_residual_layer_norm_fp8(const void* res, const void* x, const void* gate, void* res_out, const void* weight,
                                      const void* bias, const void* scale, const void* shift, long long mod_stride,
                                      long long mod_rows, void* out_fp8, const float* d_scale, long long rows, int dim,
@@ -312,6 +313,16 @@ int frt_b200_gemm_fp8_nt_rope_split_rowscale(const void* A, const void* W, int M
                                              const float* col_term, const void* rope, void* Q, void* Kout, void* Vout,
                                              const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim,
                                              int splits, int flags, void* stream);
+/* The QKV projection of a batch (M <= 256 rows = elements of rows_per_batch tokens, 0: one element), row-scaled as above
+ * (stats_in NULL: plain): rope row and cache row of token m are m % rows_per_batch, the K / V caches of the elements lie
+ * kv_batch_stride elements apart (qkv_split_rope per element, csrc/kernels/rope.cu:135-277).  K % 128 == 0.
+ * flags bit 10: m-tiles of at most 64 tokens (also in the row-scaled and gated-residual entry points). */
+int frt_b200_gemm_fp8_nt_rope_split_batched(const void* A, const void* W, int M, int K, const float* d_scale_a,
+                                            const float* d_scale_b, const float* stats_in, int n_stat, float eps,
+                                            const float* col_term, const void* rope, void* Q, void* Kout, void* Vout,
+                                            const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim,
+                                            int rows_per_batch, long long kv_batch_stride, int splits, int flags,
+                                            void* stream);
 /* gate|up form of the row-scaled projection: gate_geglu_merged_fp8 (csrc/kernels/activation.cu:249-279) behind it. */
 int frt_b200_gemm_fp8_nt_geglu_fp8_rowscale(const void* A, const void* W, void* out8, int M, int half, int K,
                                             const float* d_scale_a, const float* d_scale_b, const float* stats_in,

@@ -1,0 +1,95 @@
+"""GPU parity of the folded loop's launches at the row counts of a batch (65 .. 256 rows in one or more m-tiles), and of the
+attention split chosen by size."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from oracle import oracle as O  # noqa: E402
+from test_b_gemm_gpu import _check, _fp8_operand, _ref  # noqa: E402
+from test_c_attention_gpu import _run  # noqa: E402
+
+
+@pytest.mark.parametrize("batch,S,half", [(2, 33, True), (2, 64, True), (3, 43, False), (4, 64, False), (4, 50, True), (5, 13, False)])
+def test_projections_of_a_batch(batch, S, half):
+    """Row-scaled QKV (rope and cache rows per element), gated residual with the next operand and row-scaled gate|up at
+    M = batch * S: the codes, statistics and residual of every row are those of its own element run alone."""
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, f32, rand_bf16, zeros
+    rng = np.random.default_rng(batch * 100 + S)
+    M, D, H, hd, rows = batch * S, 1024, 512, 256, S + 7
+    q_dim, k_dim, v_dim = 512, 256, 256
+    ld = 128 if M <= 128 else 256
+    A, sa = _fp8_operand(rng, M, D, 1.0)
+    Wq, sq = _fp8_operand(rng, q_dim + k_dim + v_dim, D, 0.02)
+    Wg, sg = _fp8_operand(rng, 2 * H, D, 0.03)
+    Wo, so = _fp8_operand(rng, D, D, 0.02)
+    rope = rand_bf16(rng, (S, hd), 1.0)
+    res0, gate, mod = rand_bf16(rng, (M, D), 1.0), rand_bf16(rng, (D,), 0.5), rand_bf16(rng, (D,), 0.3)
+    ssq = (rng.random((16, M)) * D / 4.0).astype(np.float32)
+    cq, cg = rng.standard_normal(q_dim + k_dim + v_dim).astype(np.float32), rng.standard_normal(2 * H).astype(np.float32)
+    d_A, d_Wq, d_Wg, d_Wo, d_rope, d_gate, d_mod = (Dev(a) for a in (A, Wq, Wg, Wo, rope, gate, mod))
+    d_sa, d_sq, d_sg, d_so, d_s8, d_cq, d_cg = f32(sa), f32(sq), f32(sg), f32(so), f32(0.013), Dev(cq), Dev(cg)
+    g = fvk.GemmRunner()
+    h = dict(half_tiles=half)
+
+    def run(first, n):
+        m = n * S
+        pitch = 128 if m <= 128 else 256
+        st = np.zeros((16, pitch), np.float32)
+        st[:, :m] = ssq[:, first * S:first * S + m]
+        d_st, d_a, d_res = Dev(st), Dev(A[first * S:first * S + m]), Dev(res0[first * S:first * S + m])
+        Q, K, V = zeros((m, q_dim), np.uint16), zeros((n, rows, k_dim), np.uint16), zeros((n, rows, v_dim), np.uint16)
+        hid, q8, so_ = zeros((m, H), np.uint8), zeros((m, D), np.uint8), Dev(np.full((16, pitch), -1.0, np.float32))
+        g.fp8_nt_dev_rope_split_batched(d_a.ptr, d_Wq.ptr, m, D, d_sa.ptr, d_sq.ptr, d_st.ptr, 16, d_cq.ptr, d_rope.ptr,
+                                        Q.ptr, K.ptr + 7 * k_dim * 2, V.ptr + 7 * v_dim * 2, q_dim, k_dim, v_dim, hd, S,
+                                        rows * k_dim, 0, splits=2, tile_n=64, **h)
+        g.fp8_nt_dev_geglu_fp8_rowscale(d_a.ptr, d_Wg.ptr, hid.ptr, m, H, D, d_sa.ptr, d_sg.ptr, d_st.ptr, 16, d_cg.ptr,
+                                        d_s8.ptr, 0, splits=1, tile_n=128, **h)
+        k = g.fp8_nt_dev_gate_residual(d_a.ptr, d_Wo.ptr, m, D, D, d_sa.ptr, d_so.ptr, d_res.ptr, d_gate.ptr, so_.ptr, 0,
+                                       splits=4, tile_n=64, next_scale=d_mod.ptr, q8_out=q8.ptr, d_scale_q8=d_s8.ptr, **h)
+        assert fvk.tensor_core_status() == 0 and k == 16
+        return [a.get() for a in (Q, K, V, hid, q8, d_res)] + [so_.get()]
+
+    whole = run(0, batch)
+    assert (whole[6][:, M:] == -1.0).all() and whole[6].shape[1] == ld
+    for e in range(batch):
+        one = run(e, 1)
+        for i in (0, 3, 4, 5):
+            assert np.array_equal(whole[i][e * S:(e + 1) * S], one[i])
+        assert np.array_equal(whole[1][e], one[1][0]) and np.array_equal(whole[2][e], one[2][0])
+        assert np.array_equal(whole[6][:, e * S:(e + 1) * S], one[6][:, :S])
+    rms = 1.0 / np.sqrt(ssq.astype(np.float64).sum(0) / D + 1e-6)
+    v = (_ref(A, Wq, sa, sq).astype(np.float64) * rms[:, None] + cq[None, :])[:, q_dim + k_dim:]
+    _check(whole[2][:, 7:].reshape(M, v_dim), v.astype(np.float32))
+
+
+@pytest.mark.parametrize("B,Sq,Skv,extra", [(1, 20, 170, {}), (1, 60, 828, {}), (2, 50, 818, dict(fused_fp8=True)),
+                                            (4, 50, 818, {}), (3, 24, 792, dict(seqused=70)), (1, 16, 64, {}),
+                                            (4, 64, 150, {})])
+def test_attention_split_chosen_by_size(B, Sq, Skv, extra):
+    """flags bit 4: a bound on the splits; whatever split and number of parts is chosen matches the oracle."""
+    _run(B, Sq, Skv, 8, 1, 256, 8, seed=B + Sq, scratch=True, flags=16, **extra)
+
+
+def test_fp8_batch4_agrees_with_single_runs():
+    """200 rows per projection (two m-tiles, the rows of an element across them) through the whole captured loop."""
+    import torch
+    from flashrt_b200 import load_model
+    from flashrt_b200.pi05_decoder import synthetic_state_dict
+    from oracle import block_ref as R
+    L = 2
+    sd = synthetic_state_dict(seed=0, layers=L)
+    k, v = (t.to(torch.bfloat16) for t in R.synthetic_prefix_kv(seed=1, layers=L, prefix_len=300))
+    cal = [R.synthetic_noise(100 + j) for j in range(2)]
+    noises = np.stack([R.synthetic_noise(10 + j).to(torch.bfloat16).float().numpy() for j in range(4)])
+    models = []
+    for b in (1, 4):
+        m = load_model(sd, config="pi05", layers=L, num_steps=10, chunk_size=50, prefix_len=300, batch=b)
+        m.set_prefix(k, v)
+        m.calibrate([torch.stack([c] * b) if b > 1 else c for c in cal])
+        models.append(m)
+    got = models[1].predict(noise=noises)
+    for j in range(4):
+        one = models[0].predict(noise=noises[j])
+        assert np.abs(got[j] - one).max() <= 3e-2 * float(np.sqrt((one ** 2).mean()))
