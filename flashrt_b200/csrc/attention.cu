@@ -764,7 +764,7 @@ int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, voi
             const int chunks64 = (seqlen_k + 63) / 64;
             // Without scratch one split of this kernel (about 5 + 1.1 us per chunk) against the single-tile kernel's cluster
             // of splits (about 15 us while all clusters fit one wave): one split when the chain is short or the tiles alone
-            // cover the device (768 x 768 x 8 heads, 48 tiles: 58 us as clusters of four in two waves, one wave as one
+            // cover the device (768 x 768 x 8 heads, 48 tiles: 58 us as clusters of four in two waves, 27 us as one
             // split each).
             const bool one = p.o_accum ? tiles >= 74 : (tiles > 18 || chunks64 <= 9);
             int sp64 = kv_splits > 0 ? kv_splits : (one ? 1 : (chunks64 < 8 ? chunks64 : 8));

@@ -178,7 +178,7 @@ template <int BN, bool SWAP, int EPI, bool FP4 = false>
 __global__ void __launch_bounds__(128, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmC, GemmParams p) {
     static_assert(EPI == EPI_BF16 || SWAP, "fused epilogues exist for the small-M (swapped) kernel only");
-    static_assert(!FP4 || (BN >= 32 && EPI != EPI_GEGLU_FP8), "NVFP4: column tiles start on 32-row scale groups");
+    static_assert(!FP4 || (BN >= 32 && EPI != EPI_GEGLU_FP8), "NVFP4: scale groups of 32 rows");
     using Cfg = GemmCfg<BN, FP4>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -797,6 +797,9 @@ static int launch_gemm(const void* A, const void* W, GemmParams p, int K, int sp
     p.col_rows = SWAP ? p.M : p.N;
     p.w_is_lane = SWAP ? 1 : 0;
     if (FP4) {
+        // a tile of 32 columns has to be the only one: the second would start at an odd column of the scale factors in tensor
+        // memory, and those addresses have to be even
+        if (BN == 32 && p.col_rows > 32) return FRT_ERR_UNSUPPORTED;
         if (SWAP) { const uint8_t* t = p.sf_lane; p.sf_lane = p.sf_col; p.sf_col = t; }   // callers pass (A, W) order
         p.sf_katoms = K / 64;
         p.sf_col_rblocks = (p.col_rows + 127) / 128;
@@ -906,13 +909,27 @@ static int dispatch_small_m(const void* A, const void* W, GemmParams p, int K, i
 #include "gemm_pair.cuh"
 #include "gemm_tok.cuh"
 
+// NVFP4, M <= 256.  Column tiles of 64 tokens while all of them fit one wave, since the finish of a tile grows with its
+// columns -- us per wave 4.5 / 6.2 / 8.8 for 64 / 128 / 256 (200 x 1024 x 2048: 12.6 as one tile of 256, 6.7 as four of 64;
+// 200 x 8192 x 1024: 9.0 / 6.6 (128) / 9.9 (64, two waves)) -- and the k split only as far as it leaves them in one wave
+// (200 x 2560 x 1024: 11 with split 4, 4.7 without; the action expert's loop at 4 x 50 rows 65.4 -> 57.3 us per block).
 template <int EPI>
 static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, int K, int M, int tiles, int splits,
                                   bool pdl, cudaStream_t s) {
     int sp = pick_splits(tiles, p.kb_total, splits);
+    const long long sms = device_sm_count();
+    while (splits <= 0 && sp > 1 && (long long)tiles * ((M + 63) / 64) * sp > sms) sp /= 2;
     if (M <= 32) return launch_gemm<32, true, EPI, true>(A, W, p, K, sp, pdl, s);
-    if (M <= 64) return launch_gemm<64, true, EPI, true>(A, W, p, K, sp, pdl, s);
-    if (M <= 128) return launch_gemm<128, true, EPI, true>(A, W, p, K, sp, pdl, s);
+    static const int wave_cost[3] = {45, 62, 88};
+    int bn = 0;
+    long long best = 0;
+    for (int i = 0; i < 3 && (i == 0 || (32 << i) < M); ++i) {
+        const long long ctas = (long long)tiles * ((M + (64 << i) - 1) / (64 << i)) * sp;
+        const long long cost = (ctas + sms - 1) / sms * wave_cost[i];
+        if (bn == 0 || cost < best) { best = cost; bn = 64 << i; }
+    }
+    if (bn == 64) return launch_gemm<64, true, EPI, true>(A, W, p, K, sp, pdl, s);
+    if (bn == 128) return launch_gemm<128, true, EPI, true>(A, W, p, K, sp, pdl, s);
     return launch_gemm<256, true, EPI, true>(A, W, p, K, sp, pdl, s);
 }
 

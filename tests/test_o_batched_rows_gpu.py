@@ -93,3 +93,22 @@ def test_fp8_batch4_agrees_with_single_runs():
     for j in range(4):
         one = models[0].predict(noise=noises[j])
         assert np.abs(got[j] - one).max() <= 3e-2 * float(np.sqrt((one ** 2).mean()))
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 256, 512), (65, 256, 512), (128, 384, 256), (200, 1024, 512), (256, 1024, 2560),
+                                   (200, 6144, 256), (200, 16384, 256)])
+def test_nvfp4_column_tiles(M, N, K):
+    """Exact products with a different power-of-two scale in every block: column tiles of 64 (both halves of a 128-row group
+    of scales), 128 and 256 tokens equal the oracle bit for bit."""
+    from test_h_nvfp4_gpu import _run_gemm
+    rng = np.random.default_rng(M + N)
+
+    def make(rows):
+        e = rng.integers(-3, 3, (rows, K // 16))
+        x = rng.choice(np.array([-4, -3, -2, -1, 0, 1, 2, 3, 4, 6, -6], np.float32), (rows, K))
+        x = x * np.repeat(np.exp2(e).astype(np.float32), 16, axis=1)
+        x[:, ::16] = 6.0 * np.exp2(e).astype(np.float32)
+        return O.quantize_nvfp4(x.astype(np.float32), 1)
+
+    a, w = make(M), make(N)
+    assert np.array_equal(_run_gemm(*a, *w, M, N, K, alpha=0.125), O.gemm_nvfp4(*a, *w, alpha=0.125))
