@@ -13,6 +13,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libflashrt_b200.so")
+CALLS = os.path.join(HERE, "_native_calls.so")
 OBJ = os.path.join(CSRC, "build")
 
 NVCC_FLAGS = [
@@ -23,6 +24,70 @@ NVCC_FLAGS = [
 
 def sources() -> list[str]:
     return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+
+
+def calls_source(protos: dict[str, list[str]]) -> str:
+    """C source of the extension module that calls the entry points: one function per prototype, positional arguments.
+
+    A small product is bound by the host: through ctypes a call with 14-16 arguments costs 2.5-3 us on top of its launch
+    (attribute lookup, one converter object per argument), the vectorcall functions written here about 0.3 us.  A pointer is
+    an int or None, a number an int or a float; anything else (a ctypes object, a wrong count) returns NotImplemented and the
+    caller takes the ctypes path, which converts or refuses it as it always did.  The GIL is released around the call."""
+    cnum = {"int": ("long long", "PyLong_Check", "PyLong_AsLongLong"),
+            "long long": ("long long", "PyLong_Check", "PyLong_AsLongLong"),
+            "unsigned": ("long long", "PyLong_Check", "PyLong_AsLongLong"),
+            "unsigned long long": ("unsigned long long", "PyLong_Check", "PyLong_AsUnsignedLongLong"),
+            "ptr": ("unsigned long long", "PyLong_Check", "PyLong_AsUnsignedLongLong"),
+            "float": ("double", "PyFloat_Check", "PyFloat_AsDouble")}
+    out = ["#define PY_SSIZE_T_CLEAN", "#include <Python.h>", ""]
+    table = []
+    for name, types in protos.items():
+        n = len(types)
+        ctypes_ = ["const void*" if t == "ptr" else t for t in types]
+        out.append(f"int {name}({', '.join(ctypes_) or 'void'});")
+        out.append(f"static PyObject* w_{name}(PyObject* self, PyObject* const* a, Py_ssize_t n) {{")
+        out.append(f"    if (n != {n}) Py_RETURN_NOTIMPLEMENTED;")
+        for i, t in enumerate(types):
+            c, check, conv = cnum[t]
+            out.append(f"    {c} v{i} = 0;")
+            if t == "ptr":
+                out.append(f"    if (a[{i}] != Py_None) {{ if (!{check}(a[{i}])) Py_RETURN_NOTIMPLEMENTED; "
+                           f"v{i} = {conv}(a[{i}]); }}")
+            elif t == "float":
+                out.append(f"    if (PyFloat_Check(a[{i}])) v{i} = PyFloat_AS_DOUBLE(a[{i}]); "
+                           f"else if (PyLong_Check(a[{i}])) v{i} = PyLong_AsDouble(a[{i}]); else Py_RETURN_NOTIMPLEMENTED;")
+            else:
+                out.append(f"    if (!{check}(a[{i}])) Py_RETURN_NOTIMPLEMENTED; v{i} = {conv}(a[{i}]);")
+        if n:
+            out.append("    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NOTIMPLEMENTED; }")
+        args = ", ".join(f"(const void*)(uintptr_t)v{i}" if t == "ptr" else f"({t})v{i}" for i, t in enumerate(types))
+        out.append("    int rc;")
+        out.append(f"    Py_BEGIN_ALLOW_THREADS rc = {name}({args}); Py_END_ALLOW_THREADS")
+        out.append("    return PyLong_FromLong(rc);\n}")
+        table.append(f'    {{"{name}", (PyCFunction)(void*)w_{name}, METH_FASTCALL, NULL}},')
+    out += ["static PyMethodDef methods[] = {", *table, "    {NULL, NULL, 0, NULL}};",
+            'static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native_calls", NULL, -1, methods};',
+            "PyMODINIT_FUNC PyInit__native_calls(void) { return PyModule_Create(&module); }", ""]
+    return "\n".join(out)
+
+
+def build_calls(force: bool = False) -> str | None:
+    """The extension module behind ``_lib.call``; None where the interpreter's headers or a C compiler are missing (the ctypes
+    path then serves every call)."""
+    import sysconfig
+    from ._lib import HEADER_PATH, parse_header
+    inc, cc = sysconfig.get_paths()["include"], shutil.which("gcc") or shutil.which("cc")
+    if cc is None or not os.path.exists(os.path.join(inc, "Python.h")):
+        return None
+    if force or _stale(CALLS, [HEADER_PATH, os.path.abspath(__file__), LIB]):
+        src = os.path.join(OBJ, "native_calls.c")
+        with open(src, "w") as f:
+            f.write(calls_source(parse_header()))
+        r = subprocess.run([cc, "-O2", "-fPIC", "-shared", "-I", inc, src, "-o", CALLS, "-L", HERE, "-l:libflashrt_b200.so",
+                            "-Wl,-rpath,$ORIGIN"], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("gcc failed:\n" + r.stdout + r.stderr)
+    return CALLS
 
 
 def _nvcc() -> str:
@@ -77,6 +142,7 @@ def build_native(force: bool = False, verbose: bool = False) -> str:
             print("\n".join(logs))
     if jobs or force or _stale(LIB, objs):
         run([nvcc, "-shared", "-o", LIB] + objs)
+    build_calls(force)
     return LIB
 
 

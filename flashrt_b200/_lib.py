@@ -1,7 +1,8 @@
 """ctypes binding of ``libflashrt_b200.so`` (the C-ABI CUDA library).
 
 The prototypes are read from ``include/flashrt_b200.h`` so the header stays the
-single statement of the ABI.  There is no fallback: if the shared object is
+single statement of the ABI; calls go through the extension module generated from the same
+prototypes (``_build.calls_source``).  There is no fallback: if the shared object is
 missing or a call returns a non-zero status, an exception is raised.
 """
 from __future__ import annotations
@@ -52,6 +53,7 @@ def parse_header(path: str = HEADER_PATH) -> dict[str, list[str]]:
 
 _lib = None
 _protos: dict[str, list[str]] | None = None
+_fns: dict = {}             # name -> function: of the native call module where it was built, else of the ctypes library
 
 
 def load() -> C.CDLL:
@@ -71,6 +73,11 @@ def load() -> C.CDLL:
             raise KernelLibraryMissing(f"{LIB_PATH} does not export {name}; rebuild it") from e
         fn.restype = C.c_int
         fn.argtypes = [C.c_void_p if t == "ptr" else _CTYPE[t] for t in types]
+    try:
+        from . import _native_calls as native
+    except ImportError:
+        native = None
+    _fns.update({name: getattr(native, name, None) or getattr(lib, name) for name in _protos})
     _lib = lib
     return lib
 
@@ -84,15 +91,24 @@ _ERRORS = {-1: "invalid argument", -2: "unsupported shape or feature", -3: "boun
            -4: "request larger than the library's built-in fixed-size scratch"}
 
 
+def call_status(name: str, *args) -> int:
+    """Call an entry point whose return value is data or a status the caller inspects."""
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(load(), name)
+    rc = fn(*args)
+    return getattr(_lib, name)(*args) if rc is NotImplemented else rc       # an argument that ctypes has to convert
+
+
 def call(name: str, *args) -> int:
     """Call entry point ``name``; raise :class:`KernelError` on a non-zero status."""
-    rc = getattr(load(), name)(*args)
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(load(), name)
+    rc = fn(*args)
+    if rc is NotImplemented:
+        rc = getattr(_lib, name)(*args)
     if rc != 0:
         why = _ERRORS.get(rc, f"CUDA error {-rc - 1000}" if rc <= -1000 else "error")
         raise KernelError(f"{name} failed: status {rc} ({why})")
     return rc
-
-
-def call_status(name: str, *args) -> int:
-    """Call an entry point whose return value is data or a status the caller inspects."""
-    return getattr(load(), name)(*args)

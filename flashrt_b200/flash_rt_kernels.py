@@ -246,9 +246,12 @@ def fp8_gemm_descale_bf16out(A, B, C, M, N, K, act_descale, w_descale, stream=0,
     call("frt_b200_gemm_fp8_nt", A, B, C, M, N, K, act_descale, w_descale, 1.0, None, splits, _f(pdl), stream)
 
 
+_TILE_HINTS = {0: 0, 64: 1 << 8, 128: 2 << 8, 256: 3 << 8}
+
+
 def _tile_hint(tile_n: int) -> int:
     """flags bits 8-9 of the small-M FP8 GEMM entry points: pinned tile width of the token-major kernel."""
-    return {0: 0, 64: 1, 128: 2, 256: 3}[int(tile_n)] << 8
+    return _TILE_HINTS[int(tile_n)]
 
 
 class GemmRunner:
