@@ -75,7 +75,7 @@ small_gemm_bf16_kernel(const void* __restrict__ Av, const __nv_bfloat16* __restr
 }
 
 // ------------------------------------------------------------------ boundary between two Euler steps, one launch
-// Per token (one CTA, dim / 8 threads, 8 features each -- the layout of norm_row_kernel):
+// Per token one CTA of dim / 2 threads; the norms run on its first dim / 8 (8 features each -- the layout of norm_row_kernel):
 //   [has_prev]  xn = bf16(adaRMS(x; style_prev))                      final norm of the step that ends
 //               noise += xn . W_out + b_out                            action out-projection (pre-scaled by dt) + Euler
 //   [has_next]  x = bf16(bf16(noise) . W_in + b_in)                    action in-projection of the step that begins
@@ -85,11 +85,17 @@ small_gemm_bf16_kernel(const void* __restrict__ Av, const __nv_bfloat16* __restr
 // the old value), so the results are theirs bit for bit.  ACTION = 32 columns of the action space.
 constexpr int SB_ACTION = 32;
 
+// Latency bounds it (50 CTAs, a chain of two norms and two small products), so the serial stretches are short: one K-slice of
+// the out-projection and two columns of the in-projection per thread.  (With dim / 8 threads, four slices and eight columns
+// each: 15.3 us per launch in the loop at 50 x 1024, now 6.5.)
+
+// 1 / rms of the row whose 8-feature sums of squares the first dim / 8 threads hold; every thread reaches both barriers
 __device__ __forceinline__ float sb_block_rms(float ssq, float* warp_tot, int dim, float eps) {
-    ssq = warp_sum_butterfly(ssq);
-    const int nwarps = blockDim.x >> 5;
+    const int nwarps = dim >> 8;
+    const int warp = threadIdx.x >> 5;
+    if (warp < nwarps) ssq = warp_sum_butterfly(ssq);
     __syncthreads();                                    // warp_tot may still be read from the previous use
-    if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = ssq;
+    if (warp < nwarps && (threadIdx.x & 31) == 0) warp_tot[warp] = ssq;
     __syncthreads();
     float tot = warp_tot[0];
     for (int w = 1; w < nwarps; ++w) tot = __fadd_rn(tot, warp_tot[w]);
@@ -97,64 +103,78 @@ __device__ __forceinline__ float sb_block_rms(float ssq, float* warp_tot, int di
     return __fdiv_rn(1.0f, __fsqrt_rn(var));
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, const __nv_bfloat16* __restrict__ style_prev,
                      const __nv_bfloat16* __restrict__ w_out, const __nv_bfloat16* __restrict__ b_out,
                      const __nv_bfloat16* __restrict__ w_in, const __nv_bfloat16* __restrict__ b_in,
                      const __nv_bfloat16* __restrict__ style_next, uint8_t* __restrict__ act8,
                      const float* __restrict__ d_scale, int dim, float eps) {
     extern __shared__ float sb_smem[];
-    float* a_s = sb_smem;                               // [dim] normalised row (bf16 values)
+    float* a_s = sb_smem;                               // [dim] normalised row, then the new row (bf16 values)
     float* part = a_s + dim;                            // [16][32] K-slice partials of the out-projection
-    float* nz = part + 16 * SB_ACTION;                  // [32] action row, fp32
+    float* nz = part + 16 * SB_ACTION;                  // [32] action row, rounded to bf16
     float* warp_tot = nz + SB_ACTION;                   // [32]
     __nv_bfloat16* w_s = reinterpret_cast<__nv_bfloat16*>(warp_tot + 32);   // [dim][32] out-projection weights
-    const int t = blockIdx.x, tid = threadIdx.x, col = tid * 8;
+    const int t = blockIdx.x, tid = threadIdx.x, col = tid * 8, col2 = tid * 2;
+    const bool norm_thread = col < dim;
     const size_t roff = (size_t)t * dim + col;
     pdl_launch_dependents();
     if (style_prev) {
         // the out-projection weights do not depend on the kernel in front: all 16-byte loads in flight, into shared memory
         const uint4* src = reinterpret_cast<const uint4*>(w_out);
         uint4* dst = reinterpret_cast<uint4*>(w_s);
+#pragma unroll 8
         for (int i = tid; i < dim * SB_ACTION / 8; i += blockDim.x) dst[i] = src[i];
     }
-    // so do this thread's 8 columns of the in-projection weights (32 rows), held in registers across the first half
-    uint4 wrow[SB_ACTION];
+    // so do this thread's two columns of the in-projection weights (32 rows), held in registers across the first half
+    uint32_t wrow[SB_ACTION];
     if (style_next) {
 #pragma unroll
-        for (int k = 0; k < SB_ACTION; ++k) wrow[k] = ld_global_v4(w_in + (size_t)k * dim + col);
+        for (int k = 0; k < SB_ACTION; ++k) wrow[k] = *reinterpret_cast<const uint32_t*>(w_in + (size_t)k * dim + col2);
     }
     pdl_wait();
+    uint4 nsc = make_uint4(0, 0, 0, 0), nsh = nsc;
+    if (style_next && norm_thread) {
+        nsc = ld_global_v4(style_next + col);
+        nsh = ld_global_v4(style_next + dim + col);
+    }
     if (style_prev) {
-        const uint4 rv = ld_global_v4(x + roff);
-        const uint4 sc = ld_global_v4(style_prev + col), sh = ld_global_v4(style_prev + dim + col);
-        const uint32_t* rw = &rv.x;
         float r[8], ssq = 0.0f;
+        uint4 sc = make_uint4(0, 0, 0, 0), sh = sc;
+        if (norm_thread) {
+            const uint4 rv = ld_global_v4(x + roff);
+            sc = ld_global_v4(style_prev + col);
+            sh = ld_global_v4(style_prev + dim + col);
+            const uint32_t* rw = &rv.x;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            unpack_bf16x2(rw[i], r[2 * i], r[2 * i + 1]);
-            ssq = __fmaf_rn(r[2 * i], r[2 * i], ssq);
-            ssq = __fmaf_rn(r[2 * i + 1], r[2 * i + 1], ssq);
+            for (int i = 0; i < 4; ++i) {
+                unpack_bf16x2(rw[i], r[2 * i], r[2 * i + 1]);
+                ssq = __fmaf_rn(r[2 * i], r[2 * i], ssq);
+                ssq = __fmaf_rn(r[2 * i + 1], r[2 * i + 1], ssq);
+            }
         }
+        const float old = tid < SB_ACTION ? noise[(size_t)t * SB_ACTION + tid] : 0.0f;
         const float rms = sb_block_rms(ssq, warp_tot, dim, eps);
-        const uint32_t* scw = &sc.x;
-        const uint32_t* shw = &sh.x;
+        if (norm_thread) {
+            const uint32_t* scw = &sc.x;
+            const uint32_t* shw = &sh.x;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float s0, s1, h0, h1;
-            unpack_bf16x2(scw[i], s0, s1);
-            unpack_bf16x2(shw[i], h0, h1);
-            const float n0 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i], rms), 1.0f), __fadd_rn(1.0f, s0), h0);
-            const float n1 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i + 1], rms), 1.0f), __fadd_rn(1.0f, s1), h1);
-            a_s[col + 2 * i] = bf16_round(n0);
-            a_s[col + 2 * i + 1] = bf16_round(n1);
+            for (int i = 0; i < 4; ++i) {
+                float s0, s1, h0, h1;
+                unpack_bf16x2(scw[i], s0, s1);
+                unpack_bf16x2(shw[i], h0, h1);
+                const float n0 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i], rms), 1.0f), __fadd_rn(1.0f, s0), h0);
+                const float n1 = __fmaf_rn(__fmul_rn(__fmul_rn(r[2 * i + 1], rms), 1.0f), __fadd_rn(1.0f, s1), h1);
+                a_s[col + 2 * i] = bf16_round(n0);
+                a_s[col + 2 * i + 1] = bf16_round(n1);
+            }
         }
         __syncthreads();
         // out-projection: column n, K-slices ks = k mod 16; thread (n, g) forms the slices g, g + groups, ...
         const int n = tid % SB_ACTION, g = tid / SB_ACTION, groups = blockDim.x / SB_ACTION;
         for (int ks = g; ks < 16; ks += groups) {
             float acc = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
             for (int k = ks; k < dim; k += 16) acc = fmaf(a_s[k], __bfloat162float(w_s[k * SB_ACTION + n]), acc);
             part[ks * SB_ACTION + n] = acc;
         }
@@ -164,51 +184,51 @@ step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, c
 #pragma unroll
             for (int q = 0; q < 16; ++q) s += part[q * SB_ACTION + tid];
             if (b_out) s += __bfloat162float(b_out[tid]);
-            s += noise[(size_t)t * SB_ACTION + tid];
+            s += old;
             noise[(size_t)t * SB_ACTION + tid] = s;
-            nz[tid] = s;
+            nz[tid] = bf16_round(s);
         }
     } else if (tid < SB_ACTION) {
-        nz[tid] = noise[(size_t)t * SB_ACTION + tid];
+        nz[tid] = bf16_round(noise[(size_t)t * SB_ACTION + tid]);
     }
     if (!style_next) return;
     __syncthreads();
     // in-projection: a = bf16(noise); 16 slices of two terms each, partials added in slice order, then the bias
-    float xb[8], ssq = 0.0f;
     {
-        float a[SB_ACTION];
+        float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
-        for (int k = 0; k < SB_ACTION; ++k) a[k] = bf16_round(nz[k]);
-        const uint4 bv = b_in ? ld_global_v4(b_in + col) : make_uint4(0, 0, 0, 0);
-        const uint32_t* bw = &bv.x;
-        uint4 ov;
-        uint32_t* ow = &ov.x;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float s = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const uint32_t w0 = (&wrow[q].x)[j >> 1], w1 = (&wrow[q + 16].x)[j >> 1];
-                float acc = fmaf(a[q], bf16_bits_to_f32((w0 >> ((j & 1) * 16)) & 0xffffu), 0.0f);
-                acc = fmaf(a[q + 16], bf16_bits_to_f32((w1 >> ((j & 1) * 16)) & 0xffffu), acc);
-                s += acc;
-            }
-            if (b_in) s += bf16_bits_to_f32((bw[j >> 1] >> ((j & 1) * 16)) & 0xffffu);
-            xb[j] = bf16_round(s);
+        for (int q = 0; q < 16; ++q) {
+            const float a0 = nz[q], a1 = nz[q + 16];
+            float w00, w01, w10, w11;
+            unpack_bf16x2(wrow[q], w00, w01);
+            unpack_bf16x2(wrow[q + 16], w10, w11);
+            s0 += fmaf(a1, w10, fmaf(a0, w00, 0.0f));
+            s1 += fmaf(a1, w11, fmaf(a0, w01, 0.0f));
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            ow[i] = pack_bf16x2(xb[2 * i], xb[2 * i + 1]);
-            ssq = __fmaf_rn(xb[2 * i], xb[2 * i], ssq);
-            ssq = __fmaf_rn(xb[2 * i + 1], xb[2 * i + 1], ssq);
+        if (b_in) {
+            float b0, b1;
+            unpack_bf16x2(*reinterpret_cast<const uint32_t*>(b_in + col2), b0, b1);
+            s0 += b0;
+            s1 += b1;
         }
-        st_global_v4(x + roff, ov);
+        a_s[col2] = bf16_round(s0);
+        a_s[col2 + 1] = bf16_round(s1);
+        *reinterpret_cast<uint32_t*>(x + (size_t)t * dim + col2) = pack_bf16x2(s0, s1);
+    }
+    __syncthreads();
+    float xb[8], ssq = 0.0f;
+    if (norm_thread) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            xb[i] = a_s[col + i];
+            ssq = __fmaf_rn(xb[i], xb[i], ssq);
+        }
     }
     const float rms = sb_block_rms(ssq, warp_tot, dim, eps);
+    if (!norm_thread) return;
     const float inv_scale = __fdiv_rn(1.0f, *d_scale);
-    const uint4 sc = ld_global_v4(style_next + col), sh = ld_global_v4(style_next + dim + col);
-    const uint32_t* scw = &sc.x;
-    const uint32_t* shw = &sh.x;
+    const uint32_t* scw = &nsc.x;
+    const uint32_t* shw = &nsh.x;
     float v[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -280,7 +300,7 @@ int frt_b200_step_boundary(void* x, float* noise, const void* style_prev, const 
     if (rows == 0) return FRT_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows);
-    cfg.blockDim = dim3(dim / 8);
+    cfg.blockDim = dim3(dim / 2);
     const size_t smem = (size_t)(dim + 16 * SB_ACTION + 2 * SB_ACTION) * sizeof(float) + (size_t)dim * SB_ACTION * 2;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
