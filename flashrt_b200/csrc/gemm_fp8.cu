@@ -1123,7 +1123,10 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
     return dispatch_small_m<EPI_ROPE_SPLIT>(A, W, p, K, M, (p.N + 127) / 128, splits, flags & 1, (cudaStream_t)stream);
 }
 
-// gate|up projection with the GeGLU -> FP8 epilogue fused (M <= 256):
+// gate|up projection with the GeGLU -> FP8 epilogue fused (M <= 256, or any M when half % 128 == 0; larger M runs on CTA pairs
+// whose 256 columns are 128 gate and 128 up features: the activation, 30 instructions per value, runs under the MMAs of the
+// next tile instead of in a pass of its own over 2 x M x 2 half bytes -- 768 x 32768 x 2048: 41 + 26 us as two launches, 54 as
+// one):
 //   W (2*half, K): rows [0, half) = gate, [half, 2*half) = up.  out8 (M, half) =
 //   e4m3(clamp(gelu_tanh(bf16(gate)) * bf16(up) * (1 / *d_out_scale), +-448)).  half % 64 == 0.
 // Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_geglu_fp8.  flags bit 6: SiLU gate instead of GELU
@@ -1132,7 +1135,9 @@ int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int
                                    const float* d_scale_a, const float* d_scale_b, const float* d_out_scale,
                                    int splits, int flags, void* stream) {
     if (!A || !W || !out8 || !d_out_scale || M < 0 || half <= 0 || K <= 0) return FRT_ERR_INVALID;
-    if ((K % 16) || M > 256 || (half % 64)) return FRT_ERR_UNSUPPORTED;
+    if ((K % 16) || (half % 64)) return FRT_ERR_UNSUPPORTED;
+    if (M > 256 && ((half % 128) || (reinterpret_cast<uintptr_t>(out8) & 15) || (flags & (16 | 64 | 128))))
+        return FRT_ERR_UNSUPPORTED;
     if (M == 0) return FRT_OK;
     GemmParams p = {};
     p.sa = d_scale_a;
@@ -1145,6 +1150,7 @@ int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int
     p.out_scale = d_out_scale;
     p.half = half;
     // SiLU gate (bit 6) and the hardware-tanh GELU (bit 7): built in the token-major kernel only
+    if (M > 256) return launch_gemm_pair<256, EPI_P_GEGLU_FP8>(A, W, p, K, (cudaStream_t)stream);
     const bool silu = (flags & 64) != 0, fast = (flags & 128) != 0;
     if (silu && fast) return FRT_ERR_INVALID;
     if ((silu || fast) && !(tok_eligible(M, p.N, K, flags) && M <= 128)) return FRT_ERR_UNSUPPORTED;

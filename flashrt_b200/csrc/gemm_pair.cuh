@@ -16,7 +16,7 @@
 //   * the leader's MMA thread waits for full[s], issues four MMAs (K = 32 each) and commits to empty[s] of both CTAs,
 //     likewise for acc_full[buf];
 //   * eight epilogue warps per CTA drain that CTA's accumulator and arrive on the leader's acc_empty[buf]
-//     (512 arrivals), which the leader's MMA thread waits for before it reuses the buffer.
+//     (one arrival per epilogue thread of both), which the leader's MMA thread waits for before it reuses the buffer.
 // Tensor memory is allocated and freed with the cta_group::2 forms by the same warp of both CTAs.  Every wait is
 // bounded by the kernel deadline; the CTAs meet at a cluster barrier before either leaves.
 #pragma once
@@ -30,8 +30,11 @@ struct GemmPairCfg {
     static constexpr int EPI_STAGE_BYTES = 8 * 32 * 128;    // line staging of the eight epilogue warps
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;             // two accumulators
-    static constexpr int EPI_THREADS = 256;
 };
+// epilogue threads per CTA: the GeGLU finish is a chain of 30 dependent instructions per value, which sixteen warps hide
+// where eight do not
+template <int EPI>
+constexpr int pair_epi_threads() { return EPI == EPI_P_GEGLU_FP8 ? 512 : 256; }
 
 namespace tc {
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {   // same warp of both CTAs
@@ -77,8 +80,9 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }  // namespace tc
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(64 + pair_epi_threads<EPI>(), 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmParams p) {
+    static_assert(EPI != EPI_P_GEGLU_FP8 || BN == 256, "GeGLU: 128 gate and 128 up columns");
     using Cfg = GemmPairCfg<BN>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -86,7 +90,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);   // used in the leader only
     uint64_t* empty = full + STAGES;          // one per CTA: the leader's commits arrive on both
     uint64_t* acc_full = empty + STAGES;      // [2] one per CTA
-    uint64_t* acc_empty = acc_full + 2;       // [2] used in the leader only: 512 arrivals
+    uint64_t* acc_empty = acc_full + 2;       // [2] used in the leader only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -108,7 +112,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&acc_full[i], 1);
-            tc::mbar_init(&acc_empty[i], 2 * Cfg::EPI_THREADS);
+            tc::mbar_init(&acc_empty[i], 2 * pair_epi_threads<EPI>());
         }
         *abort_flag = 0;
         tc::mbar_fence_init();
@@ -137,7 +141,9 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         for (int t = pair; t < total; t += npairs) {
             int mt, nt;
             order.at(t, mt, nt);
-            const int m0 = mt * 256 + (int)rank * 128, n0 = nt * BN + (int)rank * (BN / 2);
+            const int m0 = mt * 256 + (int)rank * 128;
+            // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
+            const int n0 = EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
             for (int kb = 0; kb < kbt; ++kb) {
                 if (!tc::warp_wait(empty_a + 8 * s, ph, ready, deadline, abort_flag)) {
                     if (lane == 0 && !*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
@@ -201,7 +207,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         // ---------------- epilogue (both CTAs): this CTA's 128 rows x 256 columns
         pdl_wait();
         const int q = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int half = (warp - 2) >> 2;                 // column half (GeGLU: quarter) of this warp
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         float alpha = p.alpha_host;
         if (p.sa) alpha *= *p.sa;
@@ -221,8 +227,14 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             tc::tc_fence_after_sync();
             int mt, nt;
             order.at(t, mt, nt);
-            epilogue_rows<EPI, BN / 2>(p, tmem + buf * BN + half * (BN / 2) + lane_off, mt * 256 + (int)rank * 128 + q * 32,
-                                       nt * BN + half * (BN / 2), stg, lines, alpha, inv_os);
+            const uint32_t t_acc = tmem + buf * BN + lane_off;
+            const int m_base = mt * 256 + (int)rank * 128 + q * 32;
+            if constexpr (EPI == EPI_P_GEGLU_FP8)
+                epilogue_geglu_rows(p, t_acc + half * 32, t_acc + BN / 2 + half * 32, m_base, nt * (BN / 2) + half * 32, alpha,
+                                    inv_os);
+            else
+                epilogue_rows<EPI, BN / 2>(p, t_acc + half * (BN / 2), m_base, nt * BN + half * (BN / 2), stg, lines, alpha,
+                                           inv_os);
             tc::tc_fence_before_sync();
             tc::mbar_arrive_cluster(tc::dsmem_map(tc::smem_u32(&acc_empty[buf]), 0));
         }
@@ -255,7 +267,7 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
     const int pairs = total < sms / 2 ? total : sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(320);
+    cfg.blockDim = dim3(64 + pair_epi_threads<EPI>());
     cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];

@@ -15,7 +15,8 @@
 
 // EPI_P_BIAS_GELU_FAST_FP8: the same epilogue with the GELU through the hardware tanh -- a template value, not a run-time
 // flag: a select inside the unrolled loop over a thread's values costs as much as the arithmetic it chooses between
-enum { EPI_P_BF16 = 0, EPI_P_BIAS_GELU_FP8 = 1, EPI_P_BIAS_GELU_FAST_FP8 = 2 };
+// EPI_P_GEGLU_FP8 (CTA pairs only): the tile's columns are 128 gate features and the 128 up features that belong to them.
+enum { EPI_P_BF16 = 0, EPI_P_BIAS_GELU_FP8 = 1, EPI_P_BIAS_GELU_FAST_FP8 = 2, EPI_P_GEGLU_FP8 = 3 };
 
 // tanh-form GELU with explicitly rounded fp32 operations, the same sequence as bias_gelu_fp8_kernel
 // (csrc/quantize/bias_gelu_quantize_fp8.cu:24-49 in the reference)
@@ -218,6 +219,33 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_sr
         __syncwarp();
     }
 }
+
+// The same for 32 gate columns (t_gate) and their 32 up columns (t_up): e4m3(gelu_tanh(bf16(gate)) * bf16(up) / scale) at
+// features h0 .. h0 + 31 of out8 (M, half), the rounding points of GEMM -> geglu_fp8.  A thread's 32 bytes are one sector.
+__device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_t t_gate, uint32_t t_up, int m_base, int h0,
+                                                    float alpha, float inv_os) {
+    uint32_t g[32], u[32], w[8];
+    tc::tmem_ld32(t_gate, g);
+    tc::tmem_ld32(t_up, u);
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        float o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float gt = bf16_round(__uint_as_float(g[j + e]) * alpha), up = bf16_round(__uint_as_float(u[j + e]) * alpha);
+            o[e] = clamp448(__fmul_rn(__fmul_rn(det_gelu_tanh(gt), up), inv_os));
+        }
+        w[j / 4] = f32x4_to_e4m3x4(o[0], o[1], o[2], o[3]);
+    }
+    const int m = m_base + (threadIdx.x & 31);
+    if (m < p.M) {
+        uint8_t* dst = p.out8 + (size_t)m * p.half + h0;
+        st_global_v4(dst, make_uint4(w[0], w[1], w[2], w[3]));
+        st_global_v4(dst + 16, make_uint4(w[4], w[5], w[6], w[7]));
+    }
+}
+
 // whole-line stores are possible: 16-byte rows and bias
 template <int EPI>
 __device__ __forceinline__ bool epilogue_lines(const GemmParams& p) {

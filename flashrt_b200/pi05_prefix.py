@@ -159,12 +159,16 @@ class Pi05PrefixEncoderB200:
                              out_fp8=self.attn8.data_ptr(), out_scale=self._sp(i, "o"))
             self._gemm(self.attn8, self.w_o[i], self.ws_o_t[i], self.xn, seq, ENC_D, ENC_NH * ENC_HD, self._sp(i, "o"), st)
             self._norm(seq, self.xn, i, "gu", st, calibrate)
-            self._gemm(self.act8, self.w_gu[i], self.ws_gu_t[i], self.merged, seq, 2 * ENC_H, ENC_D, self._sp(i, "gu"), st)
+            if calibrate or seq <= 256:
+                self._gemm(self.act8, self.w_gu[i], self.ws_gu_t[i], self.merged, seq, 2 * ENC_H, ENC_D, self._sp(i, "gu"), st)
             if calibrate:
                 fvk.gate_geglu_merged(self.merged.data_ptr(), self.hidden.data_ptr(), seq, ENC_H, st)
                 self._dyn_quant(self.hidden[:seq], self.hid8[:seq], i, "d", st)
-            else:
+            elif seq <= 256:
                 fvk.gate_geglu_merged_fp8(self.merged.data_ptr(), self.hid8.data_ptr(), seq, ENC_H, self._sp(i, "d"), st)
+            else:               # one launch: the activation under the product's MMAs
+                self.gemm.fp8_nt_dev_geglu_fp8(self.act8.data_ptr(), self.w_gu[i].data_ptr(), self.hid8.data_ptr(), seq, ENC_H,
+                                               ENC_D, self._sp(i, "gu"), self.ws_gu_t[i].data_ptr(), self._sp(i, "d"), st)
             self._gemm(self.hid8, self.w_d[i], self.ws_d_t[i], self.xn, seq, ENC_D, ENC_H, self._sp(i, "d"), st)
 
     # ------------------------------------------------------------------

@@ -140,7 +140,8 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
                                     int flags, void* stream);
 /* gate|up projection + gate_geglu_merged_fp8 (csrc/bindings.cpp:1037-1044 -> csrc/kernels/activation.cu:249-279):
  *   W (2*half, K), rows [0, half) = gate, [half, 2*half) = up; out8 (M, half) e4m3 with scale *d_out_scale.
- *   half % 64 == 0.  Byte-identical to frt_b200_gemm_fp8_nt (same `splits`) followed by frt_b200_geglu_fp8.
+ *   half % 64 == 0; M > 256: half % 128 == 0, out8 16-byte aligned.  Byte-identical to frt_b200_gemm_fp8_nt (same `splits`)
+ *   followed by frt_b200_geglu_fp8.
  *   flags bit 6: SiLU gate (SwiGLU; M <= 128 and K % 128 == 0 only, else -2), byte-identical to frt_b200_geglu_fp8
  *   with its flags bit 1 behind the same GEMM.
  *   flags bit 7 (here and in the _rowscale / norm_gemm forms): GELU(tanh) through the hardware tanh (tanh.approx.f32,

@@ -112,3 +112,21 @@ def test_nvfp4_column_tiles(M, N, K):
 
     a, w = make(M), make(N)
     assert np.array_equal(_run_gemm(*a, *w, M, N, K, alpha=0.125), O.gemm_nvfp4(*a, *w, alpha=0.125))
+
+
+@pytest.mark.parametrize("M,half,K", [(257, 128, 256), (300, 384, 1024), (768, 2048, 128), (2000, 1280, 512)])
+def test_geglu_projection_of_many_rows(M, half, K):
+    """M > 256: the pair kernel's GeGLU epilogue gives the bytes of product -> geglu_fp8, ragged rows included."""
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, f32, zeros
+    rng = np.random.default_rng(M + half)
+    A, sa = _fp8_operand(rng, M, K, 1.0)
+    W, sb = _fp8_operand(rng, 2 * half, K, 0.05)
+    d_A, d_W, d_sa, d_sb, d_so = Dev(A), Dev(W), f32(sa), f32(sb), f32(0.004)
+    merged, two, one = zeros((M, 2 * half), np.uint16), zeros((M, half), np.uint8), Dev(np.full((M + 1, half), 0x5A, np.uint8))
+    g = fvk.GemmRunner()
+    g.fp8_nt_dev(d_A.ptr, d_W.ptr, merged.ptr, M, 2 * half, K, d_sa.ptr, d_sb.ptr)
+    fvk.gate_geglu_merged_fp8(merged.ptr, two.ptr, M, half, d_so.ptr, 0)
+    g.fp8_nt_dev_geglu_fp8(d_A.ptr, d_W.ptr, one.ptr, M, half, K, d_sa.ptr, d_sb.ptr, d_so.ptr)
+    assert fvk.tensor_core_status() == 0
+    assert np.array_equal(one.get()[:M], two.get()) and (one.get()[M] == 0x5A).all() and (two.get() != 0).mean() > 0.5
