@@ -46,7 +46,8 @@ class VLAModel:
         fe = self._fe
         if encoder.layers != fe.layers:
             raise ValueError(f"encoder has {encoder.layers} layers, the action expert {fe.layers}")
-        seq = encoder.encode(embeds, fe.k_cache[:, slot], fe.v_cache[:, slot])
+        seq = encoder.enqueue(embeds, fe.k_cache[:, slot], fe.v_cache[:, slot], after=fe.stream)
+        fe.stream.wait_stream(encoder.stream)
         if seq != fe.prefix_len and not getattr(fe, "fixed_shape", False):
             raise ValueError(f"prefix of {seq} tokens, model built for {fe.prefix_len} (use fixed_shape=True)")
         if getattr(fe, "fixed_shape", False):

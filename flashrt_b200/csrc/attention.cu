@@ -747,7 +747,7 @@ int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, voi
     p.Hkv = num_heads_kv;
     p.G = G;
     p.scale_log2 = softmax_scale * 1.4426950408889634f;
-    p.kv_static_rows = kv_static_rows;
+    p.kv_static_rows = kv_static_rows < 0 && !seqused_k ? 0 : kv_static_rows;
     p.flags = flags;
     if (o_accum && lse_accum && counters) {
         p.o_accum = o_accum;

@@ -262,9 +262,9 @@ class StepIO:
         common = (fe.batch, S, T, DEC_NH, DEC_NKV, DEC_HD, qs, ks, ks, qs, 1.0 / math.sqrt(DEC_HD), fe.sm_count, stream)
         q, k, v, o = (self.q.data_ptr(), fe.k_cache[layer].data_ptr(), fe.v_cache[layer].data_ptr(),
                       self.attn.data_ptr())
-        if fe.fixed_shape:      # keys beyond *dec_seqused are masked; nothing may be fetched before the producer ends
+        if fe.fixed_shape:      # keys beyond *dec_seqused are masked; only its last S rows are new
             fa2.fwd_bf16_seqused_splitkv(q, k, v, o, 0, fe.dec_seqused.data_ptr(), self.lse_accum.data_ptr(),
-                                         self.o_accum.data_ptr(), *common, kv_static_rows=0, **kw)
+                                         self.o_accum.data_ptr(), *common, kv_static_rows=-S, **kw)
         else:
             fa2.fwd_bf16(q, k, v, o, 0, self.lse_accum.data_ptr(), self.o_accum.data_ptr(), *common,
                          kv_static_rows=fe.prefix_len, **kw)
@@ -715,6 +715,7 @@ class Pi05DecoderB200:
         for n in ("action_in_w", "action_in_b", "action_out_w", "action_out_b"):
             setattr(self, n, getattr(self, n).contiguous().to(dev))
         self.rope = rope_table(prefix_len, chunk_size).to(dev)
+        self._rope_all = None
         self.dec_devpos = torch.full((1,), prefix_len, dtype=torch.int32, device=dev)
         self.dec_seqused = torch.full((1,), prefix_len + chunk_size, dtype=torch.int32, device=dev)
         # one cache per batch element: (layers, batch, prefix + chunk, 256)
@@ -746,9 +747,11 @@ class Pi05DecoderB200:
         if prefix_k.dim() == 3:
             prefix_k, prefix_v = (t.unsqueeze(1).expand(-1, self.batch, -1, -1) for t in (prefix_k, prefix_v))
         assert prefix_k.shape == (self.layers, self.batch, self.prefix_len, DEC_NKV * DEC_HD), prefix_k.shape
+        here = torch.cuda.current_stream(self.device)
+        here.wait_stream(self.stream)             # a loop in flight still reads the cache
         self.k_cache[:, :, :self.prefix_len].copy_(prefix_k.to(BF16))
         self.v_cache[:, :, :self.prefix_len].copy_(prefix_v.to(BF16))
-        torch.cuda.synchronize(self.device)
+        self.stream.wait_stream(here)
 
     def set_valid_prefix_len(self, valid: int) -> None:
         """Fixed-shape mode: the first ``valid`` rows of the prefix are real, the rest padding.  Updates the three
@@ -760,10 +763,15 @@ class Pi05DecoderB200:
         if not 0 <= valid <= self.prefix_len:
             raise ValueError(f"valid prefix length {valid} outside [0, {self.prefix_len}]")
         self.valid_prefix_len = int(valid)
-        self.dec_devpos.fill_(valid)
-        self.dec_seqused.fill_(valid + self.chunk_size)
-        self.rope.copy_(rope_table(valid, self.chunk_size).to(self.device))
-        torch.cuda.synchronize(self.device)
+        if self._rope_all is None:      # every position's row, laid out once
+            self._rope_all = rope_table(0, self.prefix_len + self.chunk_size).to(self.device)
+        here = torch.cuda.current_stream(self.device)
+        self.stream.wait_stream(here)
+        with torch.cuda.stream(self.stream):      # in order with the loop; nothing waits on the host
+            self.dec_devpos.fill_(valid)
+            self.dec_seqused.fill_(valid + self.chunk_size)
+            self.rope.copy_(self._rope_all[valid:valid + self.chunk_size])
+        here.wait_stream(self.stream)
 
     def set_prefix_pair(self, cond_k, cond_v, uncond_k, uncond_v) -> None:
         """Conditioned / unconditioned prefixes of the classifier-free-guidance pair

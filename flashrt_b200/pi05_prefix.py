@@ -204,11 +204,22 @@ class Pi05PrefixEncoderB200:
     def encode(self, embeds: torch.Tensor, k_out: torch.Tensor, v_out: torch.Tensor) -> int:
         """embeds (seq, 2048) -> rows [0, seq) of k_out[i], v_out[i] for every layer (K with its RoPE, in the
         interleaved feature order the decoder's Q uses).  Returns seq."""
+        seq = self.enqueue(embeds, k_out, v_out)
+        self.stream.synchronize()
+        return seq
+
+    def enqueue(self, embeds: torch.Tensor, k_out: torch.Tensor, v_out: torch.Tensor, after=None) -> int:
+        """``encode`` without the wait on the host: the work goes to ``self.stream``, behind the current stream (and the
+        stream ``after``), and the current stream waits for it."""
         if not self.calibrated:
             raise RuntimeError("calibrate() first: the encoder runs with static activation scales")
         seq = self._check(embeds, k_out, v_out)
+        here = torch.cuda.current_stream(self.device)
+        self.stream.wait_stream(here)
+        if after is not None:
+            self.stream.wait_stream(after)
         with torch.cuda.stream(self.stream):
             self.x[:seq].copy_(embeds.to(self.device, BF16), non_blocking=True)
             self.transformer_encoder(seq, k_out, v_out, self.stream.cuda_stream, False)
-        self.stream.synchronize()
+        here.wait_stream(self.stream)
         return seq

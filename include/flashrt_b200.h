@@ -168,6 +168,7 @@ int frt_b200_gemm_status(int reset);
  *   kv_splits: 0 = choose, else 1..8, rounded down to a power of two (combined inside a thread-block cluster;
  *   no scratch buffers).  kv_static_rows: leading K/V rows that the previous kernel in the stream does not
  *   write (with flags bit0 they are fetched before that kernel has finished); pass 0 if unsure.
+ *   With seqused_k, -n: all valid rows but the last n, and *seqused_k is not written by that kernel either.
  *   o_accum, lse_accum, counters: optional split-KV scratch (all three or none): o_accum (splits, batch,
  *   num_heads_q, seqlen_q, head_dim) fp32 and lse_accum (splits, batch, num_heads_q, seqlen_q) fp32 -- the
  *   reference's FA2 split-kv buffers -- and counters = 2 unsigned per (128-row tile, kv head, batch), zeroed once
