@@ -901,26 +901,36 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
         if (!(p.flags & 16)) {
             place(splits, 4);
         } else {
-            // kv_splits is a bound: the cheapest split that fits, by the times of the captured action-expert loop (10-64
-            // queries x 8 heads, 100-1088 keys, batch 1-4; units of 0.1 us): 1.6 us per chunk of a split's chain, 1.7
-            // more when a CTA moves out 128 columns of O instead of 64, and for the combine through the scratch
-            // 2.3 more in four parts, 6.0 in one.  (2 x 50 x 768 + 50 keys: 4 splits of 4 parts 12.3 -> 9.8 us.)
-            const long long one = (long long)tiles * groups * splits;
-            int best = 16 * ((p.chunks_total + splits - 1) / splits) + (one * 4 <= sms && splits <= 8 ? 23 : 60);
-            if (one > sms) best = 1 << 30;                  // does not fit as scratch
-            int bc = 0, bp = 0;
+            // kv_splits is a bound: the cheapest form that fits, by the times of the captured action-expert loop (10-64 queries
+            // x 8 heads, 100-1088 keys, batch 1-4) and of the prefix encoder's launches (96-1024 x 8 heads on themselves), in
+            // units of 0.1 us over the cluster exchange in four parts: 1.6 us per chunk of a split's chain, 1.7 more when a
+            // CTA moves out 128 columns of O; one CTA per (tile, split) 1.9 per chunk and 1 without a combine, 4.5 with one
+            // through the scratch; 2.3 for the scratch in four parts.  (2 x 50 on 818 keys: 4 splits of 4 parts
+            // 12.3 -> 9.8 us; 768 on 768: 2 splits through the scratch 23.3 -> 18.6.)
+            const long long ctas1 = (long long)tiles * groups;
+            auto chain = [&](int c) { return (p.chunks_total + c - 1) / c; };
+            int best = 19 * p.chunks_total + 10, bc = 1, bp = 0;                 // bp: 0 = not a cluster
             for (int c = 8; c >= 2; c >>= 1) {
                 if (c > bound || c / 2 >= p.chunks_total) continue;
                 for (int parts = 4; parts >= 2; parts -= 2) {
-                    const int cost = 16 * ((p.chunks_total + c - 1) / c) + (parts == 2 ? 17 : 0);
+                    const int cost = 16 * chain(c) + (parts == 2 ? 17 : 0);
                     if (cost < best && (fits(c, parts, false) || (parts == 4 && tail && fits(c, 4, true)))) {
                         best = cost;
                         bc = c;
                         bp = parts;
                     }
                 }
+                if (ctas1 * c > sms) continue;
+                const int cost = ctas1 * c * 4 <= sms ? 16 * chain(c) + 23 : 19 * chain(c) + 45;
+                if (cost < best) {
+                    best = cost;
+                    bc = c;
+                    bp = 0;
+                }
             }
-            if (bc) place(bc, bp);
+            if (bp) place(bc, bp);
+            splits = bc;
+            if (bc == 1) p.o_accum = nullptr;
         }
     }
     if (p.o_accum && !xc) {

@@ -31,6 +31,7 @@ from .weight_loader import (DictSource, FlatCat, FoldNorm, FusedGateUp, FusedQKV
 ENC_D, ENC_H, ENC_NH, ENC_NKV, ENC_HD, ENC_L = 2048, 16384, 8, 1, 256, 18
 QKV_N = (ENC_NH + 2 * ENC_NKV) * ENC_HD
 BF16 = torch.bfloat16
+ATTN_SPLITS = 4             # most key splits of the encoder's attention
 SITES = ("qkv", "o", "gu", "d")
 EP = "paligemma_with_expert.paligemma.model.language_model.layers.{i}"
 
@@ -108,6 +109,10 @@ class Pi05PrefixEncoderB200:
         self.hid8 = z(S, ENC_H, dtype=torch.uint8)
         self.ones = torch.ones(ENC_D, dtype=BF16, device=dev)
         self.rope = rope_rows(S).to(dev)
+        # scratch of the attention's key splits (the split is chosen by the prefix length)
+        self.o_accum = torch.empty(ATTN_SPLITS, ENC_NH, S, ENC_HD, dtype=torch.float32, device=dev)
+        self.lse_accum = torch.empty(ATTN_SPLITS, ENC_NH, S, dtype=torch.float32, device=dev)
+        self.attn_counters = z(2 * ((S * ENC_NH + 127) // 128), dtype=torch.int32)
         self.act_scale = torch.ones(layers, len(SITES), dtype=torch.float32, device=dev)
         self.scratch_scale = torch.zeros(1, dtype=torch.float32, device=dev)
         self.gemm = fvk.GemmRunner()
@@ -154,8 +159,10 @@ class Pi05PrefixEncoderB200:
                              1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs, ks, ks, qs, 1.0 / math.sqrt(ENC_HD), 0, st)
                 self._dyn_quant(self.attn[:seq], self.attn8[:seq], i, "o", st)
             else:
-                fa2.fwd_bf16(self.q.data_ptr(), k_out[i].data_ptr(), v_out[i].data_ptr(), self.attn.data_ptr(), 0, 0, 0,
-                             1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs, ks, ks, qs, 1.0 / math.sqrt(ENC_HD), 0, st,
+                fa2.fwd_bf16(self.q.data_ptr(), k_out[i].data_ptr(), v_out[i].data_ptr(), self.attn.data_ptr(), 0,
+                             self.lse_accum.data_ptr(), self.o_accum.data_ptr(), 1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs,
+                             ks, ks, qs, 1.0 / math.sqrt(ENC_HD), 0, st, kv_splits=ATTN_SPLITS, flags=16,
+                             counters=self.attn_counters.data_ptr(),
                              out_fp8=self.attn8.data_ptr(), out_scale=self._sp(i, "o"))
             self._gemm(self.attn8, self.w_o[i], self.ws_o_t[i], self.xn, seq, ENC_D, ENC_NH * ENC_HD, self._sp(i, "o"), st)
             self._norm(seq, self.xn, i, "gu", st, calibrate)

@@ -181,7 +181,8 @@ int frt_b200_gemm_status(int reset);
  *   (b) through the scratch, published with an arrival counter per tile.  (a) and (b) give the same bits.
  *   flags: bit 0 = programmatic dependent launch; bit 1 = keep the single-tile kernel; head_dim 256 with scratch:
  *   bit 2 = one CTA per (tile, split) instead of four head-dim parts, bit 3 = always (b), bit 4 = kv_splits (> 0) is an upper
- *   bound: the number of splits (2, 4 or 8, one of them possibly without keys) and of parts (4 or 2) is chosen by size. */
+ *   bound: the number of splits (1, 2, 4 or 8, one of them possibly without keys) and the form of the combine are chosen by
+ *   size; no size is refused. */
 int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, void* O, void* O_fp8,
                                 const float* out_scale, float* lse, const int* seqused_k, int batch, int seqlen_q,
                                 int seqlen_k, int num_heads_q, int num_heads_kv, int head_dim,

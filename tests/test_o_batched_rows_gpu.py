@@ -66,7 +66,8 @@ def test_projections_of_a_batch(batch, S, half):
 
 @pytest.mark.parametrize("B,Sq,Skv,extra", [(1, 20, 170, {}), (1, 60, 828, {}), (2, 50, 818, dict(fused_fp8=True)),
                                             (4, 50, 818, {}), (3, 24, 792, dict(seqused=70)), (1, 16, 64, {}),
-                                            (4, 64, 150, {})])
+                                            (4, 64, 150, {}), (1, 300, 300, {}), (1, 541, 541, dict(fused_fp8=True)),
+                                            (1, 768, 768, {}), (1, 1040, 200, {})])
 def test_attention_split_chosen_by_size(B, Sq, Skv, extra):
     """flags bit 4: a bound on the splits; whatever split and number of parts is chosen matches the oracle."""
     _run(B, Sq, Skv, 8, 1, 256, 8, seed=B + Sq, scratch=True, flags=16, **extra)
@@ -130,3 +131,22 @@ def test_geglu_projection_of_many_rows(M, half, K):
     g.fp8_nt_dev_geglu_fp8(d_A.ptr, d_W.ptr, one.ptr, M, half, K, d_sa.ptr, d_sb.ptr, d_so.ptr)
     assert fvk.tensor_core_status() == 0
     assert np.array_equal(one.get()[:M], two.get()) and (one.get()[M] == 0x5A).all() and (two.get() != 0).mean() > 0.5
+
+
+@pytest.mark.parametrize("used", [1, 65, 333, 818])
+def test_attention_length_read_early(used):
+    """kv_static_rows = -n: the splits share the chunks that hold keys; same bound against the oracle."""
+    from flashrt_b200 import flash_rt_fa2 as fa2
+    from gpu_util import Dev, rand_bf16, zeros
+    rng = np.random.default_rng(used)
+    S, T, H, D = 50, 818, 8, 256
+    q, k, v = rand_bf16(rng, (1, S, H, D)), rand_bf16(rng, (1, T, 1, D)), rand_bf16(rng, (1, T, 1, D))
+    d_q, d_k, d_v, d_o, d_u = Dev(q), Dev(k), Dev(v), zeros((1, S, H, D), np.uint16), Dev(np.array([used], np.int32))
+    acc, lse, cnt = zeros((8, 1, H, S, D), np.float32), zeros((8, 1, H, S), np.float32), zeros((16,), np.int32)
+    qs, ks = (S * H * D, H * D, D), (T * D, D, D)
+    fa2.fwd_bf16_seqused_splitkv(d_q.ptr, d_k.ptr, d_v.ptr, d_o.ptr, 0, d_u.ptr, lse.ptr, acc.ptr, 1, S, T, H, 1, D, qs, ks,
+                                 ks, qs, 1.0 / 16.0, 148, 0, kv_splits=8, counters=cnt.ptr, kv_static_rows=-S, pdl=True)
+    ref, _ = O.attention(q, k, v, 1.0 / 16.0, used)
+    got = O.bf16_bits_to_f32(d_o.get())
+    assert fa2.attention_status() == 0
+    assert (np.abs(got - ref) <= 2e-2 * np.sqrt((ref.astype(np.float64) ** 2).mean()) + np.abs(ref) * 2.0 ** -8).all()
