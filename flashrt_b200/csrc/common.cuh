@@ -208,6 +208,8 @@ __device__ __forceinline__ void st_global_v2(void* p, uint2 v) {
 // drains, about 1 us per launch.  Behind a kernel that never calls launch_dependents the attribute changes nothing.  The
 // caller's flag says more: weights, styles and scales do not come from the kernel in front and may be read before the wait
 // (`early`).
+// Inputs that the kernel in front may have written are no `const __restrict__` parameters: loads from such are invariant to
+// the compiler, which may then issue them above the wait.
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -52,8 +52,8 @@ static int launch(K kernel, unsigned grid, unsigned block, cudaStream_t stream, 
 // merged row = [gate(0..H) | up(H..2H)] bf16; out (rows, H) fp8.
 template <int ACT>
 __global__ void __launch_bounds__(256)
-geglu_fp8_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict__ out, int rows, int H,
-                 const float* __restrict__ d_scale) {
+geglu_fp8_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ out, int rows, int H,
+                 const float* d_scale) {
     pdl_launch_dependents();
     pdl_wait();
     const float inv_scale = __fdiv_rn(1.0f, *d_scale);
@@ -87,7 +87,7 @@ geglu_fp8_kernel(const __nv_bfloat16* __restrict__ merged, uint8_t* __restrict__
 // merged -> bf16 (non-quantised sibling, reference gate_geglu_merged)
 template <int ACT>
 __global__ void __launch_bounds__(256)
-geglu_bf16_kernel(const __nv_bfloat16* __restrict__ merged, __nv_bfloat16* __restrict__ out, int rows, int H) {
+geglu_bf16_kernel(const __nv_bfloat16* merged, __nv_bfloat16* __restrict__ out, int rows, int H) {
     pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = H >> 3;
@@ -116,8 +116,8 @@ geglu_bf16_kernel(const __nv_bfloat16* __restrict__ merged, __nv_bfloat16* __res
 
 // ------------------------------------------------------------------ bf16 -> FP8, given scale
 __global__ void __launch_bounds__(256)
-quantize_fp8_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict__ out, long long n,
-                    const float* __restrict__ d_scale) {
+quantize_fp8_kernel(const __nv_bfloat16* in, uint8_t* __restrict__ out, long long n,
+                    const float* d_scale) {
     pdl_launch_dependents();
     pdl_wait();
     const float inv_scale = __fdiv_rn(1.0f, *d_scale);
@@ -149,7 +149,7 @@ quantize_fp8_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict__ 
 
 // absmax into *d_amax (float, non-negative: ordered as int)
 __global__ void __launch_bounds__(256)
-absmax_kernel(const __nv_bfloat16* __restrict__ in, long long n, float* d_amax) {
+absmax_kernel(const __nv_bfloat16* in, long long n, float* d_amax) {
     float m = 0.0f;
     const long long nvec = n >> 3;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
@@ -183,8 +183,8 @@ __global__ void accumulate_scale_max_kernel(const float* src, float* dst) {
 // MODE 0: res += x            MODE 1: res += x + bias[col]      MODE 2: res += x * gate
 template <int MODE>
 __global__ void __launch_bounds__(256)
-add_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
-           const __nv_bfloat16* __restrict__ aux, long long aux_stride, long long rows, int dim) {
+add_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* x,
+           const __nv_bfloat16* aux, long long aux_stride, long long rows, int dim) {
     pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = dim >> 3;
@@ -231,9 +231,9 @@ add_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
 // Q goes to (seq, q_dim); K and V rows land at row (pos + t) of their caches,
 // pos = *devpos when devpos is given, else 0 (the caller pre-offsets K/V).
 __global__ void __launch_bounds__(256)
-qkv_split_rope_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ rope,
+qkv_split_rope_kernel(const __nv_bfloat16* qkv, const __nv_bfloat16* rope,
                       __nv_bfloat16* __restrict__ Q, __nv_bfloat16* __restrict__ K,
-                      __nv_bfloat16* __restrict__ V, const int* __restrict__ devpos, int seq, int q_dim,
+                      __nv_bfloat16* __restrict__ V, const int* devpos, int seq, int q_dim,
                       int k_dim, int v_dim, int head_dim) {
     pdl_launch_dependents();
     pdl_wait();
@@ -276,7 +276,7 @@ qkv_split_rope_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16
 // residual[i] += v_uncond[i] + beta * (v_cond[i] - v_uncond[i])   (one fma for the guided velocity, one add)
 template <typename T>
 __global__ void __launch_bounds__(256)
-cfg_combine_kernel(T* __restrict__ residual, const T* __restrict__ v_cond, const T* __restrict__ v_uncond,
+cfg_combine_kernel(T* __restrict__ residual, const T* v_cond, const T* v_uncond,
                    float beta, long long n) {
     pdl_launch_dependents();
     pdl_wait();

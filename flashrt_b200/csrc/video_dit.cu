@@ -48,10 +48,10 @@ __device__ __forceinline__ float det_gelu_tanh_form(float x) {
 // y = (x - mean) * inv_std [* w + b] [* (1 + scale) + shift]; out = fp8(clamp(bf16(y) / s)) or bf16(y)
 template <bool OUT_FP8>
 __global__ void __launch_bounds__(1024)
-layer_norm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ weight,
-                      const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ scale,
-                      const __nv_bfloat16* __restrict__ shift, long long mod_stride, void* __restrict__ out,
-                      const float* __restrict__ d_scale, int dim, float eps) {
+layer_norm_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* weight,
+                      const __nv_bfloat16* bias, const __nv_bfloat16* scale,
+                      const __nv_bfloat16* shift, long long mod_stride, void* __restrict__ out,
+                      const float* d_scale, int dim, float eps) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float warp_tot[32];
@@ -312,11 +312,11 @@ layer_norm_warp_kernel(ResNormArgs a) {
 // ------------------------------------------------------------------ QKV split + q/k RMSNorm + 3-D RoPE
 // packed (rows, 3*dim) bf16 = [q | k | v]; q_out / k_out (rows, dim); row = b * L + t
 __global__ void __launch_bounds__(1024)
-qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_bfloat16* __restrict__ wq,
-                           const __nv_bfloat16* __restrict__ wk, const float* __restrict__ fre,
-                           const float* __restrict__ fim, __nv_bfloat16* __restrict__ q_out,
+qkv_split_norm_rope_kernel(const __nv_bfloat16* packed, const __nv_bfloat16* wq,
+                           const __nv_bfloat16* wk, const float* fre,
+                           const float* fim, __nv_bfloat16* __restrict__ q_out,
                            __nv_bfloat16* __restrict__ k_out, int L, int dim, int D_h, int seq_len, float eps,
-                           const float* __restrict__ ext_ssq_q, const float* __restrict__ ext_ssq_k, int full_dim) {
+                           const float* ext_ssq_q, const float* ext_ssq_k, int full_dim) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float warp_tot[32];
@@ -396,11 +396,11 @@ qkv_split_norm_rope_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_
 // Many rows: one warp per (row, q or k); see layer_norm_warp_kernel.  20480 x 3 x 3072: 163 -> 82 us (6.2 TB/s).
 template <int NS>
 __global__ void __launch_bounds__(128)
-qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const __nv_bfloat16* __restrict__ wq,
-                                const __nv_bfloat16* __restrict__ wk, const float* __restrict__ fre,
-                                const float* __restrict__ fim, __nv_bfloat16* __restrict__ q_out,
+qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* packed, const __nv_bfloat16* wq,
+                                const __nv_bfloat16* wk, const float* fre,
+                                const float* fim, __nv_bfloat16* __restrict__ q_out,
                                 __nv_bfloat16* __restrict__ k_out, int L, int dim, int D_h, int seq_len, float eps,
-                                const float* __restrict__ ext_ssq_q, const float* __restrict__ ext_ssq_k, int full_dim,
+                                const float* ext_ssq_q, const float* ext_ssq_k, int full_dim,
                                 int rows) {
     pdl_launch_dependents();
     pdl_wait();
@@ -484,8 +484,8 @@ qkv_split_norm_rope_warp_kernel(const __nv_bfloat16* __restrict__ packed, const 
 
 // ------------------------------------------------------------------ bias + GELU(tanh) -> FP8
 __global__ void __launch_bounds__(256)
-bias_gelu_fp8_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ bias,
-                     uint8_t* __restrict__ out, const float* __restrict__ d_scale, long long rows, int N) {
+bias_gelu_fp8_kernel(const __nv_bfloat16* in, const __nv_bfloat16* bias,
+                     uint8_t* __restrict__ out, const float* d_scale, long long rows, int N) {
     pdl_launch_dependents();
     pdl_wait();
     const float inv_s = __fdiv_rn(1.0f, *d_scale);
@@ -519,8 +519,8 @@ bias_gelu_fp8_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* 
 // MODE 0: res += (x + bias) * gate     MODE 1: x += bias (in place, res == x)
 template <int MODE>
 __global__ void __launch_bounds__(256)
-bias_gate_res_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ x,
-                     const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ gate,
+bias_gate_res_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* x,
+                     const __nv_bfloat16* bias, const __nv_bfloat16* gate,
                      long long gate_stride, long long rows, int dim) {
     pdl_launch_dependents();
     pdl_wait();
@@ -566,7 +566,7 @@ bias_gate_res_kernel(__nv_bfloat16* __restrict__ res, const __nv_bfloat16* __res
 // ------------------------------------------------------------------ six modulation tensors
 // out_j[b, s, :] = bf16(adaln_params[b, s, j, :] + layer_modulation[j, :]), fp32 inputs
 __global__ void __launch_bounds__(256)
-modulation6_kernel(const float* __restrict__ params, const float* __restrict__ layer_mod,
+modulation6_kernel(const float* params, const float* layer_mod,
                    __nv_bfloat16* o0, __nv_bfloat16* o1, __nv_bfloat16* o2, __nv_bfloat16* o3, __nv_bfloat16* o4,
                    __nv_bfloat16* o5, int D, long long n) {
     pdl_launch_dependents();
@@ -585,7 +585,7 @@ modulation6_kernel(const float* __restrict__ params, const float* __restrict__ l
 // ------------------------------------------------------------------ tensor-parallel helpers for full-width norms
 // out[r] (+)= sum over `ncols` columns of x[r, col0 + c]^2   (one warp per row, fp32)
 __global__ void __launch_bounds__(256)
-row_sumsq_kernel(const __nv_bfloat16* __restrict__ x, long long row_stride, int col0, int ncols,
+row_sumsq_kernel(const __nv_bfloat16* x, long long row_stride, int col0, int ncols,
                  float* __restrict__ out, long long rows) {
     pdl_launch_dependents();
     pdl_wait();
@@ -611,8 +611,8 @@ row_sumsq_kernel(const __nv_bfloat16* __restrict__ x, long long row_stride, int 
 
 // y[r, :] = bf16(x[r, :] * rsqrt(ssq[r] / full_dim + eps) * w[:]) on a column slice of width `dim`
 __global__ void __launch_bounds__(256)
-rms_norm_ext_kernel(const __nv_bfloat16* __restrict__ x, long long x_stride, const __nv_bfloat16* __restrict__ w,
-                    const float* __restrict__ ssq, __nv_bfloat16* __restrict__ out, long long out_stride,
+rms_norm_ext_kernel(const __nv_bfloat16* x, long long x_stride, const __nv_bfloat16* w,
+                    const float* ssq, __nv_bfloat16* __restrict__ out, long long out_stride,
                     long long rows, int dim, int full_dim, float eps) {
     pdl_launch_dependents();
     pdl_wait();
