@@ -15,42 +15,60 @@ namespace frt {
 // serves move < 100 KB; the shape of the grid only has to cover the machine.
 constexpr int SG_COLS = 32, SG_KS = 16, SG_ROWS = 2, SG_KCHUNK = 1024;
 
+// Element of A, rounded to bf16.  Volatile: a plain load of a const operand may be moved above the wait for the kernel that
+// writes it.
+template <bool A_F32>
+__device__ __forceinline__ float load_a(const void* A, size_t i) {
+    if (A_F32) return bf16_round(reinterpret_cast<const volatile float*>(A)[i]);
+    return bf16_bits_to_f32(reinterpret_cast<const volatile uint16_t*>(A)[i]);
+}
+
+// The sums are formed as 16 interleaved K-slices (k mod 16), added in slice order.  Latency bounds these products, so a
+// chunk's weights of a thread are all in flight together, before the wait for the kernel in front when they may be (`early`).
 template <bool A_F32, bool D_F32>
 __global__ void __launch_bounds__(SG_COLS * SG_KS)
-small_gemm_bf16_kernel(const void* __restrict__ Av, const __nv_bfloat16* __restrict__ B,
+small_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* __restrict__ B,
                        void* __restrict__ Dv, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
-                       int accumulate) {
-    const __nv_bfloat16* A = reinterpret_cast<const __nv_bfloat16*>(Av);
-    const float* Af = reinterpret_cast<const float*>(Av);
+                       int accumulate, int early) {
     __nv_bfloat16* D = reinterpret_cast<__nv_bfloat16*>(Dv);
     float* Df = reinterpret_cast<float*>(Dv);
     __shared__ float a_s[SG_ROWS][SG_KCHUNK];
     __shared__ float part[SG_KS][SG_ROWS][SG_COLS];
+    constexpr int PER = SG_KCHUNK / SG_KS;
     const int tx = threadIdx.x % SG_COLS;
     const int ks = threadIdx.x / SG_COLS;
     const int n = blockIdx.x * SG_COLS + tx;
     const int m0 = blockIdx.y * SG_ROWS;
     pdl_launch_dependents();     // the dependent kernel still waits for this grid to complete
-    pdl_wait();
+    if (!early) pdl_wait();
     float acc[SG_ROWS] = {};
     for (int k0 = 0; k0 < K; k0 += SG_KCHUNK) {
         const int kc = K - k0 < SG_KCHUNK ? K - k0 : SG_KCHUNK;
+        __nv_bfloat16 b[PER];
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int k = ks + i * SG_KS;
+            b[i] = k < kc && n < N ? B[(size_t)(k0 + k) * N + n] : __float2bfloat16_rn(0.0f);
+        }
+        if (k0 == 0) pdl_wait();
         __syncthreads();
-        for (int i = threadIdx.x; i < SG_ROWS * kc; i += blockDim.x) {
-            const int r = i / kc, k = i - r * kc;
-            const size_t ai = (size_t)(m0 + r) * K + k0 + k;
-            // an fp32 operand is rounded to bf16 first: the projection multiplies bf16 by bf16
-            a_s[r][k] = (m0 + r < M) ? (A_F32 ? bf16_round(Af[ai]) : __bfloat162float(A[ai]))
-                                     : 0.0f;
+#pragma unroll
+        for (int r = 0; r < SG_ROWS; ++r) {
+#pragma unroll
+            for (int i = 0; i < SG_KCHUNK / (SG_COLS * SG_KS); ++i) {
+                const int k = threadIdx.x + i * SG_COLS * SG_KS;
+                const size_t ai = (size_t)(m0 + r) * K + k0 + k;
+                // an fp32 operand is rounded to bf16 first: the projection multiplies bf16 by bf16
+                if (k < kc) a_s[r][k] = m0 + r < M ? (load_a<A_F32>(Av, ai)) : 0.0f;
+            }
         }
         __syncthreads();
-        if (n < N) {
-            // the loads of B do not depend on one another: keep 16 of them in flight per thread
-#pragma unroll 16
-            for (int k = ks; k < kc; k += SG_KS) {
-                const float b = __bfloat162float(B[(size_t)(k0 + k) * N + n]);
 #pragma unroll
-                for (int r = 0; r < SG_ROWS; ++r) acc[r] = fmaf(a_s[r][k], b, acc[r]);
+        for (int i = 0; i < PER; ++i) {
+            const int k = ks + i * SG_KS;
+            if (k < kc) {
+#pragma unroll
+                for (int r = 0; r < SG_ROWS; ++r) acc[r] = fmaf(a_s[r][k], __bfloat162float(b[i]), acc[r]);
             }
         }
     }
@@ -70,6 +88,65 @@ small_gemm_bf16_kernel(const void* __restrict__ Av, const __nv_bfloat16* __restr
         } else {
             if (accumulate) s += __bfloat162float(D[o]);
             D[o] = __float2bfloat16_rn(s);
+        }
+    }
+}
+
+// K = 32 (the action in-projection): a thread forms two columns of four rows, its 32 weight pairs in registers, in the slice
+// order of the kernel above -- the same bits with one load round trip and no exchange between threads (200 x 1024: 18 us
+// as 3200 CTAs of 512 threads before).  N even, B and D 4-byte aligned.
+constexpr int SK_K = 32, SK_ROWS = 4, SK_THREADS = 128;
+template <bool A_F32, bool D_F32>
+__global__ void __launch_bounds__(SK_THREADS)
+short_k_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* __restrict__ B, void* __restrict__ Dv,
+                         const __nv_bfloat16* __restrict__ bias, int M, int N, int accumulate, int early) {
+    __shared__ float a_s[SK_ROWS][SK_K];
+    const int n = (blockIdx.x * SK_THREADS + threadIdx.x) * 2;
+    const int m0 = blockIdx.y * SK_ROWS;
+    const bool live = n < N;
+    pdl_launch_dependents();
+    if (!early) pdl_wait();
+    uint32_t w[SK_K];
+#pragma unroll
+    for (int k = 0; k < SK_K; ++k) w[k] = live ? *reinterpret_cast<const uint32_t*>(B + (size_t)k * N + n) : 0u;
+    pdl_wait();
+    {
+        const int r = threadIdx.x / SK_K, k = threadIdx.x % SK_K;
+        const size_t ai = (size_t)(m0 + r) * SK_K + k;
+        a_s[r][k] = m0 + r < M ? (load_a<A_F32>(Av, ai)) : 0.0f;
+    }
+    __syncthreads();
+    if (!live) return;
+#pragma unroll
+    for (int r = 0; r < SK_ROWS; ++r) {
+        if (m0 + r >= M) break;
+        float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            float w00, w01, w10, w11;
+            unpack_bf16x2(w[q], w00, w01);
+            unpack_bf16x2(w[q + 16], w10, w11);
+            s0 += fmaf(a_s[r][q + 16], w10, fmaf(a_s[r][q], w00, 0.0f));
+            s1 += fmaf(a_s[r][q + 16], w11, fmaf(a_s[r][q], w01, 0.0f));
+        }
+        if (bias) {
+            s0 += __bfloat162float(bias[n]);
+            s1 += __bfloat162float(bias[n + 1]);
+        }
+        const size_t o = (size_t)(m0 + r) * N + n;
+        if (D_F32) {
+            float* d = reinterpret_cast<float*>(Dv) + o;
+            d[0] = accumulate ? s0 + d[0] : s0;
+            d[1] = accumulate ? s1 + d[1] : s1;
+        } else {
+            uint32_t* d = reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(Dv) + o);
+            if (accumulate) {
+                float d0, d1;
+                unpack_bf16x2(*d, d0, d1);
+                s0 += d0;
+                s1 += d1;
+            }
+            *d = pack_bf16x2(s0, s1);
         }
     }
 }
@@ -258,8 +335,6 @@ int frt_b200_gemm_bf16_nn_small(const void* A, const void* B, void* D, const voi
     if (!A || !B || !D || M < 0 || N <= 0 || K <= 0) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((N + SG_COLS - 1) / SG_COLS, (M + SG_ROWS - 1) / SG_ROWS);
-    cfg.blockDim = dim3(SG_COLS * SG_KS);
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -268,12 +343,28 @@ int frt_b200_gemm_bf16_nn_small(const void* A, const void* B, void* D, const voi
     cfg.numAttrs = 1;
     const __nv_bfloat16* Bp = (const __nv_bfloat16*)B;
     const __nv_bfloat16* bp = (const __nv_bfloat16*)bias;
+    const int early = flags & 1;                                  // B is weights: not written by the kernel in front
+    const int blocks_m = (M + SK_ROWS - 1) / SK_ROWS;
     cudaError_t e;
+    if (K == SK_K && (N & 1) == 0 && blocks_m <= 65535 && (reinterpret_cast<uintptr_t>(B) & 3) == 0 &&
+        (reinterpret_cast<uintptr_t>(D) & 3) == 0) {
+        cfg.gridDim = dim3((N / 2 + SK_THREADS - 1) / SK_THREADS, blocks_m);
+        cfg.blockDim = dim3(SK_THREADS);
+        switch (io & 3) {
+            case 0: e = cudaLaunchKernelEx(&cfg, short_k_gemm_bf16_kernel<false, false>, A, Bp, D, bp, M, N, accumulate, early); break;
+            case 1: e = cudaLaunchKernelEx(&cfg, short_k_gemm_bf16_kernel<true, false>, A, Bp, D, bp, M, N, accumulate, early); break;
+            case 2: e = cudaLaunchKernelEx(&cfg, short_k_gemm_bf16_kernel<false, true>, A, Bp, D, bp, M, N, accumulate, early); break;
+            default: e = cudaLaunchKernelEx(&cfg, short_k_gemm_bf16_kernel<true, true>, A, Bp, D, bp, M, N, accumulate, early); break;
+        }
+        return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
+    }
+    cfg.gridDim = dim3((N + SG_COLS - 1) / SG_COLS, (M + SG_ROWS - 1) / SG_ROWS);
+    cfg.blockDim = dim3(SG_COLS * SG_KS);
     switch (io & 3) {
-        case 0: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<false, false>, A, Bp, D, bp, M, N, K, accumulate); break;
-        case 1: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<true, false>, A, Bp, D, bp, M, N, K, accumulate); break;
-        case 2: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<false, true>, A, Bp, D, bp, M, N, K, accumulate); break;
-        default: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<true, true>, A, Bp, D, bp, M, N, K, accumulate); break;
+        case 0: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<false, false>, A, Bp, D, bp, M, N, K, accumulate, early); break;
+        case 1: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<true, false>, A, Bp, D, bp, M, N, K, accumulate, early); break;
+        case 2: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<false, true>, A, Bp, D, bp, M, N, K, accumulate, early); break;
+        default: e = cudaLaunchKernelEx(&cfg, small_gemm_bf16_kernel<true, true>, A, Bp, D, bp, M, N, K, accumulate, early); break;
     }
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

@@ -135,6 +135,21 @@ __device__ __forceinline__ uint32_t pack8(const float* v, float inv) {
     for (int i = 0; i < 8; ++i) x[i] = e2m1_off_tie<FAMILY>(__fmaf_rn(v[i], inv, 0.0f));   // + 0: a zero product is +0
     return cvt8(x);
 }
+// four values -> two bytes
+template <int FAMILY>
+__device__ __forceinline__ uint16_t pack4(const float* v, float inv) {
+    float x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = e2m1_off_tie<FAMILY>(__fmaf_rn(v[i], inv, 0.0f));
+    uint16_t w;
+    asm("{\n\t.reg .b8 b0, b1;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+        "mov.b16 %0, {b0, b1};\n\t}"
+        : "=h"(w)
+        : "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]));
+    return w;
+}
 // bf16 values of a block with scale s; inv from inv_off_ties
 template <int FAMILY>
 __device__ __forceinline__ uint32_t pack8_bf16(const float* v, float s, float2 inv) {

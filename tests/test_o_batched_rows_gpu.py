@@ -150,3 +150,30 @@ def test_attention_length_read_early(used):
     got = O.bf16_bits_to_f32(d_o.get())
     assert fa2.attention_status() == 0
     assert (np.abs(got - ref) <= 2e-2 * np.sqrt((ref.astype(np.float64) ** 2).mean()) + np.abs(ref) * 2.0 ** -8).all()
+
+
+@pytest.mark.parametrize("M,N,K,io,acc", [(50, 1024, 32, 1, False), (3, 30, 32, 0, True), (201, 1026, 32, 3, True),
+                                          (50, 33, 32, 0, False), (5, 32, 1024, 2, True), (2, 40, 1500, 0, False)])
+def test_action_projection_sums(M, N, K, io, acc):
+    """Both forms of the small bf16 product: 16 interleaved K-slices added in order, then bias, then the old value."""
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, rand_bf16
+    rng = np.random.default_rng(M + N + K)
+    b, bias = rand_bf16(rng, (K, N), 0.5), rand_bf16(rng, (N,), 0.5)
+    a = rng.standard_normal((M, K)).astype(np.float32) if io & 1 else rand_bf16(rng, (M, K))
+    d = rng.standard_normal((M, N)).astype(np.float32) if io & 2 else rand_bf16(rng, (M, N))
+    d_a, d_b, d_bias, d_d = Dev(a), Dev(b), Dev(bias), Dev(d)
+    fvk.call("frt_b200_gemm_bf16_nn_small", d_a.ptr, d_b.ptr, d_d.ptr, d_bias.ptr, M, N, K, int(acc), io, 1, 0)
+    af = O.bf16_bits_to_f32(O.f32_to_bf16_bits(a) if io & 1 else a)
+    bf = O.bf16_bits_to_f32(b)
+    s = np.zeros((M, N), np.float32)
+    for q in range(16):
+        part = np.zeros((M, N), np.float32)
+        for k in range(q, K, 16):                       # products of two bf16 values are exact in fp64: one rounding per term
+            part = (af[:, k:k + 1].astype(np.float64) * bf[k].astype(np.float64) + part).astype(np.float32)
+        s = s + part
+    s = s + O.bf16_bits_to_f32(bias)
+    if acc:
+        s = s + (d if io & 2 else O.bf16_bits_to_f32(d))
+    got = d_d.get()
+    assert np.array_equal(got, s if io & 2 else O.f32_to_bf16_bits(s))
