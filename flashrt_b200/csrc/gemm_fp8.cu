@@ -1190,10 +1190,20 @@ int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const 
     bool pdl = flags & 1;
     if (M <= 256) return dispatch_small_m_nvfp4<EPI_BF16>(A, W, p, K, M, (N + 127) / 128, splits, pdl, s);
     int sp = splits > 0 ? pick_splits(1, p.kb_total, splits > 8 ? 8 : splits) : 1;
-    // Persistent kernel with two 128-column accumulators: measured faster than the 128 x 256 one-tile kernel while
-    // the per-tile prologue / epilogue dominates (K < 3072); at larger K the wider tile's lower operand traffic wins.
-    if (sp == 1 && N > 64 && !(flags & 2) && (K < 3072 || N < 256 || (flags & 4)))
-        return launch_gemm_persistent<128, EPI_P_BF16, true>(A, W, p, K, s);
+    // Persistent kernel on 128 x 128 tiles (the finish of a tile under the MMAs of the next: 0.32 us per k-block and wave, not
+    // under 2.4) or one CTA per 128 x 256 tile (fewer operand bytes, but every wave pays its set-up and finish: 5.4 + 0.40 per
+    // k-block), whichever is cheaper by whole waves; fitted to M 300 .. 8192, N 1024 .. 14336, K 1024 .. 14336, where it picks
+    // the faster one (8192 x 14336 x 3072: 209 us against 261; 2501 x 1024 x 8192: 25.3 against 18.0).
+    if (sp == 1 && N > 64 && !(flags & 2)) {
+        const int sms = device_sm_count();
+        const long long mt = (M + 127) / 128;
+        const double kb = p.kb_total;
+        const double wave_p = 0.32 * kb + 0.2 > 2.4 ? 0.32 * kb + 0.2 : 2.4;
+        const double t_persistent = 4.6 + wave_p * (double)((mt * ((N + 127) / 128) + sms - 1) / sms);
+        const double t_one = 0.6 + (5.4 + 0.40 * kb) * (double)((mt * ((N + 255) / 256) + sms - 1) / sms);
+        if (N < 256 || (flags & 4) || t_persistent <= t_one)
+            return launch_gemm_persistent<128, EPI_P_BF16, true>(A, W, p, K, s);
+    }
     if (N >= 256) return launch_gemm<256, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     return launch_gemm<64, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
