@@ -111,6 +111,9 @@ struct GemmParams {
     int w_kn;                  // large-M persistent kernel: weights stored (K, N) row-major
     int tile_gm;               // large-M kernels: m-tiles per group of the tile order
     int early;                 // the weights may be read before the kernel in front has finished
+    float* split_ws;           // CTA-pair kernel with split K: partials and one counter per epilogue warp of a tile
+    int* split_cnt;
+    int ksplits;
 };
 
 enum { EPI_BF16 = 0, EPI_ROPE_SPLIT = 1, EPI_GEGLU_FP8 = 2, EPI_GATE_RES_NORM_FP8 = 3 };
@@ -1045,6 +1048,42 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     if (N >= 256) return launch_gemm<256, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
     return launch_gemm<64, false, EPI_BF16>(A, W, p, K, sp, pdl, s);
+}
+
+// The same product for a caller with a workspace: above 256 rows a long K on few tiles may be split over CTA pairs, the
+// partials (fp32) added in split order by whichever warp of a tile comes last.  counters: 16 ints per 256 x 256 tile, zeroed
+// once by the caller, zero again behind every launch.  One launch at a time may use a workspace.
+int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
+                                const float* d_scale_b, const void* bias, float* workspace, long long workspace_bytes,
+                                int* counters, int flags, void* stream) {
+    if (!workspace || !counters || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FRT_ERR_INVALID;
+    if (A && W && D && M > 256 && N >= 256 && K > 0 && K % 16 == 0) {
+        // As many splits as one wave of pairs holds: 5.6 + 0.34 per k-block of a split (the pair kernel's cost) and 8 for the
+        // exchange of the partials (write, count, read the others') against the best unsplit kernel: 768 x 2048 x 16384 as
+        // three splits 31.2 -> 26.5 us, 300 x 2048 x 16384 as four 29.2 -> 23.8; K = 8192 (17.9 against 19.8) stays whole.
+        const int tiles = ((M + 255) / 256) * ((N + 255) / 256), kbt = (K + 127) / 128, pairs = device_sm_count() / 2;
+        int S = tiles > 0 ? pairs / tiles : 0;
+        if (S > 4) S = 4;
+        if (S > kbt) S = kbt;
+        double t_one = 0.0;
+        pick_large(M, N, K, false, &t_one);
+        if (S >= 2 && (long long)tiles * S * 262144 <= workspace_bytes && 13.6 + 0.34 * ((kbt + S - 1) / S) < t_one) {
+            GemmParams p = {};
+            p.out = (__nv_bfloat16*)D;
+            p.sa = d_scale_a;
+            p.sb = d_scale_b;
+            p.alpha_host = 1.0f;
+            p.bias = (const __nv_bfloat16*)bias;
+            p.M = M;
+            p.N = N;
+            p.kb_total = kbt;
+            p.split_ws = workspace;
+            p.split_cnt = counters;
+            p.ksplits = S;
+            return launch_gemm_pair<256, EPI_P_BF16, true>(A, W, p, K, (cudaStream_t)stream);
+        }
+    }
+    return frt_b200_gemm_fp8_nt(A, W, D, M, N, K, d_scale_a, d_scale_b, 1.0f, bias, 0, flags & 1, stream);
 }
 
 // The same product with the weights stored (K, N) row-major -- GemmRunner::fp8_nn_dev, the reference's default

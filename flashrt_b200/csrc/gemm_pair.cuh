@@ -79,7 +79,62 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 }  // namespace tc
 
-template <int BN, int EPI>
+// Split K: an epilogue warp's 32 rows x NC columns of one split.  It leaves its partial in the workspace ([unit][warp][NC / 4]
+// [lane][4] floats: 512 bytes per store), then counts itself in; the last of the tile's S warps adds the partials in split
+// order, its own from tensor memory, and puts the sum back there for the finish.  Nobody waits.  False: not the last.
+template <int NC>
+__device__ __forceinline__ bool split_k_sum(const GemmParams& p, uint32_t t_src, int unit, int S, int slot) {
+    const int lane = threadIdx.x & 31;
+    const int mine = unit % S, first = unit - mine;
+    auto base = [&](int u) { return p.split_ws + ((size_t)u * 16 + slot) * (32 * NC) + lane * 4; };
+    float* out = base(unit);
+#pragma unroll 1
+    for (int c = 0; c < NC; c += 32) {
+        uint32_t v[32];
+        tc::tmem_ld32(t_src + c, v);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            __stcg(reinterpret_cast<uint4*>(out + (c + j) * 32), make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+    }
+    __threadfence();
+    __syncwarp();
+    int seen = 0;
+    if (lane == 0) seen = atomicAdd(p.split_cnt + (unit / S) * 16 + slot, 1);
+    seen = __shfl_sync(0xffffffffu, seen, 0);
+    if (seen != S - 1) return false;
+    __threadfence();
+    if (lane == 0) p.split_cnt[(unit / S) * 16 + slot] = 0;          // for the next launch
+#pragma unroll 1
+    for (int c = 0; c < NC; c += 32) {
+        uint32_t v[32];
+        float a[32];
+        tc::tmem_ld32(t_src + c, v);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) a[j] = 0.0f;
+        for (int s = 0; s < S; ++s) {
+            if (s == mine) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) a[j] += __uint_as_float(v[j]);
+            } else {
+                const float* in = base(first + s);
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 x = __ldcg(reinterpret_cast<const float4*>(in + (c + j) * 32));
+                    a[j] += x.x; a[j + 1] += x.y; a[j + 2] += x.z; a[j + 3] += x.w;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(a[j]);
+        tc::tmem_st32(t_src + c, v);
+    }
+    tc::tmem_st_wait();
+    return true;
+}
+
+template <int BN, int EPI, bool SPLIT = false>
 __global__ void __launch_bounds__(64 + pair_epi_threads<EPI>(), 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmParams p) {
     static_assert(EPI != EPI_P_GEGLU_FP8 || BN == 256, "GeGLU: 128 gate and 128 up columns");
@@ -101,9 +156,12 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int m_tiles = (p.M + 255) / 256;
     const int n_tiles = (p.N + BN - 1) / BN;
-    const int total = m_tiles * n_tiles;
-    const int kbt = p.kb_total;
+    // SPLIT: a unit is (tile, K split), the splits of a tile next to one another and all of them resident at once
+    const int S = SPLIT ? p.ksplits : 1;
+    const int total = m_tiles * n_tiles * S;
     const TileOrder order = {p.tile_gm, m_tiles, n_tiles};
+    auto k_begin = [&](int t) { return SPLIT ? (int)((long long)p.kb_total * (t % S) / S) : 0; };
+    auto k_end = [&](int t) { return SPLIT ? (int)((long long)p.kb_total * (t % S + 1) / S) : p.kb_total; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -140,11 +198,12 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         bool ready = true;
         for (int t = pair; t < total; t += npairs) {
             int mt, nt;
-            order.at(t, mt, nt);
+            order.at(SPLIT ? t / S : t, mt, nt);
             const int m0 = mt * 256 + (int)rank * 128;
             // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
             const int n0 = EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
-            for (int kb = 0; kb < kbt; ++kb) {
+            const int kb1 = k_end(t);
+            for (int kb = k_begin(t); kb < kb1; ++kb) {
                 if (!tc::warp_wait(empty_a + 8 * s, ph, ready, deadline, abort_flag)) {
                     if (lane == 0 && !*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
                     *abort_flag = 1;
@@ -181,7 +240,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
             tc::tc_fence_after_sync();
             const uint32_t d_tm = tmem + buf * BN;
-            for (int kb = 0; kb < kbt; ++kb) {
+            const int kb0 = k_begin(t), kb1 = k_end(t);
+            for (int kb = kb0; kb < kb1; ++kb) {
                 if (!tc::warp_wait(full_a + 8 * s, ph, ready, deadline, abort_flag)) {
                     if (lane == 0 && !*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
                     *abort_flag = 1;
@@ -196,9 +256,9 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (tc::elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        tc::mma_f8_pair(d_tm, dA0 + so + 2 * k, dB0 + so + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        tc::mma_f8_pair(d_tm, dA0 + so + 2 * k, dB0 + so + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     tc::mma_commit_both(done);
-                    if (kb == kbt - 1) tc::mma_commit_both(accF_a + 8 * buf);
+                    if (kb == kb1 - 1) tc::mma_commit_both(accF_a + 8 * buf);
                 }
             }
             if (failed) break;
@@ -226,13 +286,16 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
             tc::tc_fence_after_sync();
             int mt, nt;
-            order.at(t, mt, nt);
+            order.at(SPLIT ? t / S : t, mt, nt);
             const uint32_t t_acc = tmem + buf * BN + lane_off;
+            bool finish = true;
+            if constexpr (SPLIT)
+                finish = split_k_sum<BN / 2>(p, t_acc + half * (BN / 2), t, S, (int)rank * 8 + (warp - 2));
             const int m_base = mt * 256 + (int)rank * 128 + q * 32;
             if constexpr (EPI == EPI_P_GEGLU_FP8)
                 epilogue_geglu_rows(p, t_acc + half * 32, t_acc + BN / 2 + half * 32, m_base, nt * (BN / 2) + half * 32, alpha,
                                     inv_os);
-            else
+            else if (finish)
                 epilogue_rows<EPI, BN / 2>(p, t_acc + half * (BN / 2), m_base, nt * BN + half * (BN / 2), stg, lines, alpha,
                                            inv_os);
             tc::tc_fence_before_sync();
@@ -245,14 +308,14 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (warp == 1) tc::tmem_dealloc_pair(tmem, Cfg::TMEM_COLS);
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool SPLIT = false>
 static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, cudaStream_t stream) {
     using Cfg = GemmPairCfg<BN>;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
     const int sms = device_sm_count();
     if (attr_once.need(attr_dev)) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              Cfg::SMEM_BYTES);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         attr_once.set(attr_dev);
@@ -264,7 +327,8 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
     if (rc) return rc;
     const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + BN - 1) / BN, total = m_tiles * n_tiles;
     p.tile_gm = tile_group(m_tiles, n_tiles, 256, BN, sms / 2);
-    const int pairs = total < sms / 2 ? total : sms / 2;
+    const int units = SPLIT ? total * p.ksplits : total;
+    const int pairs = units < sms / 2 ? units : sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(64 + pair_epi_threads<EPI>());
@@ -282,6 +346,6 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
     ++na;
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI>, tmA, tmW, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI, SPLIT>, tmA, tmW, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

@@ -275,6 +275,12 @@ class GemmRunner:
              | (16 if swapped else 0)
              | _tile_hint(tile_n), stream)
 
+    def fp8_nt_dev_splitk(self, A, B, D, M, N, K, d_scale_a, d_scale_b, workspace, workspace_bytes, counters, stream=0, *,
+                          pdl=False, bias=None):
+        """``fp8_nt_dev`` that may split K through the caller's workspace (M > 256; the form is chosen by size)."""
+        call("frt_b200_gemm_fp8_nt_splitk", A, B, D, M, N, K, d_scale_a, d_scale_b, bias, workspace, workspace_bytes, counters,
+             _f(pdl), stream)
+
     # -- the decoder's projections with the norm kernel between them folded in ------------------------------
     def fp8_nt_dev_gate_residual(self, A, B, M, N, K, d_scale_a, d_scale_b, residual, gate, stats_out, stream=0, *,
                                  pdl=False, splits=0, tile_n=0, next_scale=0, q8_out=0, d_scale_q8=0,

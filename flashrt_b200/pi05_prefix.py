@@ -112,6 +112,10 @@ class Pi05PrefixEncoderB200:
         # scratch of the attention's key splits (the split is chosen by the prefix length)
         self.o_accum = torch.empty(ATTN_SPLITS, ENC_NH, S, ENC_HD, dtype=torch.float32, device=dev)
         self.lse_accum = torch.empty(ATTN_SPLITS, ENC_NH, S, dtype=torch.float32, device=dev)
+        # partials of the down projection's K splits: one wave of CTA pairs
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        self.splitk_ws = torch.empty(sms // 2 * 65536, dtype=torch.float32, device=dev)
+        self.splitk_counters = z(8 * sms, dtype=torch.int32)
         self.attn_counters = z(2 * ((S * ENC_NH + 127) // 128), dtype=torch.int32)
         self.act_scale = torch.ones(layers, len(SITES), dtype=torch.float32, device=dev)
         self.scratch_scale = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -176,7 +180,9 @@ class Pi05PrefixEncoderB200:
             else:               # one launch: the activation under the product's MMAs
                 self.gemm.fp8_nt_dev_geglu_fp8(self.act8.data_ptr(), self.w_gu[i].data_ptr(), self.hid8.data_ptr(), seq, ENC_H,
                                                ENC_D, self._sp(i, "gu"), self.ws_gu_t[i].data_ptr(), self._sp(i, "d"), st)
-            self._gemm(self.hid8, self.w_d[i], self.ws_d_t[i], self.xn, seq, ENC_D, ENC_H, self._sp(i, "d"), st)
+            self.gemm.fp8_nt_dev_splitk(self.hid8.data_ptr(), self.w_d[i].data_ptr(), self.xn.data_ptr(), seq, ENC_D, ENC_H,
+                                        self._sp(i, "d"), self.ws_d_t[i].data_ptr(), self.splitk_ws.data_ptr(),
+                                        self.splitk_ws.numel() * 4, self.splitk_counters.data_ptr(), st)
 
     # ------------------------------------------------------------------
     def _check(self, embeds, k_out, v_out):

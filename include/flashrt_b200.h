@@ -120,6 +120,14 @@ int frt_b200_qkv_split_rope(const void* qkv, const void* rope, void* Q, void* K,
 int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
                          const float* d_scale_b, float alpha_host, const void* bias, int splits, int flags,
                          void* stream);
+/* frt_b200_gemm_fp8_nt for a caller with a workspace (the split K of cuBLASLt behind csrc/gemm/gemm_runner.cu:67-76, whose
+ * workspace the runner owns): above 256 rows a long K on few tiles may be split, the fp32 partials added in a fixed order.
+ * workspace: 16-byte aligned, 256 KB per (256 x 256 tile, split), at most one wave of CTA pairs (SMs / 2 x 256 KB is always
+ * enough; with less the product is not split); counters: 16 ints per tile (8 x SMs suffice), zeroed once.  Launches that share
+ * them must not overlap; after a non-zero status word zero the counters again.  flags bit 0 as above. */
+int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
+                                const float* d_scale_b, const void* bias, float* workspace, long long workspace_bytes,
+                                int* counters, int flags, void* stream);
 /* GemmRunner::fp8_nn_dev (csrc/bindings.cpp:706-716 -> csrc/gemm/gemm_runner.cu:67-76), the reference's default weight
  * layout: B stored (K, N) row-major.  D(M,N) bf16 = alpha_host * (*d_scale_a) * (*d_scale_b) * A(M,K) . B(K,N) + bias.
  * The weight tiles are loaded as 128 K-rows x 128 N-bytes and consumed as an MN-major MMA operand; the result equals
@@ -182,7 +190,7 @@ int frt_b200_gemm_status(int reset);
  *   flags: bit 0 = programmatic dependent launch; bit 1 = keep the single-tile kernel; head_dim 256 with scratch:
  *   bit 2 = one CTA per (tile, split) instead of four head-dim parts, bit 3 = always (b), bit 4 = kv_splits (> 0) is an upper
  *   bound: the number of splits (1, 2, 4 or 8, one of them possibly without keys) and the form of the combine are chosen by
- *   size; no size is refused. */
+ *   size; no size is refused (the splits of csrc/fa2_bindings.cpp:173-183). */
 int frt_b200_attention_fwd_bf16(const void* Q, const void* K, const void* V, void* O, void* O_fp8,
                                 const float* out_scale, float* lse, const int* seqused_k, int batch, int seqlen_q,
                                 int seqlen_k, int num_heads_q, int num_heads_kv, int head_dim,

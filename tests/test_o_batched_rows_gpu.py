@@ -177,3 +177,29 @@ def test_action_projection_sums(M, N, K, io, acc):
         s = s + (d if io & 2 else O.bf16_bits_to_f32(d))
     got = d_d.get()
     assert np.array_equal(got, s if io & 2 else O.f32_to_bf16_bits(s))
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 256, 16384), (768, 2048, 16384), (541, 2000, 16400), (300, 2056, 12288), (768, 2048, 2048),
+                                   (50, 1024, 4096)])
+def test_split_k_product(M, N, K):
+    """K split through a workspace: exact products (integers) give the oracle's bits, twice on the same counters."""
+    import torch
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, f32, rand_bf16, zeros
+    rng = np.random.default_rng(M + N + K)
+    vals = np.array([-2, -1, 0, 1, 2], np.float32)
+    e4 = lambda *s: torch.from_numpy(rng.choice(vals, s)).to(torch.float8_e4m3fn).view(torch.uint8).numpy()  # noqa: E731
+    A, W, bias = e4(M, K), e4(N, K), rand_bf16(rng, (N,), 0.2)
+    d_A, d_W, d_b, d_sa, d_sb = Dev(A), Dev(W), Dev(bias), f32(0.5), f32(0.25)
+    ws, cnt = torch.empty(74 * 65536, dtype=torch.float32, device="cuda"), zeros((1184,), np.int32)
+    plain = zeros((M, N), np.uint16)
+    g = fvk.GemmRunner()
+    g.fp8_nt_dev(d_A.ptr, d_W.ptr, plain.ptr, M, N, K, d_sa.ptr, d_sb.ptr, bias=d_b.ptr)
+    _check(plain.get(), _ref(A, W, 0.5, 0.25, bias))
+    for _ in range(2):
+        d_D = Dev(np.full((M + 1, N), 0x5A5A, np.uint16))
+        g.fp8_nt_dev_splitk(d_A.ptr, d_W.ptr, d_D.ptr, M, N, K, d_sa.ptr, d_sb.ptr, ws.data_ptr(), ws.numel() * 4, cnt.ptr,
+                            bias=d_b.ptr)
+        got = d_D.get()
+        assert fvk.tensor_core_status() == 0
+        assert np.array_equal(got[:M], plain.get()) and (got[M] == 0x5A5A).all() and (cnt.get() == 0).all()
