@@ -937,18 +937,21 @@ static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, in
 }
 
 // ------------------------------------------------------------------ choice among the large-M FP8 kernels
-enum { LARGE_128 = 0, LARGE_256 = 1, LARGE_PAIR = 2, LARGE_PAIR_128 = 3 };
+enum { LARGE_128 = 0, LARGE_256 = 1, LARGE_PAIR = 2, LARGE_PAIR_128 = 3, LARGE_PAIR_192 = 4 };
 
 // Microseconds of a launch: a fixed part, then whole waves of tiles, each as long as its k-blocks of 128.  The constants are
 // fitted to a sweep of graph-launched products on one B200 (M 130 .. 8192, N 1024 .. 32768, K 1024 .. 16384; the choice was
 // within 3 % of the best kernel on all but a few of its points):
 //   128 x 128 tile per CTA 3.6 + 0.32 per k-block, 128 x 256 per CTA 4.5 + 0.40, 256 x 256 per CTA pair 5.6 + 0.34,
-//   256 x 128 per CTA pair 4.6 + 0.225.
+//   256 x 128 per CTA pair 4.6 + 0.225, 256 x 192 per CTA pair 5.0 + 0.265.
 // The pair of 256 x 256 moves the fewest operand bytes per flop and wins wherever its tile list is long; the others win
 // where a short list of large tiles would leave the last wave nearly empty, or rows of a half-empty 256-row tile.
+// (256 x 192 fills the gap between one and two waves of the wide tile: 2048 x 3072 x 3072 20.1 -> 17.0 us, 2048 x 3072 x 14336
+// 70.4 -> 61.3, 600 x 9216 x 3072 20.3 -> 17.6.)
 static double large_cost(int kind, int M, int N, int K) {
-    static const struct { int tm, tn, pair; double fixed, per_kb; } c[4] = {
-        {128, 128, 0, 3.6, 0.32}, {128, 256, 0, 4.5, 0.40}, {256, 256, 1, 5.6, 0.34}, {256, 128, 1, 4.6, 0.225}};
+    static const struct { int tm, tn, pair; double fixed, per_kb; } c[5] = {
+        {128, 128, 0, 3.6, 0.32}, {128, 256, 0, 4.5, 0.40}, {256, 256, 1, 5.6, 0.34}, {256, 128, 1, 4.6, 0.225},
+        {256, 192, 1, 5.0, 0.265}};
     const int workers = device_sm_count() / (c[kind].pair ? 2 : 1);
     const long long tiles = (long long)((M + c[kind].tm - 1) / c[kind].tm) * ((N + c[kind].tn - 1) / c[kind].tn);
     return c[kind].fixed + (double)((tiles + workers - 1) / workers) * ((K + 127) / 128) * c[kind].per_kb;
@@ -956,7 +959,7 @@ static double large_cost(int kind, int M, int N, int K) {
 static int pick_large(int M, int N, int K, bool no_pair, double* cost = nullptr) {
     int best = LARGE_128;
     double t = large_cost(LARGE_128, M, N, K);
-    for (int k = LARGE_256; k <= LARGE_PAIR_128 && N >= 256; ++k) {
+    for (int k = LARGE_256; k <= LARGE_PAIR_192 && N >= 256; ++k) {
         if (k >= LARGE_PAIR && no_pair) break;
         const double tk = large_cost(k, M, N, K);
         if (tk < t) { t = tk; best = k; }
@@ -969,6 +972,7 @@ template <int EPI>
 static int launch_large(int kind, const void* A, const void* W, const GemmParams& p, int K, cudaStream_t s) {
     if (kind == LARGE_PAIR) return launch_gemm_pair<256, EPI>(A, W, p, K, s);
     if (kind == LARGE_PAIR_128) return launch_gemm_pair<128, EPI>(A, W, p, K, s);
+    if (kind == LARGE_PAIR_192) return launch_gemm_pair<192, EPI>(A, W, p, K, s);
     if (kind == LARGE_256) return launch_gemm_persistent<256, EPI>(A, W, p, K, s);
     return launch_gemm_persistent<128, EPI>(A, W, p, K, s);
 }

@@ -26,10 +26,10 @@ struct GemmPairCfg {
     static constexpr int A_BYTES = 128 * 128;
     static constexpr int B_BYTES = BN / 2 * 128;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
-    static constexpr int STAGES = BN == 256 ? 6 : 8;
+    static constexpr int STAGES = BN >= 192 ? 6 : 8;
     static constexpr int EPI_STAGE_BYTES = 8 * 32 * 128;    // line staging of the eight epilogue warps
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_STAGE_BYTES;
-    static constexpr int TMEM_COLS = 2 * BN;             // two accumulators
+    static constexpr int TMEM_COLS = BN == 128 ? 256 : 512;  // two accumulators
 };
 // epilogue threads per CTA: the GeGLU finish is a chain of 30 dependent instructions per value, which sixteen warps hide
 // where eight do not
@@ -137,6 +137,8 @@ __device__ __forceinline__ bool split_k_sum(const GemmParams& p, uint32_t t_src,
 template <int BN, int EPI, bool SPLIT = false>
 __global__ void __launch_bounds__(64 + pair_epi_threads<EPI>(), 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmParams p) {
+    static_assert(BN == 128 || BN == 192 || BN == 256, "tile widths");
+    static_assert(!SPLIT || BN == 256, "split K: 256 x 256 tiles");
     static_assert(EPI != EPI_P_GEGLU_FP8 || BN == 256, "GeGLU: 128 gate and 128 up columns");
     using Cfg = GemmPairCfg<BN>;
     constexpr int STAGES = Cfg::STAGES;
@@ -295,7 +297,10 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             if constexpr (EPI == EPI_P_GEGLU_FP8)
                 epilogue_geglu_rows(p, t_acc + half * 32, t_acc + BN / 2 + half * 32, m_base, nt * (BN / 2) + half * 32, alpha,
                                     inv_os);
-            else if (finish)
+            else if constexpr (BN == 192) {                  // whole 64-column blocks: 128 + 64
+                if (half == 0) epilogue_rows<EPI, 128>(p, t_acc, m_base, nt * BN, stg, lines, alpha, inv_os);
+                else epilogue_rows<EPI, 64>(p, t_acc + 128, m_base, nt * BN + 128, stg, lines, alpha, inv_os);
+            } else if (finish)
                 epilogue_rows<EPI, BN / 2>(p, t_acc + half * (BN / 2), m_base, nt * BN + half * (BN / 2), stg, lines, alpha,
                                            inv_os);
             tc::tc_fence_before_sync();

@@ -203,3 +203,22 @@ def test_split_k_product(M, N, K):
         got = d_D.get()
         assert fvk.tensor_core_status() == 0
         assert np.array_equal(got[:M], plain.get()) and (got[M] == 0x5A5A).all() and (cnt.get() == 0).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(541, 9216, 2048), (2001, 3080, 2064), (1030, 2600, 2048)])
+def test_pair_tiles_of_192_columns(M, N, K):
+    """Sizes whose cheapest tile is 256 x 192, ragged in both directions: exact products plus bias give the oracle's bits."""
+    import torch
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, f32, rand_bf16
+    rng = np.random.default_rng(M + N)
+    e4 = lambda *s: torch.from_numpy(rng.choice(np.array([-2, -1, 0, 1, 2], np.float32), s)).to(torch.float8_e4m3fn)  # noqa: E731
+    A, W, bias = e4(M, K), e4(N, K), rand_bf16(rng, (N,), 0.5)
+    d_A, d_W, d_b, d_sa, d_sb = Dev(A.view(torch.uint8).numpy()), Dev(W.view(torch.uint8).numpy()), Dev(bias), f32(0.5), f32(0.0625)
+    d_D = Dev(np.full((M + 1, N), 0x5A5A, np.uint16))
+    g = fvk.GemmRunner()
+    g.fp8_nt_dev(d_A.ptr, d_W.ptr, d_D.ptr, M, N, K, d_sa.ptr, d_sb.ptr, bias=d_b.ptr)
+    acc = (A.float().cuda() @ W.float().cuda().T).cpu().numpy() * np.float32(0.03125)          # integers: exact
+    got = d_D.get()
+    assert fvk.tensor_core_status() == 0 and (got[M] == 0x5A5A).all()
+    assert np.array_equal(got[:M], O.f32_to_bf16_bits((acc + O.bf16_bits_to_f32(bias)).astype(np.float32)))
