@@ -210,7 +210,7 @@ def test_pair_tiles_of_192_columns(M, N, K):
     """Sizes whose cheapest tile is 256 x 192, ragged in both directions: exact products plus bias give the oracle's bits."""
     import torch
     from flashrt_b200 import flash_rt_kernels as fvk
-    from gpu_util import Dev, f32, rand_bf16
+    from gpu_util import Dev, f32, rand_bf16, zeros
     rng = np.random.default_rng(M + N)
     e4 = lambda *s: torch.from_numpy(rng.choice(np.array([-2, -1, 0, 1, 2], np.float32), s)).to(torch.float8_e4m3fn)  # noqa: E731
     A, W, bias = e4(M, K), e4(N, K), rand_bf16(rng, (N,), 0.5)
@@ -222,3 +222,9 @@ def test_pair_tiles_of_192_columns(M, N, K):
     got = d_D.get()
     assert fvk.tensor_core_status() == 0 and (got[M] == 0x5A5A).all()
     assert np.array_equal(got[:M], O.f32_to_bf16_bits((acc + O.bf16_bits_to_f32(bias)).astype(np.float32)))
+    # and bias + GELU + FP8 in the finish equals the separate launch
+    d_mid, d_two, d_one, d_so = zeros((M, N), np.uint16), zeros((M, N), np.uint8), zeros((M, N), np.uint8), f32(0.05)
+    g.fp8_nt_dev(d_A.ptr, d_W.ptr, d_mid.ptr, M, N, K, d_sa.ptr, d_sb.ptr)
+    fvk.bias_gelu_quantize_fp8_static_bf16(d_mid.ptr, d_b.ptr, d_two.ptr, d_so.ptr, M, N, 0)
+    g.fp8_nt_dev_bias_gelu_fp8(d_A.ptr, d_W.ptr, d_one.ptr, M, N, K, d_sa.ptr, d_sb.ptr, d_b.ptr, d_so.ptr, 0)
+    assert np.array_equal(d_one.get(), d_two.get())
