@@ -185,11 +185,13 @@ int* expert_loop_status_device_ptr();
 __device__ __forceinline__ uint4 ld_global_v4(const void* p) {
     return *reinterpret_cast<const uint4*>(p);
 }
-// streaming (read-once) 16-byte load that does not allocate in L1
+// streaming (read-once) 16-byte load that does not allocate in L1.  A coherent load: the non-coherent form (.nc) promises that
+// nobody writes the data while the kernel lives, and a kernel launched programmatically lives before its producer has ended
+// (some callers also write the row back in the same kernel).
 __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
     uint4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
     return r;
 }
 __device__ __forceinline__ float4 ld_global_f4(const float* p) {
@@ -208,8 +210,9 @@ __device__ __forceinline__ void st_global_v2(void* p, uint2 v) {
 // drains, about 1 us per launch.  Behind a kernel that never calls launch_dependents the attribute changes nothing.  The
 // caller's flag says more: weights, styles and scales do not come from the kernel in front and may be read before the wait
 // (`early`).
-// Inputs that the kernel in front may have written are no `const __restrict__` parameters: loads from such are invariant to
-// the compiler, which may then issue them above the wait.
+// Inputs are no `const __restrict__` parameters and are not read with non-coherent loads (.nc, __ldg): loads from such are
+// invariant to the compiler, which may then issue them above the wait, and need not see what the kernel in front wrote while
+// this one was already resident.
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

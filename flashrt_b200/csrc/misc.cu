@@ -27,8 +27,8 @@ __device__ __forceinline__ float load_a(const void* A, size_t i) {
 // chunk's weights of a thread are all in flight together, before the wait for the kernel in front when they may be (`early`).
 template <bool A_F32, bool D_F32>
 __global__ void __launch_bounds__(SG_COLS * SG_KS)
-small_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* __restrict__ B,
-                       void* __restrict__ Dv, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
+small_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* B,
+                       void* __restrict__ Dv, const __nv_bfloat16* bias, int M, int N, int K,
                        int accumulate, int early) {
     __nv_bfloat16* D = reinterpret_cast<__nv_bfloat16*>(Dv);
     float* Df = reinterpret_cast<float*>(Dv);
@@ -98,8 +98,8 @@ small_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* __restrict__ B,
 constexpr int SK_K = 32, SK_ROWS = 4, SK_THREADS = 128;
 template <bool A_F32, bool D_F32>
 __global__ void __launch_bounds__(SK_THREADS)
-short_k_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* __restrict__ B, void* __restrict__ Dv,
-                         const __nv_bfloat16* __restrict__ bias, int M, int N, int accumulate, int early) {
+short_k_gemm_bf16_kernel(const void* Av, const __nv_bfloat16* B, void* __restrict__ Dv,
+                         const __nv_bfloat16* bias, int M, int N, int accumulate, int early) {
     __shared__ float a_s[SK_ROWS][SK_K];
     const int n = (blockIdx.x * SK_THREADS + threadIdx.x) * 2;
     const int m0 = blockIdx.y * SK_ROWS;
@@ -181,11 +181,10 @@ __device__ __forceinline__ float sb_block_rms(float ssq, float* warp_tot, int di
 }
 
 __global__ void __launch_bounds__(1024)
-step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, const __nv_bfloat16* __restrict__ style_prev,
-                     const __nv_bfloat16* __restrict__ w_out, const __nv_bfloat16* __restrict__ b_out,
-                     const __nv_bfloat16* __restrict__ w_in, const __nv_bfloat16* __restrict__ b_in,
-                     const __nv_bfloat16* __restrict__ style_next, uint8_t* __restrict__ act8,
-                     const float* __restrict__ d_scale, int dim, float eps) {
+step_boundary_kernel(__nv_bfloat16* __restrict__ x, float* __restrict__ noise, const __nv_bfloat16* style_prev,
+                     const __nv_bfloat16* w_out, const __nv_bfloat16* b_out, const __nv_bfloat16* w_in,
+                     const __nv_bfloat16* b_in, const __nv_bfloat16* style_next, uint8_t* __restrict__ act8,
+                     const float* d_scale, int dim, float eps) {
     extern __shared__ float sb_smem[];
     float* a_s = sb_smem;                               // [dim] normalised row, then the new row (bf16 values)
     float* part = a_s + dim;                            // [16][32] K-slice partials of the out-projection

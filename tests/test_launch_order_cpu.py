@@ -1,0 +1,29 @@
+"""A kernel that waits for the one in front (``pdl_wait``) is resident while that one still writes, so what it reads has to
+come through coherent loads that stay behind the wait.  Read from the sources: the order of loads cannot be seen in results."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashrt_b200", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+
+
+WAITING = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and "pdl_wait()" in source(f))
+
+
+@pytest.mark.parametrize("name", WAITING)
+def test_kernels_that_wait_read_coherently(name):
+    text = source(name)
+    for word in ("ld.global.nc", "__ldg(", "__ldlu(", "ld_global_nc"):
+        assert word not in text, f"{name}: {word}"
+    text = re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", text)
+    kernels = re.findall(r"__global__\s+void\s+(\w+)\s*\(([^{;]*)\)\s*\{", text)
+    assert len(kernels) == text.count("__global__")
+    for kernel, params in kernels:
+        for p in params.split(","):
+            assert not ("const" in p and "*" in p and "__restrict__" in p), f"{name}: {kernel}: {' '.join(p.split())}"
