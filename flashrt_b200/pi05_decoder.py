@@ -817,6 +817,7 @@ class Pi05DecoderB200:
         self.calibration_source = "measured"
         tables = p.scale_tables()
         per_sample = [[] for _ in tables]
+        self.stream.wait_stream(torch.cuda.current_stream(self.device))      # what still writes the samples or the cache
         with torch.cuda.stream(self.stream):
             for nz in noises:
                 for t in tables:

@@ -200,6 +200,7 @@ class Pi05PrefixEncoderB200:
         k = torch.zeros(self.layers, self.max_seq, ENC_HD, dtype=BF16, device=self.device)
         v = torch.zeros_like(k)
         per = []
+        self.stream.wait_stream(torch.cuda.current_stream(self.device))      # what still writes the samples (and k, v)
         with torch.cuda.stream(self.stream):
             for e in embeds_list:
                 seq = self._check(e, k, v)
