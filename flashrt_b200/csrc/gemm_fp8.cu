@@ -112,7 +112,7 @@ struct GemmParams {
     int tile_gm;               // large-M kernels: m-tiles per group of the tile order
     int early;                 // the weights may be read before the kernel in front has finished
     float* split_ws;           // CTA-pair kernel with split K: partials and one counter per epilogue warp of a tile
-    int* split_cnt;
+    unsigned* split_cnt;
     int ksplits;
 };
 
@@ -1056,7 +1056,8 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
 
 // The same product for a caller with a workspace: above 256 rows a long K on few tiles may be split over CTA pairs, the
 // partials (fp32) added in split order by whichever warp of a tile comes last.  counters: 16 ints per 256 x 256 tile, zeroed
-// once by the caller, zero again behind every launch.  One launch at a time may use a workspace.
+// once by the caller, zero again behind every launch (also one whose bounded wait gave up).  One launch at a time may use a
+// workspace.
 int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
                                 const float* d_scale_b, const void* bias, float* workspace, long long workspace_bytes,
                                 int* counters, int flags, void* stream) {
@@ -1082,7 +1083,7 @@ int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, in
             p.N = N;
             p.kb_total = kbt;
             p.split_ws = workspace;
-            p.split_cnt = counters;
+            p.split_cnt = reinterpret_cast<unsigned*>(counters);
             p.ksplits = S;
             return launch_gemm_pair<256, EPI_P_BF16, true>(A, W, p, K, (cudaStream_t)stream);
         }

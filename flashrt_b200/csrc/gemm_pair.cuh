@@ -79,6 +79,13 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 }  // namespace tc
 
+// One of the S arrivals at a (tile, epilogue warp) counter, by one lane: the number of arrivals before it.  The S-th takes the
+// counter back to zero in the same operation, so a launch leaves all of them at zero as long as every unit arrives once --
+// a warp whose wait gave up arrives for its remaining units too (the sums it spoils are reported by the status word).
+__device__ __forceinline__ int split_k_arrive(const GemmParams& p, int unit, int S, int slot) {
+    return (int)atomicInc(p.split_cnt + (unit / S) * 16 + slot, (unsigned)(S - 1));
+}
+
 // Split K: an epilogue warp's 32 rows x NC columns of one split.  It leaves its partial in the workspace ([unit][warp][NC / 4]
 // [lane][4] floats: 512 bytes per store), then counts itself in; the last of the tile's S warps adds the partials in split
 // order, its own from tensor memory, and puts the sum back there for the finish.  Nobody waits.  False: not the last.
@@ -100,11 +107,10 @@ __device__ __forceinline__ bool split_k_sum(const GemmParams& p, uint32_t t_src,
     __threadfence();
     __syncwarp();
     int seen = 0;
-    if (lane == 0) seen = atomicAdd(p.split_cnt + (unit / S) * 16 + slot, 1);
+    if (lane == 0) seen = split_k_arrive(p, unit, S, slot);
     seen = __shfl_sync(0xffffffffu, seen, 0);
     if (seen != S - 1) return false;
     __threadfence();
-    if (lane == 0) p.split_cnt[(unit / S) * 16 + slot] = 0;          // for the next launch
 #pragma unroll 1
     for (int c = 0; c < NC; c += 32) {
         uint32_t v[32];
@@ -284,6 +290,9 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             if (!__all_sync(0xffffffffu, ok)) {
                 if (!*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_EPILOGUE | (blockIdx.x << 8));
                 *abort_flag = 1;
+                if constexpr (SPLIT)
+                    for (; t < total; t += npairs)
+                        if (lane == 0) split_k_arrive(p, t, S, (int)rank * 8 + (warp - 2));
                 break;
             }
             tc::tc_fence_after_sync();

@@ -123,8 +123,8 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
 /* frt_b200_gemm_fp8_nt for a caller with a workspace (the split K of cuBLASLt behind csrc/gemm/gemm_runner.cu:67-76, whose
  * workspace the runner owns): above 256 rows a long K on few tiles may be split, the fp32 partials added in a fixed order.
  * workspace: 16-byte aligned, 256 KB per (256 x 256 tile, split), at most one wave of CTA pairs (SMs / 2 x 256 KB is always
- * enough; with less the product is not split); counters: 16 ints per tile (8 x SMs suffice), zeroed once.  Launches that share
- * them must not overlap; after a non-zero status word zero the counters again.  flags bit 0 as above. */
+ * enough; with less the product is not split); counters: 16 ints per tile (8 x SMs suffice), zeroed once: every launch leaves
+ * them at zero, one whose bounded wait gave up included.  Launches that share them must not overlap.  flags bit 0 as above. */
 int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
                                 const float* d_scale_b, const void* bias, float* workspace, long long workspace_bytes,
                                 int* counters, int flags, void* stream);

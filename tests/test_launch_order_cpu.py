@@ -27,3 +27,16 @@ def test_kernels_that_wait_read_coherently(name):
     for kernel, params in kernels:
         for p in params.split(","):
             assert not ("const" in p and "*" in p and "__restrict__" in p), f"{name}: {kernel}: {' '.join(p.split())}"
+
+
+def test_split_k_counters_end_at_zero_when_a_wait_gives_up():
+    """The counters of the split-K product belong to the caller, who zeroes them once.  Every unit of a launch has to arrive
+    exactly once with an operation that wraps at S, on the path of a warp whose wait gave up as well: a count left between
+    0 and S would make the first arrival of the next launch take itself for the last and add a stale partial."""
+    text = source("gemm_pair.cuh")
+    uses = re.findall(r"[^\n]*split_cnt[^\n]*", text)
+    assert len(uses) == 1 and re.search(r"atomicInc\(p\.split_cnt \+ .*, \(unsigned\)\(S - 1\)\)", uses[0]), uses
+    gave_up = re.search(r"ERR_EPILOGUE(.*?)break;", text, flags=re.S).group(1)
+    assert re.search(r"if constexpr \(SPLIT\)\s+for \(; t < total; t \+= npairs\)\s+if \(lane == 0\) split_k_arrive\(p, t, S, ",
+                     gave_up), gave_up
+    assert text.count("split_k_arrive(") == 3          # the definition, the sum, the path that gave up
