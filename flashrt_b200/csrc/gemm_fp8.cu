@@ -1095,8 +1095,9 @@ int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, in
 // ("kn") layout (csrc/bindings.cpp:706-716, flash_rt/models/pi05/pipeline_rtx.py:550-562):
 //   D(M,N) bf16 = alpha_host * (*d_scale_a) * (*d_scale_b) * A(M,K) . B(K,N) + bias.
 // The weight tiles arrive as boxes of 128 K-rows x 128 N-bytes and feed the MMA as an MN-major operand; accumulation
-// order and result are those of frt_b200_gemm_fp8_nt on the transposed weights (bit for bit).  K % 128 == 0,
-// N % 16 == 0; M <= 256 runs the token-major kernel, larger M the persistent kernel (N >= 128).
+// order and result are those of frt_b200_gemm_fp8_nt on the transposed weights (bit for bit) at M > 256 and wherever both
+// are given the same splits of 1, 2, 4 or 8.  K % 128 == 0, N % 16 == 0; M <= 256 runs the token-major kernel, larger M the
+// persistent kernel (N >= 128).
 int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, int K, const float* d_scale_a,
                          const float* d_scale_b, float alpha_host, const void* bias, int splits, int flags,
                          void* stream) {
@@ -1128,7 +1129,9 @@ int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, in
 // QKV projection with the RoPE + split + KV-append epilogue fused (M <= 256):
 //   row = alpha * A(M,K) . W(N,K)^T rounded to bf16, N = q_dim + k_dim + v_dim; q and k parts rotated pairwise
 //   with rope (M, head_dim) = [cos0, sin0, ...]; Q -> (M, q_dim); K, V rows -> row (*devpos + m) (devpos NULL: m).
-// Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_qkv_split_rope.
+// Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_qkv_split_rope at the same splits of 1, 2, 4 or 8 (without
+// one the plain product may go to the unsplit kernels of the large products, which have no such finish: another order of
+// sums).
 int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, const float* d_scale_a,
                                     const float* d_scale_b, const void* rope, void* Q, void* Kout, void* Vout,
                                     const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim, int splits,
@@ -1173,7 +1176,8 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
 // one):
 //   W (2*half, K): rows [0, half) = gate, [half, 2*half) = up.  out8 (M, half) =
 //   e4m3(clamp(gelu_tanh(bf16(gate)) * bf16(up) * (1 / *d_out_scale), +-448)).  half % 64 == 0.
-// Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_geglu_fp8.  flags bit 6: SiLU gate instead of GELU
+// Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_geglu_fp8 at the same splits of 1, 2, 4 or 8 (M > 256: at
+// splits 0 or 1).  flags bit 6: SiLU gate instead of GELU
 // (SwiGLU; M <= 128, K % 128 == 0: the token-major kernel), byte-identical to frt_b200_geglu_fp8 with its bit 1.
 int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int M, int half, int K,
                                    const float* d_scale_a, const float* d_scale_b, const float* d_out_scale,

@@ -373,8 +373,8 @@ class GemmRunner:
     def fp8_nn_dev(self, A, B, D, M, N, K, d_scale_a, d_scale_b, stream=0, *, pdl=False, splits=0, bias=None,
                    tile_n=0):
         """D(M,N) bf16 = sa*sb * A(M,K) . B(K,N) — weights stored (K,N), the reference's default ``fp8_layout == "kn"``
-        form (csrc/bindings.cpp:706-716).  Same result as ``fp8_nt_dev`` on the transposed weights.  K % 128 == 0,
-        N % 16 == 0, N >= 128."""
+        form (csrc/bindings.cpp:706-716).  Same bits as ``fp8_nt_dev`` on the transposed weights for M > 256 and at the
+        same ``splits`` of 1, 2, 4 or 8; otherwise K may be summed in another order.  K % 128 == 0, N % 16 == 0, N >= 128."""
         call("frt_b200_gemm_fp8_nn", A, B, D, M, N, K, d_scale_a, d_scale_b, 1.0, bias, splits,
              _f(pdl) | _tile_hint(tile_n), stream)
 

@@ -14,7 +14,7 @@ What differs from the reference's composition (same arithmetic, fewer launches a
     one copy per action token; the gate of the next residual is read straight from the style row;
   * the attention kernel also emits the FP8 copy the output projection reads (no separate quantise launch);
   * RoPE + split + KV append run in the epilogue of the QKV GEMM and GeGLU -> FP8 in the epilogue of the gate|up
-    GEMM (byte-identical to the separate kernels, which the calibration pass still uses);
+    GEMM (at a given split of K byte-identical to the separate kernels, which the calibration pass uses without one);
   * FP8 weights are (N, K) K-contiguous (``fp8_nt_dev``);
   * the action out-projection adds its bias and accumulates into the noise buffer in the same launch, and that
     Euler state is held in fp32 (the reference keeps it in bf16, whose half-ulp at |x| ~ 4 is already 0.016);

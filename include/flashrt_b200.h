@@ -131,7 +131,9 @@ int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, in
 /* GemmRunner::fp8_nn_dev (csrc/bindings.cpp:706-716 -> csrc/gemm/gemm_runner.cu:67-76), the reference's default weight
  * layout: B stored (K, N) row-major.  D(M,N) bf16 = alpha_host * (*d_scale_a) * (*d_scale_b) * A(M,K) . B(K,N) + bias.
  * The weight tiles are loaded as 128 K-rows x 128 N-bytes and consumed as an MN-major MMA operand; the result equals
- * frt_b200_gemm_fp8_nt on the transposed weights bit for bit.  K % 128 == 0, N % 16 == 0, N >= 128. */
+ * frt_b200_gemm_fp8_nt on the transposed weights bit for bit at M > 256 (no split), and at M <= 256 when both are given the
+ * same `splits` of 1, 2, 4 or 8.  With splits = 0 each entry point takes what is fastest for it -- split K or not -- and the
+ * results agree to the rounding of another order of sums.  K % 128 == 0, N % 16 == 0, N >= 128. */
 int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, int K, const float* d_scale_a,
                          const float* d_scale_b, float alpha_host, const void* bias, int splits, int flags,
                          void* stream);
@@ -140,16 +142,17 @@ int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, in
  * QKV projection + qkv_split_rope[_devpos] (csrc/bindings.cpp:1071-1099 -> csrc/kernels/rope.cu:135-277):
  *   the (M, q_dim+k_dim+v_dim) result is rounded to bf16, q and k parts are rotated pairwise with
  *   rope (M, head_dim) = [cos0, sin0, cos1, sin1, ...]; Q -> (M, q_dim); K / V rows -> row (*devpos + m)
- *   of Kout / Vout (devpos NULL: row m).  Byte-identical to frt_b200_gemm_fp8_nt (same `splits`) followed by
- *   frt_b200_qkv_split_rope. */
+ *   of Kout / Vout (devpos NULL: row m).  Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_qkv_split_rope when
+ *   both are given the same `splits` of 1, 2, 4 or 8; with splits = 0 the two choose on their own (see
+ *   frt_b200_gemm_fp8_nn). */
 int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, const float* d_scale_a,
                                     const float* d_scale_b, const void* rope, void* Q, void* Kout, void* Vout,
                                     const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim, int splits,
                                     int flags, void* stream);
 /* gate|up projection + gate_geglu_merged_fp8 (csrc/bindings.cpp:1037-1044 -> csrc/kernels/activation.cu:249-279):
  *   W (2*half, K), rows [0, half) = gate, [half, 2*half) = up; out8 (M, half) e4m3 with scale *d_out_scale.
- *   half % 64 == 0; M > 256: half % 128 == 0, out8 16-byte aligned.  Byte-identical to frt_b200_gemm_fp8_nt (same `splits`)
- *   followed by frt_b200_geglu_fp8.
+ *   half % 64 == 0; M > 256: half % 128 == 0, out8 16-byte aligned.  Byte-identical to frt_b200_gemm_fp8_nt followed by
+ *   frt_b200_geglu_fp8 when both are given the same `splits` of 1, 2, 4 or 8 (M > 256: when that product is not split).
  *   flags bit 6: SiLU gate (SwiGLU; M <= 128 and K % 128 == 0 only, else -2), byte-identical to frt_b200_geglu_fp8
  *   with its flags bit 1 behind the same GEMM.
  *   flags bit 7 (here and in the _rowscale / norm_gemm forms): GELU(tanh) through the hardware tanh (tanh.approx.f32,
@@ -359,7 +362,7 @@ int frt_b200_norm_gemm_fp8_nt_geglu_fp8(const void* x, const float* stats_in, in
 /* fp8 GEMM (GemmRunner::fp8_nt_dev, csrc/bindings.cpp:717-727) + bias_gelu_quantize_fp8_static_bf16
  * (csrc/bindings.cpp:3427-3440 -> csrc/quantize/bias_gelu_quantize_fp8.cu:24-49) in one launch, M > 256, N >= 128:
  *   out8 (M, N) e4m3 = clamp(gelu_tanh(bf16(sa * sb * A . W^T) + bias) * (1 / *d_out_scale), +-448)
- * byte-identical to the two separate calls.  flags bit 7: GELU through the hardware tanh (tanh.approx.f32, 2^-11
+ * byte-identical to the two separate calls (the product not split).  flags bit 7: GELU through the hardware tanh (tanh.approx.f32, 2^-11
  * relative) -- at K = 3072 the exact form (about 36 instructions per value on 8 epilogue warps) takes longer than the
  * MMAs of the tile; codes then differ from the exact form by single last-place flips. */
 int frt_b200_gemm_fp8_nt_bias_gelu_fp8(const void* A, const void* W, void* out8, int M, int N, int K,
