@@ -52,15 +52,17 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// 2^x of a pair on the fma pipe: x = n + f with n = floor(x) (round-down addition of 1.5 * 2^23), 2^f on [0, 1) by a
-// polynomial of degree 5 with p(0) = 1 (own least-squares fit of the relative error, reweighted towards its maximum: 1.4e-7 in
-// fp32 arithmetic, the accuracy of ex2.approx), n added to the exponent field.  x is clamped at -127, where the result is 0.
+// 2^x of a pair on the fma pipe: x = n + f with n = floor(x), 2^f on [0, 1) by a polynomial of degree 5 with p(0) = 1 (own
+// least-squares fit of the relative error, reweighted towards its maximum: 1.4e-7 in fp32 arithmetic, the accuracy of
+// ex2.approx), n added to the exponent field.  The reduction and the exponent put together as an integer are Cody and Waite's
+// (Software Manual for the Elementary Functions, 1980), the round-down addition of 1.5 * 2^23 gives floor(x) in the low bits;
+// a share of the softmax's exponentials taken off the exponential unit this way is the scheme published with FlashAttention-4.
+// x is clamped at -127, where the result is 0.  A NaN comes out as 0 as well; the kernel keeps it in the row's maximum, which
+// makes every other probability of the chunk NaN (2^n as a factor instead would keep it here, at 6 % of the kernel's time).
 __device__ __forceinline__ void exp2_pair(uint64_t x, float& e0, float& e1) {
     float x0, x1;
     f32x2_parts(x, x0, x1);
-    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x0));      // a NaN score must not come out as probability 0
-    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x1));
-    x = f32x2(x0, x1);
+    x = f32x2(fmaxf(x0, -127.0f), fmaxf(x1, -127.0f));
     const uint64_t magic = f32x2(12582912.0f, 12582912.0f);
     uint64_t t, f;
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(t) : "l"(x), "l"(magic));
@@ -76,6 +78,11 @@ __device__ __forceinline__ void exp2_pair(uint64_t x, float& e0, float& e1) {
     f32x2_parts(t, t0, t1);
     e0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
     e1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 __global__ void __launch_bounds__(320, 1)
 attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -264,12 +271,12 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
             for (int i = 0; i < BKV; i += 4) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(mx4[q], __uint_as_float(sv[i + q]));
+                for (int q = 0; q < 4; ++q) mx4[q] = max_nan(mx4[q], __uint_as_float(sv[i + q]));
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            const float mx = max_nan(max_nan(mx4[0], mx4[1]), max_nan(mx4[2], mx4[3]));
             const float mx_s = mx * p.scale_log2;               // scale_log2 > 0
-            // keep the stale maximum unless it is exceeded by more than the threshold
-            const bool grow = mx_s > m_run + Cfg::RESCALE_THRESHOLD || (m_run == -INFINITY && mx_s > -INFINITY);
+            // keep the stale maximum unless it is exceeded by more than the threshold; a NaN always replaces it
+            const bool grow = !(mx_s <= m_run + Cfg::RESCALE_THRESHOLD);
             const float m_new = grow ? mx_s : m_run;
             if (__any_sync(0xffffffffu, grow && j > 0)) {       // warp-uniform: tcgen05.ld / st are collective
                 const float alpha = grow ? tc::ex2_approx(m_run - m_new) : 1.0f;   // m_run = -inf -> 0
@@ -332,7 +339,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int tok = tok0 + t * tok_per_tile + row / p.G;
                 const int hq = hk * p.G + row % p.G;
                 const bool store = tok < p.Sq;
-                const float invl = l_run > 0.0f ? 1.0f / l_run : 0.0f;
+                // a score of +inf: inf - inf (its exponential may have been one of exp2_pair's)
+                const float invl = m_run == INFINITY ? NAN : l_run > 0.0f ? 1.0f / l_run : 0.0f;
                 const float inv_os = p.O_fp8 ? __fdiv_rn(1.0f, *p.out_scale) : 0.0f;
                 const size_t obase = (size_t)b * p.o_bs + (size_t)(store ? tok : 0) * p.o_rs + (size_t)hq * p.o_hs;
 #pragma unroll 1
