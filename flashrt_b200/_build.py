@@ -8,12 +8,13 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libflashrt_b200.so")
-CALLS = os.path.join(HERE, "_native_calls.so")
+CALLS = os.path.join(HERE, "_native_calls" + sysconfig.get_config_var("EXT_SUFFIX"))     # one per interpreter version
 OBJ = os.path.join(CSRC, "build")
 
 NVCC_FLAGS = [
@@ -73,13 +74,18 @@ def calls_source(protos: dict[str, list[str]]) -> str:
 
 def build_calls(force: bool = False) -> str | None:
     """The extension module behind ``_lib.call``; None where the interpreter's headers or a C compiler are missing (the ctypes
-    path then serves every call)."""
-    import sysconfig
+    path then serves every call).  A module of another header or library, or one without an interpreter tag (any version
+    would import it), does not stay behind."""
     from ._lib import HEADER_PATH, parse_header
     inc, cc = sysconfig.get_paths()["include"], shutil.which("gcc") or shutil.which("cc")
+    stale = force or _stale(CALLS, [HEADER_PATH, os.path.abspath(__file__), LIB])
+    untagged = os.path.join(os.path.dirname(CALLS), "_native_calls.so")
+    for old in {untagged, CALLS} if stale else {untagged} - {CALLS}:
+        if os.path.exists(old):
+            os.remove(old)
     if cc is None or not os.path.exists(os.path.join(inc, "Python.h")):
-        return None
-    if force or _stale(CALLS, [HEADER_PATH, os.path.abspath(__file__), LIB]):
+        return None if stale else CALLS
+    if stale:
         src = os.path.join(OBJ, "native_calls.c")
         with open(src, "w") as f:
             f.write(calls_source(parse_header()))

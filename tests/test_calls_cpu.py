@@ -22,3 +22,21 @@ def test_native_calls_agree_with_ctypes():
         _lib.call_status("frt_b200_norm_fp8", *args[:9], 1.5, *args[10:])
     with pytest.raises(_lib.KernelError):
         _lib.call("frt_b200_norm_fp8", *args)
+
+
+def test_call_module_belongs_to_one_interpreter(monkeypatch, tmp_path):
+    """The module's file carries the interpreter's tag, and where it cannot be built again neither a stale one nor one that any
+    interpreter would import stays behind."""
+    import os
+    import sysconfig
+    from flashrt_b200 import _build
+    native = pytest.importorskip("flashrt_b200._native_calls")
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert suffix != ".so" and native.__file__ == _build.CALLS and _build.CALLS.endswith("_native_calls" + suffix)
+    calls, untagged = tmp_path / ("_native_calls" + suffix), tmp_path / "_native_calls.so"
+    monkeypatch.setattr(_build, "CALLS", str(calls))
+    monkeypatch.setattr(_build.shutil, "which", lambda name: None)
+    for f in (calls, untagged):
+        f.write_bytes(b"")
+        os.utime(f, (1, 1))
+    assert _build.build_calls() is None and not calls.exists() and not untagged.exists()
