@@ -355,9 +355,10 @@ def run_ours(args):
                                     "gemm_tok_kernel (M=%d projections of the loop: weight streaming)" % M),
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4),
-                         # not measured in this run: dram read + write of one launch from the ncu capture under
-                         # profiles/ (1.005 x the algorithmic read bytes; the result stays in L2), scaled by bytes
-                         "traffic": int(1.005 * (gemm_bytes - gemm_out_bytes)),
+                         # not measured in this run: dram read + write of one launch from the ncu capture of the
+                         # attention-out projection under profiles/ (2.335 MB, 1.013 x the algorithmic read bytes; the
+                         # result stays in L2), scaled by bytes
+                         "traffic": int(1.013 * (gemm_bytes - gemm_out_bytes)),
                          "traffic_source": "carried over from the ncu capture in profiles/, scaled by bytes",
                          "peak_source": peak_src,
                          "avg_launch_us": round(gemm_us, 3), "algorithmic_bytes_per_launch": int(gemm_bytes)},
@@ -372,7 +373,7 @@ def run_ours(args):
 
 
 def nvfp4_summary(args, local: int) -> dict:
-    """configs[3] in short: the NVFP4 loop at batch 1 and batch 4, graph replay only (ms per loop)."""
+    """The NVFP4 loop in short: at batch 1 and batch 4, graph replay only (ms per loop)."""
     import torch
     from flashrt_b200 import load_model
     from flashrt_b200.pi05_decoder import ACTION_DIM
@@ -697,7 +698,7 @@ def ops_table(args, quick: bool):
 
 
 def ops_summary(args) -> dict:
-    """configs[1] in short for the default line: worst norm fraction of HBM peak, the FP8 GEMM fractions at M >= 2048
+    """The operator sweep in short for the default line: worst norm fraction of HBM peak, the FP8 GEMM fractions at M >= 2048
     (of 2 x the measured bf16 burst), how many of the 18 reach 0.60, and the ratio to cuBLASLt per shape."""
     table, _, _ = ops_table(args, quick=True)
     norm = [r for r in table if r["op"] == "residual_add_rms_norm_fp8"]
@@ -721,9 +722,8 @@ def run_ops(args):
             "config": {"workload": "configs[1] operator sweep", "peaks": peaks,
                        "l2": ("norm and M <= 256 GEMM cases cycle through distinct row / weight buffers totalling more than "
                               "L2; M >= 2048 GEMM cases alternate two weight buffers (tensor-bound)"),
-                       "large_m_fp8_kernel": ("cta pair (256 x 256 tiles) forced" if args.cta_pair else
-                                              "library's choice: cta pair for >= 2 waves of 256 x 256 tiles at "
-                                              "K >= 2048, else persistent one-CTA tiles"),
+                       "large_m_fp8_kernel": ("256 x 256 tiles on CTA pairs, forced" if args.cta_pair else
+                                              "library's choice by a cost of whole waves of tiles"),
                        "library_baseline": "torch._scaled_mm (cuBLASLt FP8) and torch SDPA on the same tensors",
                        "tensor_core_status": fvk.tensor_core_status(), "table": table},
             "gpu_launches": launches}
@@ -922,8 +922,7 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--calib-samples", type=int, default=8, help="calibration noises (8 = the named config)")
     ap.add_argument("--no-pdl", action="store_true",
-                    help="chain kernels with plain stream order instead of programmatic dependent launch "
-                         "(Nsight Compute cannot profile programmatically dependent launches)")
+                    help="no early reads: nothing but set-up happens in a kernel before the one in front of it has ended")
     ap.add_argument("--persistent-loop", action="store_true",
                     help="pi05 / fp8: run the whole denoise loop as one persistent cooperative kernel")
     ap.add_argument("--cta-pair", action="store_true",
@@ -936,10 +935,10 @@ def main():
     ap.add_argument("--lean", action="store_true",
                     help="skip the CPU baseline and the GEMM roofline leg (for short runs under a profiler)")
     ap.add_argument("--workload", default="pi05", choices=["pi05", "wan", "ops", "prefix", "timeline"],
-                    help="pi05 = the headline action-expert loop (default); wan = the video-DiT step (configs[4]); "
-                         "ops = the operator sweep of configs[1] (norm / FP8 GEMM / NVFP4 GEMM)")
+                    help="pi05 = the headline action-expert loop (default); wan = the video-DiT step; "
+                         "ops = the operator sweep (norm / FP8 GEMM / NVFP4 GEMM)")
     ap.add_argument("--precision", default="fp8", choices=["fp8", "nvfp4"],
-                    help="pi05 workload: fp8 = configs[2] (default, the headline), nvfp4 = configs[3]")
+                    help="pi05 workload: fp8 (default, the headline) or nvfp4")
     ap.add_argument("--batch", type=int, default=1, help="pi05 workload with --precision nvfp4: chunks per loop (1 or 4)")
     ap.add_argument("--wan-layers", type=int, default=30)
     ap.add_argument("--wan-exact-gelu", action="store_true",

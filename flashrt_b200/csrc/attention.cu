@@ -814,8 +814,8 @@ static void* g_attn_static_ptr[64] = {nullptr};
 // caller's stream in front of the kernel: make that first call before any stream capture (inside a capture it is
 // refused with -1).  Every call uses the same array, which keeps whatever the previous call left in it (the kernel
 // overwrites the partials it reads and its arrival counters only ever grow), so two calls whose kernels can overlap on the
-// GPU -- different streams, or graph branches -- would corrupt each other.  After a call whose bounded wait gave up
-// (frt_b200_attention_status != 0) the counters are stale: frt_b200_attention_status(1) clears them as well.
+// GPU -- different streams, or graph branches -- would corrupt each other.  A call whose bounded wait gave up has counted all
+// its CTAs in as well; frt_b200_attention_status(1) clears the counters after one all the same.
 int frt_b200_attention_fwd_bf16_static_scratch(const void* Q, const void* K, const void* V, void* O, void* O_fp8,
                                                const float* out_scale, float* lse, const int* seqused_k, int batch,
                                                int seqlen_q, int seqlen_k, int num_heads_q, int num_heads_kv,
@@ -874,8 +874,8 @@ extern "C" {
 
 // returns (and optionally clears) the attention kernels' device status word; 0 = no bounded wait gave up.
 // code 0x11 = TMA producer, 0x12 = MMA issuer, 0x13 = softmax warps.  Synchronises the device.  Clearing a
-// non-zero status also clears the arrival counters of the built-in scratch on the current device (a kernel that
-// gave up leaves them mid-count, and the static-scratch caller has no buffer of its own to re-zero).
+// non-zero status also clears the arrival counters of the built-in scratch on the current device (they stand at a multiple
+// of 256 behind every launch, also one that gave up; a caller's own counters need no clearing either).
 int frt_b200_attention_status(int reset) {
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return FRT_CUDA_ERR(e);

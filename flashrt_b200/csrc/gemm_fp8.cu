@@ -1002,8 +1002,9 @@ extern "C" {
 // D(M,N) bf16 = alpha_host * (*d_scale_a) * (*d_scale_b) * A(M,K) . W(N,K)^T + bias
 // A, W: FP8 E4M3 row-major, K contiguous.  K % 16 == 0; A, W 16-byte aligned.
 // splits: 0 = choose, otherwise the split-K factor (clamped to [1, 8]).
-// flags: bit0 = programmatic dependent launch; bit1 = one-tile-per-CTA kernel for M > 256; bit3 = force the CTA-pair
-// kernel (256 x 256 tiles, M > 256, N >= 256, no split-K; chosen by itself for long tile lists), bit5 = never use it.
+// flags: bit0 = the weights are settled and may be read before the kernel in front has ended; bit1 = one-tile-per-CTA kernel
+// for M > 256; bit3 = 256 x 256 tiles on CTA pairs (M > 256, N >= 256, no split-K), bit5 = no CTA pairs; without them the
+// tiles are chosen by large_cost.
 int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
                          const float* d_scale_b, float alpha_host, const void* bias, int splits, int flags,
                          void* stream) {
@@ -1172,8 +1173,8 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
 
 // gate|up projection with the GeGLU -> FP8 epilogue fused (M <= 256, or any M when half % 128 == 0; larger M runs on CTA pairs
 // whose 256 columns are 128 gate and 128 up features: the activation, 30 instructions per value, runs under the MMAs of the
-// next tile instead of in a pass of its own over 2 x M x 2 half bytes -- 768 x 32768 x 2048: 41 + 26 us as two launches, 54 as
-// one):
+// next tile instead of in a pass of its own over 2 x M x 2 half bytes -- 768 x 32768 x 2048: 43 + 29 us as two launches, 42 as
+// one; 541 rows: 44 + 20 against 54):
 //   W (2*half, K): rows [0, half) = gate, [half, 2*half) = up.  out8 (M, half) =
 //   e4m3(clamp(gelu_tanh(bf16(gate)) * bf16(up) * (1 / *d_out_scale), +-448)).  half % 64 == 0.
 // Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_geglu_fp8 at the same splits of 1, 2, 4 or 8 (M > 256: at

@@ -9,8 +9,9 @@ on a non-zero status instead of failing silently.  Entry points of the reference
 lie outside the denoise path raise :class:`NotBuilt` (the analogue of the reference's
 "extension not built" refusal, ``flash_rt/_extensions.py:67-108``).
 
-Optional keyword ``pdl=True`` (not in the reference) launches with programmatic
-dependent launch; the B200 pipeline uses it, reference call sites never pass it.
+Optional keyword ``pdl=True`` (not in the reference): weights, scales and styles are settled
+and may be read before the launches in front have ended; the B200 pipeline uses it, reference
+call sites never pass it.
 """
 from __future__ import annotations
 
@@ -266,10 +267,9 @@ class GemmRunner:
                    one_tile_per_cta=False, cta_pair=None, swapped=False, tile_n=0):
         """D(M,N) bf16 = sa*sb * A(M,K) . B(N,K)^T — weights stored (N,K), the ``fp8_layout == "nk"`` form.
         ``one_tile_per_cta`` selects the non-persistent large-M kernel (same result; kept for comparison runs);
-        ``cta_pair`` True / False forces / forbids the 256 x 256-tile kernel on CTA pairs (M > 256, N >= 256; by
-        default the library uses it for tile lists of at least two waves at K >= 2048).  M <= 256: ``swapped``
-        keeps the weights-on-lanes kernel instead of the token-major one, ``tile_n`` (64 / 128 / 256) pins the
-        token-major kernel's tile width."""
+        ``cta_pair`` True forces 256 x 256 tiles on CTA pairs, False forbids pairs (M > 256, N >= 256; by default the
+        tiles are chosen by a cost of whole waves).  M <= 256: ``swapped`` keeps the weights-on-lanes kernel instead of
+        the token-major one, ``tile_n`` (64 / 128 / 256) pins the token-major kernel's tile width."""
         call("frt_b200_gemm_fp8_nt", A, B, D, M, N, K, d_scale_a, d_scale_b, 1.0, bias, splits,
              _f(pdl) | (2 if one_tile_per_cta else 0) | (8 if cta_pair else 0) | (32 if cta_pair is False else 0)
              | (16 if swapped else 0)

@@ -176,9 +176,9 @@ def rope_table(start: int, count: int) -> torch.Tensor:
 def projection_tiles(rows: int):
     """Tile width / split-K of the four projections (QKV, attention-out, gate|up, FFN-down) of the folded loop, from timings
     of the whole captured loop.  Up to 64 rows one m-tile does; up to 128 rows two tiles of 64 beat one of 128 (the narrow
-    N = 1024 / 2560 products leave the chip idle: 100 rows 7.00 ms per loop against 7.09-7.9); above, the MMA's fixed cost per
-    128-row weight tile makes two tiles of up to 128 better than four of 64 (200 rows 8.45 against 9.3), except for the
-    QKV product, where both do the same."""
+    N = 1024 / 2560 products leave the chip idle: 100 rows 6.23 ms per loop against 6.71, and 9.0 with the library's own
+    choice); above, the MMA's fixed cost per 128-row weight tile makes two tiles of up to 128 better than four of 64 (200 rows
+    8.06 ms against 9.80, 150 rows 7.10 against 8.81), except for the QKV product, where both do the same."""
     if rows <= 64:
         return (dict(splits=4, tile_n=64), dict(splits=8, tile_n=64), dict(splits=2, tile_n=128), dict(splits=8, tile_n=64))
     half = rows <= 128
@@ -663,7 +663,7 @@ class Pi05DecoderB200:
         # the four launches between two Euler steps (final norm, action out-projection, action in-projection, first norm)
         # as one launch per step boundary, bit-identical to the four (batch 1 without guidance, folded norms)
         self.fuse_step_io = bool(fuse_step_io) and self.fold_norms
-        # the whole loop as one cooperative kernel (phases separated by grid barriers) instead of 1300 launches
+        # the whole loop as one cooperative kernel (phases separated by grid barriers) instead of 912 launches
         self.persistent_loop = bool(persistent_loop)
         if self.persistent_loop and precision != "fp8":
             raise ValueError("persistent_loop is built for the FP8 loop")

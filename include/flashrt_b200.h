@@ -14,10 +14,12 @@
  *   -4  the request exceeds a built-in fixed-size buffer (entry points that say so)
  *   -(1000 + cudaError_t) for a CUDA runtime failure at launch.
  *
- * `flags` bit 0: launch with programmatic dependent launch (the kernel starts
- * its input-independent prologue before the previous kernel in the stream has
- * finished; only set it when scales / weights / styles are not written by that
- * previous kernel).
+ * Kernels are launched programmatically: their set-up runs while the kernel in
+ * front drains, and they wait for it before they touch anything it writes.
+ * `flags` bit 0: scales / weights / styles may be read before that wait.  Set it
+ * only when they were settled before the run of launches began: the kernel in
+ * front is not the only one that may still be running by then, since it lets its
+ * successor start before its own wait has returned.
  *
  * Citations name the reference entry point each function stands in for, as
  * path:line inside the FlashRT source tree.
@@ -109,14 +111,16 @@ int frt_b200_qkv_split_rope(const void* qkv, const void* rope, void* Q, void* K,
  *   splits: 0 = choose; else split-K factor in [1, 16] (reduced inside a thread-block cluster).  At M > 256 the
  *   library never chooses a split itself: a 128 x 256 fp32 tile per rank through distributed shared memory costs
  *   several times what the split saves (measured 2048 x 3072 x 14336: 92 us unsplit, 284 us with splits = 2).
- *   M > 256 runs as a persistent kernel (one CTA per SM walking the tile list, two accumulators in tensor memory so
- *   that the epilogue overlaps the next tile's MMAs); flags bit 1 selects the one-tile-per-CTA kernel instead;
- *   tile lists of at least two waves with K >= 2048 (or flags bit 3; M > 256, N >= 256, no split-K) run a kernel with
- *   one 256 x 256 tile per CTA pair (tcgen05 cta_group::2: each CTA stages its 128 rows of A and 128 of the 256 weight
- *   rows, the leader issues the MMAs for both); flags bit 5 keeps the one-CTA persistent kernel.
- *   M <= 128 (up to 256 with a pinned tile width or split) with K % 128 == 0 and N % 8 == 0 runs the token-major kernel (activation rows on the 128 accumulator
- *   lanes, up to 256 weight rows on the columns, split-K in {1, 2, 4, 8} over a cluster); flags bit 4 keeps the
- *   swapped kernel (weights on the lanes) instead; flags bits 8-9 pin the tile width (1 = 64, 2 = 128, 3 = 256). */
+ *   M > 256 runs as a persistent kernel (two accumulators in tensor memory, so that the epilogue overlaps the next tile's
+ *   MMAs) on the tiles that a cost by whole waves finds cheapest: 128 x 128 or 128 x 256 per CTA, or 256 x 128, 192 or 256
+ *   per CTA pair (tcgen05 cta_group::2: each CTA stages its 128 rows of A and half of the weight rows, the leader issues
+ *   the MMAs for both).  flags bit 1 selects the one-tile-per-CTA kernel instead, bit 3 256 x 256 tiles on pairs (N >= 256),
+ *   bit 5 keeps the one-CTA tiles.
+ *   M <= 128 (up to 256 with a pinned tile width or split) with K % 128 == 0 and N % 8 == 0 runs the token-major kernel
+ *   (activation rows on the 128 accumulator lanes, up to 256 weight rows on the columns, split-K in {1, 2, 4, 8} over a
+ *   cluster), other M <= 256 the swapped kernel (weights on the lanes, split-K too); without a split or a hint the kernels of
+ *   M > 256 take 17 .. 256 rows as well where the same costs put them in front.  flags bit 4 keeps the swapped kernel, bits
+ *   8-9 pin the token-major tile width (1 = 64, 2 = 128, 3 = 256). */
 int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, int K, const float* d_scale_a,
                          const float* d_scale_b, float alpha_host, const void* bias, int splits, int flags,
                          void* stream);
@@ -177,13 +181,13 @@ int frt_b200_gemm_status(int reset);
  *   e4m3(clamp(O * (1 / *out_scale), +-448)) written with O's indexing (NULL to skip).
  *   lse: optional (batch, num_heads_q, seqlen_q) fp32; seqused_k: optional device int (valid keys).
  *   kv_splits: 0 = choose, else 1..8, rounded down to a power of two (combined inside a thread-block cluster;
- *   no scratch buffers).  kv_static_rows: leading K/V rows that the previous kernel in the stream does not
- *   write (with flags bit0 they are fetched before that kernel has finished); pass 0 if unsure.
- *   With seqused_k, -n: all valid rows but the last n, and *seqused_k is not written by that kernel either.
+ *   no scratch buffers).  kv_static_rows: leading K/V rows that no launch in flight writes (with flags bit 0 they are
+ *   fetched before the kernel in front has finished); pass 0 if unsure.
+ *   With seqused_k, -n: all valid rows but the last n, and *seqused_k is not written by a launch in flight either.
  *   o_accum, lse_accum, counters: optional split-KV scratch (all three or none): o_accum (splits, batch,
  *   num_heads_q, seqlen_q, head_dim) fp32 and lse_accum (splits, batch, num_heads_q, seqlen_q) fp32 -- the
  *   reference's FA2 split-kv buffers -- and counters = 2 unsigned per (128-row tile, kv head, batch), zeroed once
- *   by the caller.  Given scratch, the head_dim-256 kernel may run more CTAs than (tiles x splits): the grid
+ *   by the caller (every launch adds 256 to the counters it uses, one whose bounded wait gave up included).  Given scratch, the head_dim-256 kernel may run more CTAs than (tiles x splits): the grid
  *   (tiles x kv heads x batch x splits) must then fit the device in one wave, else -2 is returned.  When four times
  *   that grid fits as well, every (tile, split) is cut into four head-dim parts, and the kv splits of a part
  *   exchange their partials (a) as one thread-block cluster through distributed shared memory -- scratch and counters

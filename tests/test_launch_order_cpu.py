@@ -40,3 +40,12 @@ def test_split_k_counters_end_at_zero_when_a_wait_gives_up():
     assert re.search(r"if constexpr \(SPLIT\)\s+for \(; t < total; t \+= npairs\)\s+if \(lane == 0\) split_k_arrive\(p, t, S, ",
                      gave_up), gave_up
     assert text.count("split_k_arrive(") == 3          # the definition, the sum, the path that gave up
+
+
+@pytest.mark.parametrize("name", ["attention.cu", "attention_d256.cuh"])
+def test_attention_counters_count_every_cta(name):
+    """A tile's arrival counter stands at a multiple of 256 behind every launch: each CTA arrives, whether its waits returned
+    or gave up."""
+    text = re.sub(r"\s*ATT_STAMP\(\d+\);", "", source(name))
+    found = re.findall(r"__threadfence\(\);\s*__syncthreads\(\);\s*if \(threadIdx\.x == 0\) \{\s*asm volatile\(\"red\.relaxed\.gpu", text)
+    assert len(found) == text.count("red.relaxed.gpu") == 1
