@@ -716,10 +716,10 @@ def run_ops(args):
     table, launches, peaks = ops_table(args, quick=False)
     from flashrt_b200 import flash_rt_kernels as fvk
     big = [r for r in table if r["op"] == "gemm_fp8" and r["M"] >= 2048]
-    line = {"metric": "operator sweep (configs[1])", "value": round(statistics.mean(r["frac_tensor"] for r in big), 4),
+    line = {"metric": "operator sweep", "value": round(statistics.mean(r["frac_tensor"] for r in big), 4),
             "unit": "mean fraction of 2 x measured bf16 peak over the FP8 GEMMs with M >= 2048", "n_gpus": 1,
             "steps": 1, "warmup": 3, "higher_is_better": True, "data": "synthetic", "dtype": "fp8_e4m3 / nvfp4 / bf16",
-            "config": {"workload": "configs[1] operator sweep", "peaks": peaks,
+            "config": {"workload": "operator sweep", "peaks": peaks,
                        "l2": ("norm and M <= 256 GEMM cases cycle through distinct row / weight buffers totalling more than "
                               "L2; M >= 2048 GEMM cases alternate two weight buffers (tensor-bound)"),
                        "large_m_fp8_kernel": ("256 x 256 tiles on CTA pairs, forced" if args.cta_pair else
