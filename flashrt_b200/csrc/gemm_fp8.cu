@@ -1173,13 +1173,13 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
 
 // gate|up projection with the GeGLU -> FP8 epilogue fused (M <= 256, or any M when half % 128 == 0; larger M runs on CTA pairs
 // whose 256 columns are 128 gate and 128 up features: the activation, 30 instructions per value, runs under the MMAs of the
-// next tile instead of in a pass of its own over 2 x M x 2 half bytes -- 768 x 32768 x 2048: 43 + 29 us as two launches, 42 as
-// one; 541 rows: 44 + 20 against 54):
+// next tile instead of in a pass of its own over 2 x M x 2 half bytes -- 768 x 32768 x 2048 with gate values of unit variance:
+// 45 + 25 us as two launches, 45 as one; 541 rows: 42 + 21 against 49-60):
 //   W (2*half, K): rows [0, half) = gate, [half, 2*half) = up.  out8 (M, half) =
 //   e4m3(clamp(gelu_tanh(bf16(gate)) * bf16(up) * (1 / *d_out_scale), +-448)).  half % 64 == 0.
 // Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_geglu_fp8 at the same splits of 1, 2, 4 or 8 (M > 256: at
-// splits 0 or 1).  flags bit 6: SiLU gate instead of GELU
-// (SwiGLU; M <= 128, K % 128 == 0: the token-major kernel), byte-identical to frt_b200_geglu_fp8 with its bit 1.
+// splits 0 or 1).  flags bit 6: SiLU gate instead of GELU (SwiGLU; M <= 128, K % 128 == 0: the token-major kernel),
+// byte-identical to frt_b200_geglu_fp8 with its bit 1.
 int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int M, int half, int K,
                                    const float* d_scale_a, const float* d_scale_b, const float* d_out_scale,
                                    int splits, int flags, void* stream) {
