@@ -129,6 +129,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_sr
 #pragma unroll 1
         for (int c = 0; c < NC; c += 32) {
             uint32_t v[32];
+            __syncwarp();                                   // tcgen05.ld is the whole warp's; lanes beyond M skip the stores
             tc::tmem_ld32(t_src + c, v);
             tc::tmem_ld_wait();
             if (m >= p.M) continue;

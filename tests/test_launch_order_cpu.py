@@ -49,3 +49,12 @@ def test_attention_counters_count_every_cta(name):
     text = re.sub(r"\s*ATT_STAMP\(\d+\);", "", source(name))
     found = re.findall(r"__threadfence\(\);\s*__syncthreads\(\);\s*if \(threadIdx\.x == 0\) \{\s*asm volatile\(\"red\.relaxed\.gpu", text)
     assert len(found) == text.count("red.relaxed.gpu") == 1
+
+
+def test_lanes_that_skip_stores_meet_before_the_next_collective_load():
+    """tcgen05.ld is executed by a whole warp: the loop around one whose lanes may take a ``continue`` starts with a warp
+    barrier."""
+    text = source("gemm_persistent.cuh")
+    head = text[:text.index("if (m >= p.M) continue;")]
+    head = head[head.rindex("for (int c"):]
+    assert 0 < head.find("__syncwarp();") < head.index("tmem_ld") and text.count("continue;") == 1
