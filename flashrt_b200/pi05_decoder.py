@@ -738,6 +738,7 @@ class Pi05DecoderB200:
         self._dev_status = torch.zeros(4, dtype=torch.int32, device=dev)
         self._pinned_status = torch.zeros(4, dtype=torch.int32).pin_memory()
         self.latency_records: list[float] = []
+        self.stream.wait_stream(torch.cuda.current_stream(dev))       # weights, tables and buffers were written there
 
     # ---- prefix (what the encoder would have written) ---------------------
     def set_prefix(self, prefix_k: torch.Tensor, prefix_v: torch.Tensor) -> None:

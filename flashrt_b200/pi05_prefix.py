@@ -121,6 +121,7 @@ class Pi05PrefixEncoderB200:
         self.scratch_scale = torch.zeros(1, dtype=torch.float32, device=dev)
         self.gemm = fvk.GemmRunner()
         self.stream = torch.cuda.Stream(device=dev)
+        self.stream.wait_stream(torch.cuda.current_stream(dev))       # weights, tables and buffers were written there
         self.calibrated = False
 
     # ------------------------------------------------------------------

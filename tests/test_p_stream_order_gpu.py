@@ -42,3 +42,20 @@ def test_encoder_calibration_waits_for_its_samples():
     want = enc.act_scale.clone()
     enc.calibrate([_late(embeds)])
     assert torch.equal(enc.act_scale, want)
+
+
+@pytest.mark.parametrize("precision", ["fp8", "nvfp4"])
+def test_models_start_behind_the_stream_that_loaded_them(precision, monkeypatch):
+    """Weights, tables and buffers are written on the caller's stream; the model's own stream waits for them, whatever call
+    comes first."""
+    from flashrt_b200 import load_model
+    from flashrt_b200.pi05_decoder import synthetic_state_dict
+    from flashrt_b200.pi05_prefix import Pi05PrefixEncoderB200
+    waits, wait = [], torch.cuda.Stream.wait_stream
+    monkeypatch.setattr(torch.cuda.Stream, "wait_stream", lambda s, other: (waits.append((s, other)), wait(s, other))[1])
+    with torch.cuda.stream(torch.cuda.Stream()):
+        here = torch.cuda.current_stream()
+        fe = load_model(synthetic_state_dict(seed=0, layers=1), config="pi05", layers=1, chunk_size=16, prefix_len=64,
+                        precision=precision)._fe
+        enc = Pi05PrefixEncoderB200("synthetic:0", layers=1, max_seq=64)
+    assert (fe.stream, here) in waits and (enc.stream, here) in waits
