@@ -74,6 +74,22 @@ int make_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
     return r == CUDA_SUCCESS ? FRT_OK : FRT_ERR_INVALID;
 }
 
+// Scale atoms of the block-scaled products: a row of 128 operand rows is katoms atoms of 512 bytes, seen as 64-bit words; box =
+// the four atoms of a k-block (2048 bytes) x box_rows, no swizzle.  Atom rows beyond the buffer arrive as zeros.
+static int make_tmap_sf(CUtensorMap* out, const void* base, uint64_t rblocks, uint64_t katoms, uint32_t box_rows) {
+    int rc = ensure_encode();
+    if (rc) return rc;
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (katoms & 3)) return FRT_ERR_INVALID;
+    cuuint64_t dims[2] = {katoms * 64, rblocks};
+    cuuint64_t strides[1] = {katoms * 512};
+    cuuint32_t box[2] = {256, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? FRT_OK : FRT_ERR_INVALID;
+}
+
 // ------------------------------------------------------------------ kernel
 struct GemmParams {
     __nv_bfloat16* out;        // (M, N) row-major
@@ -748,9 +764,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
 
 // ------------------------------------------------------------------ host launch
 struct TmapKey {
-    const void* base; uint64_t rows, row_bytes, pitch; uint32_t box_rows;
+    const void* base; uint64_t rows, row_bytes, pitch; uint32_t box_rows; bool sf;
     bool operator==(const TmapKey& o) const {
-        return base == o.base && rows == o.rows && row_bytes == o.row_bytes && pitch == o.pitch && box_rows == o.box_rows;
+        return base == o.base && rows == o.rows && row_bytes == o.row_bytes && pitch == o.pitch && box_rows == o.box_rows &&
+               sf == o.sf;
     }
 };
 struct TmapKeyHash {
@@ -758,26 +775,32 @@ struct TmapKeyHash {
         size_t h = std::hash<const void*>()(k.base);
         h ^= k.rows * 0x9e3779b97f4a7c15ull + (h << 6);
         h ^= k.row_bytes * 0xc2b2ae3d27d4eb4full + (h >> 3);
-        h ^= (k.pitch << 8) ^ k.box_rows;
+        h ^= (k.pitch << 8) ^ (k.box_rows << 1) ^ (k.sf ? 1 : 0);
         return h;
     }
 };
 static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> g_tmaps;
 
-int get_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch,
-                   uint32_t box_rows) {
-    TmapKey k{base, rows, row_bytes, pitch, box_rows};
+static int get_tmap(CUtensorMap* out, const TmapKey& k) {
     {
         std::lock_guard<std::mutex> lk(g_mu);
         auto it = g_tmaps.find(k);
         if (it != g_tmaps.end()) { *out = it->second; return FRT_OK; }
     }
-    int rc = make_tmap_2d_u8(out, base, rows, row_bytes, pitch, box_rows);
+    int rc = k.sf ? make_tmap_sf(out, k.base, k.rows, k.row_bytes / 512, k.box_rows)
+                  : make_tmap_2d_u8(out, k.base, k.rows, k.row_bytes, k.pitch, k.box_rows);
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_tmaps.size() > 65536) g_tmaps.clear();
     g_tmaps[k] = *out;
     return FRT_OK;
+}
+int get_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch,
+                   uint32_t box_rows) {
+    return get_tmap(out, TmapKey{base, rows, row_bytes, pitch, box_rows, false});
+}
+static int get_tmap_sf(CUtensorMap* out, const void* base, int rblocks, int katoms, uint32_t box_rows) {
+    return get_tmap(out, TmapKey{base, (uint64_t)rblocks, (uint64_t)katoms * 512, 0, box_rows, true});
 }
 
 // K counts elements; a row holds K bytes (FP8) or K / 2 bytes (packed NVFP4)
@@ -912,28 +935,63 @@ static int dispatch_small_m(const void* A, const void* W, GemmParams p, int K, i
 #include "gemm_pair.cuh"
 #include "gemm_tok.cuh"
 
+// NVFP4 small-M kernel: k split and column tile (tokens per CTA) of M <= 256 rows, and what the launch takes in us.
+struct Nvfp4Small { int bn, splits; double us; };
+
 // NVFP4, M <= 256.  Column tiles of 64 tokens while all of them fit one wave, since the finish of a tile grows with its
 // columns -- us per wave 4.5 / 6.2 / 8.8 for 64 / 128 / 256 (200 x 1024 x 2048: 12.6 as one tile of 256, 6.7 as four of 64;
 // 200 x 8192 x 1024: 9.0 / 6.6 (128) / 9.9 (64, two waves)) -- and the k split only as far as it leaves them in one wave
 // (200 x 2560 x 1024: 11 with split 4, 4.7 without; the action expert's loop at 4 x 50 rows 65.4 -> 57.3 us per block).
-template <int EPI>
-static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, int K, int M, int tiles, int splits,
-                                  bool pdl, cudaStream_t s) {
-    int sp = pick_splits(tiles, p.kb_total, splits);
+// `us`: fitted to 150 products of 16 .. 256 rows, N 1024 .. 14336, K 1024 .. 14336 in a graph (5 % standard deviation).
+static Nvfp4Small pick_small_m_nvfp4(int M, int N, int K, int splits) {
+    const int tiles = (N + 127) / 128, kb = K / 256;
     const long long sms = device_sm_count();
+    int sp = pick_splits(tiles, kb, splits);
     while (splits <= 0 && sp > 1 && (long long)tiles * ((M + 63) / 64) * sp > sms) sp /= 2;
-    if (M <= 32) return launch_gemm<32, true, EPI, true>(A, W, p, K, sp, pdl, s);
     static const int wave_cost[3] = {45, 62, 88};
-    int bn = 0;
-    long long best = 0;
-    for (int i = 0; i < 3 && (i == 0 || (32 << i) < M); ++i) {
-        const long long ctas = (long long)tiles * ((M + (64 << i) - 1) / (64 << i)) * sp;
-        const long long cost = (ctas + sms - 1) / sms * wave_cost[i];
-        if (bn == 0 || cost < best) { best = cost; bn = 64 << i; }
+    static const double fixed[4] = {3.2, 4.35, 6.15, 8.0}, per_kb[4] = {0.31, 0.317, 0.346, 0.462};
+    int bn = 32;
+    long long best = 0, waves = 1;
+    for (int i = 0; M > 32 && i < 3 && (i == 0 || (32 << i) < M); ++i) {
+        const long long w = ((long long)tiles * ((M + (64 << i) - 1) / (64 << i)) * sp + sms - 1) / sms;
+        if (bn == 32 || w * wave_cost[i] < best) { best = w * wave_cost[i]; bn = 64 << i; waves = w; }
     }
-    if (bn == 64) return launch_gemm<64, true, EPI, true>(A, W, p, K, sp, pdl, s);
-    if (bn == 128) return launch_gemm<128, true, EPI, true>(A, W, p, K, sp, pdl, s);
-    return launch_gemm<256, true, EPI, true>(A, W, p, K, sp, pdl, s);
+    const int c = bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3;
+    const double us = waves * (fixed[c] + per_kb[c] * ((kb + sp - 1) / sp) + (sp > 1 ? 1.2 + 0.005 * M : 0.0)) - 0.1;
+    return {bn, sp, us};
+}
+template <int EPI>
+static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, int K, int M, int splits, bool pdl,
+                                  cudaStream_t s) {
+    const Nvfp4Small c = pick_small_m_nvfp4(M, p.N, K, splits);
+    if (c.bn == 32) return launch_gemm<32, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
+    if (c.bn == 64) return launch_gemm<64, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
+    if (c.bn == 128) return launch_gemm<128, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
+    return launch_gemm<256, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
+}
+
+// NVFP4 on CTA pairs: columns of the 256-row tile (0: the small-M kernel is the faster one), by a cost of whole waves -- a fixed
+// part, then per wave a finish and the k-blocks of 256: 3.1 + waves (0.54 + 0.252 kb) for 128 columns, 3.2 + (0.94 + 0.283 kb)
+// for 192, 3.1 + (1.34 + 0.315 kb) for 256.  Fitted to 270 products (M 50 .. 16384, N 1024 .. 14336, K 1024 .. 14336, standard
+// deviation 6-8 %); the choice is within 1 % of the fastest on average.  Against the kernels that served M > 256 before (128 x
+// 128 tiles of one CTA, persistent, or 128 x 256, one tile each): 16384 x 14336 x 14336 1756 -> 1099 us (6.1 PFLOP/s), 8192 x
+// 3072 x 3072 52 -> 33, 2501 x 3072 x 3072 22.2 -> 13.9, 300 x 1024 x 1024 5.3 -> 4.4.  At most 64 rows stay with the small-M
+// kernel: a pair's 256-row boxes are mostly padding there (16 x 8192 x 14336: 18.8 against 31), and in a chain of launches its
+// larger CTAs on twice the SMs keep the next launches from fetching their weights early (the loop of 50 tokens, with one
+// product or all four on pairs: 7.06 -> 7.08 .. 7.43 ms; with 4 x 50 tokens 10.1 -> 9.2).
+static int pick_nvfp4_pair(int M, int N, int K) {
+    if (M <= 64 || (M > 256 && N <= 64)) return 0;
+    static const struct { int tn; double fixed, wave, per_kb; } c[3] = {
+        {128, 3.1, 0.54, 0.252}, {192, 3.2, 0.94, 0.283}, {256, 3.1, 1.34, 0.315}};
+    const int pairs = device_sm_count() / 2;
+    int best = 0;
+    double t = M <= 256 ? pick_small_m_nvfp4(M, N, K, 0).us : 1e30;
+    for (const auto& k : c) {
+        const long long tiles = (long long)((M + 255) / 256) * ((N + k.tn - 1) / k.tn);
+        const double tk = k.fixed + (double)((tiles + pairs - 1) / pairs) * (k.wave + k.per_kb * (K / 256));
+        if (tk < t) { t = tk; best = k.tn; }
+    }
+    return best;
 }
 
 // ------------------------------------------------------------------ choice among the large-M FP8 kernels
@@ -1237,22 +1295,17 @@ int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const 
     p.sf_col = (const uint8_t*)SFW;
     cudaStream_t s = (cudaStream_t)stream;
     bool pdl = flags & 1;
-    if (M <= 256) return dispatch_small_m_nvfp4<EPI_BF16>(A, W, p, K, M, (N + 127) / 128, splits, pdl, s);
-    int sp = splits > 0 ? pick_splits(1, p.kb_total, splits > 8 ? 8 : splits) : 1;
-    // Persistent kernel on 128 x 128 tiles (the finish of a tile under the MMAs of the next: 0.32 us per k-block and wave, not
-    // under 2.4) or one CTA per 128 x 256 tile (fewer operand bytes, but every wave pays its set-up and finish: 5.4 + 0.40 per
-    // k-block), whichever is cheaper by whole waves; fitted to M 300 .. 8192, N 1024 .. 14336, K 1024 .. 14336, where it picks
-    // the faster one (8192 x 14336 x 3072: 209 us against 261; 2501 x 1024 x 8192: 25.3 against 18.0).
-    if (sp == 1 && N > 64 && !(flags & 2)) {
-        const int sms = device_sm_count();
-        const long long mt = (M + 127) / 128;
-        const double kb = p.kb_total;
-        const double wave_p = 0.32 * kb + 0.2 > 2.4 ? 0.32 * kb + 0.2 : 2.4;
-        const double t_persistent = 4.6 + wave_p * (double)((mt * ((N + 127) / 128) + sms - 1) / sms);
-        const double t_one = 0.6 + (5.4 + 0.40 * kb) * (double)((mt * ((N + 255) / 256) + sms - 1) / sms);
-        if (N < 256 || (flags & 4) || t_persistent <= t_one)
-            return launch_gemm_persistent<128, EPI_P_BF16, true>(A, W, p, K, s);
+    p.early = pdl ? 1 : 0;
+    int pair = 0;
+    if (splits <= 1 && !(flags & 2)) {
+        pair = ((flags >> 8) & 3) ? 64 + 64 * ((flags >> 8) & 3) : pick_nvfp4_pair(M, N, K);
+        if (splits == 1 && M <= 256) pair = 0;
     }
+    if (pair == 128) return launch_gemm_pair<128, EPI_P_BF16, false, true>(A, W, p, K, s);
+    if (pair == 192) return launch_gemm_pair<192, EPI_P_BF16, false, true>(A, W, p, K, s);
+    if (pair == 256) return launch_gemm_pair<256, EPI_P_BF16, false, true>(A, W, p, K, s);
+    if (M <= 256) return dispatch_small_m_nvfp4<EPI_BF16>(A, W, p, K, M, splits, pdl, s);
+    int sp = splits > 0 ? pick_splits(1, p.kb_total, splits > 8 ? 8 : splits) : 1;
     if (N >= 256) return launch_gemm<256, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     if (N > 64) return launch_gemm<128, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
     return launch_gemm<64, false, EPI_BF16, true>(A, W, p, K, sp, pdl, s);
@@ -1287,8 +1340,14 @@ int frt_b200_gemm_nvfp4_nt_rope_split(const void* A, const void* SFA, const void
     p.k_dim = k_dim;
     p.v_dim = v_dim;
     p.head_dim = head_dim;
-    return dispatch_small_m_nvfp4<EPI_ROPE_SPLIT>(A, W, p, K, M, (p.N + 127) / 128, splits, flags & 1,
-                                                  (cudaStream_t)stream);
+    // on CTA pairs where the plain product goes there: the same sums, so the pair of launches gives the same bytes
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(rope) | reinterpret_cast<uintptr_t>(Q) |
+                           reinterpret_cast<uintptr_t>(Kout) | reinterpret_cast<uintptr_t>(Vout);
+    if (splits <= 0 && !(ptrs & 15) && !((q_dim | k_dim | v_dim | head_dim) & 7) && pick_nvfp4_pair(M, p.N, K)) {
+        p.early = flags & 1;
+        return launch_gemm_pair<128, EPI_P_ROPE, false, true>(A, W, p, K, (cudaStream_t)stream);
+    }
+    return dispatch_small_m_nvfp4<EPI_ROPE_SPLIT>(A, W, p, K, M, splits, flags & 1, (cudaStream_t)stream);
 }
 
 // Row-parallel projection of the action expert with the following norm kernel fused (M <= 64, N = 128 .. 1024):

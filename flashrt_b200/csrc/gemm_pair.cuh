@@ -21,15 +21,30 @@
 // bounded by the kernel deadline; the CTAs meet at a cluster barrier before either leaves.
 #pragma once
 
-template <int BN>                                         // columns of the pair's tile (BN / 2 weight rows per CTA)
+//
+// NVFP4 (FP4 = true): the same protocol with k-blocks of 256 packed e2m1 elements (128 bytes a row) and, behind the operand
+// tiles of a stage, the block scales: the CTA's own 128 rows of A (2 KB) and ALL the tile's columns (2 KB per 128; 192 columns
+// touch two atom rows wherever they start, at row 0 or 64 of the first), since each SM multiplies its 128 rows by every
+// column.  They go to tensor memory with tcgen05.cp in front of the k-block's MMAs.  What bounds this product is the operand
+// traffic from L2: a 128 x 128 tile per CTA takes 36 KB per 270 clocks of math, a pair of 256 x 256 38 KB per 540.
+// 256 columns: two accumulators and the 48 scale columns are more than the 512 of tensor memory, so the accumulators share
+// 64 columns (0..255 and 192..447).  The warps that hold the shared columns read them first and release them at once; the
+// MMAs of the next tile wait for that one read (about 0.3 us per tile) and not for the finish.
+template <int BN, bool FP4 = false>                       // columns of the pair's tile (BN / 2 weight rows per CTA)
 struct GemmPairCfg {
     static constexpr int A_BYTES = 128 * 128;
     static constexpr int B_BYTES = BN / 2 * 128;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
-    static constexpr int STAGES = BN >= 192 ? 6 : 8;
+    static constexpr int SFA_BYTES = FP4 ? 2048 : 0;
+    static constexpr int SFB_ROWS = (BN + 127) / 128;       // 128-row atom rows of the columns' scales
+    static constexpr int SFB_BYTES = FP4 ? SFB_ROWS * 2048 : 0;
+    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;   // per CTA
+    static constexpr int STAGES = FP4 ? (BN >= 192 ? 5 : 6) : BN >= 192 ? 6 : 8;
     static constexpr int EPI_STAGE_BYTES = 8 * 32 * 128;    // line staging of the eight epilogue warps
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_STAGE_BYTES;
-    static constexpr int TMEM_COLS = BN == 128 ? 256 : 512;  // two accumulators
+    static constexpr int TMEM_COLS = BN == 128 && !FP4 ? 256 : 512;  // two accumulators (and the scales)
+    static constexpr bool OVERLAP = FP4 && BN == 256;
+    static constexpr int ACC_STRIDE = OVERLAP ? 192 : BN;   // columns from one accumulator to the other
+    static constexpr int SF_COL = ACC_STRIDE + BN;          // scales of A: 4 columns per K = 64; of W: 4 per atom row
 };
 // epilogue threads per CTA: the GeGLU finish is a chain of 30 dependent instructions per value, which sixteen warps hide
 // where eight do not
@@ -73,9 +88,6 @@ __device__ __forceinline__ void mma_commit_both(uint32_t bar_addr) {
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar_addr),
         "h"((uint16_t)3)
         : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 }  // namespace tc
 
@@ -140,13 +152,17 @@ __device__ __forceinline__ bool split_k_sum(const GemmParams& p, uint32_t t_src,
     return true;
 }
 
-template <int BN, int EPI, bool SPLIT = false>
+// tmSA, tmSW: scale atoms of the NVFP4 form (copies of the operand maps otherwise)
+template <int BN, int EPI, bool SPLIT = false, bool FP4 = false>
 __global__ void __launch_bounds__(64 + pair_epi_threads<EPI>(), 1)
-gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmParams p) {
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
+                     const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSW, GemmParams p) {
     static_assert(BN == 128 || BN == 192 || BN == 256, "tile widths");
     static_assert(!SPLIT || BN == 256, "split K: 256 x 256 tiles");
     static_assert(EPI != EPI_P_GEGLU_FP8 || BN == 256, "GeGLU: 128 gate and 128 up columns");
-    using Cfg = GemmPairCfg<BN>;
+    static_assert(!FP4 || (!SPLIT && (EPI == EPI_P_BF16 || (EPI == EPI_P_ROPE && BN == 128))), "forms of the NVFP4 product");
+    static_assert(EPI != EPI_P_ROPE || FP4, "RoPE finish: NVFP4");
+    using Cfg = GemmPairCfg<BN, FP4>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -184,6 +200,10 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tc::mbar_fence_init();
         tc::tma_prefetch_desc(&tmA);
         tc::tma_prefetch_desc(&tmW);
+        if (FP4) {
+            tc::tma_prefetch_desc(&tmSA);
+            tc::tma_prefetch_desc(&tmSW);
+        }
     }
     if (warp == 1) {
         tc::tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
@@ -196,8 +216,30 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
     pdl_launch_dependents();
 
+    // weight tile (and column scales) of a k-block of n-tile nt; the leader posts the byte count of the whole stage first
+    auto load_weights = [&](uint32_t dst, uint32_t bar, uint32_t own, int kb, int nt) {
+        // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
+        const int n0 = EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
+        if (rank == 0) tc::mbar_arrive_expect_tx(own, 2 * Cfg::STAGE_BYTES);
+        tc::tma_load_2d_pair(dst + Cfg::A_BYTES, &tmW, bar, kb * 128, n0);
+        if constexpr (FP4)
+            tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES, &tmSW, bar, kb * 256, nt * BN / 128);
+    };
+
     if (warp == 0) {
         // ---------------- TMA producer (whole warp, see warp_wait; both CTAs): its half of A and of the weight rows, bytes posted at the leader
+        // Settled weights (p.early): the pair's first ring of weight tiles is fetched before the wait for the kernel in front
+        int ahead = 0;                // k-blocks of the first tile whose weights are on their way
+        if (p.early && pair < total) {
+            int mt, nt;
+            order.at(SPLIT ? pair / S : pair, mt, nt);
+            const int kb0 = k_begin(pair), n = k_end(pair) - kb0;
+            ahead = n < STAGES ? n : STAGES;
+            const uint32_t ring = tc::smem_u32(smem), full_a = tc::smem_u32(full);
+            if (tc::elect_one())
+                for (int s = 0; s < ahead; ++s)
+                    load_weights(ring + s * Cfg::STAGE_BYTES, tc::dsmem_map(full_a, 0) + 8 * s, full_a + 8 * s, kb0 + s, nt);
+        }
         pdl_wait();
         const uint32_t ring = tc::smem_u32(smem), empty_a = tc::smem_u32(empty), full_a = tc::smem_u32(full);
         const uint32_t lead_full = tc::dsmem_map(full_a, 0);
@@ -208,8 +250,6 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             int mt, nt;
             order.at(SPLIT ? t / S : t, mt, nt);
             const int m0 = mt * 256 + (int)rank * 128;
-            // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
-            const int n0 = EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
             const int kb1 = k_end(t);
             for (int kb = k_begin(t); kb < kb1; ++kb) {
                 if (!tc::warp_wait(empty_a + 8 * s, ph, ready, deadline, abort_flag)) {
@@ -223,15 +263,19 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (++s == STAGES) { s = 0; ph ^= 1; }
                 ready = tc::mbar_test(empty_a + 8 * s, ph);
                 if (tc::elect_one()) {
-                    if (rank == 0) tc::mbar_arrive_expect_tx(own, 2 * Cfg::STAGE_BYTES);
+                    if (ahead <= 0) load_weights(dst, bar, own, kb, nt);
                     tc::tma_load_2d_pair(dst, &tmA, bar, kb * 128, m0);
-                    tc::tma_load_2d_pair(dst + Cfg::A_BYTES, &tmW, bar, kb * 128, n0);
+                    if constexpr (FP4)
+                        tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES, &tmSA, bar, kb * 256, m0 / 128);
                 }
+                --ahead;
             }
         }
     } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer (whole warp, leader only): accumulator i & 1 for the pair's i-th tile
-        constexpr uint32_t idesc = tc::make_idesc(0, 0, 0, 0, 256, BN);
+        constexpr uint32_t idesc = FP4 ? tc::make_idesc_nvfp4(256, BN) : tc::make_idesc(0, 0, 0, 0, 256, BN);
+        const uint32_t sf0 = tc::smem_u32(smem + Cfg::A_BYTES + Cfg::B_BYTES);
+        const uint32_t tmem_sfa = tmem + Cfg::SF_COL, tmem_sfw = tmem_sfa + 16;
         const uint64_t dA0 = tc::make_desc_kmajor_sw128(tc::smem_u32(smem));
         const uint64_t dB0 = tc::make_desc_kmajor_sw128(tc::smem_u32(smem + Cfg::A_BYTES));
         const uint32_t full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty);
@@ -241,13 +285,24 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         bool ready = false, failed = false;
         for (int t = pair; t < total; t += npairs, ++i) {
             const int buf = i & 1;
-            if (!tc::warp_wait(accE_a + 8 * buf, (uint32_t)(((i >> 1) - 1) & 1), i < 2, deadline, abort_flag)) {
+            // this accumulator's tile before the last one is drained; with shared columns: those of the last tile are read
+            const bool free_acc = Cfg::OVERLAP
+                ? tc::warp_wait(accE_a + 8 * (buf ^ 1), (uint32_t)(((i - 1) >> 1) & 1), i < 1, deadline, abort_flag)
+                : tc::warp_wait(accE_a + 8 * buf, (uint32_t)(((i >> 1) - 1) & 1), i < 2, deadline, abort_flag);
+            if (!free_acc) {
                 if (lane == 0 && !*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_MMA | (blockIdx.x << 8));
                 *abort_flag = 1;
                 break;
             }
             tc::tc_fence_after_sync();
-            const uint32_t d_tm = tmem + buf * BN;
+            const uint32_t d_tm = tmem + buf * Cfg::ACC_STRIDE;
+            // the tile's first column is row 0 or (192-wide tiles) row 64 of its first scale atom: two columns further on
+            uint32_t sfw_tm = tmem_sfw;
+            if constexpr (FP4 && BN == 192) {
+                int mt, nt;
+                order.at(t, mt, nt);
+                sfw_tm += (uint32_t)(nt & 1) * 2;
+            }
             const int kb0 = k_begin(t), kb1 = k_end(t);
             for (int kb = kb0; kb < kb1; ++kb) {
                 if (!tc::warp_wait(full_a + 8 * s, ph, ready, deadline, abort_flag)) {
@@ -258,10 +313,24 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
                 tc::tc_fence_after_sync();
                 const uint64_t so = (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
-                const uint32_t done = empty_a + 8 * s;
+                const uint32_t sf = sf0 + (uint32_t)(s * Cfg::STAGE_BYTES), done = empty_a + 8 * s;
                 if (++s == STAGES) { s = 0; ph ^= 1; }
                 ready = tc::mbar_test(full_a + 8 * s, ph);
                 if (tc::elect_one()) {
+                    if constexpr (FP4) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            tc::tmem_cp_sf_atom_pair(tmem_sfa + 4 * k, sf + 512 * k);
+#pragma unroll
+                            for (int j = 0; j < Cfg::SFB_ROWS; ++j)
+                                tc::tmem_cp_sf_atom_pair(tmem_sfw + (k * Cfg::SFB_ROWS + j) * 4,
+                                                         sf + Cfg::SFA_BYTES + j * 2048 + 512 * k);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            tc::mma_nvfp4_pair(d_tm, dA0 + so + 2 * k, dB0 + so + 2 * k, idesc, tmem_sfa + 4 * k,
+                                               sfw_tm + k * Cfg::SFB_ROWS * 4, (kb > kb0 || k > 0) ? 1u : 0u);
+                    } else
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
                         tc::mma_f8_pair(d_tm, dA0 + so + 2 * k, dB0 + so + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
@@ -280,12 +349,19 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         float alpha = p.alpha_host;
         if (p.sa) alpha *= *p.sa;
         if (p.sb) alpha *= *p.sb;
-        const float inv_os = (EPI != EPI_P_BF16) ? __fdiv_rn(1.0f, *p.out_scale) : 0.0f;
+        const float inv_os = EPI != EPI_P_BF16 && EPI != EPI_P_ROPE ? __fdiv_rn(1.0f, *p.out_scale) : 0.0f;
         const bool lines = epilogue_lines<EPI>(p);
+        const int pos = EPI == EPI_P_ROPE && p.devpos ? *p.devpos : 0;
         uint8_t* stg = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * (32 * 128);
         int i = 0;
         for (int t = pair; t < total; t += npairs, ++i) {
             const int buf = i & 1;
+            uint4 tab[EPI == EPI_P_ROPE ? 8 : 1];
+            if constexpr (EPI == EPI_P_ROPE) {
+                int mt, nt;
+                order.at(t, mt, nt);
+                rope_table_rows(p, mt * 256 + (int)rank * 128 + q * 32 + lane, nt * BN + half * 64, tab);
+            }
             const bool ok = tc::mbar_wait_until(&acc_full[buf], (uint32_t)((i >> 1) & 1), deadline, abort_flag);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (!*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_EPILOGUE | (blockIdx.x << 8));
@@ -298,12 +374,28 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             tc::tc_fence_after_sync();
             int mt, nt;
             order.at(SPLIT ? t / S : t, mt, nt);
-            const uint32_t t_acc = tmem + buf * BN + lane_off;
+            const uint32_t t_acc = tmem + buf * Cfg::ACC_STRIDE + lane_off;
             bool finish = true;
             if constexpr (SPLIT)
                 finish = split_k_sum<BN / 2>(p, t_acc + half * (BN / 2), t, S, (int)rank * 8 + (warp - 2));
             const int m_base = mt * 256 + (int)rank * 128 + q * 32;
-            if constexpr (EPI == EPI_P_GEGLU_FP8)
+            if constexpr (Cfg::OVERLAP) {
+                // shared with the other accumulator: the last 64 columns of the first, the first 64 of the second.  Their warps
+                // arrive when they have read them, the others now: they are through with the tiles before this one
+                const bool shared = half != buf;
+                const uint32_t bar = tc::dsmem_map(tc::smem_u32(&acc_empty[buf]), 0);
+                if (!shared) {
+                    tc::tc_fence_before_sync();
+                    tc::mbar_arrive_cluster(bar);
+                }
+                const int flip = buf == 0 && half == 1 ? 64 : 0;
+                const int c0 = half * 128 + flip, c1 = half * 128 + (64 - flip);
+                epilogue_rows<EPI, 64>(p, t_acc + c0, m_base, nt * BN + c0, stg, lines, alpha, inv_os, shared ? bar : 0u);
+                epilogue_rows<EPI, 64>(p, t_acc + c1, m_base, nt * BN + c1, stg, lines, alpha, inv_os);
+                continue;
+            } else if constexpr (EPI == EPI_P_ROPE)
+                epilogue_rope_rows(p, t_acc + half * 64, m_base + lane, nt * BN + half * 64, alpha, pos, tab);
+            else if constexpr (EPI == EPI_P_GEGLU_FP8)
                 epilogue_geglu_rows(p, t_acc + half * 32, t_acc + BN / 2 + half * 32, m_base, nt * (BN / 2) + half * 32, alpha,
                                     inv_os);
             else if constexpr (BN == 192) {                  // whole 64-column blocks: 128 + 64
@@ -322,23 +414,33 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (warp == 1) tc::tmem_dealloc_pair(tmem, Cfg::TMEM_COLS);
 }
 
-template <int BN, int EPI, bool SPLIT = false>
+template <int BN, int EPI, bool SPLIT = false, bool FP4 = false>
 static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, cudaStream_t stream) {
-    using Cfg = GemmPairCfg<BN>;
+    using Cfg = GemmPairCfg<BN, FP4>;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
     const int sms = device_sm_count();
     if (attr_once.need(attr_dev)) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             Cfg::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel<BN, EPI, SPLIT, FP4>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         attr_once.set(attr_dev);
     }
-    CUtensorMap tmA, tmW;
-    int rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, (uint64_t)K, (uint64_t)K, 128);
+    CUtensorMap tmA, tmW, tmSA, tmSW;
+    const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
+    int rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, row_bytes, row_bytes, 128);
     if (rc) return rc;
-    rc = get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, (uint64_t)K, (uint64_t)K, BN / 2);
+    rc = get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, row_bytes, row_bytes, BN / 2);
     if (rc) return rc;
+    if (FP4) {
+        rc = get_tmap_sf(&tmSA, p.sf_lane, (p.M + 127) / 128, K / 64, 1);
+        if (rc) return rc;
+        rc = get_tmap_sf(&tmSW, p.sf_col, (p.N + 127) / 128, K / 64, Cfg::SFB_ROWS);
+        if (rc) return rc;
+    } else {
+        tmSA = tmA;
+        tmSW = tmW;
+    }
     const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + BN - 1) / BN, total = m_tiles * n_tiles;
     p.tile_gm = tile_group(m_tiles, n_tiles, 256, BN, sms / 2);
     const int units = SPLIT ? total * p.ksplits : total;
@@ -360,6 +462,6 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
     ++na;
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI, SPLIT>, tmA, tmW, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI, SPLIT, FP4>, tmA, tmW, tmSA, tmSW, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

@@ -16,7 +16,8 @@
 // EPI_P_BIAS_GELU_FAST_FP8: the same epilogue with the GELU through the hardware tanh -- a template value, not a run-time
 // flag: a select inside the unrolled loop over a thread's values costs as much as the arithmetic it chooses between
 // EPI_P_GEGLU_FP8 (CTA pairs only): the tile's columns are 128 gate features and the 128 up features that belong to them.
-enum { EPI_P_BF16 = 0, EPI_P_BIAS_GELU_FP8 = 1, EPI_P_BIAS_GELU_FAST_FP8 = 2, EPI_P_GEGLU_FP8 = 3 };
+// EPI_P_ROPE (NVFP4 CTA pairs): the QKV projection's RoPE + split + KV append, as EPI_ROPE_SPLIT of the small-M kernel.
+enum { EPI_P_BF16 = 0, EPI_P_BIAS_GELU_FP8 = 1, EPI_P_BIAS_GELU_FAST_FP8 = 2, EPI_P_GEGLU_FP8 = 3, EPI_P_ROPE = 4 };
 
 // tanh-form GELU with explicitly rounded fp32 operations, the same sequence as bias_gelu_fp8_kernel
 // (csrc/quantize/bias_gelu_quantize_fp8.cu:24-49 in the reference)
@@ -56,7 +57,7 @@ static int tile_group(int m_tiles, int n_tiles, int tm, int tn, int workers) {
 // where nothing hides it).
 template <int NC, bool BIAS>
 __device__ __forceinline__ void epilogue_bf16_lines(const GemmParams& p, uint32_t t_src, int m_base, int n0, uint8_t* stg,
-                                                    float alpha) {
+                                                    float alpha, uint32_t release) {
     const int lane = threadIdx.x & 31;
     const uint32_t stg_w = tc::smem_u32(stg) + lane * 128, sw = (uint32_t)(lane & 7) << 4;
     const int ch = lane & 7, r0 = lane >> 3;
@@ -68,6 +69,10 @@ __device__ __forceinline__ void epilogue_bf16_lines(const GemmParams& p, uint32_
         tc::tmem_ld32(t_src + c, v);
         tc::tmem_ld32(t_src + c + 32, v + 32);
         tc::tmem_ld_wait();
+        if (NC == 64 && release) {                          // these columns may be overwritten from here on
+            tc::tc_fence_before_sync();
+            tc::mbar_arrive_cluster(release);
+        }
         const int nb = n0 + c;
         // this thread's row: 64 results -> bf16 -> eight 16-byte chunks, chunk index xor (row & 7)
 #pragma unroll
@@ -115,15 +120,16 @@ __device__ __forceinline__ void epilogue_bf16_lines(const GemmParams& p, uint32_
 // quadrant and first column) -> bf16 (+ bias) or bias + GELU + FP8.  `stg` = 4 KB of this warp: tcgen05.ld delivers "thread
 // = row"; through shared memory the store instructions become whole lines (8 threads = 128 bytes of a row) instead of 32
 // separate half-sectors.  `lines`: rows and bias are 16-byte aligned; otherwise every thread stores its row directly.
+// `release` (bf16, NC = 64): a barrier on which every thread arrives as soon as the accumulator's columns are in registers.
 template <int EPI, int NC>
 __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_src, int m_base, int n0, uint8_t* stg,
-                                              bool lines, float alpha, float inv_os) {
+                                              bool lines, float alpha, float inv_os, uint32_t release = 0) {
     const int lane = threadIdx.x & 31;
     const int m = m_base + lane;
     if (EPI == EPI_P_BF16) {
         if (lines) {
-            if (p.bias) epilogue_bf16_lines<NC, true>(p, t_src, m_base, n0, stg, alpha);
-            else epilogue_bf16_lines<NC, false>(p, t_src, m_base, n0, stg, alpha);
+            if (p.bias) epilogue_bf16_lines<NC, true>(p, t_src, m_base, n0, stg, alpha, release);
+            else epilogue_bf16_lines<NC, false>(p, t_src, m_base, n0, stg, alpha, release);
             return;
         }
 #pragma unroll 1
@@ -157,6 +163,10 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_sr
                                 p.bias != nullptr));
                 }
             }
+        }
+        if (release) {
+            tc::tc_fence_before_sync();
+            tc::mbar_arrive_cluster(release);
         }
         return;
     }
@@ -247,6 +257,56 @@ __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_
     }
 }
 
+// 64 features of the fused q|k|v row of one token per thread: bf16(alpha * acc) rotated (V: copied), the rounding points of
+// EPI_ROPE_SPLIT.  `tab`: the token's 64 table values, fetched while the MMAs run (rope_table_rows).
+__device__ __forceinline__ int rope_column(const GemmParams& p, int n) {     // feature within its q, k or v part
+    return n < p.q_dim ? n : n < p.q_dim + p.k_dim ? n - p.q_dim : n - p.q_dim - p.k_dim;
+}
+__device__ __forceinline__ void rope_table_rows(const GemmParams& p, int m, int n0, uint4* tab) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const int n = n0 + 8 * c;
+        tab[c] = make_uint4(0, 0, 0, 0);
+        if (m < p.M && n < p.q_dim + p.k_dim)
+            tab[c] = ld_global_v4(p.rope + (size_t)m * p.head_dim + rope_column(p, n) % p.head_dim);
+    }
+}
+__device__ __forceinline__ void epilogue_rope_rows(const GemmParams& p, uint32_t t_src, int m, int n0, float alpha, int pos,
+                                                   const uint4* tab) {
+    uint32_t a[64];
+    tc::tmem_ld32(t_src, a);
+    tc::tmem_ld32(t_src + 32, a + 32);
+    tc::tmem_ld_wait();
+    if (m >= p.M) return;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const int n = n0 + 8 * c;
+        if (n >= p.N) break;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = bf16_round(__uint_as_float(a[8 * c + j]) * alpha);
+        const bool is_q = n < p.q_dim, is_k = !is_q && n < p.q_dim + p.k_dim;
+        const int nr = rope_column(p, n);
+        uint4 o;
+        if (is_q || is_k) {
+            const uint32_t* tw = &tab[c].x;
+            uint32_t* ow = &o.x;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float cs, sn;
+                unpack_bf16x2(tw[k], cs, sn);
+                ow[k] = pack_bf16x2(__fmaf_rn(v[2 * k], cs, -__fmul_rn(v[2 * k + 1], sn)),
+                                    __fmaf_rn(v[2 * k + 1], cs, __fmul_rn(v[2 * k], sn)));
+            }
+        } else {
+            o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        }
+        __nv_bfloat16* dst = is_q ? p.outQ + (size_t)m * p.q_dim + nr
+                                  : (is_k ? p.outK + (size_t)(pos + m) * p.k_dim + nr : p.outV + (size_t)(pos + m) * p.v_dim + nr);
+        st_global_v4(dst, o);
+    }
+}
+
 // whole-line stores are possible: 16-byte rows and bias
 template <int EPI>
 __device__ __forceinline__ bool epilogue_lines(const GemmParams& p) {
@@ -256,29 +316,26 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p) {
     return (p.N % 16) == 0 && (reinterpret_cast<uintptr_t>(p.out8) & 15) == 0;
 }
 
-template <int BN, bool FP4 = false>
+template <int BN>
 struct PGemmCfg {
-    static_assert(!FP4 || BN == 128, "NVFP4: two 128-column accumulators plus the scale columns fill tensor memory");
     static constexpr int L_BYTES = 128 * 128;
     static constexpr int C_BYTES = BN * 128;
-    static constexpr int SF_BYTES = FP4 ? 2048 : 0;    // four 512-byte scale atoms (one per K = 64 step) per operand
-    static constexpr int STAGE_BYTES = L_BYTES + C_BYTES + 2 * SF_BYTES;
+    static constexpr int STAGE_BYTES = L_BYTES + C_BYTES;
     static constexpr int MAX_STAGES = (227 * 1024 - 2048) / STAGE_BYTES;
     static constexpr int STAGES = MAX_STAGES > 6 ? 6 : MAX_STAGES;
     // bf16 epilogue staging: every epilogue warp owns 32 rows x 128 bytes, through which its 32 x 64 block of results is
     // turned from "thread = row" (what tcgen05.ld gives) into "8 threads = one 128-byte line" for the global store
-    static constexpr int EPI_STAGE_BYTES = FP4 ? 0 : 8 * 32 * 128;
+    static constexpr int EPI_STAGE_BYTES = 8 * 32 * 128;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + EPI_STAGE_BYTES;
-    static constexpr int SF_COL = 2 * BN;             // NVFP4: 16 scale columns per operand behind the accumulators
-    static constexpr int TMEM_COLS = FP4 ? 512 : 2 * BN;   // BN in {128, 256}
+    static constexpr int TMEM_COLS = 2 * BN;          // BN in {128, 256}
     static constexpr int EPI_THREADS = 256;
 };
 
-template <int BN, int EPI, bool FP4 = false>
+template <int BN, int EPI>
 __global__ void __launch_bounds__(320, 1)
 gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                            GemmParams p) {
-    using Cfg = PGemmCfg<BN, FP4>;
+    using Cfg = PGemmCfg<BN>;
     constexpr int STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -355,29 +412,20 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                 if (tc::elect_one()) {
                     tc::mbar_arrive_expect_tx(bar, Cfg::STAGE_BYTES);
                     tc::tma_load_2d(dst, &tmA, bar, kb * 128, m0);
-                    if (!FP4 && p.w_kn) {      // (K, N) weights: one 128 x 128-byte box per 128 output features
+                    if (p.w_kn) {      // (K, N) weights: one 128 x 128-byte box per 128 output features
 #pragma unroll
                         for (int j = 0; j < BN / 128; ++j)
                             tc::tma_load_2d(dst + Cfg::L_BYTES + j * 16384, &tmW, bar, n0 + j * 128, kb * 128);
                     } else {
                         tc::tma_load_2d(dst + Cfg::L_BYTES, &tmW, bar, kb * 128, n0);
                     }
-                    if (FP4) {      // activations are the lane operand here: sf_lane = SFA, sf_col = SFW
-                        const uint32_t sf = dst + Cfg::L_BYTES + Cfg::C_BYTES;
-                        tc::bulk_load(sf, p.sf_lane + ((size_t)(m0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512, 2048, bar);
-                        tc::bulk_load(sf + 2048, p.sf_col + ((size_t)(n0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512, 2048,
-                                      bar);
-                    }
                 }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (whole warp): accumulator i & 1 for the CTA's i-th tile
-        const bool w_kn = !FP4 && p.w_kn;
-        const uint32_t idesc = FP4 ? tc::make_idesc_nvfp4(128, BN)
-                                   : (tc::make_idesc(0, 0, 0, 0, 128, BN) | (w_kn ? (1u << 16) : 0u));
-        const uint32_t sf_smem0 = tc::smem_u32(smem + Cfg::L_BYTES + Cfg::C_BYTES);
-        const uint32_t tmem_sfa = tmem + Cfg::SF_COL, tmem_sfw = tmem + Cfg::SF_COL + 16;
+        const bool w_kn = p.w_kn;
+        const uint32_t idesc = tc::make_idesc(0, 0, 0, 0, 128, BN) | (w_kn ? (1u << 16) : 0u);
         const uint64_t dL0 = tc::make_desc_kmajor_sw128(tc::smem_u32(smem));
         const uint64_t dC0 = w_kn ? tc::make_desc_mnmajor_sw128(tc::smem_u32(smem + Cfg::L_BYTES), 16384)
                                   : tc::make_desc_kmajor_sw128(tc::smem_u32(smem + Cfg::L_BYTES));
@@ -405,25 +453,13 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                 }
                 tc::tc_fence_after_sync();
                 const uint64_t so = (uint64_t)(s * (Cfg::STAGE_BYTES >> 4));
-                const uint32_t sf = sf_smem0 + (uint32_t)(s * Cfg::STAGE_BYTES), done = empty_a + 8 * s;
+                const uint32_t done = empty_a + 8 * s;
                 if (++s == STAGES) { s = 0; ph ^= 1; }
                 ready = tc::mbar_test(full_a + 8 * s, ph);
                 if (tc::elect_one()) {
-                    if (FP4) {
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            tc::tmem_cp_sf_atom(tmem_sfa + 4 * k, sf + 512 * k);
-                            tc::tmem_cp_sf_atom(tmem_sfw + 4 * k, sf + 2048 + 512 * k);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc::mma_nvfp4(d_tm, dL0 + so + 2 * k, dC0 + so + 2 * k, idesc, tmem_sfa + 4 * k,
-                                          tmem_sfw + 4 * k, (kb > 0 || k > 0) ? 1u : 0u);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            tc::mma_f8(d_tm, dL0 + so + 2 * k, dC0 + so + cstep * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < 4; ++k)
+                        tc::mma_f8(d_tm, dL0 + so + 2 * k, dC0 + so + cstep * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc::mma_commit(done);
                     if (kb == kbt - 1) tc::mma_commit(accF_a + 8 * buf);
                 }
@@ -440,7 +476,7 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
         if (p.sa) alpha *= *p.sa;
         if (p.sb) alpha *= *p.sb;
         const float inv_os = (EPI != EPI_P_BF16) ? __fdiv_rn(1.0f, *p.out_scale) : 0.0f;
-        const bool lines = Cfg::EPI_STAGE_BYTES > 0 && epilogue_lines<EPI>(p);
+        const bool lines = epilogue_lines<EPI>(p);
         uint8_t* stg = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * (32 * 128);
         int i = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
@@ -466,25 +502,23 @@ gemm_fp8_persistent_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     if (warp == 1) tc::tmem_dealloc(tmem, Cfg::TMEM_COLS);
 }
 
-template <int BN, int EPI, bool FP4 = false>
+template <int BN, int EPI>
 static int launch_gemm_persistent(const void* A, const void* W, GemmParams p, int K, cudaStream_t stream) {
-    using Cfg = PGemmCfg<BN, FP4>;
+    using Cfg = PGemmCfg<BN>;
     static PerDeviceOnce attr_once;
     int attr_dev = 0;
     const int sms = device_sm_count();
     if (attr_once.need(attr_dev)) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_persistent_kernel<BN, EPI, FP4>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(gemm_fp8_persistent_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             Cfg::SMEM_BYTES);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         attr_once.set(attr_dev);
     }
     CUtensorMap tmA, tmW;
-    const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
-    if (FP4) p.sf_katoms = K / 64;
-    int rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, row_bytes, row_bytes, 128);
+    int rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, (uint64_t)K, (uint64_t)K, 128);
     if (rc) return rc;
-    rc = (!FP4 && p.w_kn) ? get_tmap_2d_u8(&tmW, W, (uint64_t)K, (uint64_t)p.N, (uint64_t)p.N, 128)
-                          : get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, row_bytes, row_bytes, BN);
+    rc = p.w_kn ? get_tmap_2d_u8(&tmW, W, (uint64_t)K, (uint64_t)p.N, (uint64_t)p.N, 128)
+                : get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, (uint64_t)K, (uint64_t)K, BN);
     if (rc) return rc;
     const int m_tiles = (p.M + 127) / 128, n_tiles = (p.N + BN - 1) / BN, total = m_tiles * n_tiles;
     p.tile_gm = tile_group(m_tiles, n_tiles, 128, BN, sms);
@@ -498,6 +532,6 @@ static int launch_gemm_persistent(const void* A, const void* W, GemmParams p, in
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;                   // nothing global is read before the wait
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_persistent_kernel<BN, EPI, FP4>, tmA, tmW, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_persistent_kernel<BN, EPI>, tmA, tmW, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }

@@ -337,6 +337,21 @@ __device__ __forceinline__ void mma_nvfp4(uint32_t tmem_d, uint64_t adesc, uint6
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
         : "memory");
 }
+// The forms of a CTA pair (cta_group::2), issued by one thread of the leader: the copy takes the atom at this shared-memory
+// offset of EACH CTA into that CTA's tensor memory (every CTA stages the scales of its own 128 rows of A and of ALL columns).
+__device__ __forceinline__ void tmem_cp_sf_atom_pair(uint32_t taddr, uint32_t saddr) {
+    const uint64_t desc = make_smem_desc(saddr, 0, 128, 0);
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void mma_nvfp4_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
+        : "memory");
+}
 // all MMAs issued so far by this thread -> one arrival on `bar` when they complete
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -378,6 +393,9 @@ __device__ __forceinline__ void st_async_b32(uint32_t peer_addr, uint32_t peer_b
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
                  ::"r"(peer_addr), "r"(a), "r"(peer_bar)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 __device__ __forceinline__ float dsmem_ld_f32(uint32_t cluster_addr) {
     float v;

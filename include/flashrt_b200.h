@@ -411,7 +411,10 @@ int frt_b200_norm_nvfp4(void* residual, const void* x, const void* gate_in, long
 /* cutlass_fp4_gemm_variant, cutlass_fp4_sq_fp16   csrc/fp4_bindings.cpp:85-99,355-370 -> csrc/gemm/fp4/cutlass_fp4_gemm.cu
  * cutlass_fp4_gemm_bias_bf16                       csrc/fp4_bindings.cpp:1139-1155
  *   D(M,N) bf16 = alpha * (*d_alpha) * (A.SFA)(M,K) . (W.SFW)(N,K)^T + bias;  d_alpha, bias optional;  K % 256 == 0;
- *   beta is not supported (the decoder path calls with beta = 0).  One kernel for every variant index. */
+ *   beta is not supported (the decoder path calls with beta = 0).  One kernel for every variant index.
+ *   splits: 0 = choose (1: M <= 256 rows on one split of the small-M kernel); flags: bit0 = the weights are settled and may be
+ *   read before the kernel in front has ended, bit1 = one-tile-per-CTA kernel for M > 256 (bits 0-1 as frt_b200_gemm_fp8_nt),
+ *   bits 8-9 = tile columns on CTA pairs (1 = 128, 2 = 192, 3 = 256; 0 = choose). */
 int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const void* SFW, void* D, int M, int N,
                            int K, float alpha, const float* d_alpha, const void* bias, int splits, int flags,
                            void* stream);

@@ -241,3 +241,50 @@ def test_gemm_nvfp4_persistent_equals_one_tile_per_cta(M, N, K):
     assert fvk.tensor_core_status() == 0
     assert np.array_equal(d_1.get(), d_2.get())
     _check(d_1.get(), O.gemm_nvfp4(Ap, Asf, Wp, Wsf, want_f32=True))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 256), (65, 2560, 1024), (129, 136, 512), (256, 1040, 768), (257, 64, 256),
+                                   (513, 1936, 1280), (1000, 4104, 1536), (2501, 3072, 2048)])
+@pytest.mark.parametrize("cols", [128, 192, 256])
+@pytest.mark.parametrize("pdl", [False, True])
+def test_gemm_nvfp4_pair_tiles_give_the_same_bytes(M, N, K, cols, pdl):
+    """256 x cols tiles on CTA pairs: one tile and several per pair, last tiles of a few rows or columns, scale rows that start
+    at 64 (192 columns), accumulators that share columns (256), weights fetched ahead (pdl).  Unsplit sums in K order: the
+    bytes of the one-tile-per-CTA kernels."""
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import Dev, zeros
+    rng = np.random.default_rng(M + N + K)
+    Ap, Asf = _operand(rng, M, K, 1.0)
+    Wp, Wsf = _operand(rng, N, K, 0.02)
+    bias = O.f32_to_bf16_bits((rng.standard_normal(N) * 0.1).astype(np.float32))
+    d = [Dev(Ap), Dev(Asf), Dev(Wp), Dev(Wsf)]
+    d_b, d_1, d_2 = Dev(bias), zeros((M, N), np.uint16), zeros((M, N), np.uint16)
+    for out, splits, flags in ((d_1, 1, 2), (d_2, 0, ((cols - 64) // 64) << 8 | pdl)):
+        _lib.call("frt_b200_gemm_nvfp4_nt", d[0].ptr, d[1].ptr, d[2].ptr, d[3].ptr, out.ptr, M, N, K, 0.5, None, d_b.ptr,
+                  splits, flags, 0)
+    assert fvk.tensor_core_status() == 0
+    assert np.array_equal(d_1.get(), d_2.get())
+
+
+@pytest.mark.parametrize("M,k_dim,pos", [(65, 256, 768), (100, 128, 3), (200, 256, 0), (256, 64, 541)])
+def test_gemm_nvfp4_pair_rope_split_equals_pair_of_launches(M, k_dim, pos):
+    """More than 64 tokens: the RoPE finish of the CTA pairs against GEMM -> qkv_split_rope, byte for byte."""
+    from flashrt_b200 import flash_rt_fp4 as fp4, flash_rt_kernels as fvk
+    from gpu_util import Dev, rand_bf16, zeros
+    rng = np.random.default_rng(M + k_dim)
+    K, q_dim, hd = 1024, 8 * k_dim, k_dim
+    N = q_dim + 2 * k_dim
+    Ap, Asf = _operand(rng, M, K, 1.0)
+    Wp, Wsf = _operand(rng, N, K, 0.02)
+    d = [Dev(Ap), Dev(Asf), Dev(Wp), Dev(Wsf)]
+    d_rope, d_pos, d_qkv = Dev(rand_bf16(rng, (M, hd), 0.7)), Dev(np.array([pos], np.int32)), zeros((M, N), np.uint16)
+    out = [[zeros((M, q_dim), np.uint16), zeros((pos + M, k_dim), np.uint16), zeros((pos + M, k_dim), np.uint16)]
+           for _ in range(2)]
+    assert fp4.cutlass_fp4_gemm_variant(0, *(x.ptr for x in d), d_qkv.ptr, M, N, K, 0.5) == 0
+    fvk.qkv_split_rope(d_qkv.ptr, d_rope.ptr, out[0][0].ptr, out[0][1].ptr + pos * k_dim * 2,
+                       out[0][2].ptr + pos * k_dim * 2, M, q_dim, k_dim, k_dim, hd, 0)
+    assert fp4.cutlass_fp4_gemm_rope_split(*(x.ptr for x in d), d_rope.ptr, *(x.ptr for x in out[1]), M, K, q_dim, k_dim,
+                                           k_dim, hd, devpos=d_pos.ptr, alpha=0.5) == 0
+    assert fvk.tensor_core_status() == 0
+    for a, b in zip(*out):
+        assert np.array_equal(a.get(), b.get())
