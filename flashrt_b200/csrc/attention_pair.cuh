@@ -34,24 +34,6 @@ struct PairCfg {
     static constexpr float RESCALE_THRESHOLD = 8.0f;     // log2 domain
 };
 
-__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f32x2_parts(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // 2^x of a pair on the fma pipe: x = n + f with n = floor(x), 2^f on [0, 1) by a polynomial of degree 5 with p(0) = 1 (own
 // least-squares fit of the relative error, reweighted towards its maximum: 1.4e-7 in fp32 arithmetic, the accuracy of
 // ex2.approx), n added to the exponent field.  The reduction and the exponent put together as an integer are Cody and Waite's

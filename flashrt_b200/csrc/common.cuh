@@ -54,6 +54,40 @@ __device__ __forceinline__ float bf16_round(float v) {
     return __uint_as_float(r);
 }
 
+// two fp32 values in one register pair: one instruction for two correctly rounded products or fmas
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f32x2_parts(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t unpack_bf16x2(uint32_t w) {
+    return f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+// larger magnitude of each half (a NaN loses), its sign the xor of both
+__device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
 // ---------------------------------------------------------------- fp8 e4m3
 // clamp to +-448 (NaN -> -448, as fminf(fmaxf(v, -448), 448) gives) in front of a saturating E4M3 conversion: the
 // conversion itself does the upper bound, so one instruction remains
@@ -193,6 +227,20 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
     asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
     return r;
+}
+// 32 bytes: one instruction where the pointer is 32-byte aligned (`wide`), else two of 16, the second one only if it is there
+__device__ __forceinline__ void ld_stream_32(const void* p, bool wide, bool second, uint32_t* r) {
+    if (wide) {
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "l"(p) : "memory");
+    } else {
+        const uint4 a = ld_stream_v4(p);
+        uint4 b = make_uint4(0, 0, 0, 0);
+        if (second) b = ld_stream_v4(static_cast<const uint8_t*>(p) + 16);
+        r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+        r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+    }
 }
 __device__ __forceinline__ float4 ld_global_f4(const float* p) {
     return *reinterpret_cast<const float4*>(p);

@@ -196,113 +196,189 @@ norm_row_kernel(NormArgs a) {
     if (HAS_STYLE && a.gate_out) st_global_v4(a.gate_out + roff, gt);
 }
 
-// Many rows: one WARP per row, the row in registers (NS slices of 256 columns, 16 bytes per lane and slice, bf16 bits).
-// The one-CTA-per-row kernel above is bound by its latency chain -- one load, one block barrier and a serial sum of warp
-// totals per 6 KB row, with five CTAs of 384 threads on an SM.  Here every lane has NS loads in flight, there is no barrier,
-// and 16-24 rows share an SM.  Same sums in the same order (warp_row_total), same bits.  RMSNorm -> FP8: 8192 x 3072 27.2 ->
-// 18.2 us, 20480 x 3072 63.7 -> 36.9 us (5.1 TB/s); -> NVFP4: 20480 x 3072 85.7 -> 59.9 us (bound by its instructions).
-template <int OUT, int NS>
+// Many rows: a warp, or WPR of the CTA's four warps, takes a row; it stays in registers, 16 neighbouring values per lane and piece
+// of 512 columns, NP pieces per warp.  The one-CTA-per-row kernel above is bound by its latency chain -- one load, one block barrier
+// and a serial sum of warp totals per row, a few rows on an SM.  Here every lane has NP loads of 32 bytes in flight and 16-24 rows
+// share an SM.  A lane's 16 values are one block of the NVFP4 result, whose scale, reciprocal and conversions are then made once
+// (twice with 8 values per lane), products and fmas run two at a time, the largest magnitude on packed bf16: what bounds the
+// NVFP4 result is still its instructions, about 95 per 8 values.  Same sums in the same order as the CTA kernel, same bits.
+// us, one warp per row with 8 values per lane (above 4096 columns: one CTA per row) -> now: to NVFP4 20480 x 3072 59.8 -> 45.2, 8192
+// x 8192 101 -> 50, 2501 x 3072 11.4 -> 8.7; to FP8 20480 x 3072 34.2 -> 32.5 (5.8 TB/s), 8192 x 4096 22.5 -> 19.7, 8192 x 8192 84.8 ->
+// 36.7.
+template <int OUT, int NP, int WPR>
 __global__ void __launch_bounds__(128)
-norm_warp_kernel(NormArgs a) {
+norm_block_kernel(NormArgs a) {
     constexpr bool OUT_FP8 = OUT == OUT_E4M3;
     constexpr bool OUT_FP4 = OUT == OUT_NVFP4_A || OUT == OUT_NVFP4_B;
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    constexpr int P = NP <= 1 ? 1 : NP <= 2 ? 2 : NP <= 4 ? 4 : 8;
+    constexpr uint32_t HI = 0xffff0000u;
+    static_assert(NP <= 8 && (WPR == 1 || WPR == 2 || WPR == 4), "slice pairs per warp, warps per row");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.x * (4 / WPR) + warp / WPR, part = warp % WPR;
     pdl_launch_dependents();
     pdl_wait();
-    float inv_scale = 1.0f;
-    if (OUT_FP8) inv_scale = __fdiv_rn(1.0f, *a.d_scale);
-    if (row >= a.rows) return;
-    const int n = (a.dim + 255) >> 8;                       // slices of this row, n <= NS
-    const size_t rbase = (size_t)row * a.dim + lane * 8;
-    const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
-    uint8_t* sf = nullptr;                                  // scale byte of this lane's block: + 4 atoms per slice
-    const bool sf_words = OUT_FP4 && (a.dim & 63) == 0;
-    if (OUT_FP4) sf = a.sf_out + nvfp4::sf_offset(row, (lane >> 3) * 4, (a.dim + 63) >> 6);
-    uint4 rv[NS];
-    float ssq[NS];
+    const float inv_scale = OUT_FP8 ? __fdiv_rn(1.0f, *a.d_scale) : 1.0f;
+    const bool live = row < a.rows;
+    if (WPR == 1 && !live) return;
+    // whole: every lane's piece is 32 bytes at a multiple of 32, its result one aligned store; otherwise by halves of 8 values
+    const bool wide = ((reinterpret_cast<uintptr_t>(a.residual) & 31) | (a.dim & 15)) == 0;
+    const bool whole = ((reinterpret_cast<uintptr_t>(a.out) & 15) | (a.dim & 15)) == 0;
+    const int col0 = part * 512 + lane * 16;                // pair i of this lane: columns col0 + i * WPR * 512 ..
+    const size_t rbase = (size_t)row * a.dim + col0;
+    const int left = live ? a.dim - col0 : 0;
+    uint32_t x[NP][8];
 #pragma unroll
-    for (int w = 0; w < NS; ++w) {
-        rv[w] = make_uint4(0, 0, 0, 0);
-        if (w * 256 < left) rv[w] = ld_stream_v4(a.residual + rbase + w * 256);
+    for (int i = 0; i < NP; ++i) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[i][j] = 0u;
+        if (i * WPR * 512 < left) ld_stream_32(a.residual + rbase + i * WPR * 512, wide, i * WPR * 512 + 8 < left, x[i]);
     }
+    // Sums of squares: the chain over 8 values of both halves at once; then the butterfly over the 32 chunks of a slice.  A
+    // lane holds chunks 2 lane and 2 lane + 1 of a pair's 64, so the exchanges at distance 16, 8, 4, 2 of a chunk are 8, 4, 2, 1 of a
+    // lane, and the last one is between the halves: the tree of the one-CTA-per-row kernel.  Every exchange hands half of the
+    // values held to the partner (see warp_row_total).
+    float v[2 * P];
 #pragma unroll
-    for (int w = 0; w < NS; ++w) {
-        const uint32_t* rw = &rv[w].x;
-        float s = 0.0f;
+    for (int i = 0; i < P; ++i) {
+        uint64_t s = f32x2(0.0f, 0.0f);
+        if (i < NP) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float r0, r1;
-            unpack_bf16x2(rw[i], r0, r1);
-            s = __fmaf_rn(r0, r0, s);
-            s = __fmaf_rn(r1, r1, s);
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t e = f32x2(__uint_as_float(x[i][j] << 16), __uint_as_float(x[i][4 + j] << 16));
+                const uint64_t o = f32x2(__uint_as_float(x[i][j] & HI), __uint_as_float(x[i][4 + j] & HI));
+                s = fma_f32x2(o, o, fma_f32x2(e, e, s));
+            }
         }
-        ssq[w] = s;
+        f32x2_parts(s, v[i], v[P + i]);
     }
-    const float tot = warp_row_total<NS>(ssq, n);
+    int d = 8;
+#pragma unroll
+    for (int h = P; h >= 1; h >>= 1, d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, d));
+        }
+    }
+#pragma unroll
+    for (; d >= 1; d >>= 1) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], d));
+    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 8));
+    // slice 2 (i WPR + part) is in lanes i * (8 / P) .., the one behind it 16 lanes further on
+    const int n = (a.dim + 255) >> 8;
+    float tot = 0.0f;
+    if (WPR == 1) {
+        tot = __shfl_sync(0xffffffffu, v[0], 0);
+#pragma unroll
+        for (int w = 1; w < 2 * NP; ++w) {
+            const float y = __shfl_sync(0xffffffffu, v[0], (w >> 1) * (8 / P) + (w & 1) * 16);
+            if (w < n) tot = __fadd_rn(tot, y);
+        }
+    } else {
+        __shared__ float slices[4 / WPR][2 * NP * WPR];
+        float* sl = slices[warp / WPR];
+        const int i = (lane & 7) / (8 / P);
+        if ((lane & 8) == 0 && (lane & 7) % (8 / P) == 0 && i < NP) sl[2 * (i * WPR + part) + (lane >> 4)] = v[0];
+        __syncthreads();
+        if (!live) return;
+        tot = sl[0];
+#pragma unroll
+        for (int w = 1; w < 2 * NP * WPR; ++w) {
+            const float y = sl[w];
+            if (w < n) tot = __fadd_rn(tot, y);
+        }
+    }
     const float var = __fadd_rn(__fdiv_rn(tot, (float)a.dim), a.eps);
     const float rms = __fdiv_rn(1.0f, __fsqrt_rn(var));
+    const uint64_t rms2 = f32x2(rms, rms), zero2 = f32x2(0.0f, 0.0f);
+    uint8_t* sf = nullptr;                                  // scale byte of this lane's block of pair 0
+    const bool sf_words = OUT_FP4 && (a.dim & 63) == 0;
+    if (OUT_FP4) sf = a.sf_out + nvfp4::sf_offset(row, (part * 32 + lane) & ~3, (a.dim + 63) >> 6);
 #pragma unroll
-    for (int w = 0; w < NS; ++w) {
-        const bool on = w * 256 < left;
-        uint4 wv = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-        if (on && a.weight) wv = ld_global_v4(a.weight + lane * 8 + w * 256);
-        const uint32_t* rw = &rv[w].x;
-        const uint32_t* ww = &wv.x;
-        float v[8];
+    for (int i = 0; i < NP; ++i) {
+        const bool on = i * WPR * 512 < left, on2 = i * WPR * 512 + 8 < left;
+        uint32_t wv[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float r0, r1, w0, w1;
-            unpack_bf16x2(rw[i], r0, r1);
-            unpack_bf16x2(ww[i], w0, w1);
-            v[2 * i] = __fmul_rn(__fmul_rn(r0, rms), w0);
-            v[2 * i + 1] = __fmul_rn(__fmul_rn(r1, rms), w1);
+        for (int j = 0; j < 8; ++j) wv[j] = 0x3f803f80u;
+        if (on && a.weight) {
+            const __nv_bfloat16* wp = a.weight + col0 + i * WPR * 512;
+            const uint4 w0 = ld_global_v4(wp), w1 = on2 ? ld_global_v4(wp + 8) : w0;
+            wv[0] = w0.x; wv[1] = w0.y; wv[2] = w0.z; wv[3] = w0.w;
+            wv[4] = w1.x; wv[5] = w1.y; wv[6] = w1.z; wv[7] = w1.w;
         }
-        const size_t roff = rbase + w * 256;
-        if (OUT_FP4) {
-            constexpr int FAM = OUT == OUT_NVFP4_A ? 0 : 1;
-            float amax = 0.0f;
+        uint64_t y[8];
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                unpack_bf16x2(pack_bf16x2(v[i], v[i + 1]), v[i], v[i + 1]);
-                amax = fmaxf(amax, fmaxf(fabsf(v[i]), fabsf(v[i + 1])));
+        for (int j = 0; j < 8; ++j) y[j] = mul_f32x2(mul_f32x2(unpack_bf16x2(x[i][j]), rms2), unpack_bf16x2(wv[j]));
+        const size_t roff = rbase + i * WPR * 512;
+        if (OUT_FP8) {
+            const uint64_t is2 = f32x2(inv_scale, inv_scale);
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float q0, q1, q2, q3;
+                f32x2_parts(mul_f32x2(y[2 * j], is2), q0, q1);
+                f32x2_parts(mul_f32x2(y[2 * j + 1], is2), q2, q3);
+                o[j] = f32x4_to_e4m3x4(clamp448(q0), clamp448(q1), clamp448(q2), clamp448(q3));
             }
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            float s;
-            uint32_t sb = nvfp4::block_scale<FAM>(amax, s);
-            const float2 inv = nvfp4::inv_off_ties<FAM>(nvfp4::inverse<FAM>(s), s);
-            const uint32_t pk = nvfp4::pack8_bf16<FAM>(v, s, inv);
-            if (on) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(a.out) + (roff >> 1)) = pk;
-            // the scale bytes of four neighbouring blocks (eight lanes) are one aligned word of the scale layout
-            if (sf_words) {
-                sb |= __shfl_down_sync(0xffffffffu, sb, 2) << 8;
-                sb |= __shfl_down_sync(0xffffffffu, sb, 4) << 16;
-                if (on && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf + w * 2048) = sb;
-            } else if (on && (lane & 1) == 0) {
-                sf[w * 2048 + ((lane >> 1) & 3)] = (uint8_t)sb;
+            uint8_t* dst = reinterpret_cast<uint8_t*>(a.out) + roff;
+            if (whole) {
+                if (on) st_global_v4(dst, make_uint4(o[0], o[1], o[2], o[3]));
+            } else {
+                if (on) st_global_v2(dst, make_uint2(o[0], o[1]));
+                if (on2) st_global_v2(dst + 8, make_uint2(o[2], o[3]));
             }
-        } else if (OUT_FP8) {
-            uint2 o;
-            o.x = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[0], inv_scale)), clamp448(__fmul_rn(v[1], inv_scale)),
-                                  clamp448(__fmul_rn(v[2], inv_scale)), clamp448(__fmul_rn(v[3], inv_scale)));
-            o.y = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[4], inv_scale)), clamp448(__fmul_rn(v[5], inv_scale)),
-                                  clamp448(__fmul_rn(v[6], inv_scale)), clamp448(__fmul_rn(v[7], inv_scale)));
-            if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + roff, o);
-        } else {
-            uint4 o;
-            o.x = pack_bf16x2(v[0], v[1]);
-            o.y = pack_bf16x2(v[2], v[3]);
-            o.z = pack_bf16x2(v[4], v[5]);
-            o.w = pack_bf16x2(v[6], v[7]);
-            if (on) st_global_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + roff, o);
+            continue;
+        }
+        uint32_t b[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float y0, y1;
+            f32x2_parts(y[j], y0, y1);
+            b[j] = pack_bf16x2(y0, y1);
+        }
+        if (!OUT_FP4) {
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + roff;
+            if (on) st_global_v4(dst, make_uint4(b[0], b[1], b[2], b[3]));
+            if (on2) st_global_v4(dst + 8, make_uint4(b[4], b[5], b[6], b[7]));
+            continue;
+        }
+        constexpr int FAM = OUT == OUT_NVFP4_A ? 0 : 1;
+        const uint32_t m = absmax_bf16x2(absmax_bf16x2(absmax_bf16x2(b[0], b[1]), absmax_bf16x2(b[2], b[3])),
+                                         absmax_bf16x2(absmax_bf16x2(b[4], b[5]), absmax_bf16x2(b[6], b[7]))) & 0x7fff7fffu;
+        const float amax = fmaxf(0.0f, fmaxf(__uint_as_float(m << 16), __uint_as_float(m & HI)));
+        float s;
+        uint32_t sb = nvfp4::block_scale<FAM>(amax, s);
+        const float2 inv = nvfp4::inv_off_ties<FAM>(nvfp4::inverse<FAM>(s), s);
+        uint32_t q[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float e[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float y0, y1;
+                f32x2_parts(unpack_bf16x2(b[4 * h + j]), y0, y1);
+                const uint64_t i2 = FAM == 0 ? f32x2(inv.x, inv.x)
+                                             : f32x2(fabsf(y0) < s ? inv.x : inv.y, fabsf(y1) < s ? inv.x : inv.y);
+                f32x2_parts(fma_f32x2(f32x2(y0, y1), i2, zero2), e[2 * j], e[2 * j + 1]);
+            }
+            q[h] = nvfp4::cvt8(e);
+        }
+        if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + (roff >> 1), make_uint2(q[0], q[1]));
+        // the scale bytes of four neighbouring blocks (lanes) are one aligned word of the scale layout
+        if (sf_words) {
+            sb |= __shfl_down_sync(0xffffffffu, sb, 1) << 8;
+            sb |= __shfl_down_sync(0xffffffffu, sb, 2) << 16;
+            if (on && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf + i * WPR * 4096) = sb;
+        } else if (on) {
+            sf[i * WPR * 4096 + (lane & 3)] = (uint8_t)sb;
         }
     }
 }
 
-template <int OUT, int NS>
-static int launch_norm_warp(const NormArgs& a, cudaStream_t stream) {
+template <int OUT, int NP, int WPR>
+static int launch_norm_block(const NormArgs& a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((a.rows + 3) / 4));
+    cfg.gridDim = dim3((unsigned)((a.rows + 4 / WPR - 1) / (4 / WPR)));
     cfg.blockDim = dim3(128);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -310,35 +386,45 @@ static int launch_norm_warp(const NormArgs& a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, norm_warp_kernel<OUT, NS>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, norm_block_kernel<OUT, NP, WPR>, a);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
+template <int OUT, int WPR>
+static int dispatch_norm_block(const NormArgs& a, cudaStream_t stream) {
+    switch ((a.dim + 512 * WPR - 1) / (512 * WPR)) {
+        case 1: return launch_norm_block<OUT, 1, WPR>(a, stream);
+        case 2: return launch_norm_block<OUT, 2, WPR>(a, stream);
+        case 3: return launch_norm_block<OUT, 3, WPR>(a, stream);
+        case 4: return launch_norm_block<OUT, 4, WPR>(a, stream);
+        case 5: return launch_norm_block<OUT, 5, WPR>(a, stream);
+        case 6: return launch_norm_block<OUT, 6, WPR>(a, stream);
+        case 7: return launch_norm_block<OUT, 7, WPR>(a, stream);
+        case 8: return launch_norm_block<OUT, 8, WPR>(a, stream);
+        default: return FRT_ERR_UNSUPPORTED;
+    }
+}
 
-// Rows from which the warp-per-row kernel wins (graph of back-to-back launches, dim 1024 .. 4096): below, the rows of the
-// CTA kernel are all on the chip at once and its chain is shorter.  The NVFP4 result needs twice the instructions per
-// value, so more rows have to share an SM before the load latency is what counts.  The residual form stays with the CTA
-// kernel at every size (it already streams 5.6 TB/s; two register-held rows per lane were slower).
+// From 3 Mi values on (1536 x 2048, 1024 x 3072) the rows of the CTA kernel no longer fit the chip at once and its chain per row is
+// what counts; below, that chain is the shorter one (512 x 3072 to NVFP4: 3.7 us against 4.0; 1024 x 2048: 3.9 against 4.3).  Warps
+// per row: 1 up to 1024 columns, 2 up to 3072, 4 above, so that a lane holds one to four 32-byte pieces (20480 x 4096 to NVFP4 with
+// 1 / 2 / 4 warps: 70.5 / 61.9 / 58.0 us; 20480 x 1024: 15.8 / 17.6 / 31.0).  The residual form stays with the CTA kernel at every size (it
+// already streams 5.6 TB/s; two register-held rows per lane were slower).
 template <int OUT>
-static constexpr int norm_warp_rows() { return OUT == OUT_BF16 || OUT == OUT_E4M3 ? 1536 : 3072; }
+static int launch_norm_rows(const NormArgs& a, cudaStream_t stream) {
+    if (a.dim <= 1024) return dispatch_norm_block<OUT, 1>(a, stream);
+    if (a.dim <= 3072) return dispatch_norm_block<OUT, 2>(a, stream);
+    return dispatch_norm_block<OUT, 4>(a, stream);
+}
 
 template <bool HAS_X, bool HAS_GATE, bool HAS_STYLE, int OUT>
 static int launch_norm(NormArgs a, cudaStream_t stream, bool pdl) {
     a.early = pdl ? 1 : 0;
     if (a.rows < 0 || a.dim <= 0 || (a.dim & 7) || a.dim > 8192) return FRT_ERR_UNSUPPORTED;
     if (a.rows == 0) return FRT_OK;
-    if (!HAS_X && !HAS_STYLE && a.rows >= norm_warp_rows<OUT>() && a.dim > 512 &&
-        (reinterpret_cast<uintptr_t>(a.sf_out) & 3) == 0) {
-        switch ((a.dim + 511) / 512) {
-            case 2: return launch_norm_warp<OUT, 4>(a, stream);
-            case 3: return launch_norm_warp<OUT, 6>(a, stream);
-            case 4: return launch_norm_warp<OUT, 8>(a, stream);
-            case 5: return launch_norm_warp<OUT, 10>(a, stream);
-            case 6: return launch_norm_warp<OUT, 12>(a, stream);
-            case 7: return launch_norm_warp<OUT, 14>(a, stream);
-            case 8: return launch_norm_warp<OUT, 16>(a, stream);
-            default: break;                                  // wider rows: the CTA kernel
-        }
-    }
+    if (!HAS_X && !HAS_STYLE && (long long)a.rows * a.dim >= 3ll << 20 && a.dim > 512 &&
+        (OUT == OUT_BF16 || OUT == OUT_E4M3 ||
+         ((reinterpret_cast<uintptr_t>(a.sf_out) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 7) == 0)))
+        return launch_norm_rows<OUT>(a, stream);
     int threads = ((a.dim / 8 + 31) / 32) * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.rows);

@@ -106,3 +106,30 @@ def test_qkv_split_norm_rope_rows(L, heads, hd, seq):
                                          k.ptr + r * dim * 2, 1, n, heads, hd, max(0, min(n, seq - r)), 1e-6, 0)
         outs.append((q.get(), k.get()))
     assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("rows,dim", [(3073, 1024), (3077, 1040), (1027, 3072), (1111, 3088), (769, 4112), (389, 8192)])
+@pytest.mark.parametrize("kind", ["fp8", "nvfp4_0", "nvfp4_1"])
+def test_norm_blocks_of_unaligned_rows(rows, dim, kind):
+    """One, two and four warps per row: the last piece of a row partly there, rows and results that start 16 (8) bytes off the
+    widest access, values of every class."""
+    from flashrt_b200 import _lib
+    from gpu_util import f32, rand_bf16, zeros
+    x = _rows(rows + dim, rows, dim)
+    x[9, 3], x[11, 17], x[13, 40:48] = 0x7f80, 0x7fc0, 0x0001      # inf, NaN, subnormal values
+    w, sc, katoms, got = _dev(rand_bf16(np.random.default_rng(1), (dim,))), f32(0.011), (dim + 63) // 64, []
+    buf = np.zeros(rows * dim + 8, np.uint16)
+    for off, step in ((0, rows), (8, rows), (0, 256)):
+        buf[off:off + rows * dim] = x.reshape(-1)
+        d_x, d_o, d_sf = _dev(buf), zeros((rows * dim + 8,), np.uint8), zeros(((rows + 127) // 128 * katoms * 512,), np.uint8)
+        for r in range(0, rows, step):
+            n, xp = min(step, rows - r), d_x.ptr + (r * dim + off) * 2
+            if kind == "fp8":
+                _lib.call("frt_b200_norm_fp8", xp, None, None, 0, w.ptr, None, 0, d_o.ptr + r * dim + off, None, n, dim, 1e-6,
+                          sc.ptr, 0, 0)
+            else:
+                _lib.call("frt_b200_norm_nvfp4", xp, None, None, 0, w.ptr, None, 0, d_o.ptr + r * dim // 2 + off,
+                          d_sf.ptr + r // 128 * katoms * 512, None, n, dim, 1e-6, int(kind[-1]), 0, 0)
+        got.append((d_o.get()[off:off + rows * dim // (1 if kind == "fp8" else 2)], d_sf.get()))
+    for g in got[:2]:
+        assert np.array_equal(g[0], got[2][0]) and np.array_equal(g[1], got[2][1])
