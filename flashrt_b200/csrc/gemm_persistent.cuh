@@ -235,10 +235,17 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_sr
 // features h0 .. h0 + 31 of out8 (M, half), the rounding points of GEMM -> geglu_fp8.  A thread's 32 bytes are one sector.
 __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_t t_gate, uint32_t t_up, int m_base, int h0,
                                                     float alpha, float inv_os) {
+    if (m_base >= p.M) return;
+    const int m = m_base + (threadIdx.x & 31);
     uint32_t g[32], u[32], w[8];
     tc::tmem_ld32(t_gate, g);
     tc::tmem_ld32(t_up, u);
     tc::tmem_ld_wait();
+    // rows beyond M hold zeros, and a zero takes the slow path of the activation's division (541 rows: 48 us a launch with it)
+    if (m >= p.M) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) g[j] = 0x3f800000u;
+    }
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
         float o[4];
@@ -249,7 +256,6 @@ __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_
         }
         w[j / 4] = f32x4_to_e4m3x4(o[0], o[1], o[2], o[3]);
     }
-    const int m = m_base + (threadIdx.x & 31);
     if (m < p.M) {
         uint8_t* dst = p.out8 + (size_t)m * p.half + h0;
         st_global_v4(dst, make_uint4(w[0], w[1], w[2], w[3]));
