@@ -4,7 +4,8 @@
 //
 // The single-tile kernel keeps one K and one V chunk of 112 keys in shared memory (Q + K + V + P fill it), so every
 // chunk pays a full TMA round trip before its MMAs: measured 4.5 us per additional chunk.  Here
-//   * chunks are 64 keys, K/V are double-buffered (Q 64 KB + 2 x (32 + 32) KB), the producer runs two chunks ahead;
+//   * chunks are 64 keys, K/V are double-buffered (Q 64 KB + 2 x (32 + 32) KB), the producer runs two chunks ahead; a stage's K
+//     is released behind its Q.K^T and its V behind its P.V (both behind P.V before: 1.44 -> 0.95 us per chunk of a long chain)
 //   * S is double-buffered in TMEM (2 x 64 columns) so QK(j+1) is issued before the softmax of chunk j has finished;
 //   * P (bf16) overlays its S buffer and feeds the PV MMA as the A operand from TMEM -- no shared-memory round trip;
 //   * the row of S lives in registers (one tcgen05.wait per chunk); O is rescaled only when a row maximum grows by
@@ -93,14 +94,15 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
     uint64_t* q_full = bars + 0;
     uint64_t* k_full = bars + 1;      // [2]
     uint64_t* v_full = bars + 3;      // [2]
-    uint64_t* kv_empty = bars + 5;    // [2]
+    uint64_t* k_empty = bars + 5;     // [2] Q.K^T of the chunk in the stage has completed
     uint64_t* s_full = bars + 7;      // [2] one per S buffer
     uint64_t* p_ready = bars + 9;     // [2] 128 arrivals per chunk, one barrier per S / P buffer
     uint64_t* o_full = bars + 11;     // PV of a chunk has completed (read only where the count is known to within one)
     uint64_t* o_done = bars + 12;     // every PV of this CTA has completed
     uint64_t* c_full = bars + 13;     // the C column slices of the combine have landed
     uint64_t* q_part = bars + 14;     // [3] the second .. fourth 64-column block of Q (q_full covers the first)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+    uint64_t* v_empty = bars + 17;    // [2] P.V of it
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const uint64_t deadline = tc::global_timer_ns() + FRT_KERNEL_DEADLINE_NS;
@@ -137,7 +139,8 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&k_full[i], 1);
             tc::mbar_init(&v_full[i], 1);
-            tc::mbar_init(&kv_empty[i], 1);
+            tc::mbar_init(&k_empty[i], 1);
+            tc::mbar_init(&v_empty[i], 1);
             tc::mbar_init(&s_full[i], 1);
         }
         tc::mbar_init(&p_ready[0], 128);
@@ -171,13 +174,19 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
 
     if (warp == 4) {
         // ---------------- TMA producer (whole warp)
-        auto load_kv = [&](int j) {
+        auto load_k = [&](int j) {
             const int st = j & 1;
             const int key0 = (c_begin + j) * BKV;
             if (tc::elect_one()) {
                 tc::mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
                 for (int db = 0; db < 4; ++db)
                     tc::tma_load_4d(sK + st * Cfg::KV_BYTES + db * (BKV * 128), &tmK, &k_full[st], db * 64, hk, key0, b);
+            }
+        };
+        auto load_v = [&](int j) {
+            const int st = j & 1;
+            const int key0 = (c_begin + j) * BKV;
+            if (tc::elect_one()) {
                 tc::mbar_arrive_expect_tx(&v_full[st], V_BYTES);
                 for (int db = 0; db < DV / 64; ++db)
                     tc::tma_load_4d(sV + st * V_BYTES + db * (BKV * 128), &tmV, &v_full[st], dq * DV + db * 64, hk, key0, b);
@@ -186,7 +195,8 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
         // chunks that lie inside the rows the previous kernel does not write may be fetched while it still runs
         int early = 0;
         while (early < 2 && early < nchunks && (c_begin + early + 1) * BKV <= static_rows) {
-            load_kv(early);
+            load_k(early);
+            load_v(early);
             ++early;
         }
         pdl_wait();
@@ -202,9 +212,23 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
                 tc::tma_load_5d(sQ + db * (128 * 128), &tmQ, qb, db * 64, 0, hk, tok0, b);
             }
         }
-        for (int j = early; j < nchunks; ++j) {
-            if (j >= 2 && !attn_warp_wait(&kv_empty[j & 1], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER, deadline, abort_flag)) break;
-            load_kv(j);
+        for (int j = early; j < 2 && j < nchunks; ++j) {
+            load_k(j);
+            load_v(j);
+        }
+        // A stage's K is free when its Q.K^T has completed, a chunk and a half before its V: K runs one chunk ahead of V.  (Both
+        // released behind P.V, a stage's way round -- 64 KB from L2, Q.K^T, softmax, P.V -- was what a chunk took: 1.6 us.)
+        auto k_next = [&](int j) {
+            if (j >= nchunks) return true;
+            if (!attn_warp_wait(&k_empty[j & 1], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER, deadline, abort_flag)) return false;
+            load_k(j);
+            return true;
+        };
+        bool ok = k_next(2);
+        for (int j = 2; ok && j < nchunks; ++j) {
+            ok = k_next(j + 1) &&
+                 attn_warp_wait(&v_empty[j & 1], (uint32_t)(((j >> 1) - 1) & 1), AERR_PRODUCER, deadline, abort_flag);
+            if (ok) load_v(j);
         }
     } else if (warp == 5) {
         // ---------------- MMA issuer (whole warp)
@@ -213,7 +237,8 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
         const uint64_t dq_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sQ));
         const uint64_t dk_base = tc::make_desc_kmajor_sw128(tc::smem_u32(sK));
         const uint64_t dv_base = tc::make_desc_mnmajor_sw128(tc::smem_u32(sV), BKV * 128);
-        const uint32_t s_full_a = tc::smem_u32(s_full), kv_empty_a = tc::smem_u32(kv_empty), o_full_a = tc::smem_u32(o_full);
+        const uint32_t s_full_a = tc::smem_u32(s_full), k_empty_a = tc::smem_u32(k_empty),
+                       v_empty_a = tc::smem_u32(v_empty), o_full_a = tc::smem_u32(o_full);
         // the 64-column block `blk` of Q . K^T(j)
         auto qk_block = [&](int j, int blk) {
             const uint64_t dk = dk_base + (uint64_t)((j & 1) * (Cfg::KV_BYTES >> 4) + blk * ((BKV * 128) >> 4));
@@ -223,7 +248,10 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     tc::mma_f16(d_tm, dqb + 2 * k, dk + 2 * k, idesc_s, (blk > 0 || k > 0) ? 1u : 0u);
-                if (blk == 3) tc::mma_commit(s_full_a + 8 * (j & 1));
+                if (blk == 3) {
+                    tc::mma_commit(s_full_a + 8 * (j & 1));
+                    if (j + 2 < nchunks) tc::mma_commit(k_empty_a + 8 * (j & 1));
+                }
             }
         };
         bool ok = attn_warp_wait(q_full, 0u, AERR_MMA, deadline, abort_flag);
@@ -260,7 +288,7 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
                 for (int k = 0; k < BKV / 16; ++k)
                     tc::mma_f16_ts(tmem + Cfg::O_COL, a_tm + 8 * k, dv + (uint64_t)(k * ((16 * 128) >> 4)), idesc_o,
                                    (j > 0 || k > 0) ? 1u : 0u);
-                tc::mma_commit(kv_empty_a + 8 * (j & 1));
+                if (j + 2 < nchunks) tc::mma_commit(v_empty_a + 8 * (j & 1));
                 tc::mma_commit(o_full_a);
             }
         }
@@ -903,17 +931,17 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
         } else {
             // kv_splits is a bound: the cheapest form that fits, by the times of the captured action-expert loop (10-64 queries
             // x 8 heads, 100-1088 keys, batch 1-4) and of the prefix encoder's launches (96-1024 x 8 heads on themselves), in
-            // units of 0.1 us over the cluster exchange in four parts: 1.6 us per chunk of a split's chain, 1.7 more when a
-            // CTA moves out 128 columns of O; one CTA per (tile, split) 1.9 per chunk and 1 without a combine, 4.5 with one
-            // through the scratch; 2.3 for the scratch in four parts.  (2 x 50 on 818 keys: 4 splits of 4 parts
-            // 12.3 -> 9.8 us; 768 on 768: 2 splits through the scratch 23.3 -> 18.6.)
+            // units of 0.05 us over the cluster exchange in four parts: 0.8 us per chunk of a split's chain, 0.9 and 1.9 once
+            // when a CTA moves out 128 columns of O; one CTA per tile 0.93 per chunk, per (tile, split) through the scratch 1.1 and
+            // 4.3 once; 2.3 for the scratch in four parts.  (2 x 50 on 818 keys 8.8 us as 4 splits of 4 parts, 10.9 as 2; 768 on
+            // 768: one CTA per tile 15.8, two splits through the scratch 16.1.)
             const long long ctas1 = (long long)tiles * groups;
             auto chain = [&](int c) { return (p.chunks_total + c - 1) / c; };
-            int best = 19 * p.chunks_total + 10, bc = 1, bp = 0;                 // bp: 0 = not a cluster
+            int best = 19 * p.chunks_total - 6, bc = 1, bp = 0;                 // bp: 0 = not a cluster
             for (int c = 8; c >= 2; c >>= 1) {
                 if (c > bound || c / 2 >= p.chunks_total) continue;
                 for (int parts = 4; parts >= 2; parts -= 2) {
-                    const int cost = 16 * chain(c) + (parts == 2 ? 17 : 0);
+                    const int cost = parts == 2 ? 18 * chain(c) + 38 : 16 * chain(c);
                     if (cost < best && (fits(c, parts, false) || (parts == 4 && tail && fits(c, 4, true)))) {
                         best = cost;
                         bc = c;
@@ -921,7 +949,7 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
                     }
                 }
                 if (ctas1 * c > sms) continue;
-                const int cost = ctas1 * c * 4 <= sms ? 16 * chain(c) + 23 : 19 * chain(c) + 45;
+                const int cost = ctas1 * c * 4 <= sms ? 16 * chain(c) + 46 : 22 * chain(c) + 86;
                 if (cost < best) {
                     best = cost;
                     bc = c;
