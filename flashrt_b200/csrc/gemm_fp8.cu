@@ -1080,6 +1080,7 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     p.kb_total = (K + 127) / 128;
     cudaStream_t s = (cudaStream_t)stream;
     bool pdl = flags & 1;
+    p.early = pdl ? 1 : 0;
     // M <= 256 without a hint: the kernels below it stream the weights through clusters that split K, which wins while the
     // product is small or K is long; from about 8 MB of weights (M <= 128), or for most of 129 .. 256, the persistent kernels
     // of the large products do.  Microseconds again: token-major 5 + 0.3 per MB of weights (5.2 + 0.45 above 64 rows),
@@ -1144,6 +1145,7 @@ int frt_b200_gemm_fp8_nt_splitk(const void* A, const void* W, void* D, int M, in
             p.split_ws = workspace;
             p.split_cnt = reinterpret_cast<unsigned*>(counters);
             p.ksplits = S;
+            p.early = flags & 1;
             return launch_gemm_pair<256, EPI_P_BF16, true>(A, W, p, K, (cudaStream_t)stream);
         }
     }
@@ -1256,6 +1258,7 @@ int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int
     p.out8 = (uint8_t*)out8;
     p.out_scale = d_out_scale;
     p.half = half;
+    p.early = flags & 1;
     // SiLU gate (bit 6) and the hardware-tanh GELU (bit 7): built in the token-major kernel only
     if (M > 256) return launch_gemm_pair<256, EPI_P_GEGLU_FP8>(A, W, p, K, (cudaStream_t)stream);
     const bool silu = (flags & 64) != 0, fast = (flags & 128) != 0;
@@ -1405,6 +1408,7 @@ int frt_b200_gemm_fp8_nt_bias_gelu_fp8(const void* A, const void* W, void* out8,
     p.kb_total = (K + 127) / 128;
     p.out8 = (uint8_t*)out8;
     p.out_scale = d_out_scale;
+    p.early = flags & 1;
     const int kind = pick_large(M, N, K, false);
     if (flags & 128) return launch_large<EPI_P_BIAS_GELU_FAST_FP8>(kind, A, W, p, K, (cudaStream_t)stream);
     return launch_large<EPI_P_BIAS_GELU_FP8>(kind, A, W, p, K, (cudaStream_t)stream);

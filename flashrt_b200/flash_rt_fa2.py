@@ -10,12 +10,20 @@ shared memory.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 from ._lib import call, call_status, KernelError  # noqa: F401
 
 
+@functools.lru_cache(maxsize=256)
 def _s3(t):
     return (C.c_longlong * 3)(int(t[0]), int(t[1]), int(t[2]))
+
+
+def _strides(*arrays):
+    """Host arrays of three strides each (to be held until the call has returned; their addresses go through the native call
+    module, where ctypes pointers take the slow path: 11 us a call)."""
+    return [_s3(tuple(a)) for a in arrays]
 
 
 _COUNTERS = {}
@@ -41,10 +49,10 @@ def _fwd(Q, K, V, O, softmax_lse, seqused_k, lse_accum, o_accum, batch, seqlen_q
         counters = _default_counters(2 * ((seqlen_q * g + 127) // 128) * num_heads_kv * batch)
     if not (lse_accum and o_accum):
         lse_accum = o_accum = counters = 0
+    strides = _strides(q_strides, k_strides, v_strides, o_strides)
     call("frt_b200_attention_fwd_bf16", Q, K, V, O, out_fp8 or None, out_scale or None, softmax_lse or None,
          seqused_k or None, batch, seqlen_q, seqlen_k, num_heads_q, num_heads_kv, head_dim,
-         C.cast(_s3(q_strides), C.c_void_p), C.cast(_s3(k_strides), C.c_void_p),
-         C.cast(_s3(v_strides), C.c_void_p), C.cast(_s3(o_strides), C.c_void_p),
+         *map(C.addressof, strides),
          softmax_scale, kv_splits, kv_static_rows, o_accum or None, lse_accum or None, counters or None,
          (1 if pdl else 0) | (flags & ~1), stream)
 
@@ -87,8 +95,8 @@ def fwd_bf16_static_scratch(Q, K, V, O, softmax_lse, batch, seqlen_q, seqlen_k, 
     reference): the partials live in a fixed array inside the library instead of caller-provided buffers.  Raises
     :class:`KernelError` (status -4) when the shape exceeds that array (8 splits, 512 query rows x heads, head_dim
     256).  Make the first call on a device outside stream capture; do not let two calls overlap on the GPU."""
+    strides = _strides(q_strides, k_strides, v_strides, o_strides)
     call("frt_b200_attention_fwd_bf16_static_scratch", Q, K, V, O, out_fp8 or None, out_scale or None,
          softmax_lse or None, seqused_k or None, batch, seqlen_q, seqlen_k, num_heads_q, num_heads_kv, head_dim,
-         C.cast(_s3(q_strides), C.c_void_p), C.cast(_s3(k_strides), C.c_void_p),
-         C.cast(_s3(v_strides), C.c_void_p), C.cast(_s3(o_strides), C.c_void_p),
+         *map(C.addressof, strides),
          softmax_scale, kv_splits, kv_static_rows, 1 if pdl else 0, stream)

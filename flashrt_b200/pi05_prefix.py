@@ -120,13 +120,21 @@ class Pi05PrefixEncoderB200:
         self.act_scale = torch.ones(layers, len(SITES), dtype=torch.float32, device=dev)
         self.scratch_scale = torch.zeros(1, dtype=torch.float32, device=dev)
         self.gemm = fvk.GemmRunner()
+        # Addresses of what an encoder owns for its lifetime, taken once: a pass is 140 launches from Python, and indexing the
+        # tensors for them took 6 of the 10 us that each one cost the host (a pass over 100 rows 1.43 ms on 1.08 ms of device time)
+        buffers = ("x", "xn", "h_bf16", "qkv", "q", "attn", "merged", "hidden", "act8", "attn8", "hid8", "ones", "rope", "o_accum",
+                   "lse_accum", "splitk_ws", "splitk_counters", "attn_counters", "scratch_scale")
+        self._p = {n: getattr(self, n).data_ptr() for n in buffers}
+        weights = ("w_qkv", "ws_qkv_t", "w_o", "ws_o_t", "w_gu", "ws_gu_t", "w_d", "ws_d_t")
+        self._w = [{n: getattr(self, n)[i].data_ptr() for n in weights} for i in range(layers)]
+        self._scales = [{site: self.act_scale[i, j].data_ptr() for j, site in enumerate(SITES)} for i in range(layers)]
         self.stream = torch.cuda.Stream(device=dev)
         self.stream.wait_stream(torch.cuda.current_stream(dev))       # weights, tables and buffers were written there
         self.calibrated = False
 
     # ------------------------------------------------------------------
     def _sp(self, layer, site):
-        return self.act_scale[layer, SITES.index(site)].data_ptr()
+        return self._scales[layer][site]
 
     def _dyn_quant(self, src, dst8, layer, site, st):
         fvk.quantize_fp8_device(src.data_ptr(), dst8.data_ptr(), self.scratch_scale.data_ptr(), src.numel(), st)
@@ -134,56 +142,55 @@ class Pi05PrefixEncoderB200:
         fvk.quantize_fp8_static(src.data_ptr(), dst8.data_ptr(), self._sp(layer, site), src.numel(), st)
 
     def _norm(self, seq, delta, layer, site, st, calibrate):
-        """(x += delta) ; RMSNorm with unit weight -> FP8 input of ``site``."""
+        """(x += delta) ; RMSNorm with unit weight -> FP8 input of ``site``.  ``delta``: address or None."""
+        p = self._p
         if not calibrate:
-            fvk.call("frt_b200_norm_fp8", self.x.data_ptr(), delta.data_ptr() if delta is not None else None, None, 0,
-                     self.ones.data_ptr(), None, 0, self.act8.data_ptr(), None, seq, ENC_D, 1e-6,
-                     self._sp(layer, site), 0, st)
+            fvk.call("frt_b200_norm_fp8", p["x"], delta, None, 0, p["ones"], None, 0, p["act8"], None, seq, ENC_D, 1e-6,
+                     self._sp(layer, site), 1, st)
             return
-        fvk.call("frt_b200_norm_bf16", self.x.data_ptr(), delta.data_ptr() if delta is not None else None, None, 0,
-                 self.ones.data_ptr(), None, 0, self.h_bf16.data_ptr(), None, seq, ENC_D, 1e-6, 0, st)
+        fvk.call("frt_b200_norm_bf16", p["x"], delta, None, 0, p["ones"], None, 0, p["h_bf16"], None, seq, ENC_D, 1e-6, 0, st)
         self._dyn_quant(self.h_bf16[:seq], self.act8[:seq], layer, site, st)
 
-    def _gemm(self, a8, w8, ws, out, M, N, K, sp, st):
-        self.gemm.fp8_nt_dev(a8.data_ptr(), w8.data_ptr(), out.data_ptr(), M, N, K, sp, ws.data_ptr(), st)
+    def _gemm(self, a8, w8, ws, out, M, N, K, sp, st, pdl):
+        # pdl (not while calibrating): weights, tables and scales are settled before a pass begins and may be fetched early
+        self.gemm.fp8_nt_dev(a8, w8, out, M, N, K, sp, ws, st, pdl=pdl)
 
     def transformer_encoder(self, seq: int, k_out: torch.Tensor, v_out: torch.Tensor, st: int, calibrate: bool):
         """Runs the layers on ``self.x[:seq]``; layer i writes rows [0, seq) of k_out[i] / v_out[i] ((rows, 256))."""
-        L = self.layers
-        qs = (seq * ENC_NH * ENC_HD, ENC_NH * ENC_HD, ENC_HD)
+        L, p, pdl = self.layers, self._p, not calibrate
+        QD, KD = ENC_NH * ENC_HD, ENC_NKV * ENC_HD
+        qs, ks = (seq * QD, QD, ENC_HD), (k_out.shape[1] * ENC_HD, ENC_HD, ENC_HD)
+        k0, v0 = k_out.data_ptr(), v_out.data_ptr()
+        k_step, v_step = k_out.stride(0) * k_out.element_size(), v_out.stride(0) * v_out.element_size()
+        scale = 1.0 / math.sqrt(ENC_HD)
         for i in range(L):
-            self._norm(seq, self.xn if i > 0 else None, i, "qkv", st, calibrate)
-            self._gemm(self.act8, self.w_qkv[i], self.ws_qkv_t[i], self.qkv, seq, QKV_N, ENC_D, self._sp(i, "qkv"), st)
-            fvk.qkv_split_rope(self.qkv.data_ptr(), self.rope.data_ptr(), self.q.data_ptr(), k_out[i].data_ptr(),
-                               v_out[i].data_ptr(), seq, ENC_NH * ENC_HD, ENC_NKV * ENC_HD, ENC_NKV * ENC_HD, ENC_HD, st)
+            w, k, v = self._w[i], k0 + i * k_step, v0 + i * v_step
+            self._norm(seq, p["xn"] if i > 0 else None, i, "qkv", st, calibrate)
+            self._gemm(p["act8"], w["w_qkv"], w["ws_qkv_t"], p["qkv"], seq, QKV_N, ENC_D, self._sp(i, "qkv"), st, pdl)
+            fvk.qkv_split_rope(p["qkv"], p["rope"], p["q"], k, v, seq, QD, KD, KD, ENC_HD, st, pdl=pdl)
             if i == L - 1:
                 return
-            ks = (k_out[i].shape[0] * ENC_HD, ENC_HD, ENC_HD)
             if calibrate:
-                fa2.fwd_bf16(self.q.data_ptr(), k_out[i].data_ptr(), v_out[i].data_ptr(), self.attn.data_ptr(), 0, 0, 0,
-                             1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs, ks, ks, qs, 1.0 / math.sqrt(ENC_HD), 0, st)
+                fa2.fwd_bf16(p["q"], k, v, p["attn"], 0, 0, 0, 1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs, ks, ks, qs, scale, 0, st)
                 self._dyn_quant(self.attn[:seq], self.attn8[:seq], i, "o", st)
             else:
-                fa2.fwd_bf16(self.q.data_ptr(), k_out[i].data_ptr(), v_out[i].data_ptr(), self.attn.data_ptr(), 0,
-                             self.lse_accum.data_ptr(), self.o_accum.data_ptr(), 1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs,
-                             ks, ks, qs, 1.0 / math.sqrt(ENC_HD), 0, st, kv_splits=ATTN_SPLITS, flags=16,
-                             counters=self.attn_counters.data_ptr(),
-                             out_fp8=self.attn8.data_ptr(), out_scale=self._sp(i, "o"))
-            self._gemm(self.attn8, self.w_o[i], self.ws_o_t[i], self.xn, seq, ENC_D, ENC_NH * ENC_HD, self._sp(i, "o"), st)
-            self._norm(seq, self.xn, i, "gu", st, calibrate)
+                fa2.fwd_bf16(p["q"], k, v, p["attn"], 0, p["lse_accum"], p["o_accum"], 1, seq, seq, ENC_NH, ENC_NKV, ENC_HD, qs,
+                             ks, ks, qs, scale, 0, st, kv_splits=ATTN_SPLITS, flags=16, counters=p["attn_counters"], pdl=True,
+                             out_fp8=p["attn8"], out_scale=self._sp(i, "o"))
+            self._gemm(p["attn8"], w["w_o"], w["ws_o_t"], p["xn"], seq, ENC_D, QD, self._sp(i, "o"), st, pdl)
+            self._norm(seq, p["xn"], i, "gu", st, calibrate)
             if calibrate or seq <= 256:
-                self._gemm(self.act8, self.w_gu[i], self.ws_gu_t[i], self.merged, seq, 2 * ENC_H, ENC_D, self._sp(i, "gu"), st)
+                self._gemm(p["act8"], w["w_gu"], w["ws_gu_t"], p["merged"], seq, 2 * ENC_H, ENC_D, self._sp(i, "gu"), st, pdl)
             if calibrate:
-                fvk.gate_geglu_merged(self.merged.data_ptr(), self.hidden.data_ptr(), seq, ENC_H, st)
+                fvk.gate_geglu_merged(p["merged"], p["hidden"], seq, ENC_H, st)
                 self._dyn_quant(self.hidden[:seq], self.hid8[:seq], i, "d", st)
             elif seq <= 256:
-                fvk.gate_geglu_merged_fp8(self.merged.data_ptr(), self.hid8.data_ptr(), seq, ENC_H, self._sp(i, "d"), st)
+                fvk.gate_geglu_merged_fp8(p["merged"], p["hid8"], seq, ENC_H, self._sp(i, "d"), st, pdl=True)
             else:               # one launch: the activation under the product's MMAs
-                self.gemm.fp8_nt_dev_geglu_fp8(self.act8.data_ptr(), self.w_gu[i].data_ptr(), self.hid8.data_ptr(), seq, ENC_H,
-                                               ENC_D, self._sp(i, "gu"), self.ws_gu_t[i].data_ptr(), self._sp(i, "d"), st)
-            self.gemm.fp8_nt_dev_splitk(self.hid8.data_ptr(), self.w_d[i].data_ptr(), self.xn.data_ptr(), seq, ENC_D, ENC_H,
-                                        self._sp(i, "d"), self.ws_d_t[i].data_ptr(), self.splitk_ws.data_ptr(),
-                                        self.splitk_ws.numel() * 4, self.splitk_counters.data_ptr(), st)
+                self.gemm.fp8_nt_dev_geglu_fp8(p["act8"], w["w_gu"], p["hid8"], seq, ENC_H, ENC_D, self._sp(i, "gu"),
+                                               w["ws_gu_t"], self._sp(i, "d"), st, pdl=True)
+            self.gemm.fp8_nt_dev_splitk(p["hid8"], w["w_d"], p["xn"], seq, ENC_D, ENC_H, self._sp(i, "d"), w["ws_d_t"],
+                                        p["splitk_ws"], self.splitk_ws.numel() * 4, p["splitk_counters"], st, pdl=pdl)
 
     # ------------------------------------------------------------------
     def _check(self, embeds, k_out, v_out):
