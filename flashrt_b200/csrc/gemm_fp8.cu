@@ -964,6 +964,20 @@ template <int EPI>
 static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, int K, int M, int splits, bool pdl,
                                   cudaStream_t s) {
     const Nvfp4Small c = pick_small_m_nvfp4(M, p.N, K, splits);
+    // the push exchange of the token-major kernel where it is the faster one; asked for splits (0 or a power of two): the same bytes
+    if (M <= 64) {
+        const TokPlan pl = pick_tok_nvfp4(M, p.N, K, splits <= 0 ? 0 : c.splits);
+        if (pl.S && (splits > 1 || tok_nvfp4_us(M, p.N, K, pl.BN, pl.S) < c.us - 0.9)) {
+            TokParams t = {};
+            t.M = M; t.N = p.N; t.sa = p.sa; t.sb = p.sb; t.alpha_host = p.alpha_host;
+            t.out = p.out; t.bias = p.bias; t.sf_a = p.sf_lane; t.sf_w = p.sf_col;
+            t.rope = p.rope; t.outQ = p.outQ; t.outK = p.outK; t.outV = p.outV; t.devpos = p.devpos;
+            t.q_dim = p.q_dim; t.k_dim = p.k_dim; t.v_dim = p.v_dim; t.head_dim = p.head_dim;
+            constexpr int TEPI = EPI == EPI_ROPE_SPLIT ? TOK_EPI_ROPE : TOK_EPI_BF16;
+            if (pl.BN == 128) return launch_gemm_tok<128, TOK_PRO_TMA, TEPI, 0, true>(A, W, t, K, pl, pdl, s);
+            return launch_gemm_tok<64, TOK_PRO_TMA, TEPI, 0, true>(A, W, t, K, pl, pdl, s);
+        }
+    }
     if (c.bn == 32) return launch_gemm<32, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
     if (c.bn == 64) return launch_gemm<64, true, EPI, true>(A, W, p, K, c.splits, pdl, s);
     if (c.bn == 128) return launch_gemm<128, true, EPI, true>(A, W, p, K, c.splits, pdl, s);

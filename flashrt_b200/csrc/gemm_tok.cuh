@@ -113,20 +113,29 @@ struct TokParams {
     uint8_t* q8_out;
     const __nv_bfloat16* q8_mod;
     const float* q8_scale;
+    // NVFP4: block scales of both operands in atoms of 128 rows x 4 blocks, atoms along K = K / 64
+    const uint8_t* sf_a;
+    const uint8_t* sf_w;
+    int sf_katoms;
 #ifdef FRT_PHASE_STAMPS
     int trace_slot;
 #endif
 };
 
-template <int BN>
+// FP4 (BF16 and RoPE finishes, at most 64 tokens): k-blocks of 256 packed e2m1 elements, the scale atoms of both operands behind the
+// operand tiles.  The block-scaled MMA has M = 128 only: with at most 64 tokens its upper 64 lanes read the weight tile behind the
+// 8 KB of tokens and their results are never looked at.
+template <int BN, bool FP4 = false>
 struct TokCfg {
+    static_assert(!FP4 || BN <= 128, "NVFP4: one atom row of column scales");
     static constexpr int W_BYTES = BN * 128;
+    static constexpr int SF_BYTES = FP4 ? 2048 : 0;           // per operand: four atoms of a k-block
     // A tile of a stage: 128 (or, for at most 64 tokens, 64) token rows x 128 K-bytes
     static constexpr int a_bytes(bool m64) { return m64 ? 64 * 128 : 128 * 128; }
-    static constexpr int stage_bytes(bool m64) { return a_bytes(m64) + W_BYTES; }
+    static constexpr int stage_bytes(bool m64) { return a_bytes(m64) + W_BYTES + (FP4 ? (2 * SF_BYTES + 1023) / 1024 * 1024 : 0); }
     static constexpr int MAX_STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
     static constexpr int AUX_BYTES = 2048;                    // barriers, flags, per-token 1 / rms
-    static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+    static constexpr int TMEM_COLS = FP4 ? 2 * BN : BN < 32 ? 32 : BN;      // NVFP4: 32 scale columns behind the accumulator
     // operand ring, then the receive slots [S][per][BN] fp32 of the split-K exchange (never aliased: a fast rank
     // pushes while a slow rank's MMAs still read its operands)
     static int ring_bytes(int stages, bool m64) { return stages * stage_bytes(m64); }
@@ -200,11 +209,12 @@ __device__ __forceinline__ void tok_sum8(const float* recv, int S, int per, int 
 // ACT (GeGLU epilogue only): the gate activation, 0 exact GELU(tanh), 1 SiLU, 2 GELU through the hardware tanh.  A
 // template argument, not a field of the parameters: selected at run time inside the unrolled finish the choice cost
 // 0.55 us per gate|up launch of the action-expert loop (0.10 ms per loop), a third of that epilogue's arithmetic.
-template <int BN, int PRO, int EPI, int ACT = 0>
+template <int BN, int PRO, int EPI, int ACT = 0, bool FP4 = false>
 __global__ void __launch_bounds__(256, 2)
 gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, TokParams p) {
     static_assert(EPI != TOK_EPI_GEGLU || BN >= 128, "GeGLU tiles are BN / 2 gate rows + the matching up rows");
-    using Cfg = TokCfg<BN>;
+    static_assert(!FP4 || (PRO == TOK_PRO_TMA && (EPI == TOK_EPI_BF16 || EPI == TOK_EPI_ROPE)), "forms of the NVFP4 product");
+    using Cfg = TokCfg<BN, FP4>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* aux = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* tiles = aux + Cfg::AUX_BYTES;                       // 1024-aligned
@@ -298,6 +308,14 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             } else {
                 tc::tma_load_2d(dst, &tmW, bar, kb * 128, n0);
             }
+            if constexpr (FP4)
+                tc::bulk_load(dst + Cfg::W_BYTES + Cfg::SF_BYTES, p.sf_w + ((size_t)(n0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512,
+                              2048, bar);
+        };
+        auto load_a = [&](int stage, int kb) {
+            const uint32_t dst = ring + stage * STAGE_BYTES, bar = full_a + 8 * stage;
+            tc::tma_load_2d(dst, &tmA, bar, kb * 128, m0);
+            if constexpr (FP4) tc::bulk_load(dst + A_BYTES + Cfg::W_BYTES, p.sf_a + (size_t)kb * 4 * 512, 2048, bar);
         };
         const int pre = nkb < STG ? nkb : STG;
         if (tc::elect_one()) {
@@ -309,8 +327,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         pdl_wait();
         if (tc::elect_one()) {
             if (PRO == TOK_PRO_TMA) {
-                for (int i = 0; i < pre; ++i)
-                    tc::tma_load_2d(ring + i * STAGE_BYTES, &tmA, full_a + 8 * i, (kb0 + i) * 128, m0);
+                for (int i = 0; i < pre; ++i) load_a(i, kb0 + i);
             }
             *issued = pre;
         }
@@ -325,7 +342,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             if (tc::elect_one()) {
                 tc::mbar_arrive_expect_tx(full_a + 8 * s, tx);
                 load_w(s, kb0 + i);
-                if (PRO == TOK_PRO_TMA) tc::tma_load_2d(ring + s * STAGE_BYTES, &tmA, full_a + 8 * s, (kb0 + i) * 128, m0);
+                if (PRO == TOK_PRO_TMA) load_a(s, kb0 + i);
                 *issued = i + 1;
             }
             if (++s == STG) { s = 0; ph ^= 1; }
@@ -426,7 +443,12 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
     if (warp == 1) {
         // ---------------- MMA issuer (whole warp)
-        const uint32_t idesc = tc::make_idesc(0, 0, 0, 0, m64 ? 64 : 128, BN) | (p.w_kn ? (1u << 16) : 0u);   // bit 16: B MN-major
+        const uint32_t idesc = FP4 ? tc::make_idesc_nvfp4(128, BN)
+                                   : tc::make_idesc(0, 0, 0, 0, m64 ? 64 : 128, BN) | (p.w_kn ? (1u << 16) : 0u);   // bit 16: B MN-major
+        // scales in tensor memory: four columns per K = 64 step; a tile of 64 weight rows may start at row 64 of its atom
+        const uint32_t tmem_sfa = tmem_d + BN, tmem_sfw = tmem_sfa + 16;
+        const uint32_t sfw_off = FP4 ? (uint32_t)((n0 & 127) >> 5) : 0u;
+        const uint32_t sf0 = tc::smem_u32(tiles) + A_BYTES + Cfg::W_BYTES;
         bool failed = false;
         if (PRO == TOK_PRO_NORM) failed = !tc::warp_wait(tc::smem_u32(a_ready), 0, false, deadline, abort_flag);
         const uint32_t full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty), accum_a = tc::smem_u32(accum_bar);
@@ -448,10 +470,21 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             if (i == 0 && lane == 0) g_tok_trace[p.trace_slot][(blockIdx.z * gridDim.x + blockIdx.x) % 160][10] = tc::global_timer_ns();
 #endif
             const uint64_t so = (uint64_t)((s * STAGE_BYTES) >> 4);
-            const uint32_t done = empty_a + 8 * s;
+            const uint32_t sf = sf0 + (uint32_t)(s * STAGE_BYTES), done = empty_a + 8 * s;
             if (++s == STG) { s = 0; ph ^= 1; }
             ready = tc::mbar_test(full_a + 8 * s, ph);
             if (tc::elect_one()) {
+                if constexpr (FP4) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        tc::tmem_cp_sf_atom(tmem_sfa + 4 * k, sf + 512 * k);
+                        tc::tmem_cp_sf_atom(tmem_sfw + 4 * k, sf + Cfg::SF_BYTES + 512 * k);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        tc::mma_nvfp4(tmem_d, dA0 + so + 2 * k, dW0 + so + 2 * k, idesc, tmem_sfa + 4 * k,
+                                      tmem_sfw + 4 * k + sfw_off, (i > 0 || k > 0) ? 1u : 0u);
+                } else
 #pragma unroll
                 for (int k = 0; k < 4; ++k)   // 4 x (K = 32) per 128-byte k-block; +32 bytes = +2 in the address field
                     tc::mma_f8(tmem_d, dA0 + so + 2 * k, dW0 + so + wstep * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
@@ -549,7 +582,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     cluster_wait_acquire();          // every peer has initialised its receive barrier (arrived during its set-up)
     {
         const int quad = warp & 3, chalf = warp >> 2;
-        const int qrows = m64 ? 16 : 32;                       // accumulator rows per 32-lane quadrant
+        const int qrows = m64 && !FP4 ? 16 : 32;               // accumulator rows per 32-lane quadrant
         const int row = lane < qrows ? quad * qrows + lane : Mt;   // token inside the m-tile (none on the idle lanes)
         if (have_acc && quad * qrows < Mt) {
             const uint32_t trow = tmem_d + ((uint32_t)(quad * 32) << 16);
@@ -847,11 +880,13 @@ static bool tok_plan(int N, int K, int m_tiles, int mt, int epi, int pro, int sm
 // m-tiles of at most 128 tokens, or (half) of at most 64: M = 64 MMAs over 8 KB operand tiles, two CTAs to an SM
 static inline int tok_m_tiles(int M, bool half) { return M <= 0 ? 1 : half ? (M + 63) / 64 : (M + 127) / 128; }
 
-template <int BN, int PRO, int EPI, int ACT = 0>
+template <int BN, int PRO, int EPI, int ACT = 0, bool FP4 = false>
 static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, const TokPlan& pl, bool pdl,
                            cudaStream_t stream) {
-    using Cfg = TokCfg<BN>;
-    auto kern = gemm_tok_kernel<BN, PRO, EPI, ACT>;
+    using Cfg = TokCfg<BN, FP4>;
+    auto kern = gemm_tok_kernel<BN, PRO, EPI, ACT, FP4>;
+    const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
+    if (FP4) p.sf_katoms = K / 64;
     const int m_tiles = pl.m_tiles;
     const int mt = (p.M + m_tiles - 1) / m_tiles;             // rows spread evenly over the m-tiles
     p.m_rows = mt;
@@ -889,13 +924,13 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     CUtensorMap tmA, tmW;
     int rc;
     if (PRO == TOK_PRO_TMA) {
-        rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, (uint64_t)K, (uint64_t)K, m64 ? 64 : 128);
+        rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, row_bytes, row_bytes, m64 ? 64 : 128);
         if (rc) return rc;
     } else {
         memset(&tmA, 0, sizeof(tmA));
     }
     rc = p.w_kn ? get_tmap_2d_u8(&tmW, W, (uint64_t)K, (uint64_t)p.N, (uint64_t)p.N, 128)
-                : get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, (uint64_t)K, (uint64_t)K, EPI == TOK_EPI_GEGLU ? BN / 2 : BN);
+                : get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, row_bytes, row_bytes, EPI == TOK_EPI_GEGLU ? BN / 2 : BN);
     if (rc) return rc;
     const int tiles = EPI == TOK_EPI_GEGLU ? (p.half + BN / 2 - 1) / (BN / 2) : (p.N + BN - 1) / BN;
     cudaLaunchConfig_t cfg = {};
@@ -918,6 +953,38 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
+}
+
+// NVFP4, at most 64 rows: microseconds of a launch of N / bn tiles x S CTAs that are all resident -- fitted to 710 products of a
+// sweep (M 8 .. 64, N 1024 .. 14336, K 1024 .. 14336, in a graph, weights fetched early; 6 % standard deviation): k-blocks of a CTA,
+// KB pushed to its peers, tokens it finishes, SMs in use.
+static double tok_nvfp4_us(int M, int N, int K, int bn, int S) {
+    const int ctas = (N + bn - 1) / bn * S;
+    const double t = 2.0 + K / 256 / S * (bn == 128 ? 0.33 : 0.305) + (double)(S - 1) / S * M * bn / 256.0 * 0.09 +
+                     (M + S - 1) / S * bn / 1024.0 * 0.3;
+    return ctas > 74 ? t + (ctas - 74) * (1.35 / 74) : t;
+}
+// The cheapest plan (S = 0: none), `want` > 0 pins the split.  All CTAs resident at once, and of clusters of eight no more than fit
+// beside one another when a CTA needs an SM to itself.  50 x 2560 x 1024 6.1 -> 3.9 us against the small-M kernel and its exchange by
+// cluster barriers, 50 x 1024 x 4096 6.6 -> 4.6, 16 x 1024 x 1024 4.3 -> 2.8; unsplit products of much weight stay there (50 x 8192 x
+// 1024: 4.6 against 4.85).
+static TokPlan pick_tok_nvfp4(int M, int N, int K, int want) {
+    TokPlan best = {0, 0, 0, 0, 1};
+    double t = 1e30;
+    const int kbt = K / 256, sms = device_sm_count();
+    if ((N & 7) || M > 64) return best;
+    for (int bn = 64; bn <= 128; bn += 64) {
+        const int tiles = (N + bn - 1) / bn;
+        for (int S = 1; S <= 8; S *= 2) {
+            if (kbt % S || tiles * S > sms || (S == 8 && tiles > 14) || (want > 0 && S != want)) continue;
+            const double us = tok_nvfp4_us(M, N, K, bn, S);
+            if (us >= t) continue;
+            const int nkb = kbt / S, most = bn == 128 ? 6 : 8;
+            t = us;
+            best = {bn, S, nkb, nkb < most ? nkb : most, 1};
+        }
+    }
+    return best;
 }
 
 static int tok_sm_count() {

@@ -266,9 +266,11 @@ def test_gemm_nvfp4_pair_tiles_give_the_same_bytes(M, N, K, cols, pdl):
     assert np.array_equal(d_1.get(), d_2.get())
 
 
-@pytest.mark.parametrize("M,k_dim,pos", [(65, 256, 768), (100, 128, 3), (200, 256, 0), (256, 64, 541)])
-def test_gemm_nvfp4_pair_rope_split_equals_pair_of_launches(M, k_dim, pos):
-    """More than 64 tokens: the RoPE finish of the CTA pairs against GEMM -> qkv_split_rope, byte for byte."""
+@pytest.mark.parametrize("M,k_dim,pos", [(1, 64, 7), (64, 128, 541), (65, 256, 768), (100, 128, 3), (200, 256, 0),
+                                         (256, 64, 541)])
+def test_gemm_nvfp4_rope_finishes_equal_the_pair_of_launches(M, k_dim, pos):
+    """The RoPE finish of the token-major kernel (up to 64 tokens) and of the CTA pairs against GEMM -> qkv_split_rope, byte for
+    byte."""
     from flashrt_b200 import flash_rt_fp4 as fp4, flash_rt_kernels as fvk
     from gpu_util import Dev, rand_bf16, zeros
     rng = np.random.default_rng(M + k_dim)
@@ -288,3 +290,22 @@ def test_gemm_nvfp4_pair_rope_split_equals_pair_of_launches(M, k_dim, pos):
     assert fvk.tensor_core_status() == 0
     for a, b in zip(*out):
         assert np.array_equal(a.get(), b.get())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (17, 72, 2048), (64, 1096, 2048), (50, 200, 14336), (33, 1024, 768)])
+@pytest.mark.parametrize("splits", [0, 1, 2, 8])
+@pytest.mark.parametrize("pdl", [False, True])
+def test_gemm_nvfp4_token_major(M, N, K, splits, pdl):
+    """Up to 64 tokens: last tiles of a few weight rows, tiles that start at row 64 of a scale atom, one token per rank, more
+    k-blocks than the ring holds."""
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import Dev, zeros
+    rng = np.random.default_rng(M + N + K + splits)
+    Ap, Asf = _operand(rng, M, K, 1.0)
+    Wp, Wsf = _operand(rng, N, K, 0.02)
+    bias = O.f32_to_bf16_bits((rng.standard_normal(N) * 0.1).astype(np.float32))
+    d, d_b, d_o = [Dev(Ap), Dev(Asf), Dev(Wp), Dev(Wsf)], Dev(bias), zeros((M, N), np.uint16)
+    _lib.call("frt_b200_gemm_nvfp4_nt", d[0].ptr, d[1].ptr, d[2].ptr, d[3].ptr, d_o.ptr, M, N, K, 1.0, None, d_b.ptr, splits,
+              int(pdl), 0)
+    assert fvk.tensor_core_status() == 0
+    _check(d_o.get(), O.gemm_nvfp4(Ap, Asf, Wp, Wsf, bias=bias, want_f32=True))
