@@ -966,8 +966,8 @@ static int dispatch_small_m_nvfp4(const void* A, const void* W, GemmParams p, in
     const Nvfp4Small c = pick_small_m_nvfp4(M, p.N, K, splits);
     // the push exchange of the token-major kernel where it is the faster one; asked for splits (0 or a power of two): the same bytes
     if (M <= 64) {
-        const TokPlan pl = pick_tok_nvfp4(M, p.N, K, splits <= 0 ? 0 : c.splits);
-        if (pl.S && (splits > 1 || tok_nvfp4_us(M, p.N, K, pl.BN, pl.S) < c.us - 0.9)) {
+        const TokPlan pl = pick_tok_nvfp4(M, p.N, K, splits <= 0 ? 0 : c.splits, pdl);
+        if (pl.S && (splits > 1 || (pdl && pl.nkb <= 8) || tok_nvfp4_us(M, p.N, K, pl.BN, pl.S) < c.us - 0.9)) {
             TokParams t = {};
             t.M = M; t.N = p.N; t.sa = p.sa; t.sb = p.sb; t.alpha_host = p.alpha_host;
             t.out = p.out; t.bias = p.bias; t.sf_a = p.sf_lane; t.sf_w = p.sf_col;

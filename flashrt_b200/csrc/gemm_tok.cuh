@@ -964,15 +964,26 @@ static double tok_nvfp4_us(int M, int N, int K, int bn, int S) {
                      (M + S - 1) / S * bn / 1024.0 * 0.3;
     return ctas > 74 ? t + (ctas - 74) * (1.35 / 74) : t;
 }
-// The cheapest plan (S = 0: none), `want` > 0 pins the split.  All CTAs resident at once, and of clusters of eight no more than fit
+// The plan (S = 0: none), the cheapest by that cost; `want` > 0 pins the split.  All CTAs resident at once, and of clusters of eight no more than fit
 // beside one another when a CTA needs an SM to itself.  50 x 2560 x 1024 6.1 -> 3.9 us against the small-M kernel and its exchange by
 // cluster barriers, 50 x 1024 x 4096 6.6 -> 4.6, 16 x 1024 x 1024 4.3 -> 2.8; unsplit products of much weight stay there (50 x 8192 x
 // 1024: 4.6 against 4.85).
-static TokPlan pick_tok_nvfp4(int M, int N, int K, int want) {
+// In a chain (`chain`: the caller says the weights may be fetched early) more and smaller CTAs pay also where the launch alone is no
+// faster: every weight tile of a split waits in shared memory.  There: tiles of 64 and the largest split with a CTA per SM (or two of a
+// product that would stay whole), if its k-blocks all fit the ring.  Loops of 20 / 33 / 50 / 64 tokens on 768 / 500 / 768 / 900 keys,
+// all splits of the four products timed: 5.32 / 5.60 / 6.03 / 6.82 ms, with the cheapest launches 6.16 / 6.09 / 6.23 / 6.89.
+static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     TokPlan best = {0, 0, 0, 0, 1};
     double t = 1e30;
     const int kbt = K / 256, sms = device_sm_count();
     if ((N & 7) || M > 64) return best;
+    const int tiles64 = (N + 63) / 64;
+    for (int S = 8; chain && want <= 0 && S >= 1; S /= 2) {
+        if (kbt % S || kbt / S > 8 || tiles64 * S > sms || (S == 8 && tiles64 * 64 > sms * 7)) continue;
+        if (S == 1 && kbt % 2 == 0 &&          // two CTAs of half the k-blocks share an SM
+            TokCfg<64, true>::smem_bytes(kbt / 2, 2, (M + 1) / 2, true, TOK_ROW_PAD) <= 110 * 1024) S = 2;
+        return {64, S, kbt / S, kbt / S, 1};
+    }
     for (int bn = 64; bn <= 128; bn += 64) {
         const int tiles = (N + bn - 1) / bn;
         for (int S = 1; S <= 8; S *= 2) {
