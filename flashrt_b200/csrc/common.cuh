@@ -204,6 +204,59 @@ __device__ __forceinline__ float warp_row_total(const float (&part)[NS], int n) 
     return tot;
 }
 
+// The same total for a row whose lanes hold 16 neighbouring values per piece of 512 columns, NP pieces in this warp and WPR warps of
+// the row (piece i of warp `part` is i * WPR + part): part0 / part1 are the lane's partials of its first and second eight values.
+// A lane holds chunks 2 lane and 2 lane + 1 of a piece's 64, so the exchanges at distance 16, 8, 4, 2 of a chunk are 8, 4, 2, 1 of a
+// lane, and the last one is between the halves.  WPR > 1: `slices` = 2 * NP * WPR floats of shared memory for this row, and every
+// thread of the block has to come here.
+template <int NP, int WPR>
+__device__ __forceinline__ float piece_row_total(const float (&part0)[NP], const float (&part1)[NP], int n, int part,
+                                                 float* slices) {
+    constexpr int P = NP <= 1 ? 1 : NP <= 2 ? 2 : NP <= 4 ? 4 : 8;
+    static_assert(NP <= 8 && (WPR == 1 || WPR == 2 || WPR == 4), "pieces per warp, warps per row");
+    const int lane = threadIdx.x & 31;
+    float v[2 * P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+        v[i] = i < NP ? part0[i < NP ? i : 0] : 0.0f;
+        v[P + i] = i < NP ? part1[i < NP ? i : 0] : 0.0f;
+    }
+    int d = 8;
+#pragma unroll
+    for (int h = P; h >= 1; h >>= 1, d >>= 1) {
+        const bool up = (lane & d) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, d));
+        }
+    }
+#pragma unroll
+    for (; d >= 1; d >>= 1) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], d));
+    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 8));
+    // slice 2 (i WPR + part) is in lanes i * (8 / P) .., the one behind it 16 lanes further on
+    float tot = 0.0f;
+    if (WPR == 1) {
+        tot = __shfl_sync(0xffffffffu, v[0], 0);
+#pragma unroll
+        for (int w = 1; w < 2 * NP; ++w) {
+            const float y = __shfl_sync(0xffffffffu, v[0], (w >> 1) * (8 / P) + (w & 1) * 16);
+            if (w < n) tot = __fadd_rn(tot, y);
+        }
+    } else {
+        const int i = (lane & 7) / (8 / P);
+        if ((lane & 8) == 0 && (lane & 7) % (8 / P) == 0 && i < NP) slices[2 * (i * WPR + part) + (lane >> 4)] = v[0];
+        __syncthreads();
+        tot = slices[0];
+#pragma unroll
+        for (int w = 1; w < 2 * NP * WPR; ++w) {
+            const float y = slices[w];
+            if (w < n) tot = __fadd_rn(tot, y);
+        }
+    }
+    return tot;
+}
+
 // Element of every bf16 GEMM epilogue: alpha * acc, or alpha * acc + bias with ONE rounding.  Written out so that every
 // kernel that can serve a shape produces the same bits (the compiler is otherwise free to fuse or not, site by site).
 __device__ __forceinline__ float scale_bias(float acc, float alpha, float bias, bool has_bias) {
@@ -240,6 +293,15 @@ __device__ __forceinline__ void ld_stream_32(const void* p, bool wide, bool seco
         if (second) b = ld_stream_v4(static_cast<const uint8_t*>(p) + 16);
         r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
         r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
+    }
+}
+__device__ __forceinline__ void st_global_32(void* p, bool wide, bool second, const uint32_t* r) {
+    if (wide) {
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                     "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+    } else {
+        *reinterpret_cast<uint4*>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+        if (second) *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p) + 16) = make_uint4(r[4], r[5], r[6], r[7]);
     }
 }
 __device__ __forceinline__ float4 ld_global_f4(const float* p) {

@@ -210,9 +210,7 @@ __global__ void __launch_bounds__(128)
 norm_block_kernel(NormArgs a) {
     constexpr bool OUT_FP8 = OUT == OUT_E4M3;
     constexpr bool OUT_FP4 = OUT == OUT_NVFP4_A || OUT == OUT_NVFP4_B;
-    constexpr int P = NP <= 1 ? 1 : NP <= 2 ? 2 : NP <= 4 ? 4 : 8;
     constexpr uint32_t HI = 0xffff0000u;
-    static_assert(NP <= 8 && (WPR == 1 || WPR == 2 || WPR == 4), "slice pairs per warp, warps per row");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = blockIdx.x * (4 / WPR) + warp / WPR, part = warp % WPR;
     pdl_launch_dependents();
@@ -233,61 +231,22 @@ norm_block_kernel(NormArgs a) {
         for (int j = 0; j < 8; ++j) x[i][j] = 0u;
         if (i * WPR * 512 < left) ld_stream_32(a.residual + rbase + i * WPR * 512, wide, i * WPR * 512 + 8 < left, x[i]);
     }
-    // Sums of squares: the chain over 8 values of both halves at once; then the butterfly over the 32 chunks of a slice.  A
-    // lane holds chunks 2 lane and 2 lane + 1 of a pair's 64, so the exchanges at distance 16, 8, 4, 2 of a chunk are 8, 4, 2, 1 of a
-    // lane, and the last one is between the halves: the tree of the one-CTA-per-row kernel.  Every exchange hands half of the
-    // values held to the partner (see warp_row_total).
-    float v[2 * P];
+    // sums of squares, the chains over the 8 values of both halves at once
+    float part0[NP], part1[NP];
 #pragma unroll
-    for (int i = 0; i < P; ++i) {
+    for (int i = 0; i < NP; ++i) {
         uint64_t s = f32x2(0.0f, 0.0f);
-        if (i < NP) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint64_t e = f32x2(__uint_as_float(x[i][j] << 16), __uint_as_float(x[i][4 + j] << 16));
-                const uint64_t o = f32x2(__uint_as_float(x[i][j] & HI), __uint_as_float(x[i][4 + j] & HI));
-                s = fma_f32x2(o, o, fma_f32x2(e, e, s));
-            }
+        for (int j = 0; j < 4; ++j) {
+            const uint64_t e = f32x2(__uint_as_float(x[i][j] << 16), __uint_as_float(x[i][4 + j] << 16));
+            const uint64_t o = f32x2(__uint_as_float(x[i][j] & HI), __uint_as_float(x[i][4 + j] & HI));
+            s = fma_f32x2(o, o, fma_f32x2(e, e, s));
         }
-        f32x2_parts(s, v[i], v[P + i]);
+        f32x2_parts(s, part0[i], part1[i]);
     }
-    int d = 8;
-#pragma unroll
-    for (int h = P; h >= 1; h >>= 1, d >>= 1) {
-        const bool up = (lane & d) != 0;
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            const float keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
-            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, d));
-        }
-    }
-#pragma unroll
-    for (; d >= 1; d >>= 1) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], d));
-    v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], 8));
-    // slice 2 (i WPR + part) is in lanes i * (8 / P) .., the one behind it 16 lanes further on
-    const int n = (a.dim + 255) >> 8;
-    float tot = 0.0f;
-    if (WPR == 1) {
-        tot = __shfl_sync(0xffffffffu, v[0], 0);
-#pragma unroll
-        for (int w = 1; w < 2 * NP; ++w) {
-            const float y = __shfl_sync(0xffffffffu, v[0], (w >> 1) * (8 / P) + (w & 1) * 16);
-            if (w < n) tot = __fadd_rn(tot, y);
-        }
-    } else {
-        __shared__ float slices[4 / WPR][2 * NP * WPR];
-        float* sl = slices[warp / WPR];
-        const int i = (lane & 7) / (8 / P);
-        if ((lane & 8) == 0 && (lane & 7) % (8 / P) == 0 && i < NP) sl[2 * (i * WPR + part) + (lane >> 4)] = v[0];
-        __syncthreads();
-        if (!live) return;
-        tot = sl[0];
-#pragma unroll
-        for (int w = 1; w < 2 * NP * WPR; ++w) {
-            const float y = sl[w];
-            if (w < n) tot = __fadd_rn(tot, y);
-        }
-    }
+    __shared__ float slices[WPR == 1 ? 1 : 4 / WPR][WPR == 1 ? 1 : 2 * NP * WPR];
+    const float tot = piece_row_total<NP, WPR>(part0, part1, (a.dim + 255) >> 8, part, slices[WPR == 1 ? 0 : warp / WPR]);
+    if (!live) return;
     const float var = __fadd_rn(__fdiv_rn(tot, (float)a.dim), a.eps);
     const float rms = __fdiv_rn(1.0f, __fsqrt_rn(var));
     const uint64_t rms2 = f32x2(rms, rms), zero2 = f32x2(0.0f, 0.0f);

@@ -133,3 +133,27 @@ def test_norm_blocks_of_unaligned_rows(rows, dim, kind):
         got.append((d_o.get()[off:off + rows * dim // (1 if kind == "fp8" else 2)], d_sf.get()))
     for g in got[:2]:
         assert np.array_equal(g[0], got[2][0]) and np.array_equal(g[1], got[2][1])
+
+
+@pytest.mark.parametrize("rows,dim", [(1, 8), (5, 1000), (7, 1032), (3, 3064), (9, 4104), (6, 8192)])
+@pytest.mark.parametrize("off", [0, 8])
+def test_residual_layer_norm_pieces(rows, dim, off):
+    """The many-row kernel at its own edges (the residual form takes it at every size): last pieces half there, one to four warps
+    per row, rows 16 bytes off the widest access; against residual update and LayerNorm apart."""
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import f32, rand_bf16, zeros
+    rng = np.random.default_rng(rows * dim + off)
+    n = rows * dim
+    pad = lambda a: np.concatenate([np.zeros(off, np.uint16), a.reshape(-1)])  # noqa: E731
+    x, y = pad(rand_bf16(rng, (rows, dim))), pad(rand_bf16(rng, (rows, dim)))
+    g, sc, sh, w, b = (_dev(rand_bf16(rng, (dim,), 0.5)) for _ in range(5))
+    s8 = f32(0.02)
+    for kw, args in ((dict(scale=sc.ptr, shift=sh.ptr), (None, None, sc.ptr, sh.ptr)),
+                     (dict(weight=w.ptr, bias=b.ptr), (w.ptr, b.ptr, None, None))):
+        d_x, d_y, d_r, d_o = _dev(x), _dev(y), zeros((n + off,), np.uint16), zeros((n + off,), np.uint8)
+        fvk.residual_layer_norm_fp8(d_x.ptr + 2 * off, d_y.ptr + 2 * off, g.ptr, d_r.ptr + 2 * off, d_o.ptr + off, s8.ptr, rows,
+                                    dim, 1e-6, 0, **kw)
+        d_u, d_q = _dev(x), zeros((n + off,), np.uint8)
+        _lib.call("frt_b200_gate_mul_residual", d_u.ptr + 2 * off, d_y.ptr + 2 * off, g.ptr, 0, rows, dim, 0, 0)
+        _lib.call("frt_b200_layer_norm", d_u.ptr + 2 * off, *args, 0, d_q.ptr + off, None, s8.ptr, rows, dim, 1e-6, 0, 0)
+        assert np.array_equal(d_r.get()[off:], d_u.get()[off:]) and np.array_equal(d_o.get(), d_q.get())
