@@ -932,12 +932,13 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
             // kv_splits is a bound: the cheapest form that fits, by the times of the captured action-expert loop (10-64 queries
             // x 8 heads, 100-1088 keys, batch 1-4) and of the prefix encoder's launches (96-1024 x 8 heads on themselves), in
             // units of 0.05 us over the cluster exchange in four parts: 0.8 us per chunk of a split's chain, 0.9 and 1.9 once
-            // when a CTA moves out 128 columns of O; one CTA per tile 0.93 per chunk, per (tile, split) through the scratch 1.1 and
-            // 4.3 once; 2.3 for the scratch in four parts.  (2 x 50 on 818 keys 8.8 us as 4 splits of 4 parts, 10.9 as 2; 768 on
-            // 768: one CTA per tile 15.8, two splits through the scratch 16.1.)
+            // when a CTA moves out 128 columns of O; one CTA per tile 0.95 per chunk, per (tile, split) through the scratch 1.1 and
+            // 4.3 once; 2.3 for the scratch in four parts.  One CTA per tile is charged 0.9 more than its launch takes: its CTAs
+            // hold all of tensor memory, and the kernel behind starts late (in the encoder at 300 rows two splits of two parts save
+            // 5 us a layer, at 768 two splits through the scratch 2).  (2 x 50 on 818 keys 8.8 us as 4 splits of 4 parts, 10.9 as 2.)
             const long long ctas1 = (long long)tiles * groups;
             auto chain = [&](int c) { return (p.chunks_total + c - 1) / c; };
-            int best = 19 * p.chunks_total - 6, bc = 1, bp = 0;                 // bp: 0 = not a cluster
+            int best = 19 * p.chunks_total + 12, bc = 1, bp = 0;                 // bp: 0 = not a cluster
             for (int c = 8; c >= 2; c >>= 1) {
                 if (c > bound || c / 2 >= p.chunks_total) continue;
                 for (int parts = 4; parts >= 2; parts -= 2) {

@@ -130,6 +130,46 @@ __device__ __forceinline__ float det_gelu_tanh(float g) {
     return __fdiv_rn(g, __fadd_rn(1.0f, e));
 }
 
+// The same of two values, bit for bit, with half the instructions: products, fmas and additions run in pairs, round-to-integer is an
+// addition of 1.5 * 2^23 (whose sum's low bits are also the exponent of 2^n), and the quotient is Markstein's (IBM J. Res. Dev. 34,
+// 1990): reciprocal approximation, one Newton step, quotient, exact remainder, one correction -- correctly rounded as long as
+// nothing leaves the normal range, so gates outside 2^-60 <= |g| < 9 (zeros, tiny ones, infinities, NaN, large ones) take the scalar
+// form.  Inputs are bf16 values: all 65536 are checked against it.
+__device__ __forceinline__ uint64_t det_gelu_tanh2(uint64_t g) {
+    auto both = [](float v) { return f32x2(v, v); };
+    float g0, g1, x0, x1, t0, t1, d0, d1;
+    f32x2_parts(g, g0, g1);
+    if (!(fabsf(g0) >= 8.673617379884035e-19f && fabsf(g0) < 9.0f && fabsf(g1) >= 8.673617379884035e-19f && fabsf(g1) < 9.0f))
+        return f32x2(det_gelu_tanh(g0), det_gelu_tanh(g1));
+    const uint64_t one = both(1.0f);
+    const uint64_t inner = fma_f32x2(mul_f32x2(both(0.044715f), g), g, one);
+    f32x2_parts(mul_f32x2(mul_f32x2(both(-1.5957691216057308f), g), inner), x0, x1);
+    const uint64_t x = f32x2(fminf(fmaxf(x0, -87.0f), 88.0f), fminf(fmaxf(x1, -87.0f), 88.0f));
+    const uint64_t t = add_f32x2(mul_f32x2(x, both(1.4426950408889634f)), both(12582912.0f));
+    const uint64_t n = add_f32x2(t, both(-12582912.0f));
+    uint64_t r = fma_f32x2(n, both(-0.693145751953125f), x);
+    r = fma_f32x2(n, both(-1.4286068203094173e-06f), r);
+    uint64_t p = both(1.9841269841269841e-04f);
+    p = fma_f32x2(p, r, both(1.3888888888888889e-03f));
+    p = fma_f32x2(p, r, both(8.3333333333333332e-03f));
+    p = fma_f32x2(p, r, both(4.1666666666666664e-02f));
+    p = fma_f32x2(p, r, both(1.6666666666666666e-01f));
+    p = fma_f32x2(p, r, both(0.5f));
+    p = fma_f32x2(p, r, one);
+    p = fma_f32x2(p, r, one);
+    f32x2_parts(t, t0, t1);
+    const uint64_t s = f32x2(__uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u),
+                             __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u));
+    const uint64_t d = add_f32x2(one, mul_f32x2(p, s)), nd = mul_f32x2(d, both(-1.0f));
+    f32x2_parts(d, d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(d1));
+    uint64_t y = f32x2(d0, d1);
+    y = fma_f32x2(y, fma_f32x2(nd, y, one), y);
+    const uint64_t q = mul_f32x2(g, y);
+    return fma_f32x2(fma_f32x2(nd, q, g), y, q);
+}
+
 // SiLU: g * sigmoid(g) = g / (1 + exp(-g))  (silu_mul_split_fp8_kernel, csrc/kernels/activation.cu:291-306)
 __device__ __forceinline__ float det_silu(float g) {
     return __fdiv_rn(g, __fadd_rn(1.0f, det_expf(-g)));
@@ -146,8 +186,11 @@ __device__ __forceinline__ float fast_gelu_tanh(float g) {
 
 // gate activation of the gated FFN epilogues: 0 = GELU(tanh) (GeGLU), 1 = SiLU (SwiGLU)
 template <int ACT>
-__device__ __forceinline__ float det_gate_act(float g) {
-    return ACT == 1 ? det_silu(g) : det_gelu_tanh(g);
+__device__ __forceinline__ uint64_t det_gate_act2(uint64_t g) {
+    if (ACT == 0) return det_gelu_tanh2(g);
+    float g0, g1;
+    f32x2_parts(g, g0, g1);
+    return f32x2(det_silu(g0), det_silu(g1));
 }
 
 // ---------------------------------------------------------------- reductions

@@ -71,11 +71,11 @@ geglu_fp8_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ out, int row
         float o[8];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float g0, g1, u0, u1;
-            unpack_bf16x2(gw[k], g0, g1);
-            unpack_bf16x2(uw[k], u0, u1);
-            o[2 * k] = clamp448(__fmul_rn(__fmul_rn(det_gate_act<ACT>(g0), u0), inv_scale));
-            o[2 * k + 1] = clamp448(__fmul_rn(__fmul_rn(det_gate_act<ACT>(g1), u1), inv_scale));
+            const uint64_t v = mul_f32x2(mul_f32x2(det_gate_act2<ACT>(unpack_bf16x2(gw[k])), unpack_bf16x2(uw[k])),
+                                         f32x2(inv_scale, inv_scale));
+            f32x2_parts(v, o[2 * k], o[2 * k + 1]);
+            o[2 * k] = clamp448(o[2 * k]);
+            o[2 * k + 1] = clamp448(o[2 * k + 1]);
         }
         uint2 ov;
         ov.x = f32x4_to_e4m3x4(o[0], o[1], o[2], o[3]);
@@ -105,10 +105,9 @@ geglu_bf16_kernel(const __nv_bfloat16* merged, __nv_bfloat16* __restrict__ out, 
         uint32_t* ow = &ov.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float g0, g1, u0, u1;
-            unpack_bf16x2(gw[k], g0, g1);
-            unpack_bf16x2(uw[k], u0, u1);
-            ow[k] = pack_bf16x2(__fmul_rn(det_gate_act<ACT>(g0), u0), __fmul_rn(det_gate_act<ACT>(g1), u1));
+            float v0, v1;
+            f32x2_parts(mul_f32x2(det_gate_act2<ACT>(unpack_bf16x2(gw[k])), unpack_bf16x2(uw[k])), v0, v1);
+            ow[k] = pack_bf16x2(v0, v1);
         }
         st_global_v4(out + row * H + col, ov);
     }

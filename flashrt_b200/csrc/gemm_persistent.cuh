@@ -241,7 +241,8 @@ __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_
     tc::tmem_ld32(t_gate, g);
     tc::tmem_ld32(t_up, u);
     tc::tmem_ld_wait();
-    // rows beyond M hold zeros, and a zero takes the slow path of the activation's division (541 rows: 48 us a launch with it)
+    const uint64_t al2 = f32x2(alpha, alpha), io2 = f32x2(inv_os, inv_os);
+    // rows beyond M hold zeros, and a zero takes the activation's slow path (541 rows: 48 us a launch with it)
     if (m >= p.M) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) g[j] = 0x3f800000u;
@@ -250,11 +251,15 @@ __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_
     for (int j = 0; j < 32; j += 4) {
         float o[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float gt = bf16_round(__uint_as_float(g[j + e]) * alpha), up = bf16_round(__uint_as_float(u[j + e]) * alpha);
-            o[e] = clamp448(__fmul_rn(__fmul_rn(det_gelu_tanh(gt), up), inv_os));
+        for (int e = 0; e < 4; e += 2) {
+            auto rounded = [&](const uint32_t* v) {          // bf16(alpha * v) of two columns
+                float v0, v1;
+                f32x2_parts(mul_f32x2(f32x2(__uint_as_float(v[0]), __uint_as_float(v[1])), al2), v0, v1);
+                return unpack_bf16x2(pack_bf16x2(v0, v1));
+            };
+            f32x2_parts(mul_f32x2(mul_f32x2(det_gelu_tanh2(rounded(g + j + e)), rounded(u + j + e)), io2), o[e], o[e + 1]);
         }
-        w[j / 4] = f32x4_to_e4m3x4(o[0], o[1], o[2], o[3]);
+        w[j / 4] = f32x4_to_e4m3x4(clamp448(o[0]), clamp448(o[1]), clamp448(o[2]), clamp448(o[3]));
     }
     if (m < p.M) {
         uint8_t* dst = p.out8 + (size_t)m * p.half + h0;

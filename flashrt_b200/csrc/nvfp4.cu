@@ -87,11 +87,7 @@ geglu_nvfp4_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ packed, ui
         float amax = 0.0f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            float ga, gb, ua, ub;
-            unpack_bf16x2(gw[i], ga, gb);
-            unpack_bf16x2(uw[i], ua, ub);
-            v[2 * i] = __fmul_rn(det_gelu_tanh(ga), ua);
-            v[2 * i + 1] = __fmul_rn(det_gelu_tanh(gb), ub);
+            f32x2_parts(mul_f32x2(det_gelu_tanh2(unpack_bf16x2(gw[i])), unpack_bf16x2(uw[i])), v[2 * i], v[2 * i + 1]);
             amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
         }
         float s;
@@ -125,16 +121,11 @@ geglu_nvfp4_lanes_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ pack
         gv = *reinterpret_cast<const uint2*>(g);
         uv = *reinterpret_cast<const uint2*>(g + H);
     }
-    float g[4], u[4], v[4], amax = 0.0f;
-    unpack_bf16x2(gv.x, g[0], g[1]);
-    unpack_bf16x2(gv.y, g[2], g[3]);
-    unpack_bf16x2(uv.x, u[0], u[1]);
-    unpack_bf16x2(uv.y, u[2], u[3]);
+    float v[4], amax = 0.0f;
+    f32x2_parts(mul_f32x2(det_gelu_tanh2(unpack_bf16x2(gv.x)), unpack_bf16x2(uv.x)), v[0], v[1]);
+    f32x2_parts(mul_f32x2(det_gelu_tanh2(unpack_bf16x2(gv.y)), unpack_bf16x2(uv.y)), v[2], v[3]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        v[i] = __fmul_rn(det_gelu_tanh(g[i]), u[i]);
-        amax = fmaxf(amax, fabsf(v[i]));
-    }
+    for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fabsf(v[i]));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     float s;

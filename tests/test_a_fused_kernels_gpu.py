@@ -242,3 +242,19 @@ def test_qkv_split_rope_appends_to_cache(fvk, seq, pos, use_devpos):
     assert np.array_equal(d_Q.get(), Q_ref)
     assert np.array_equal(d_K.get(), Kr)       # rows outside [pos, pos+seq) untouched
     assert np.array_equal(d_V.get(), Vr)
+
+
+@pytest.mark.parametrize("neighbour", [0x3F80, 0x0000, 0x4120])
+def test_geglu_every_gate_value(neighbour):
+    """All 65536 bf16 gates through the paired activation (normal, zero and large neighbours) and the scalar one of the oracle."""
+    from flashrt_b200 import flash_rt_kernels as fvk
+    from gpu_util import Dev, zeros
+    gates = np.arange(65536, dtype=np.uint32).astype(np.uint16)
+    finite = (gates & 0x7F80) != 0x7F80
+    gate = np.stack([gates, np.full_like(gates, neighbour)], axis=1).reshape(64, -1)
+    up = np.random.default_rng(3).integers(0x3F00, 0x4000, gate.shape).astype(np.uint16)
+    merged = np.concatenate([gate, up], axis=1)
+    d_m, d_o = Dev(merged), zeros(gate.shape, np.uint16)
+    fvk.gate_geglu_merged(d_m.ptr, d_o.ptr, gate.shape[0], gate.shape[1], 0)
+    got, ref = d_o.get().reshape(-1, 2), O.geglu_bf16(merged).reshape(-1, 2)
+    assert np.array_equal(got[finite], ref[finite]) and np.array_equal(got[:, 1], ref[:, 1])
