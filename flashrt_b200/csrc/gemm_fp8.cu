@@ -1028,6 +1028,11 @@ static double large_cost(int kind, int M, int N, int K) {
     const long long tiles = (long long)((M + c[kind].tm - 1) / c[kind].tm) * ((N + c[kind].tn - 1) / c[kind].tn);
     return c[kind].fixed + (double)((tiles + workers - 1) / workers) * ((K + 127) / 128) * c[kind].per_kb;
 }
+// swapped kernel at 129 .. 256 rows: whole waves of 128 weight rows (256 x 32768 x 2048 is two: 34 us, on CTA pairs 16)
+static double swapped_us(int N, int kb) {
+    const int tiles = (N + 127) / 128, sms = device_sm_count();
+    return (13.0 + 0.115 * kb) * ((tiles + sms - 1) / sms);
+}
 static int pick_large(int M, int N, int K, bool no_pair, double* cost = nullptr) {
     int best = LARGE_128;
     double t = large_cost(LARGE_128, M, N, K);
@@ -1105,7 +1110,7 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
         double t_large = 0.0;
         const int kind = pick_large(M, N, K, M <= 128 || (flags & 32) != 0, &t_large);
         const double mb = (double)N * K / 1048576.0;
-        const double t_small = M > 128 ? 13.0 + 0.115 * p.kb_total : M > 64 ? 5.2 + 0.45 * mb : 5.0 + 0.3 * mb;
+        const double t_small = M > 128 ? swapped_us(N, p.kb_total) : M > 64 ? 5.2 + 0.45 * mb : 5.0 + 0.3 * mb;
         if (t_large + 0.3 < t_small) return launch_large<EPI_P_BF16>(kind, A, W, p, K, s);
     }
     // the swapped kernel's splits keep up with a long K better than the token-major kernel's exchange
@@ -1274,7 +1279,16 @@ int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int
     p.half = half;
     p.early = flags & 1;
     // SiLU gate (bit 6) and the hardware-tanh GELU (bit 7): built in the token-major kernel only
-    if (M > 256) return launch_gemm_pair<256, EPI_P_GEGLU_FP8>(A, W, p, K, (cudaStream_t)stream);
+    // 65 .. 256 rows: CTA pairs where many weights make whole waves of them cheaper than the small-M kernels (us; 256 x 16384 x 2048
+    // 42 -> 17 with the separate GeGLU launch, 100 rows 22.7 -> 17)
+    bool pairs = M > 256;
+    if (M > 64 && M <= 256 && splits <= 0 && !(flags & (16 | 64 | 128 | 0x300)) && half % 128 == 0 &&
+        !(reinterpret_cast<uintptr_t>(out8) & 15)) {
+        const int workers = device_sm_count() / 2, waves = (half / 128 + workers - 1) / workers;
+        const double mb = 2.0 * half * K / 1048576.0;
+        pairs = 7.0 + waves * (1.0 + 0.34 * p.kb_total) < (M > 128 ? swapped_us(p.N, p.kb_total) : 5.2 + 0.45 * mb);
+    }
+    if (pairs) return launch_gemm_pair<256, EPI_P_GEGLU_FP8>(A, W, p, K, (cudaStream_t)stream);
     const bool silu = (flags & 64) != 0, fast = (flags & 128) != 0;
     if (silu && fast) return FRT_ERR_INVALID;
     if ((silu || fast) && !(tok_eligible(M, p.N, K, flags) && M <= 128)) return FRT_ERR_UNSUPPORTED;

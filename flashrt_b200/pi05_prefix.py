@@ -179,12 +179,12 @@ class Pi05PrefixEncoderB200:
                              out_fp8=p["attn8"], out_scale=self._sp(i, "o"))
             self._gemm(p["attn8"], w["w_o"], w["ws_o_t"], p["xn"], seq, ENC_D, QD, self._sp(i, "o"), st, pdl)
             self._norm(seq, p["xn"], i, "gu", st, calibrate)
-            if calibrate or seq <= 256:
+            if calibrate or seq <= 64:
                 self._gemm(p["act8"], w["w_gu"], w["ws_gu_t"], p["merged"], seq, 2 * ENC_H, ENC_D, self._sp(i, "gu"), st, pdl)
             if calibrate:
                 fvk.gate_geglu_merged(p["merged"], p["hidden"], seq, ENC_H, st)
                 self._dyn_quant(self.hidden[:seq], self.hid8[:seq], i, "d", st)
-            elif seq <= 256:
+            elif seq <= 64:
                 fvk.gate_geglu_merged_fp8(p["merged"], p["hid8"], seq, ENC_H, self._sp(i, "d"), st, pdl=True)
             else:               # one launch: the activation under the product's MMAs
                 self.gemm.fp8_nt_dev_geglu_fp8(p["act8"], w["w_gu"], p["hid8"], seq, ENC_H, ENC_D, self._sp(i, "gu"),
