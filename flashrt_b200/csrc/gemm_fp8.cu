@@ -1028,10 +1028,11 @@ static double large_cost(int kind, int M, int N, int K) {
     const long long tiles = (long long)((M + c[kind].tm - 1) / c[kind].tm) * ((N + c[kind].tn - 1) / c[kind].tn);
     return c[kind].fixed + (double)((tiles + workers - 1) / workers) * ((K + 127) / 128) * c[kind].per_kb;
 }
-// swapped kernel at 129 .. 256 rows: whole waves of 128 weight rows (256 x 32768 x 2048 is two: 34 us, on CTA pairs 16)
+// swapped kernel at 129 .. 256 rows: set-up and exchange of its splits, half a microsecond per k-block of a split, whole waves of 128
+// weight rows (256 x 32768 x 2048 is two: 34 us, on CTA pairs 16)
 static double swapped_us(int N, int kb) {
-    const int tiles = (N + 127) / 128, sms = device_sm_count();
-    return (13.0 + 0.115 * kb) * ((tiles + sms - 1) / sms);
+    const int tiles = (N + 127) / 128, sms = device_sm_count(), sp = pick_splits(tiles, kb, 0);
+    return ((sp > 1 ? 13.0 : 6.0) + 0.5 * ((kb + sp - 1) / sp)) * ((tiles * sp + sms - 1) / sms);
 }
 static int pick_large(int M, int N, int K, bool no_pair, double* cost = nullptr) {
     int best = LARGE_128;
@@ -1101,16 +1102,17 @@ int frt_b200_gemm_fp8_nt(const void* A, const void* W, void* D, int M, int N, in
     bool pdl = flags & 1;
     p.early = pdl ? 1 : 0;
     // M <= 256 without a hint: the kernels below it stream the weights through clusters that split K, which wins while the
-    // product is small or K is long; from about 8 MB of weights (M <= 128), or for most of 129 .. 256, the persistent kernels
-    // of the large products do.  Microseconds again: token-major 5 + 0.3 per MB of weights (5.2 + 0.45 above 64 rows),
-    // swapped 13 + 0.115 per k-block (e.g. 256 x 4096 x 1024: swapped 14.3, persistent 6.4; 50 x 14336 x 3072: token-major
-    // 15.9, persistent 12.7).
+    // product is small or K is long; from about 8 MB of weights (M <= 128), or for most of 129 .. 256, the kernels of the large
+    // products do, CTA pairs among them.  Microseconds again: token-major 5 + 0.28 per MB of weights (5.2 + 0.33 above 64 rows),
+    // swapped as swapped_us.  Over 175 products of 16 .. 256 rows (N 1024 .. 14336, K 1024 .. 8192) the choice is within 2 % of the
+    // best kernel on average; without pairs up to 128 rows and with one cost per k-block of the swapped kernel 256 x 14336 x 8192
+    // took 40.6 us instead of 29.7, 128 x 8192 x 8192 22.1 instead of 18.6, 90 x 8192 x 5120 15.3 instead of 13.2.
     const bool hinted = splits > 0 || (flags & (16 | 0x300));
     if (M <= 256 && M > 16 && !hinted && !(flags & 2) && N >= 128) {
         double t_large = 0.0;
-        const int kind = pick_large(M, N, K, M <= 128 || (flags & 32) != 0, &t_large);
+        const int kind = pick_large(M, N, K, (flags & 32) != 0, &t_large);
         const double mb = (double)N * K / 1048576.0;
-        const double t_small = M > 128 ? swapped_us(N, p.kb_total) : M > 64 ? 5.2 + 0.45 * mb : 5.0 + 0.3 * mb;
+        const double t_small = M > 128 ? swapped_us(N, p.kb_total) : M > 64 ? 5.2 + 0.33 * mb : 5.0 + 0.28 * mb;
         if (t_large + 0.3 < t_small) return launch_large<EPI_P_BF16>(kind, A, W, p, K, s);
     }
     // the swapped kernel's splits keep up with a long K better than the token-major kernel's exchange
