@@ -116,6 +116,7 @@ struct AttnParams {
 #ifdef FRT_PHASE_STAMPS
     int trace_slot;
 #endif
+    int pair_units, pair_full; // two-tile kernel: units of two row tiles per (batch, kv head); first unit on two CTAs
 };
 
 template <int D, int BKV>

@@ -66,10 +66,13 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
-__global__ void __launch_bounds__(320, 1)
-attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, AttnParams p) {
+// SINGLE: one row tile only (warps 4-7 idle).  A compile-time form: with the choice at run time in the MMA warp's loop the two-tile
+// form lost a quarter of its rate (2 x 24 heads x 20280^2 7.5 -> 9.9 ms).
+template <bool SINGLE>
+__device__ __forceinline__ void attn_pair_body(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                               const AttnParams& p, const int by, const int tile) {
     using Cfg = PairCfg;
+    constexpr int T = SINGLE ? 1 : 2;
     constexpr int D = Cfg::D, BKV = Cfg::BKV;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -91,10 +94,10 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint64_t deadline = tc::global_timer_ns() + FRT_KERNEL_DEADLINE_NS;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int hk = blockIdx.y % p.Hkv;
-    const int b = blockIdx.y / p.Hkv;
+    const int hk = by % p.Hkv;
+    const int b = by / p.Hkv;
     const int tok_per_tile = 128 / p.G;
-    const int tok0 = blockIdx.x * 2 * tok_per_tile;
+    const int tok0 = tile * tok_per_tile;
     const int nchunks = p.chunks_total;
 
     if (threadIdx.x == 0) {
@@ -129,8 +132,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // ---------------- TMA producer (whole warp)
         pdl_wait();
         if (tc::elect_one()) {
-            tc::mbar_arrive_expect_tx(q_full, 2 * Cfg::Q_BYTES);
-            for (int t = 0; t < 2; ++t)
+            tc::mbar_arrive_expect_tx(q_full, T * Cfg::Q_BYTES);
+            for (int t = 0; t < T; ++t)
                 for (int db = 0; db < 2; ++db)
                     tc::tma_load_5d(sQ + t * Cfg::Q_BYTES + db * (128 * 128), &tmQ, q_full, db * 64, 0, hk,
                                     tok0 + t * tok_per_tile, b);
@@ -192,7 +195,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             pv(t, j, 0, false);
             if (!attn_warp_wait(&p_ready[t], ph, AERR_MMA, deadline, abort_flag)) return false;
             tc::tc_fence_after_sync();
-            pv(t, j, 1, t == 1);
+            pv(t, j, 1, t == T - 1);
             return true;
         };
         bool ok = attn_warp_wait(q_full, 0u, AERR_MMA, deadline, abort_flag);
@@ -201,7 +204,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (ok) {
                 tc::tc_fence_after_sync();
                 qk(0, 0);
-                qk(1, 0);
+                if constexpr (!SINGLE) qk(1, 0);
             }
         }
         for (int j = 0; ok && j < nchunks; ++j) {
@@ -213,12 +216,14 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 tc::tc_fence_after_sync();
                 qk(0, j + 1);
             }
-            ok = p_step(1, j);
-            if (!ok) break;
-            if (j + 1 < nchunks) qk(1, j + 1);
+            if constexpr (!SINGLE) {
+                ok = p_step(1, j);
+                if (!ok) break;
+                if (j + 1 < nchunks) qk(1, j + 1);
+            }
         }
         if (ok && tc::elect_one()) tc::mma_commit(o_done);
-    } else if (warp < 8) {
+    } else if (warp < 4 * T) {
         // ---------------- softmax: tile t, thread = row
         pdl_wait();
         const int t = warp >> 2;
@@ -373,6 +378,23 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (warp == 9) tc::tmem_dealloc(tmem, Cfg::TMEM_COLS);
 }
 
+__global__ void __launch_bounds__(320, 1)
+attn_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
+    attn_pair_body<false>(tmQ, tmK, tmV, p, (int)blockIdx.y, (int)blockIdx.x * 2);
+}
+// The same with a last wave of single tiles: units of two row tiles in (batch, kv head) order; from pair_full on, a unit is two CTAs.
+// (A kernel of its own: beside the second body the two-tile form is 1.7 % slower.)
+__global__ void __launch_bounds__(320, 1)
+attn_pair_rest_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                      const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
+    const int s = (int)blockIdx.x - p.pair_full;
+    const int unit = s < 0 ? (int)blockIdx.x : p.pair_full + (s >> 1);
+    const int by = unit / p.pair_units, tile = (unit - by * p.pair_units) * 2;
+    if (s < 0) attn_pair_body<false>(tmQ, tmK, tmV, p, by, tile);
+    else attn_pair_body<true>(tmQ, tmK, tmV, p, by, tile + (s & 1));
+}
+
 static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnParams p, const long long* qs,
                             const long long* ks, const long long* vs, cudaStream_t stream) {
     using Cfg = PairCfg;
@@ -381,6 +403,8 @@ static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnPar
     if (attr_once.need(attr_dev)) {
         cudaError_t e = cudaFuncSetAttribute(attn_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              Cfg::SMEM_BYTES);
+        if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        e = cudaFuncSetAttribute(attn_pair_rest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         attr_once.set(attr_dev);
     }
@@ -405,8 +429,15 @@ static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnPar
     p.chunks_total = (p.Skv + Cfg::BKV - 1) / Cfg::BKV;
     p.o_accum = nullptr;
     const int tiles = (p.Sq * p.G + 127) / 128;
+    // The units of a last wave that fills at most half of the SMs go as two CTAs of one tile, which take about two thirds of the time
+    // of one with two: 24 heads x 1972^2 66.8 -> 63.2 us, x 500^2 14.6 -> 11.5, 600 queries on 512 keys 15.9 -> 11.7.  From eight waves
+    // on it gives less than the second body costs.
+    p.pair_units = (tiles + 1) / 2;
+    const int units = p.pair_units * p.Hkv * p.B, sms = device_sm_count(), rest = units % sms;
+    const bool split = rest > 0 && 2 * rest <= sms && units < 8 * sms;
+    p.pair_full = units - rest;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((tiles + 1) / 2, p.Hkv * p.B, 1);
+    cfg.gridDim = split ? dim3(units + rest) : dim3(p.pair_units, p.Hkv * p.B);
     cfg.blockDim = dim3(320);
     cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
     cfg.stream = stream;
@@ -415,6 +446,6 @@ static int launch_attn_pair(const void* Q, const void* K, const void* V, AttnPar
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;                                  // nothing global is read before the wait
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_pair_kernel, tmQ, tmK, tmV, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, split ? attn_pair_rest_kernel : attn_pair_kernel, tmQ, tmK, tmV, p);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
