@@ -25,6 +25,10 @@
 // memory and each reduces 1/S of the tile's columns in fixed order (split 0, 1, ...).
 // There is no global-memory workspace and the result is deterministic.
 //
+// The other kernels of these entry points are included below: gemm_tok.cuh (tokens on the lanes, small M), gemm_persistent.cuh and
+// gemm_pair.cuh (large M).  NVFP4 (tcgen05.mma kind::mxf4nvf4) runs on the kernel of this file where neither gemm_tok.cuh (up to
+// 64 rows) nor gemm_pair.cuh takes the product.
+//
 // Each TMA copy lands in the issuing CTA's own shared memory.
 #include "common.cuh"
 #include "tc05.cuh"

@@ -1,4 +1,4 @@
-// Small-M FP8 GEMM with the TOKENS on the 128 TMEM lanes and the WEIGHTS on the accumulator columns, sm_100a.
+// Small-M FP8 / NVFP4 GEMM with the TOKENS on the 128 TMEM lanes and the WEIGHTS on the accumulator columns, sm_100a.
 //
 // Included by gemm_fp8.cu inside namespace frt (tensor-map cache, status word, arithmetic helpers).
 //
@@ -95,11 +95,18 @@ struct TokParams {
     const __nv_bfloat16* gate;
     float* stats_out;
     // TOK_PRO_NORM: x (M, K) bf16, stats_in [n_stat][stat_stride], style = [scale (K) | shift (K)] one row
-    const __nv_bfloat16* x;
+    // NVFP4 (never with TOK_PRO_NORM): block scales of both operands in atoms of 128 rows x 4 blocks, K / 64 atoms along K
+    union {
+        const __nv_bfloat16* x;
+        const uint8_t* sf_a;
+    };
     const float* stats_in;
     int n_stat;
     int K;
-    const __nv_bfloat16* style;
+    union {
+        const __nv_bfloat16* style;
+        const uint8_t* sf_w;
+    };
     float eps;
     int w_kn;                  // weights stored (K, N) row-major (the MN-major B operand) instead of (N, K)
     int early;                 // weights and style may be read before the kernel in front has finished
@@ -113,10 +120,6 @@ struct TokParams {
     uint8_t* q8_out;
     const __nv_bfloat16* q8_mod;
     const float* q8_scale;
-    // NVFP4: block scales of both operands in atoms of 128 rows x 4 blocks, atoms along K = K / 64
-    const uint8_t* sf_a;
-    const uint8_t* sf_w;
-    int sf_katoms;
 #ifdef FRT_PHASE_STAMPS
     int trace_slot;
 #endif
@@ -309,7 +312,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 tc::tma_load_2d(dst, &tmW, bar, kb * 128, n0);
             }
             if constexpr (FP4)
-                tc::bulk_load(dst + Cfg::W_BYTES + Cfg::SF_BYTES, p.sf_w + ((size_t)(n0 / 128) * p.sf_katoms + (size_t)kb * 4) * 512,
+                tc::bulk_load(dst + Cfg::W_BYTES + Cfg::SF_BYTES, p.sf_w + ((size_t)(n0 / 128) * (p.K >> 6) + (size_t)kb * 4) * 512,
                               2048, bar);
         };
         auto load_a = [&](int stage, int kb) {
@@ -886,7 +889,6 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     using Cfg = TokCfg<BN, FP4>;
     auto kern = gemm_tok_kernel<BN, PRO, EPI, ACT, FP4>;
     const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
-    if (FP4) p.sf_katoms = K / 64;
     const int m_tiles = pl.m_tiles;
     const int mt = (p.M + m_tiles - 1) / m_tiles;             // rows spread evenly over the m-tiles
     p.m_rows = mt;

@@ -179,9 +179,10 @@ def projection_tiles(rows: int, keys: int = 1024):
     N = 1024 / 2560 products leave the chip idle: 100 rows 6.23 ms per loop against 6.71, and 9.0 with the library's own
     choice); above, the MMA's fixed cost per 128-row weight tile makes two tiles of up to 128 better than four of 64 (200 rows
     8.06 ms against 9.80, 150 rows 7.10 against 8.81), except for the QKV product, where both do the same."""
-    if rows <= 64:      # 160 or 80 CTAs for the QKV product: fewer leave SMs to the attention, whose CTAs need one each (50 on 200
-        #                 keys 5.05 -> 4.89 ms, 64 on 768 5.65 -> 5.52, 24 on 300 4.42 -> 4.35); up to 16 rows it is the other way round
-        #                 (16 on 768: 4.36 against 4.61), and gate|up takes tiles of 256 (4.29)
+    if rows <= 64:
+        # 160 or 80 CTAs for the QKV product: fewer leave SMs to the attention, whose CTAs need one each (50 on 200 keys
+        # 5.05 -> 4.89 ms, 64 on 768 5.65 -> 5.52, 24 on 300 4.42 -> 4.35); up to 16 rows it is the other way round (16 on 768:
+        # 4.36 against 4.61), and gate|up takes tiles of 256 (4.29)
         qkv = 2 if rows > 16 and keys > 128 else 4
         return (dict(splits=qkv, tile_n=64), dict(splits=8, tile_n=64), dict(splits=2, tile_n=128 if rows > 16 else 256),
                 dict(splits=8, tile_n=64))
