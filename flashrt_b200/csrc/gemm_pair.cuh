@@ -216,42 +216,50 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
     pdl_launch_dependents();
 
-    // weight tile (and column scales) of a k-block of n-tile nt; the leader posts the byte count of the whole stage first
-    auto load_weights = [&](uint32_t dst, uint32_t bar, uint32_t own, int kb, int nt) {
-        // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
-        const int n0 = EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
-        if (rank == 0) tc::mbar_arrive_expect_tx(own, 2 * Cfg::STAGE_BYTES);
+    // a k-block of this CTA's activation rows / of its weight rows, with their scales
+    auto load_rows = [&](uint32_t dst, uint32_t bar, int kb, int m0) {
+        tc::tma_load_2d_pair(dst, &tmA, bar, kb * 128, m0);
+        if constexpr (FP4) tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES, &tmSA, bar, kb * 256, m0 / 128);
+    };
+    auto load_weights = [&](uint32_t dst, uint32_t bar, int kb, int n0, int sf_row) {
         tc::tma_load_2d_pair(dst + Cfg::A_BYTES, &tmW, bar, kb * 128, n0);
         if constexpr (FP4)
-            tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES, &tmSW, bar, kb * 256, nt * BN / 128);
+            tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES, &tmSW, bar, kb * 256, sf_row);
+    };
+    auto weight_row = [&](int nt) {          // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
+        return EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
     };
 
     if (warp == 0) {
         // ---------------- TMA producer (whole warp, see warp_wait; both CTAs): its half of A and of the weight rows, bytes posted at the leader
-        // Settled weights (p.early): the pair's first ring of weight tiles is fetched before the wait for the kernel in front
-        int ahead = 0;                // k-blocks of the first tile whose weights are on their way
+        // Settled weights (p.early): the pair's first ring of weight tiles is fetched before the wait for the kernel in front.
+        // Apart from the loop below: its body with one more test and the weights in front of the rows made every product of
+        // many k-blocks 1.5 % slower (2048 x 3072 x 3072 16.3 -> 16.5 us, 8192 x 3072 x 3072 59.7 -> 60.6).
+        const uint32_t ring = tc::smem_u32(smem), empty_a = tc::smem_u32(empty), full_a = tc::smem_u32(full);
+        const uint32_t lead_full = tc::dsmem_map(full_a, 0);
+        int ahead = 0, mt, nt;        // k-blocks of the first tile whose weights are on their way
         if (p.early && pair < total) {
-            int mt, nt;
             order.at(SPLIT ? pair / S : pair, mt, nt);
             const int kb0 = k_begin(pair), n = k_end(pair) - kb0;
             ahead = n < STAGES ? n : STAGES;
-            const uint32_t ring = tc::smem_u32(smem), full_a = tc::smem_u32(full);
             if (tc::elect_one())
-                for (int s = 0; s < ahead; ++s)
-                    load_weights(ring + s * Cfg::STAGE_BYTES, tc::dsmem_map(full_a, 0) + 8 * s, full_a + 8 * s, kb0 + s, nt);
+                for (int s = 0; s < ahead; ++s) {
+                    if (rank == 0) tc::mbar_arrive_expect_tx(full_a + 8 * s, 2 * Cfg::STAGE_BYTES);
+                    load_weights(ring + s * Cfg::STAGE_BYTES, lead_full + 8 * s, kb0 + s, weight_row(nt), nt * BN / 128);
+                }
         }
         pdl_wait();
-        const uint32_t ring = tc::smem_u32(smem), empty_a = tc::smem_u32(empty), full_a = tc::smem_u32(full);
-        const uint32_t lead_full = tc::dsmem_map(full_a, 0);
-        int s = 0;
-        uint32_t ph = 1;              // parity that an empty slot has completed (a fresh barrier passes parity 1)
-        bool ready = true;
+        if (ahead > 0 && tc::elect_one())
+            for (int s = 0; s < ahead; ++s)
+                load_rows(ring + s * Cfg::STAGE_BYTES, lead_full + 8 * s, k_begin(pair) + s, mt * 256 + (int)rank * 128);
+        int s = ahead % STAGES;
+        uint32_t ph = ahead < STAGES;   // parity that an empty slot has completed (a fresh barrier passes parity 1)
+        bool ready = ahead < STAGES;
         for (int t = pair; t < total; t += npairs) {
-            int mt, nt;
             order.at(SPLIT ? t / S : t, mt, nt);
-            const int m0 = mt * 256 + (int)rank * 128;
+            const int m0 = mt * 256 + (int)rank * 128, n0 = weight_row(nt), sf_row = nt * BN / 128;
             const int kb1 = k_end(t);
-            for (int kb = k_begin(t); kb < kb1; ++kb) {
+            for (int kb = k_begin(t) + (t == pair ? ahead : 0); kb < kb1; ++kb) {
                 if (!tc::warp_wait(empty_a + 8 * s, ph, ready, deadline, abort_flag)) {
                     if (lane == 0 && !*abort_flag) atomicCAS(&g_gemm_status, 0, ERR_PRODUCER | (blockIdx.x << 8));
                     *abort_flag = 1;
@@ -263,12 +271,10 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (++s == STAGES) { s = 0; ph ^= 1; }
                 ready = tc::mbar_test(empty_a + 8 * s, ph);
                 if (tc::elect_one()) {
-                    if (ahead <= 0) load_weights(dst, bar, own, kb, nt);
-                    tc::tma_load_2d_pair(dst, &tmA, bar, kb * 128, m0);
-                    if constexpr (FP4)
-                        tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES, &tmSA, bar, kb * 256, m0 / 128);
+                    if (rank == 0) tc::mbar_arrive_expect_tx(own, 2 * Cfg::STAGE_BYTES);
+                    load_rows(dst, bar, kb, m0);
+                    load_weights(dst, bar, kb, n0, sf_row);
                 }
-                --ahead;
             }
         }
     } else if (warp == 1 && rank == 0) {

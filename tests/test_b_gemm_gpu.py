@@ -272,6 +272,29 @@ def test_gemm_fp8_cta_pair_kernel(M, N, K):
     assert np.abs(a - b).max() <= 1          # bf16 bit patterns at most one step apart
 
 
+@pytest.mark.parametrize("kb", [1, 5, 6, 7, 12, 13])
+@pytest.mark.parametrize("M,N", [(300, 320), (2570, 2050)])
+def test_gemm_fp8_pair_weights_ahead(M, N, kb):
+    """A ring of weight tiles fetched ahead on CTA pairs (6 stages): fewer k-blocks than the ring, as many, more, one tile per pair
+    and several.  The same bytes as without, those within one bf16 step of the one-CTA kernel; the GeGLU finish likewise."""
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import Dev, f32, zeros
+    rng, K = np.random.default_rng(M + kb), kb * 128
+    A, sa = _fp8_operand(rng, M, K, 1.0)
+    W, sb = _fp8_operand(rng, N, K, 0.02)
+    d_A, d_W, d_sa, d_sb, d_so = Dev(A), Dev(W), f32(sa), f32(sb), f32(0.013)
+    out, half = [zeros((M, N), np.uint16) for _ in range(3)], N // 2 // 128 * 128
+    for o, flags in zip(out, (32, 8, 9)):
+        _lib.call("frt_b200_gemm_fp8_nt", d_A.ptr, d_W.ptr, o.ptr, M, N, K, d_sa.ptr, d_sb.ptr, 1.0, None, 0, flags, 0)
+    gated = [zeros((M, half), np.uint8) for _ in range(2)]
+    for early, o in enumerate(gated):
+        _lib.call("frt_b200_gemm_fp8_nt_geglu_fp8", d_A.ptr, d_W.ptr, o.ptr, M, half, K, d_sa.ptr, d_sb.ptr, d_so.ptr, 0, early, 0)
+    assert fvk.tensor_core_status() == 0
+    one, plain, early = (o.get().astype(np.int64) for o in out)
+    assert np.array_equal(plain, early) and np.abs(one - plain).max() <= 1
+    assert np.array_equal(gated[0].get(), gated[1].get())
+
+
 @pytest.mark.parametrize("M,N,K", [(2048, 1024, 1024), (1000, 200, 512), (3000, 14336 // 8, 3072)])
 def test_gemm_fp8_bias_gelu_epilogue_equals_pair(M, N, K):
     """GEMM with bias + GELU + FP8 quantise in the epilogue == GEMM -> bias_gelu_quantize_fp8, byte for byte."""
