@@ -152,11 +152,16 @@ __device__ __forceinline__ bool split_k_sum(const GemmParams& p, uint32_t t_src,
     return true;
 }
 
-// tmSA, tmSW: scale atoms of the NVFP4 form (copies of the operand maps otherwise)
+// Maps of the scale atoms (256 bytes of launch parameters): the NVFP4 form's alone.
+template <bool FP4>
+struct PairScaleMaps {};
+template <>
+struct PairScaleMaps<true> { CUtensorMap a, w; };
+
 template <int BN, int EPI, bool SPLIT = false, bool FP4 = false>
 __global__ void __launch_bounds__(64 + pair_epi_threads<EPI>(), 1)
-gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
-                     const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSW, GemmParams p) {
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, GemmParams p,
+                     const __grid_constant__ PairScaleMaps<FP4> sfm) {
     static_assert(BN == 128 || BN == 192 || BN == 256, "tile widths");
     static_assert(!SPLIT || BN == 256, "split K: 256 x 256 tiles");
     static_assert(EPI != EPI_P_GEGLU_FP8 || BN == 256, "GeGLU: 128 gate and 128 up columns");
@@ -200,9 +205,9 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tc::mbar_fence_init();
         tc::tma_prefetch_desc(&tmA);
         tc::tma_prefetch_desc(&tmW);
-        if (FP4) {
-            tc::tma_prefetch_desc(&tmSA);
-            tc::tma_prefetch_desc(&tmSW);
+        if constexpr (FP4) {
+            tc::tma_prefetch_desc(&sfm.a);
+            tc::tma_prefetch_desc(&sfm.w);
         }
     }
     if (warp == 1) {
@@ -219,12 +224,12 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     // a k-block of this CTA's activation rows / of its weight rows, with their scales
     auto load_rows = [&](uint32_t dst, uint32_t bar, int kb, int m0) {
         tc::tma_load_2d_pair(dst, &tmA, bar, kb * 128, m0);
-        if constexpr (FP4) tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES, &tmSA, bar, kb * 256, m0 / 128);
+        if constexpr (FP4) tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES, &sfm.a, bar, kb * 256, m0 / 128);
     };
     auto load_weights = [&](uint32_t dst, uint32_t bar, int kb, int n0, int sf_row) {
         tc::tma_load_2d_pair(dst + Cfg::A_BYTES, &tmW, bar, kb * 128, n0);
         if constexpr (FP4)
-            tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES, &tmSW, bar, kb * 256, sf_row);
+            tc::tma_load_2d_pair(dst + Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES, &sfm.w, bar, kb * 256, sf_row);
     };
     auto weight_row = [&](int nt) {          // GeGLU: the leader stages the gate rows of the tile, its peer the up rows
         return EPI == EPI_P_GEGLU_FP8 ? nt * (BN / 2) + (int)rank * p.half : nt * BN + (int)rank * (BN / 2);
@@ -432,20 +437,18 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
         attr_once.set(attr_dev);
     }
-    CUtensorMap tmA, tmW, tmSA, tmSW;
+    CUtensorMap tmA, tmW;
+    PairScaleMaps<FP4> sfm;
     const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
     int rc = get_tmap_2d_u8(&tmA, A, (uint64_t)p.M, row_bytes, row_bytes, 128);
     if (rc) return rc;
     rc = get_tmap_2d_u8(&tmW, W, (uint64_t)p.N, row_bytes, row_bytes, BN / 2);
     if (rc) return rc;
-    if (FP4) {
-        rc = get_tmap_sf(&tmSA, p.sf_lane, (p.M + 127) / 128, K / 64, 1);
+    if constexpr (FP4) {
+        rc = get_tmap_sf(&sfm.a, p.sf_lane, (p.M + 127) / 128, K / 64, 1);
         if (rc) return rc;
-        rc = get_tmap_sf(&tmSW, p.sf_col, (p.N + 127) / 128, K / 64, Cfg::SFB_ROWS);
+        rc = get_tmap_sf(&sfm.w, p.sf_col, (p.N + 127) / 128, K / 64, Cfg::SFB_ROWS);
         if (rc) return rc;
-    } else {
-        tmSA = tmA;
-        tmSW = tmW;
     }
     const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + BN - 1) / BN, total = m_tiles * n_tiles;
     p.tile_gm = tile_group(m_tiles, n_tiles, 256, BN, sms / 2);
@@ -468,6 +471,6 @@ static int launch_gemm_pair(const void* A, const void* W, GemmParams p, int K, c
     ++na;
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI, SPLIT, FP4>, tmA, tmW, tmSA, tmSW, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel<BN, EPI, SPLIT, FP4>, tmA, tmW, p, sfm);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
