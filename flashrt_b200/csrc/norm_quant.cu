@@ -204,7 +204,8 @@ norm_row_kernel(NormArgs a) {
 // NVFP4 result is still its instructions, about 95 per 8 values.  Same sums in the same order as the CTA kernel, same bits.
 // us, one warp per row with 8 values per lane (above 4096 columns: one CTA per row) -> now: to NVFP4 20480 x 3072 59.8 -> 45.2, 8192
 // x 8192 101 -> 50, 2501 x 3072 11.4 -> 8.7; to FP8 20480 x 3072 34.2 -> 32.5 (5.8 TB/s), 8192 x 4096 22.5 -> 19.7, 8192 x 8192 84.8 ->
-// 36.7.
+// 36.7; to bf16 (a lane's 32 bytes as one store; as two, every store touches half of each sector: 4096 x 4096 11.8 instead of 10.6)
+// 8192 x 4096 24.3 -> 21.4.
 template <int OUT, int NP, int WPR>
 __global__ void __launch_bounds__(128)
 norm_block_kernel(NormArgs a) {
@@ -220,7 +221,7 @@ norm_block_kernel(NormArgs a) {
     if (WPR == 1 && !live) return;
     // whole: every lane's piece is 32 bytes at a multiple of 32, its result one aligned store; otherwise by halves of 8 values
     const bool wide = ((reinterpret_cast<uintptr_t>(a.residual) & 31) | (a.dim & 15)) == 0;
-    const bool whole = ((reinterpret_cast<uintptr_t>(a.out) & 15) | (a.dim & 15)) == 0;
+    const bool whole = ((reinterpret_cast<uintptr_t>(a.out) & (OUT == OUT_BF16 ? 31 : 15)) | (a.dim & 15)) == 0;
     const int col0 = part * 512 + lane * 16;                // pair i of this lane: columns col0 + i * WPR * 512 ..
     const size_t rbase = (size_t)row * a.dim + col0;
     const int left = live ? a.dim - col0 : 0;
@@ -297,8 +298,7 @@ norm_block_kernel(NormArgs a) {
         }
         if (!OUT_FP4) {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + roff;
-            if (on) st_global_v4(dst, make_uint4(b[0], b[1], b[2], b[3]));
-            if (on2) st_global_v4(dst + 8, make_uint4(b[4], b[5], b[6], b[7]));
+            if (on) st_global_32(dst, whole, on2, b);
             continue;
         }
         constexpr int FAM = OUT == OUT_NVFP4_A ? 0 : 1;
@@ -334,10 +334,84 @@ norm_block_kernel(NormArgs a) {
     }
 }
 
-template <int OUT, int NP, int WPR>
-static int launch_norm_block(const NormArgs& a, cudaStream_t stream) {
+// FP8 and bf16, many short rows: one warp per row with 8 values per lane and slice of 256 columns (NS slices).  What bounds these is
+// the loads in flight, and with 16 values per lane a short row's last piece is half empty and its results take twice the registers:
+// 20480 x 768 to bf16 10.2 us there and 9.3 here, 4096 x 1024 4.2 and 3.7, 20480 x 1280 to FP8 14.9 and 13.9.  Same sums, same bits.
+template <int OUT, int NS>
+__global__ void __launch_bounds__(128)
+norm_warp_kernel(NormArgs a) {
+    static_assert(OUT == OUT_BF16 || OUT == OUT_E4M3, "results of one value per element");
+    const int lane = threadIdx.x & 31;
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    pdl_wait();
+    const float inv_scale = OUT == OUT_E4M3 ? __fdiv_rn(1.0f, *a.d_scale) : 1.0f;
+    if (row >= a.rows) return;
+    const int n = (a.dim + 255) >> 8;                       // slices of this row, n <= NS
+    const size_t rbase = (size_t)row * a.dim + lane * 8;
+    const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
+    uint4 rv[NS];
+    float ssq[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        rv[w] = make_uint4(0, 0, 0, 0);
+        if (w * 256 < left) rv[w] = ld_stream_v4(a.residual + rbase + w * 256);
+    }
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float r0, r1;
+            unpack_bf16x2(rw[i], r0, r1);
+            s = __fmaf_rn(r0, r0, s);
+            s = __fmaf_rn(r1, r1, s);
+        }
+        ssq[w] = s;
+    }
+    const float tot = warp_row_total<NS>(ssq, n);
+    const float var = __fadd_rn(__fdiv_rn(tot, (float)a.dim), a.eps);
+    const float rms = __fdiv_rn(1.0f, __fsqrt_rn(var));
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const bool on = w * 256 < left;
+        uint4 wv = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+        if (on && a.weight) wv = ld_global_v4(a.weight + lane * 8 + w * 256);
+        const uint32_t* rw = &rv[w].x;
+        const uint32_t* ww = &wv.x;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float r0, r1, w0, w1;
+            unpack_bf16x2(rw[i], r0, r1);
+            unpack_bf16x2(ww[i], w0, w1);
+            v[2 * i] = __fmul_rn(__fmul_rn(r0, rms), w0);
+            v[2 * i + 1] = __fmul_rn(__fmul_rn(r1, rms), w1);
+        }
+        const size_t roff = rbase + w * 256;
+        if (OUT == OUT_E4M3) {
+            uint2 o;
+            o.x = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[0], inv_scale)), clamp448(__fmul_rn(v[1], inv_scale)),
+                                  clamp448(__fmul_rn(v[2], inv_scale)), clamp448(__fmul_rn(v[3], inv_scale)));
+            o.y = f32x4_to_e4m3x4(clamp448(__fmul_rn(v[4], inv_scale)), clamp448(__fmul_rn(v[5], inv_scale)),
+                                  clamp448(__fmul_rn(v[6], inv_scale)), clamp448(__fmul_rn(v[7], inv_scale)));
+            if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + roff, o);
+        } else {
+            uint4 o;
+            o.x = pack_bf16x2(v[0], v[1]);
+            o.y = pack_bf16x2(v[2], v[3]);
+            o.z = pack_bf16x2(v[4], v[5]);
+            o.w = pack_bf16x2(v[6], v[7]);
+            if (on) st_global_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + roff, o);
+        }
+    }
+}
+
+// CTAs of 128 threads, `per` rows each
+static int launch_norm_rows(void (*kern)(NormArgs), const NormArgs& a, int per, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((a.rows + 4 / WPR - 1) / (4 / WPR)));
+    cfg.gridDim = dim3((unsigned)((a.rows + per - 1) / per));
     cfg.blockDim = dim3(128);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -345,34 +419,60 @@ static int launch_norm_block(const NormArgs& a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, norm_block_kernel<OUT, NP, WPR>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
     return e == cudaSuccess ? FRT_OK : FRT_CUDA_ERR(e);
 }
-template <int OUT, int WPR>
-static int dispatch_norm_block(const NormArgs& a, cudaStream_t stream) {
-    switch ((a.dim + 512 * WPR - 1) / (512 * WPR)) {
-        case 1: return launch_norm_block<OUT, 1, WPR>(a, stream);
-        case 2: return launch_norm_block<OUT, 2, WPR>(a, stream);
-        case 3: return launch_norm_block<OUT, 3, WPR>(a, stream);
-        case 4: return launch_norm_block<OUT, 4, WPR>(a, stream);
-        case 5: return launch_norm_block<OUT, 5, WPR>(a, stream);
-        case 6: return launch_norm_block<OUT, 6, WPR>(a, stream);
-        case 7: return launch_norm_block<OUT, 7, WPR>(a, stream);
-        case 8: return launch_norm_block<OUT, 8, WPR>(a, stream);
-        default: return FRT_ERR_UNSUPPORTED;
-    }
-}
 
-// From 3 Mi values on (1536 x 2048, 1024 x 3072) the rows of the CTA kernel no longer fit the chip at once and its chain per row is
-// what counts; below, that chain is the shorter one (512 x 3072 to NVFP4: 3.7 us against 4.0; 1024 x 2048: 3.9 against 4.3).  Warps
-// per row: 1 up to 1024 columns, 2 up to 3072, 4 above, so that a lane holds one to four 32-byte pieces (20480 x 4096 to NVFP4 with
-// 1 / 2 / 4 warps: 70.5 / 61.9 / 58.0 us; 20480 x 1024: 15.8 / 17.6 / 31.0).  The residual form stays with the CTA kernel at every size (it
-// already streams 5.6 TB/s; two register-held rows per lane were slower).
+// The kernel of an RMSNorm without a residual (null: the one-CTA-per-row kernel) and the rows of its CTA.  Timed at 528 .. 8192
+// columns, 256 .. 20480 rows and the three kinds of result; all give the same bits.  What decides is how many rows of a form an
+// SM holds, so the lines are in rows per SM (us, the form taken first):
+//   above 1536 columns the chain of the CTA kernel counts from 3 Mi values on, when its rows no longer fit the chip at once; below,
+//   it is the shorter one (512 x 3072 to NVFP4 3.4 against 4.5).  Two warps per row up to 3072 columns, four above, so that a lane
+//   holds two to four pieces (20480 x 4096 to NVFP4 with 4 / 2 / 1 warps: 58 / 64 / 73).  But where five pieces leave one of two warps
+//   idle in the third: one warp of 16 values at 13 to 16 rows (2304 x 2560 to FP8 5.2, two warps 6.2), the 8-value kernel up to 20,
+//   its full wave, and above 40 (20480 x 2560 to FP8 27.9, two warps 32.3).  Its full wave is also 16 to 20 rows of four pieces (2816 x
+//   2048 to bf16 4.5, two warps 5.2) and up to 16 of six (2304 x 3072 to bf16 5.8, two warps 6.8).
+//   up to 1536 columns: more than 20 rows take a warp each, with 16 values per lane to NVFP4 (its instructions count) and to FP8 where
+//   they fill more than half of the last piece (20480 x 1024 11.2, 8 values 11.6), else with 8; more than 15 take two warps each (2560
+//   x 1024 to FP8 2.8, one warp 3.0, the CTA kernel 4.1), but not to NVFP4 above 1024 columns (2560 x 1280: the CTA kernel 5.0, two
+//   warps 6.1).
+// The residual form stays with the CTA kernel at every size (it already streams 5.6 TB/s; two register-held rows per lane were
+// slower).
+struct NormRows { void (*kern)(NormArgs); int per; };
 template <int OUT>
-static int launch_norm_rows(const NormArgs& a, cudaStream_t stream) {
-    if (a.dim <= 1024) return dispatch_norm_block<OUT, 1>(a, stream);
-    if (a.dim <= 3072) return dispatch_norm_block<OUT, 2>(a, stream);
-    return dispatch_norm_block<OUT, 4>(a, stream);
+static NormRows pick_norm_rows(const NormArgs& a) {
+    constexpr bool FP4 = OUT == OUT_NVFP4_A || OUT == OUT_NVFP4_B;
+    constexpr NormRows CTA = {nullptr, 0};
+    const long long rows = a.rows, sms = device_sm_count();
+    const int pieces = (a.dim + 511) / 512;
+    const bool values = rows * a.dim >= 3ll << 20;
+    if (a.dim <= 512 || (FP4 && ((reinterpret_cast<uintptr_t>(a.sf_out) & 3) || (reinterpret_cast<uintptr_t>(a.out) & 7))))
+        return CTA;
+    if (pieces > 3) {
+        if (!values) return CTA;
+        if (pieces > 12) return {norm_block_kernel<OUT, 4, 4>, 1};
+        if (pieces > 8) return {norm_block_kernel<OUT, 3, 4>, 1};
+        if (pieces > 6) return {norm_block_kernel<OUT, 2, 4>, 1};
+        if constexpr (OUT != OUT_BF16)
+            if (pieces == 5 && rows > 12 * sms && rows <= 16 * sms) return {norm_block_kernel<OUT, 5, 1>, 4};
+        if constexpr (!FP4) {
+            if (pieces == 4 && rows > 16 * sms && rows <= 20 * sms) return {norm_warp_kernel<OUT, 8>, 4};
+            if (pieces == 5 && rows > 14 * sms && (rows <= 20 * sms || rows > 40 * sms)) return {norm_warp_kernel<OUT, 10>, 4};
+            if (pieces == 6 && rows > 14 * sms && rows <= 16 * sms) return {norm_warp_kernel<OUT, 12>, 4};
+        }
+        if (pieces == 4) return {norm_block_kernel<OUT, 2, 2>, 2};
+        return {norm_block_kernel<OUT, 3, 2>, 2};
+    }
+    if (rows > 20 * sms) {
+        if constexpr (!FP4)
+            if (OUT == OUT_BF16 || ((a.dim - 1) & 511) < 256)
+                return {pieces == 2 ? norm_warp_kernel<OUT, 4> : norm_warp_kernel<OUT, 6>, 4};
+        if constexpr (OUT != OUT_BF16)
+            return {pieces == 2 ? norm_block_kernel<OUT, 2, 1> : norm_block_kernel<OUT, 3, 1>, 4};
+    }
+    if (FP4 ? pieces == 2 && rows > 15 * sms : values || rows > 15 * sms)
+        return {pieces == 2 ? norm_block_kernel<OUT, 1, 2> : norm_block_kernel<OUT, 2, 2>, 2};
+    return CTA;
 }
 
 template <bool HAS_X, bool HAS_GATE, bool HAS_STYLE, int OUT>
@@ -380,10 +480,10 @@ static int launch_norm(NormArgs a, cudaStream_t stream, bool pdl) {
     a.early = pdl ? 1 : 0;
     if (a.rows < 0 || a.dim <= 0 || (a.dim & 7) || a.dim > 8192) return FRT_ERR_UNSUPPORTED;
     if (a.rows == 0) return FRT_OK;
-    if (!HAS_X && !HAS_STYLE && (long long)a.rows * a.dim >= 3ll << 20 && a.dim > 512 &&
-        (OUT == OUT_BF16 || OUT == OUT_E4M3 ||
-         ((reinterpret_cast<uintptr_t>(a.sf_out) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 7) == 0)))
-        return launch_norm_rows<OUT>(a, stream);
+    if constexpr (!HAS_X && !HAS_STYLE) {
+        const NormRows many = pick_norm_rows<OUT>(a);
+        if (many.kern) return launch_norm_rows(many.kern, a, many.per, stream);
+    }
     int threads = ((a.dim / 8 + 31) / 32) * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.rows);

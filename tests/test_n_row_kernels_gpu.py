@@ -1,11 +1,11 @@
-"""The warp-per-row kernels (many rows) against the one-CTA-per-row kernels on the same rows in smaller calls: the same
-bits, at partial slices, partial CTAs and both sides of the row threshold."""
+"""The kernels for many rows (one, two or four warps per row) against the one-CTA-per-row kernels on the same rows in smaller
+calls: the same bits, at partial slices, partial CTAs and both sides of the row threshold."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-STEP = 384      # rows per small call: below every threshold, whole scale-factor atoms
+STEP = 384      # rows per small call: below every threshold (up to 8191 columns), whole scale-factor atoms
 
 
 def _dev(a):
@@ -133,6 +133,41 @@ def test_norm_blocks_of_unaligned_rows(rows, dim, kind):
         got.append((d_o.get()[off:off + rows * dim // (1 if kind == "fp8" else 2)], d_sf.get()))
     for g in got[:2]:
         assert np.array_equal(g[0], got[2][0]) and np.array_equal(g[1], got[2][1])
+
+
+@pytest.mark.parametrize("dim", [520, 784, 1032, 1536, 2048, 2560, 3072])
+@pytest.mark.parametrize("per_sm", [12, 14, 15, 16, 20, 40])
+@pytest.mark.parametrize("kind", ["fp8", "bf16", "nvfp4_0", "nvfp4_1"])
+def test_norm_rows_at_the_lines_between_kernels(dim, per_sm, kind):
+    """`per_sm` rows per SM are where another kernel takes over: that many rows and one more, results on and off the widest store,
+    against the same rows in calls of 256 (the one-CTA-per-row kernel): the same bits."""
+    import torch
+    from flashrt_b200 import _lib
+    from gpu_util import f32, rand_bf16, zeros
+    last = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    dim = dim // 16 * 16 if kind.startswith("nvfp4") else dim
+    x = _rows(dim + per_sm, last + 1, dim)
+    x[9, 3], x[11, 17], x[13, 40:48] = 0x7f80, 0x7fc0, 0x0001      # inf, NaN, subnormal values
+    d_x, w, sc, katoms = _dev(x), _dev(rand_bf16(np.random.default_rng(1), (dim,))), f32(0.011), (dim + 63) // 64
+    item = {"fp8": 2, "bf16": 4}.get(kind, 1)                       # half bytes per value
+    got = []
+    for rows, off, step in ((last + 1, 0, last + 1), (last + 1, 16, last + 1), (last, 0, last), (last + 1, 0, 256)):
+        d_o, d_sf = zeros((rows * dim * item // 2 + 16,), np.uint8), zeros(((rows + 127) // 128 * katoms * 512,), np.uint8)
+        off = off // (1 if kind == "bf16" else 2)                   # the least alignment the entry points take
+        for r in range(0, rows, step):
+            n, xp, op = min(step, rows - r), d_x.ptr + r * dim * 2, d_o.ptr + off + r * dim * item // 2
+            if kind == "fp8":
+                _lib.call("frt_b200_norm_fp8", xp, None, None, 0, w.ptr, None, 0, op, None, n, dim, 1e-6, sc.ptr, 0, 0)
+            elif kind == "bf16":
+                _lib.call("frt_b200_norm_bf16", xp, None, None, 0, w.ptr, None, 0, op, None, n, dim, 1e-6, 0, 0)
+            else:
+                _lib.call("frt_b200_norm_nvfp4", xp, None, None, 0, w.ptr, None, 0, op, d_sf.ptr + r // 128 * katoms * 512, None, n,
+                          dim, 1e-6, int(kind[-1]), 0, 0)
+        got.append((d_o.get()[off:off + last * dim * item // 2], d_o.get()[off + last * dim * item // 2:][:dim * item // 2],
+                    d_sf.get()[: last // 128 * katoms * 512], rows))
+    for g in got[:3]:
+        assert np.array_equal(g[0], got[3][0]) and np.array_equal(g[2], got[3][2])
+        assert g[3] == last or np.array_equal(g[1], got[3][1])
 
 
 @pytest.mark.parametrize("rows,dim", [(1, 8), (5, 1000), (7, 1032), (3, 3064), (9, 4104), (6, 8192)])
