@@ -304,6 +304,154 @@ layer_norm_rows_kernel(ResNormArgs a) {
     }
 }
 
+// Short rows, one warp each with 8 values per lane and slice of 256 columns (NS slices): more rows on an SM than with 16 values, which
+// counts while the rows are one wave of it, and above 40 rows per SM to FP8 (pick in launch_layer_norm_rows; 2560 x 768 -> FP8 3.7 us
+// with two warps of 16 values, 3.3 here, 2900 x 2048 8.0 and 6.5).  Same sums, same bits.
+template <bool OUT_FP8, int NS, bool AFFINE, bool MOD>
+__global__ void __launch_bounds__(128, 5)
+layer_norm_warp_kernel(ResNormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    float inv_a = 1.0f;
+    if (OUT_FP8 && a.out) inv_a = __fdiv_rn(1.0f, *a.d_scale);
+    if (row >= a.rows) return;
+    const int n = (a.dim + 255) >> 8;                       // n <= NS
+    const size_t rbase = (size_t)row * a.dim + lane * 8;
+    const size_t mbase = (size_t)(row / a.mod_rows) * a.mod_stride + lane * 8;
+    const int left = a.dim - lane * 8;                      // slice w of this lane exists while w * 256 < left
+    uint4 rv[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        rv[w] = make_uint4(0, 0, 0, 0);
+        if (w * 256 < left) rv[w] = ld_stream_v4(a.res + rbase + w * 256);
+    }
+    if (a.x) {
+        constexpr int B = 4;                                // slices of x in flight
+#pragma unroll
+        for (int w0 = 0; w0 < NS; w0 += B) {
+            uint4 xv[B], gv[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                xv[j] = make_uint4(0, 0, 0, 0);
+                gv[j] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);   // no gate: x * 1 + r rounds once, as the add
+                if (w0 + j < NS && (w0 + j) * 256 < left) {
+                    xv[j] = ld_stream_v4(a.x + rbase + (w0 + j) * 256);
+                    if (a.gate) gv[j] = ld_global_v4(a.gate + mbase + (w0 + j) * 256);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < B && w0 + j < NS; ++j) {
+                const int w = w0 + j;
+                uint32_t* rw = &rv[w].x;
+                const uint32_t* xw = &xv[j].x;
+                const uint32_t* gw = &gv[j].x;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float r0, r1, x0, x1, g0, g1;
+                    unpack_bf16x2(rw[i], r0, r1);
+                    unpack_bf16x2(xw[i], x0, x1);
+                    unpack_bf16x2(gw[i], g0, g1);
+                    rw[i] = pack_bf16x2(__fmaf_rn(x0, g0, r0), __fmaf_rn(x1, g1, r1));
+                }
+                if (w * 256 < left) st_global_v4(a.res_out + rbase + w * 256, rv[w]);
+            }
+        }
+    }
+    if (!a.out) return;
+    float part[NS];
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            s = __fadd_rn(s, v0);
+            s = __fadd_rn(s, v1);
+        }
+        part[w] = s;
+    }
+    const float mean = __fdiv_rn(warp_row_total<NS>(part, n), (float)a.dim);
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const uint32_t* rw = &rv[w].x;
+        float q = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            v0 = __fsub_rn(v0, mean);
+            v1 = __fsub_rn(v1, mean);
+            q = __fmaf_rn(v0, v0, q);
+            q = __fmaf_rn(v1, v1, q);
+        }
+        part[w] = w * 256 < left ? q : 0.0f;
+    }
+    const float var = __fadd_rn(__fdiv_rn(warp_row_total<NS>(part, n), (float)a.dim), a.eps);
+    const float inv_std = __fdiv_rn(1.0f, __fsqrt_rn(var));
+#pragma unroll
+    for (int w = 0; w < NS; ++w) {
+        const bool on = w * 256 < left;
+        uint4 wv = make_uint4(0, 0, 0, 0), bv = wv, sc = wv, sh = wv;
+        if (on) {
+            if (AFFINE) {
+                wv = ld_global_v4(a.weight + lane * 8 + w * 256);
+                if (a.bias) bv = ld_global_v4(a.bias + lane * 8 + w * 256);
+            }
+            if (MOD) {
+                sc = ld_global_v4(a.scale + mbase + w * 256);
+                sh = ld_global_v4(a.shift + mbase + w * 256);
+            }
+        }
+        const uint32_t* rw = &rv[w].x;
+        const uint32_t* ww = &wv.x;
+        const uint32_t* bw = &bv.x;
+        const uint32_t* scw = &sc.x;
+        const uint32_t* shw = &sh.x;
+        uint4 o16;
+        uint32_t* ow = &o16.x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            unpack_bf16x2(rw[i], v0, v1);
+            float n0 = __fmul_rn(__fsub_rn(v0, mean), inv_std), n1 = __fmul_rn(__fsub_rn(v1, mean), inv_std);
+            if (AFFINE) {
+                float w0, w1, b0, b1;
+                unpack_bf16x2(ww[i], w0, w1);
+                unpack_bf16x2(bw[i], b0, b1);
+                n0 = __fmaf_rn(n0, w0, b0);
+                n1 = __fmaf_rn(n1, w1, b1);
+            }
+            if (MOD) {
+                float s0, s1, h0, h1;
+                unpack_bf16x2(scw[i], s0, s1);
+                unpack_bf16x2(shw[i], h0, h1);
+                n0 = __fmaf_rn(n0, __fadd_rn(1.0f, s0), h0);
+                n1 = __fmaf_rn(n1, __fadd_rn(1.0f, s1), h1);
+            }
+            ow[i] = pack_bf16x2(n0, n1);
+        }
+        if (!OUT_FP8) {
+            if (on) st_global_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + rbase + w * 256, o16);
+        } else {
+            float r[8];                                      // quantise the bf16-rounded value
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                unpack_bf16x2(ow[i], r[2 * i], r[2 * i + 1]);
+                r[2 * i] = clamp448(__fmul_rn(r[2 * i], inv_a));
+                r[2 * i + 1] = clamp448(__fmul_rn(r[2 * i + 1], inv_a));
+            }
+            uint2 o8;
+            o8.x = f32x4_to_e4m3x4(r[0], r[1], r[2], r[3]);
+            o8.y = f32x4_to_e4m3x4(r[4], r[5], r[6], r[7]);
+            if (on) st_global_v2(reinterpret_cast<uint8_t*>(a.out) + rbase + w * 256, o8);
+        }
+    }
+}
+
 // ------------------------------------------------------------------ QKV split + q/k RMSNorm + 3-D RoPE
 // packed (rows, 3*dim) bf16 = [q | k | v]; q_out / k_out (rows, dim); row = b * L + t
 __global__ void __launch_bounds__(1024)
@@ -656,20 +804,55 @@ static inline unsigned cap_grid(long long items, int threads) {
     return (unsigned)(need < 1 ? 1 : (need < cap ? need : cap));
 }
 
-// Rows from which the kernels of many rows win over one CTA per row (graph of back-to-back launches, dim 1024 .. 5120); LayerNorm also
-// from 2 Mi values on (512 x 5120 with the residual 5.9 us, one CTA per row without it 7.1).
-enum { LN_MANY_ROWS = 1024, ROPE_MANY_ROWS = 512 };
+enum { ROPE_MANY_ROWS = 512 };      // from here on one warp per row and part wins over one CTA per row
 
+// LayerNorm without a residual: more rows than one CTA each is the fastest for.  In rows per SM by pieces of 512 columns: 8 up to 1024
+// columns (1024 x 1024 -> FP8 3.2 us, with two warps per row 3.5), 6, 5, 5, 3 (512 x 3072 4.6, with four warps per row 3.7), above 3072
+// columns from 1024 rows or 2 Mi values on.
+static bool layer_norm_many(long long rows, int dim) {
+    static const int line[7] = {8, 8, 8, 6, 5, 5, 3};
+    const int pieces = (dim + 511) / 512;
+    return pieces > 6 ? rows >= 1024 || rows * dim >= 2ll << 20 : rows > (long long)line[pieces] * device_sm_count();
+}
+
+// Warps per row and values per lane, again by rows per SM: what counts is how many rows of a form an SM holds, and that no warp of a
+// row is idle in the last piece.  8 rows are one wave of four warps each, 10 of two at 2560 and 3072 columns.  With the residual (two rows in registers) the lines lie higher and four warps per row go further:
+// 1972 x 3072 with two warps 12.9 us, with four 10.8, 8192 x 3072 35.0 and 35.3.  Without, to FP8, two warps and the form taken:
+// 2560 x 1280 6.3 and 5.1 (one warp), 2304 x 2560 9.0 and 7.3 (one), 1972 x 3072 9.3 and 7.9 (four), 20480 x 3072 52.9 and 47.3 (one).
 template <bool OUT_FP8, bool AFFINE, bool MOD>
 static int launch_layer_norm_rows(const ResNormArgs& a, cudaStream_t s) {
-    auto grid = [&](int rows_per_cta) { return (unsigned)((a.rows + rows_per_cta - 1) / rows_per_cta); };
-    // up to 1024 columns: two warps per row while that keeps more of the chip busy (1972 x 1024: 5.4 us with one)
-    if (a.dim <= 1024 && a.rows < 3072) return launch_k(layer_norm_rows_kernel<OUT_FP8, 1, 2, AFFINE, MOD>, grid(2), 128, s, a);
-    if (a.dim <= 1024) return launch_k(layer_norm_rows_kernel<OUT_FP8, 2, 1, AFFINE, MOD>, grid(4), 128, s, a);
-    if (a.dim <= 2048) return launch_k(layer_norm_rows_kernel<OUT_FP8, 2, 2, AFFINE, MOD>, grid(2), 128, s, a);
-    if (a.dim <= 3072) return launch_k(layer_norm_rows_kernel<OUT_FP8, 3, 2, AFFINE, MOD>, grid(2), 128, s, a);
-    if (a.dim <= 4096) return launch_k(layer_norm_rows_kernel<OUT_FP8, 2, 4, AFFINE, MOD>, grid(1), 128, s, a);
-    return launch_k(layer_norm_rows_kernel<OUT_FP8, 4, 4, AFFINE, MOD>, grid(1), 128, s, a);
+    const int pieces = (a.dim + 511) / 512;
+    const long long sms = device_sm_count();
+    const bool res = a.x != nullptr;
+    auto over = [&](int rows_per_sm) { return a.rows > rows_per_sm * sms; };
+    auto run = [&](void (*kern)(ResNormArgs), int rows_per_cta) {
+        return launch_k(kern, (unsigned)((a.rows + rows_per_cta - 1) / rows_per_cta), 128, s, a);
+    };
+    if (pieces > 8) return run(layer_norm_rows_kernel<OUT_FP8, 4, 4, AFFINE, MOD>, 1);
+    if (pieces > 6) return run(layer_norm_rows_kernel<OUT_FP8, 2, 4, AFFINE, MOD>, 1);
+    if (pieces == 6) {
+        if (!over(res ? 30 : 16) && (over(10) || !over(8))) return run(layer_norm_rows_kernel<OUT_FP8, 2, 4, AFFINE, MOD>, 1);
+        if (OUT_FP8 && !res && over(40)) return run(layer_norm_rows_kernel<OUT_FP8, 6, 1, AFFINE, MOD>, 4);
+        return run(layer_norm_rows_kernel<OUT_FP8, 3, 2, AFFINE, MOD>, 2);
+    }
+    if (pieces == 5) {
+        if (over(30) || (!res && over(10) && !over(16))) return run(layer_norm_rows_kernel<OUT_FP8, 5, 1, AFFINE, MOD>, 4);
+        if (!over(res ? 30 : 10) && (over(10) || !over(8))) return run(layer_norm_rows_kernel<OUT_FP8, 2, 4, AFFINE, MOD>, 1);
+        return run(layer_norm_rows_kernel<OUT_FP8, 3, 2, AFFINE, MOD>, 2);
+    }
+    if (pieces == 4) {
+        if (!res && over(15) && (!over(20) || over(40))) return run(layer_norm_warp_kernel<OUT_FP8, 8, AFFINE, MOD>, 4);
+        if (!over(res ? 80 : 10)) return run(layer_norm_rows_kernel<OUT_FP8, 1, 4, AFFINE, MOD>, 1);
+        return run(layer_norm_rows_kernel<OUT_FP8, 2, 2, AFFINE, MOD>, 2);
+    }
+    if (pieces == 3) {
+        if (over(res ? 28 : OUT_FP8 ? 14 : 16)) return run(layer_norm_rows_kernel<OUT_FP8, 3, 1, AFFINE, MOD>, 4);
+        if (res || !over(8)) return run(layer_norm_rows_kernel<OUT_FP8, 1, 4, AFFINE, MOD>, 1);
+        return run(layer_norm_rows_kernel<OUT_FP8, 2, 2, AFFINE, MOD>, 2);
+    }
+    if (over(6) && !over(20)) return run(layer_norm_warp_kernel<OUT_FP8, 4, AFFINE, MOD>, 4);
+    if (over(res && pieces > 1 ? 80 : 20)) return run(layer_norm_rows_kernel<OUT_FP8, 2, 1, AFFINE, MOD>, 4);
+    return run(layer_norm_rows_kernel<OUT_FP8, 1, 2, AFFINE, MOD>, 2);
 }
 template <bool OUT_FP8>
 static int dispatch_layer_norm_warp(const ResNormArgs& a, cudaStream_t s) {
@@ -699,7 +882,7 @@ int frt_b200_layer_norm(const void* x, const void* weight, const void* bias, con
         mis(out_fp8, 8))
         return FRT_ERR_INVALID;
     if (rows == 0) return FRT_OK;
-    if (rows >= LN_MANY_ROWS || (long long)rows * dim >= 2ll << 20) {
+    if (layer_norm_many(rows, dim)) {
         ResNormArgs a = {};
         a.res = (const __nv_bfloat16*)x;
         a.weight = (const __nv_bfloat16*)weight;

@@ -88,6 +88,41 @@ def test_layer_norm_rows_and_residual_form(rows, dim, mod):
         assert np.array_equal(d_o.get(), d_o2.get())
 
 
+@pytest.mark.parametrize("dims,lines,res_lines", [((520, 1024), (8, 20), (6, 20, 80)), ((1032, 1536), (6, 8, 14, 16), (28,)),
+                                                  ((1800, 2048), (5, 10, 15, 20, 40), (80,)), ((2056, 2560), (5, 8, 10, 16, 30), (8, 10, 30)),
+                                                  ((2568, 3072), (3, 8, 10, 16, 40), (8, 10, 30))])
+@pytest.mark.parametrize("mod", ["affine", "modulated"])
+def test_layer_norm_at_the_lines_between_kernels(dims, lines, res_lines, mod):
+    """`lines` rows per SM are where another kernel takes over: one row more than that many, against the same rows in calls of 128
+    (one CTA per row; with the residual the form for few rows): the same bits.  FP8, bf16 and the residual form."""
+    import torch
+    from flashrt_b200 import _lib
+    from gpu_util import f32, rand_bf16, zeros
+    sms, rng = torch.cuda.get_device_properties(0).multi_processor_count, np.random.default_rng(dims[0])
+    s8 = f32(0.013)
+    for dim in dims:
+        vec = [_dev(rand_bf16(rng, (dim,))) for _ in range(3)]
+        aff, md = ((vec[0].ptr, vec[1].ptr), (None, None)) if mod == "affine" else ((None, None), (vec[0].ptr, vec[1].ptr))
+        top = sms * max(lines + res_lines) + 1
+        d_x, d_y = _dev(_rows(dim, top, dim)), _dev(_rows(dim + 1, top, dim))
+        for kind, per_sm in [(k, n) for k in ("fp8", "bf16") for n in lines] + [("res", n) for n in res_lines]:
+            rows, outs = per_sm * sms + 1, []
+            for step in (rows, 128):
+                d_o = torch.zeros(rows, dim, dtype=torch.uint16 if kind == "bf16" else torch.uint8, device="cuda")
+                d_r = torch.zeros(rows, dim, dtype=torch.uint16, device="cuda")
+                for r in range(0, rows, step):
+                    n, xp, yp, op = min(step, rows - r), d_x.ptr + r * dim * 2, d_y.ptr + r * dim * 2, d_o[r:].data_ptr()
+                    if kind == "res":
+                        _lib.call("frt_b200_residual_layer_norm_fp8", xp, yp, vec[2].ptr, d_r[r:].data_ptr(), *aff, *md, 0, n, op,
+                                  s8.ptr, n, dim, 1e-6, 0, 0)
+                    else:
+                        _lib.call("frt_b200_layer_norm", xp, *aff, *md, 0, op if kind == "fp8" else None,
+                                  op if kind == "bf16" else None, s8.ptr, n, dim, 1e-6, 0, 0)
+                torch.cuda.synchronize()
+                outs.append((d_o.view(torch.uint8), d_r.view(torch.uint8)))
+            assert all(torch.equal(g, w) for g, w in zip(*outs)), (dim, kind, per_sm)
+
+
 @pytest.mark.parametrize("L,heads,hd,seq", [(512, 24, 128, 512), (515, 3, 40, 400), (513, 5, 256, 513)])
 def test_qkv_split_norm_rope_rows(L, heads, hd, seq):
     from flashrt_b200 import flash_rt_kernels as fvk
