@@ -52,6 +52,7 @@ enum { TOK_EPI_BF16 = 0, TOK_EPI_ROPE = 1, TOK_EPI_GEGLU = 2, TOK_EPI_RESID = 3 
 // with rows of BN floats (a multiple of 32 banks) the four tokens of a warp hit the same banks (8 wavefronts per 16-byte
 // load instead of 4); four floats of padding rotate them apart.
 constexpr int TOK_ROW_PAD = 4;
+constexpr int TOK_MAX_SMEM = 227 * 1024;                      // shared memory of a CTA
 enum { TOK_PRO_TMA = 0, TOK_PRO_NORM = 1 };
 // floats between the per-tile rows of a statistics buffer
 static inline int tok_stat_stride(int M) { return M <= 128 ? 128 : 256; }
@@ -861,9 +862,9 @@ static bool tok_plan(int N, int K, int m_tiles, int mt, int epi, int pro, int sm
             const int stages = nkb < max_st ? nkb : max_st;
             const int per = (mt + S - 1) / S;
             const int smem = 3072 + stages * stage_bytes + S * per * (BN + TOK_ROW_PAD) * 4;
-            if (pro == TOK_PRO_NORM && smem - S * per * TOK_ROW_PAD * 4 > 227 * 1024) continue;
+            if (pro == TOK_PRO_NORM && smem - S * per * TOK_ROW_PAD * 4 > TOK_MAX_SMEM) continue;
             // the launcher shortens the ring down to two stages, not further
-            if (3072 + (stages < 2 ? stages : 2) * stage_bytes + S * per * BN * 4 > 227 * 1024) continue;
+            if (3072 + (stages < 2 ? stages : 2) * stage_bytes + S * per * BN * 4 > TOK_MAX_SMEM) continue;
             const double pushed_kb = (double)(S - 1) / S * mt * BN * 4 / 1024.0;
             double cost = nkb * 0.33 + pushed_kb * 0.06 + (S > 1 ? 0.05 * S : 0.0);
             if (pro == TOK_PRO_NORM) cost += 0.6 * nkb;
@@ -902,9 +903,9 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     const bool m64 = p.m64 != 0;
     // padded receive rows unless even a two-stage ring would not fit beside them
     const int need_stages = PRO == TOK_PRO_NORM ? pl.nkb : (p.stages < 2 ? p.stages : 2);   // the ring's lower bound
-    p.row_pad = Cfg::smem_bytes(need_stages, pl.S, p.per, m64, TOK_ROW_PAD) > 227 * 1024 ? 0 : TOK_ROW_PAD;
+    p.row_pad = Cfg::smem_bytes(need_stages, pl.S, p.per, m64, TOK_ROW_PAD) > TOK_MAX_SMEM ? 0 : TOK_ROW_PAD;
     // the operand ring shrinks until it fits beside the receive slots
-    while (p.stages > 2 && Cfg::smem_bytes(p.stages, pl.S, p.per, m64, p.row_pad) > 227 * 1024) --p.stages;
+    while (p.stages > 2 && Cfg::smem_bytes(p.stages, pl.S, p.per, m64, p.row_pad) > TOK_MAX_SMEM) --p.stages;
     if (PRO == TOK_PRO_NORM && p.stages < pl.nkb) return FRT_ERR_UNSUPPORTED;
     p.K = K;
 #ifdef FRT_PHASE_STAMPS
@@ -913,15 +914,14 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
 #endif
     const int smem = Cfg::smem_bytes(p.stages, pl.S, p.per, m64, p.row_pad);
     p.ring_bytes = Cfg::ring_bytes(p.stages, m64);
-    if (smem > 227 * 1024) return FRT_ERR_UNSUPPORTED;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    static int attr_smem[64] = {0};
-    if (dev < 0 || dev >= 64) return FRT_ERR_UNSUPPORTED;
-    if (attr_smem[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > TOK_MAX_SMEM) return FRT_ERR_UNSUPPORTED;
+    // the limit, not this launch's size: a size that grew from launch to launch could be set back by another thread's smaller one
+    static PerDeviceOnce attr_once;
+    int attr_dev = 0;
+    if (attr_once.need(attr_dev)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TOK_MAX_SMEM);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
-        attr_smem[dev] = smem;
+        attr_once.set(attr_dev);
     }
     CUtensorMap tmA, tmW;
     int rc;

@@ -58,3 +58,15 @@ def test_lanes_that_skip_stores_meet_before_the_next_collective_load():
     head = text[:text.index("if (m >= p.M) continue;")]
     head = head[head.rindex("for (int c"):]
     assert 0 < head.find("__syncwarp();") < head.index("tmem_ld") and text.count("continue;") == 1
+
+
+def test_shared_memory_limit_of_a_kernel_does_not_follow_the_launch():
+    """A kernel's limit of dynamic shared memory is one value per kernel: a size raised from launch to launch is set back when
+    another thread's smaller launch sets its own between the check and the call."""
+    values = []
+    for name in sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))):
+        values += re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*)\);", source(name))
+    assert len(values) > 10
+    for v in values:                   # no name of a variable: constants and what they make up
+        words = set(re.findall(r"[A-Za-z_]\w*", v)) - {"int", "sizeof", "float", "el", "Cfg", "smem_bytes", "ragged_smem_bytes", "true"}
+        assert all(w.isupper() for w in words), v
