@@ -959,21 +959,48 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
 
 // NVFP4, at most 64 rows: microseconds of a launch of N / bn tiles x S CTAs that are all resident -- fitted to 710 products of a
 // sweep (M 8 .. 64, N 1024 .. 14336, K 1024 .. 14336, in a graph, weights fetched early; 6 % standard deviation): k-blocks of a CTA,
-// KB pushed to its peers, tokens it finishes, SMs in use.
+// KB pushed to its peers, tokens it finishes, SMs in use beyond half of them.
 static double tok_nvfp4_us(int M, int N, int K, int bn, int S) {
-    const int ctas = (N + bn - 1) / bn * S;
+    const int ctas = (N + bn - 1) / bn * S, half = device_sm_count() / 2;
     const double t = 2.0 + K / 256 / S * (bn == 128 ? 0.33 : 0.305) + (double)(S - 1) / S * M * bn / 256.0 * 0.09 +
                      (M + S - 1) / S * bn / 1024.0 * 0.3;
-    return ctas > 74 ? t + (ctas - 74) * (1.35 / 74) : t;
+    return ctas > half ? t + (ctas - half) * (1.35 / half) : t;
 }
-// The plan (S = 0: none), the cheapest by that cost; `want` > 0 pins the split.  All CTAs resident at once, and of clusters of eight no more than fit
-// beside one another when a CTA needs an SM to itself.  50 x 2560 x 1024 6.1 -> 3.9 us against the small-M kernel and its exchange by
-// cluster barriers, 50 x 1024 x 4096 6.6 -> 4.6, 16 x 1024 x 1024 4.3 -> 2.8; unsplit products of much weight stay there (50 x 8192 x
-// 1024: 4.6 against 4.85).
+// Clusters of eight CTAs that the device holds at once where a CTA needs an SM to itself: fewer than SMs / 8, since the SMs that a
+// group of them has beyond a multiple of eight stay empty (15 on the parts measured).  Asked once per device; 4/5 of the SMs if the
+// question is refused.
+static int tok_clusters_of_8() {
+    static int known[64] = {0};
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return device_sm_count() / 10;
+    if (known[dev]) return known[dev];
+    auto kern = gemm_tok_kernel<64, TOK_PRO_TMA, TOK_EPI_BF16, 0, true>;
+    cudaLaunchConfig_t q = {};
+    q.gridDim = dim3(1, 1, 8);
+    q.blockDim = dim3(256);
+    q.dynamicSmemBytes = 120 * 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 8;
+    q.attrs = attr;
+    q.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &q) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = device_sm_count() / 10;
+    }
+    return known[dev] = n;
+}
+// The plan (S = 0: none), the cheapest by that cost; `want` > 0 pins the split.  All CTAs resident at once.  50 x 2560 x 1024 6.1 ->
+// 3.9 us against the small-M kernel and its exchange by cluster barriers, 50 x 1024 x 4096 6.6 -> 4.6, 16 x 1024 x 1024 4.3 -> 2.8;
+// unsplit products of much weight stay there (50 x 8192 x 1024: 4.6 against 4.85).
 // In a chain (`chain`: the caller says the weights may be fetched early) more and smaller CTAs pay also where the launch alone is no
 // faster: every weight tile of a split waits in shared memory.  There: tiles of 64 and the largest split with a CTA per SM (or two of a
-// product that would stay whole), if its k-blocks all fit the ring.  Loops of 20 / 33 / 50 / 64 tokens on 768 / 500 / 768 / 900 keys,
-// all splits of the four products timed: 5.32 / 5.60 / 6.03 / 6.82 ms, with the cheapest launches 6.16 / 6.09 / 6.23 / 6.89.
+// product that would stay whole), if its k-blocks all fit the ring; up to 16 clusters of eight where two CTAs share an SM.  With five
+// or six k-blocks and more they do not, and 16 clusters are two waves: 50 x 1024 x 12288 10.3 us, as four splits 6.2.  Loops of 20 /
+// 33 / 50 / 64 tokens on 768 / 500 / 768 / 900 keys, all splits of the four products timed: 5.32 / 5.60 / 6.03 / 6.82 ms, with the
+// cheapest launches 6.16 / 6.09 / 6.23 / 6.89; alone, 8192 x 1024 is slower so (16 rows 4.1 us, by cost 3.4).
 static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     TokPlan best = {0, 0, 0, 0, 1};
     double t = 1e30;
@@ -981,7 +1008,11 @@ static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     if ((N & 7) || M > 64) return best;
     const int tiles64 = (N + 63) / 64;
     for (int S = 8; chain && want <= 0 && S >= 1; S /= 2) {
-        if (kbt % S || kbt / S > 8 || tiles64 * S > sms || (S == 8 && tiles64 * 64 > sms * 7)) continue;
+        if (kbt % S || kbt / S > 8 || tiles64 * S > sms) continue;
+        if (S == 8) {
+            const bool share = TokCfg<64, true>::smem_bytes(kbt / 8, 8, (M + 7) / 8, true, TOK_ROW_PAD) <= 110 * 1024;
+            if (share ? tiles64 * 64 > sms * 7 : tiles64 > tok_clusters_of_8()) continue;
+        }
         if (S == 1 && kbt % 2 == 0 &&          // two CTAs of half the k-blocks share an SM
             TokCfg<64, true>::smem_bytes(kbt / 2, 2, (M + 1) / 2, true, TOK_ROW_PAD) <= 110 * 1024) S = 2;
         return {64, S, kbt / S, kbt / S, 1};
@@ -989,7 +1020,7 @@ static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     for (int bn = 64; bn <= 128; bn += 64) {
         const int tiles = (N + bn - 1) / bn;
         for (int S = 1; S <= 8; S *= 2) {
-            if (kbt % S || tiles * S > sms || (S == 8 && tiles > 14) || (want > 0 && S != want)) continue;
+            if (kbt % S || tiles * S > sms || (S == 8 && tiles > tok_clusters_of_8()) || (want > 0 && S != want)) continue;
             const double us = tok_nvfp4_us(M, N, K, bn, S);
             if (us >= t) continue;
             const int nkb = kbt / S, most = bn == 128 ? 6 : 8;

@@ -292,7 +292,8 @@ def test_gemm_nvfp4_rope_finishes_equal_the_pair_of_launches(M, k_dim, pos):
         assert np.array_equal(a.get(), b.get())
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (17, 72, 2048), (64, 1096, 2048), (50, 200, 14336), (33, 1024, 768)])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (17, 72, 2048), (64, 1096, 2048), (50, 200, 14336), (33, 1024, 768),
+                                   (50, 960, 12288), (64, 1024, 10240)])
 @pytest.mark.parametrize("splits", [0, 1, 2, 8])
 @pytest.mark.parametrize("pdl", [False, True])
 def test_gemm_nvfp4_token_major(M, N, K, splits, pdl):
