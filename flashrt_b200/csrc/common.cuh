@@ -134,7 +134,7 @@ __device__ __forceinline__ float det_gelu_tanh(float g) {
 // addition of 1.5 * 2^23 (whose sum's low bits are also the exponent of 2^n), and the quotient is Markstein's (IBM J. Res. Dev. 34,
 // 1990): reciprocal approximation, one Newton step, quotient, exact remainder, one correction -- correctly rounded as long as
 // nothing leaves the normal range, so gates outside 2^-60 <= |g| < 9 (zeros, tiny ones, infinities, NaN, large ones) take the scalar
-// form.  Inputs are bf16 values: all 65536 are checked against it.
+// form.  Inputs are bf16 values: every finite one is checked against it.
 __device__ __forceinline__ uint64_t det_gelu_tanh2(uint64_t g) {
     auto both = [](float v) { return f32x2(v, v); };
     float g0, g1, x0, x1, t0, t1, d0, d1;

@@ -414,7 +414,9 @@ int frt_b200_norm_nvfp4(void* residual, const void* x, const void* gate_in, long
  *   beta is not supported (the decoder path calls with beta = 0).  One kernel for every variant index.
  *   splits: 0 = choose (1: M <= 256 rows on one split of the small-M kernel); flags: bit0 = the weights are settled and may be
  *   read before the kernel in front has ended, bit1 = one-tile-per-CTA kernel for M > 256 (bits 0-1 as frt_b200_gemm_fp8_nt),
- *   bits 8-9 = tile columns on CTA pairs (1 = 128, 2 = 192, 3 = 256; 0 = choose). */
+ *   bits 8-9 = tile columns on CTA pairs (1 = 128, 2 = 192, 3 = 256; 0 = choose).
+ *   At most 64 rows: the split chosen for splits = 0, and with it the order of the sums, depends on bit 0 (a chain of launches
+ *   wants more and smaller CTAs than one launch).  The same bits with and without early reads: give the split. */
 int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const void* SFW, void* D, int M, int N,
                            int K, float alpha, const float* d_alpha, const void* bias, int splits, int flags,
                            void* stream);

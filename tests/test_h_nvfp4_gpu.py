@@ -226,8 +226,8 @@ def test_gemm_nvfp4_rope_split_equals_pair():
 
 @pytest.mark.parametrize("M,N,K", [(2048, 1024, 1024), (1000, 200, 768), (4096, 3072, 1024)])
 def test_gemm_nvfp4_persistent_equals_one_tile_per_cta(M, N, K):
-    """M > 256 runs as a persistent kernel (two accumulators + the scale columns in tensor memory); the
-    one-tile-per-CTA kernel accumulates in the same order: identical bytes."""
+    """M > 256 runs on CTA pairs that walk the list of tiles; the one-tile-per-CTA kernel accumulates in the same order:
+    identical bytes."""
     from flashrt_b200 import flash_rt_fp4 as fp4, flash_rt_kernels as fvk
     from gpu_util import Dev, zeros
     rng = np.random.default_rng(M + N + K + 1)
