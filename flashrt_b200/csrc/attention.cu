@@ -109,15 +109,25 @@ struct AttnParams {
     int kv_static_rows;          // leading K/V rows that the previous kernel in the stream does not write
     // split-KV through global scratch (same buffers and layouts as the reference's FA2 split-kv path):
     float* o_accum;              // (splits, B, Hq, Sq, D) fp32, each split's O already divided by its row sum
-    float* lse_accum;            // (splits, B, Hq, Sq) fp32, log2-domain log-sum-exp of the split (-inf if empty)
+    union {
+        float* lse_accum;        // (splits, B, Hq, Sq) fp32, log2-domain log-sum-exp of the split (-inf if empty)
+        struct {                 // two-tile kernel (no splits):
+            int pair_units;      //   units of two row tiles per (batch, kv head)
+            int pair_full;       //   first unit on two CTAs
+        };
+    };
     unsigned* counters;          // 2 words per (row tile, kv head, batch): arrivals (monotonic), spare; zero before first use
     float scale_log2;            // softmax_scale * log2(e)
     int flags;                   // the entry point's flags (head_dim-256 kernel: bit 2 keeps one CTA per (tile, split), bit 3 the global-scratch combine, bit 4: kv_splits is an upper bound)
 #ifdef FRT_PHASE_STAMPS
     int trace_slot;
 #endif
-    int pair_units, pair_full; // two-tile kernel: units of two row tiles per (batch, kv head); first unit on two CTAs
 };
+#ifndef FRT_PHASE_STAMPS
+// With three tensor maps these are 512 bytes of launch parameters.  Eight bytes more cost the head-dim-256 launch 0.08 us: the loop of 4
+// x 19 tokens on 147 keys 5.430 -> 5.444 ms.
+static_assert(sizeof(AttnParams) <= 128, "launch parameters of the attention kernels");
+#endif
 
 template <int D, int BKV>
 struct AttnCfg {
