@@ -443,9 +443,11 @@ template <int OUT>
 static NormRows pick_norm_rows(const NormArgs& a) {
     constexpr bool FP4 = OUT == OUT_NVFP4_A || OUT == OUT_NVFP4_B;
     constexpr NormRows CTA = {nullptr, 0};
-    const long long rows = a.rows, sms = device_sm_count();
+    const long long rows = a.rows;
     const int pieces = (a.dim + 511) / 512;
     const bool values = rows * a.dim >= 3ll << 20;
+    if (rows < 512 && !values) return CTA;              // below every line: the smallest calls are spared the question (0.03 us)
+    const long long sms = device_sm_count();
     if (a.dim <= 512 || (FP4 && ((reinterpret_cast<uintptr_t>(a.sf_out) & 3) || (reinterpret_cast<uintptr_t>(a.out) & 7))))
         return CTA;
     if (pieces > 3) {

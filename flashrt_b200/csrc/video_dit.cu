@@ -812,6 +812,7 @@ enum { ROPE_MANY_ROWS = 512 };      // from here on one warp per row and part wi
 static bool layer_norm_many(long long rows, int dim) {
     static const int line[7] = {8, 8, 8, 6, 5, 5, 3};
     const int pieces = (dim + 511) / 512;
+    if (rows < 128 && pieces <= 6) return false;        // below every line
     return pieces > 6 ? rows >= 1024 || rows * dim >= 2ll << 20 : rows > (long long)line[pieces] * device_sm_count();
 }
 
