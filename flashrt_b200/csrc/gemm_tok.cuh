@@ -13,7 +13,9 @@
 //     update and the row sum of squares all stay inside a thread or a group of 8-16 neighbouring lanes.
 // Split-K: rank r of the cluster finishes a contiguous range of tokens.  Every rank PUSHES the accumulator rows of a
 // token straight from registers into the owner's shared memory (st.async, 16 bytes each, completing bytes on the
-// owner's mbarrier); the owner waits for S x tokens x BN x 4 bytes and sums the S slots in fixed order 0, 1, ...
+// owner's mbarrier); the owner waits for (S - 1) x tokens x BN x 4 bytes and sums the S slots in fixed order 0, 1, ...
+// Its own rows it stores plainly: st.async takes the cluster network to its own SM as well, at 17 GB/s (of two ranks half
+// of the bytes: gate|up at 50 tokens 1.3 us from the accumulator to the last push, now 0.65; the loop 5.14 -> 4.87 ms).
 // No cluster barrier and no remote load sits between the last MMA and the result.  Measured on B200: a cluster
 // barrier costs 0.75 us and a pull-based exchange needs two of them plus two remote round trips (6.2 us per launch
 // of the attention-out projection against 4.3 us with the push); staging the rows and pushing them with
@@ -271,8 +273,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         *issued = 0;
         *consumed = 0;
         tc::mbar_fence_init();
-        // every rank (this one included) sends this rank's tokens: S slots of ntok rows
-        tc::mbar_arrive_expect_tx(recv_bar, (uint32_t)(S * ntok * BN * 4));
+        // every other rank sends this rank's tokens: S - 1 slots of ntok rows
+        tc::mbar_arrive_expect_tx(recv_bar, (uint32_t)((S - 1) * ntok * BN * 4));
         if (PRO == TOK_PRO_TMA) tc::tma_prefetch_desc(&tmA);
         tc::tma_prefetch_desc(&tmW);
     }
@@ -592,7 +594,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const uint32_t trow = tmem_d + ((uint32_t)(quad * 32) << 16);
             const int rq = (row * p.per_magic) >> 16;           // row / per
             const int owner = rq < S ? rq : 0;
-            const uint32_t dst_local = tc::smem_u32(recv) + (uint32_t)(((rank * per + (row - rq * per)) * (BN + p.row_pad)) * 4);
+            float* own = recv + (rank * per + (row - rq * per)) * (BN + p.row_pad);
+            const uint32_t dst_local = tc::smem_u32(own);
             const uint32_t dst = tc::dsmem_map(dst_local, (uint32_t)owner);
             const uint32_t bar = tc::dsmem_map(tc::smem_u32(recv_bar), (uint32_t)owner);
 #pragma unroll 1
@@ -600,7 +603,11 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 uint32_t v[32];
                 tc::tmem_ld32(trow + c, v);
                 tc::tmem_ld_wait();
-                if (row < Mt) {
+                if (row < Mt && owner == rank) {            // this rank's own tokens do not leave the SM
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<uint4*>(own + c + 4 * j) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                } else if (row < Mt) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         st_async_v4(dst + (uint32_t)(c + 4 * j) * 4u, bar, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -609,14 +616,14 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
     TOK_STAMP(5);
-    // ---------------- all S slots of this rank's tokens have landed
+    __syncthreads();                     // the own slot (and s_rms) of this rank's tokens is complete
+    // ---------------- the peers' slots of this rank's tokens have landed
     const bool got = tc::mbar_wait_until(recv_bar, 0, deadline, abort_flag);
     if (!got && !*abort_flag) {
         *abort_flag = 1;
         atomicCAS(&g_gemm_status, 0, ERR_EPILOGUE | (blockIdx.x << 8));
     }
     __syncwarp();
-    if (rowscale) __syncthreads();       // s_rms of this rank's tokens is complete
     TOK_STAMP(6);
 
     // ---------------- finish: sum the S slots in order and apply the epilogue
