@@ -175,7 +175,7 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
     // first MMA)
     if constexpr (XC) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
-    pdl_launch_dependents();
+    if constexpr (!XC) pdl_launch_dependents();
 
     if (warp == 4) {
         // ---------------- TMA producer (whole warp)
@@ -390,6 +390,8 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
             if (j == 0) ATT_STAMP(5);
         }
         ATT_STAMP(6);
+        // the kernel behind may start now: under the softmax its set-up costs more than it gains (0.75 -> 1.3 us)
+        if constexpr (XC) pdl_launch_dependents();
         const float invl = l_run > 0.0f ? 1.0f / l_run : 0.0f;
         const float lse2 = l_run > 0.0f ? m_run + log2f(l_run) : -INFINITY;
         // slot of a source split: [rows_valid][dper] bf16, then rows_valid log-sum-exps
@@ -829,8 +831,9 @@ attn_d256_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // one of 16 rows -- 16 clusters do not fit but 3 x 4 + 2 do.  blockIdx.x 0 and 1: the halves of the last tile (they
 // have the longer way to go and start first); above: part (x - 2) % 4 of tile (x - 2) / 4.  The last tile has at most
 // RAGGED_ROWS rows, which keeps its receive slots, and with them the shared memory of the launch, small enough for a
-// CTA of the previous kernel to stay resident beside it (the early start under programmatic dependent launch).
-__global__ void __launch_bounds__(192, 1)
+// CTA of the previous kernel to stay resident beside it (the early start under programmatic dependent launch).  Bounds of 256 threads
+// and two CTAs: at most 128 registers, with which a scheduler holds two of these warps and two of a projection's.
+__global__ void __launch_bounds__(256, 2)
 attn_d256_ragged_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
     const int ntiles = ((int)gridDim.x - 2) / 4 + 1;
@@ -863,6 +866,12 @@ static int launch_attn_d256(const void* Q, const void* K, const void* V, AttnPar
         e = cudaFuncSetAttribute(attn_d256_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg::ragged_smem_bytes());
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        // All of the SM's memory to shared memory: the rest beside such a CTA then holds one of the projection behind, which would wait
+        // for this CTA's end otherwise
+        for (auto kern : {attn_d256_ragged_kernel, attn_d256_kernel<4, true>, attn_d256_kernel<2, true>}) {
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        }
         attr_done[dev] = true;
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -33,6 +33,13 @@
 // (csrc/kernels/activation.cu:249-279); gated residual update + per-tile row sums of squares
 // (csrc/kernels/fusion.cu:41-64, first pass).
 //
+// Programmatic launch: the kernel behind may start (its CTAs then come to stand beside this one's) once the operand has landed, not
+// from the beginning.  A CTA that starts costs the one beside it: the softmax of the attention took 1.3 us instead of 0.75 when the
+// attention-out CTAs started under it.  gate|up lets it in when its own wait has returned, QKV and the gated residual with the
+// accumulator, the plain result (whose dependents are small) behind the push: all times and products of the loops tried.  With the
+// attention's (behind its softmax) and the carve-outs that let CTAs share an SM: loop of 50 tokens on 768 keys 4.82 -> 4.62 ms,
+// NVFP4 5.95 -> 5.82, guided 5.98 -> 5.93.
+//
 // Warps: 0 (lane 0) TMA producer, 1 (lane 0) MMA issuer, 2 TMEM owner; all 8 warps stage and finish the tile.
 // Every wait is bounded by the kernel deadline; on expiry the status word is set, the work is skipped and every
 // thread still reaches the cluster barriers and the TMEM release.
@@ -112,7 +119,8 @@ struct TokParams {
     };
     float eps;
     int w_kn;                  // weights stored (K, N) row-major (the MN-major B operand) instead of (N, K)
-    int early;                 // weights and style may be read before the kernel in front has finished
+    int early;                 // bit 0: weights and style may be read before the kernel in front has finished; bit 1: the kernel behind
+                               // may start from the beginning
     // Deferred row scale (TOK_PRO_TMA with TOK_EPI_ROPE / TOK_EPI_GEGLU, active when stats_in != NULL): the A operand
     // holds e4m3(x * (1 + scale)) WITHOUT the 1 / rms factor; the finish applies it per token and adds the column
     // term:  y[m][n] = bf16(alpha * acc[m][n] * rms[m] + col_term[n]),  rms from stats_in / n_stat / K / eps as above,
@@ -290,8 +298,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     cluster_arrive_release();
     TOK_STAMP(1);
 
-    pdl_launch_dependents();
-    if (!p.early) pdl_wait();
+    if (p.early & 2) pdl_launch_dependents();
+    if (!(p.early & 1)) pdl_wait();
 
     if (warp == 0) {
         // ---------------- TMA producer (whole warp, see warp_wait): the weights do not depend on the producer grid and start
@@ -514,6 +522,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     TOK_STAMP(2);
     pdl_wait();
     TOK_STAMP(3);
+    if (EPI == TOK_EPI_GEGLU) pdl_launch_dependents();
     constexpr int G = (EPI == TOK_EPI_GEGLU) ? BN / 16 : BN / 8;      // 8-feature groups per token that carry output
     const int items = ntok * G;
     const int items_pad = (items + 31) & ~31;                         // whole warps iterate together (shuffles below)
@@ -585,6 +594,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     __syncwarp();
     tc::tc_fence_after_sync();
     TOK_STAMP(4);
+    if (EPI == TOK_EPI_ROPE || EPI == TOK_EPI_RESID) pdl_launch_dependents();
     cluster_wait_acquire();          // every peer has initialised its receive barrier (arrived during its set-up)
     {
         const int quad = warp & 3, chalf = warp >> 2;
@@ -616,6 +626,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
     }
     TOK_STAMP(5);
+    if (EPI == TOK_EPI_BF16) pdl_launch_dependents();
     __syncthreads();                     // the own slot (and s_rms) of this rank's tokens is complete
     // ---------------- the peers' slots of this rank's tokens have landed
     const bool got = tc::mbar_wait_until(recv_bar, 0, deadline, abort_flag);
@@ -928,6 +939,10 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     if (attr_once.need(attr_dev)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TOK_MAX_SMEM);
         if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        if (EPI == TOK_EPI_GEGLU) {
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return FRT_CUDA_ERR(e);
+        }
         attr_once.set(attr_dev);
     }
     CUtensorMap tmA, tmW;
@@ -957,7 +972,9 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    p.early = pdl ? 1 : 0;
+    // more CTAs than the device holds: those that wait for a place keep the kernel behind out anyway (4 x 50 tokens, 320 CTAs of the QKV
+    // product: the loop 7.57 ms, let in late 7.64)
+    p.early = (pdl ? 1 : 0) | ((long long)tiles * m_tiles * pl.S > 2 * device_sm_count() ? 2 : 0);
     cfg.attrs = attr;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmW, p);
