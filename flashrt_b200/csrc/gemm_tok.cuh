@@ -184,35 +184,37 @@ __device__ __forceinline__ int2 tok_batch_row(int m, const TokParams& p) {
     return make_int2(b, m - b * p.rows_per_batch);
 }
 
-// Sum over the S slots (fixed order) of the 8 received fp32 values of (token t of this rank, columns c8*8 .. +7).
-template <int BN>
-__device__ __forceinline__ void tok_sum8(const float* recv, int S, int per, int pad, int t, int c8, float* a) {
-    const float4* row = reinterpret_cast<const float4*>(recv + (size_t)t * (BN + pad));
-    const int c0 = 2 * c8, c1 = 2 * c8 + 1;
+// Sum over the S slots (fixed order) of the VW received fp32 values of (token t of this rank, columns cv*VW .. +VW-1).
+template <int BN, int VW = 8>
+__device__ __forceinline__ void tok_sum(const float* recv, int S, int per, int pad, int t, int cv, float* a) {
+    constexpr int Q = VW / 4;
+    const float4* row = reinterpret_cast<const float4*>(recv + (size_t)t * (BN + pad)) + Q * cv;
     const size_t slot = (size_t)per * (BN + pad) / 4;
     // S is 1, 2, 4 or 8: the loads of four slots in flight at a time, the sums in slot order
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = 0.0f;
+    for (int j = 0; j < VW; ++j) a[j] = 0.0f;
 #pragma unroll
     for (int s0 = 0; s0 < 8; s0 += 4) {
         if (s0 < S) {
-            float4 x[4], y[4];
+            float4 x[4][Q];
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 if (s0 + s < S) {
-                    x[s] = row[(s0 + s) * slot + c0];
-                    y[s] = row[(s0 + s) * slot + c1];
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) x[s][q] = row[(s0 + s) * slot + q];
                 }
             }
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 if (s0 + s < S) {
-                    if (s0 + s == 0) {
-                        a[0] = x[s].x; a[1] = x[s].y; a[2] = x[s].z; a[3] = x[s].w;
-                        a[4] = y[s].x; a[5] = y[s].y; a[6] = y[s].z; a[7] = y[s].w;
-                    } else {
-                        a[0] += x[s].x; a[1] += x[s].y; a[2] += x[s].z; a[3] += x[s].w;
-                        a[4] += y[s].x; a[5] += y[s].y; a[6] += y[s].z; a[7] += y[s].w;
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        float* d = a + 4 * q;
+                        if (s0 + s == 0) {
+                            d[0] = x[s][q].x; d[1] = x[s][q].y; d[2] = x[s][q].z; d[3] = x[s][q].w;
+                        } else {
+                            d[0] += x[s][q].x; d[1] += x[s][q].y; d[2] += x[s][q].z; d[3] += x[s][q].w;
+                        }
                     }
                 }
             }
@@ -220,7 +222,19 @@ __device__ __forceinline__ void tok_sum8(const float* recv, int S, int per, int 
     }
 }
 
-// ACT (GeGLU epilogue only): the gate activation, 0 exact GELU(tanh), 1 SiLU, 2 GELU through the hardware tanh.  A
+// VW neighbouring bf16 values
+template <int VW>
+struct alignas(2 * VW) TokVec {
+    uint32_t w[VW / 2];
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { *this = *reinterpret_cast<const TokVec*>(p); }
+    __device__ __forceinline__ void store(__nv_bfloat16* p) const { *reinterpret_cast<TokVec*>(p) = *this; }
+};
+
+// ACT, gated residual: 1 = items of four features instead of eight.  A rank of eight splits finishes few tokens (7 of 50), whose items
+// of eight are the work of two warps with six idle, and the finish takes as long as an item's code: attention-out 0.75 -> 0.5 us from
+// the last slot to the result, the loop of 50 tokens on 768 keys 4.66 -> 4.60 ms; with 25 tokens of a rank it is two rounds instead of
+// one (4 x 50 tokens 7.54 -> 7.59).
+// ACT, GeGLU: the gate activation, 0 exact GELU(tanh), 1 SiLU, 2 GELU through the hardware tanh.  A
 // template argument, not a field of the parameters: selected at run time inside the unrolled finish the choice cost
 // 0.55 us per gate|up launch of the action-expert loop (0.10 ms per loop), a third of that epilogue's arithmetic.
 template <int BN, int PRO, int EPI, int ACT = 0, bool FP4 = false>
@@ -523,7 +537,9 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     pdl_wait();
     TOK_STAMP(3);
     if (EPI == TOK_EPI_GEGLU) pdl_launch_dependents();
-    constexpr int G = (EPI == TOK_EPI_GEGLU) ? BN / 16 : BN / 8;      // 8-feature groups per token that carry output
+    // features of an item: eight, one 16-byte store; four in the narrow form of the gated residual
+    constexpr int VW = EPI == TOK_EPI_RESID && ACT == 1 ? 4 : 8;
+    constexpr int G = (EPI == TOK_EPI_GEGLU) ? BN / 16 : BN / VW;     // groups per token that carry output
     const int items = ntok * G;
     const int items_pad = (items + 31) & ~31;                         // whole warps iterate together (shuffles below)
     float alpha = p.alpha_host;
@@ -531,8 +547,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (p.sb) alpha *= *p.sb;
     const float inv_os = (EPI == TOK_EPI_GEGLU) ? __fdiv_rn(1.0f, *p.out_scale) : 0.0f;
     const int pos = (EPI == TOK_EPI_ROPE && p.devpos) ? *p.devpos : 0;
-    uint4 pre0 = make_uint4(0, 0, 0, 0), pre1 = make_uint4(0, 0, 0, 0);   // first item's operands
-    uint4 pre2 = make_uint4(0, 0, 0, 0);
+    uint4 pre0 = make_uint4(0, 0, 0, 0);                                   // first item's operands
+    TokVec<VW> res0 = {}, res1 = {}, res2 = {};
     float4 ct0 = make_float4(0.f, 0.f, 0.f, 0.f), ct1 = ct0, ct2 = ct0, ct3 = ct0;   // first item's column terms
     const bool rowscale = PRO == TOK_PRO_TMA && (EPI == TOK_EPI_ROPE || EPI == TOK_EPI_GEGLU) && p.stats_in != nullptr;
     const bool emit_q8 = EPI == TOK_EPI_RESID && p.q8_out != nullptr;
@@ -556,7 +572,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     {
         const int it = threadIdx.x;
         if (it < items) {
-            const int m = m0 + tb + it / G, n = n0 + (it % G) * 8;
+            const int m = m0 + tb + it / G, n = n0 + (it % G) * VW;
             if (rowscale) {
                 if (EPI == TOK_EPI_GEGLU) {
                     if (n < p.half) {
@@ -571,9 +587,9 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             }
             if (EPI == TOK_EPI_RESID && n < p.N) {
-                pre0 = ld_global_v4(p.resid + (size_t)m * p.N + n);
-                pre1 = ld_global_v4(p.gate + n);
-                if (emit_q8) pre2 = ld_global_v4(p.q8_mod + n);
+                res0.load(p.resid + (size_t)m * p.N + n);
+                res1.load(p.gate + n);
+                if (emit_q8) res2.load(p.q8_mod + n);
             } else if (EPI == TOK_EPI_ROPE && n < p.q_dim + p.k_dim) {
                 const int nr = n < p.q_dim ? n : n - p.q_dim;
                 pre0 = ld_global_v4(p.rope + (size_t)tok_batch_row(m, p).y * p.head_dim + rope_col(nr, p.head_dim));
@@ -646,12 +662,12 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const int g = it % G;
             const int m = m0 + tb + t;
             const bool first = it < 256;
-            float a[8];
+            float a[VW];
             if (act) {
-                tok_sum8<BN>(recv, S, per, p.row_pad, t, g, a);
+                tok_sum<BN, VW>(recv, S, per, p.row_pad, t, g, a);
             } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) a[j] = 0.0f;
+                for (int j = 0; j < VW; ++j) a[j] = 0.0f;
             }
             if (EPI == TOK_EPI_BF16) {
                 const int n = n0 + g * 8;
@@ -735,7 +751,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const int h = n0 + g * 8;
                 if (act && h < p.half) {
                     float b[8];
-                    tok_sum8<BN>(recv, S, per, p.row_pad, t, G + g, b);
+                    tok_sum<BN>(recv, S, per, p.row_pad, t, G + g, b);
                     float q[8];
                     if (rowscale) {
                         float4 c0 = ct0, c1 = ct1, c2 = ct2, c3 = ct3;
@@ -774,55 +790,58 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
             } else {
                 // gated residual: x <- bf16(x + bf16(o) * gate); sum of squares of the UNROUNDED update per (tile, token)
-                const int n = n0 + g * 8;
-                float ssq = 0.0f;
+                const int n = n0 + g * VW;
+                float ssq = 0.0f, x[VW];
+#pragma unroll
+                for (int j = 0; j < VW; ++j) x[j] = 0.0f;      // the updated residual, unrounded
                 if (act && n < p.N) {
                     __nv_bfloat16* rp = p.resid + (size_t)m * p.N + n;
-                    uint4 rv = pre0, gv = pre1, mv = pre2;
+                    TokVec<VW> rv = res0, gv = res1, mv = res2, ob;
                     if (!first) {
-                        rv = ld_global_v4(rp);
-                        gv = ld_global_v4(p.gate + n);
-                        if (emit_q8) mv = ld_global_v4(p.q8_mod + n);
+                        rv.load(rp);
+                        gv.load(p.gate + n);
+                        if (emit_q8) mv.load(p.q8_mod + n);
                     }
-                    const uint32_t* mw = &mv.x;
-                    float u[8];
-                    const uint32_t* rw = &rv.x;
-                    const uint32_t* gw = &gv.x;
-                    uint4 ob;
-                    uint32_t* ow = &ob.x;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int k = 0; k < VW / 2; ++k) {
                         float r0, r1, g0, g1;
-                        unpack_bf16x2(rw[k], r0, r1);
-                        unpack_bf16x2(gw[k], g0, g1);
+                        unpack_bf16x2(rv.w[k], r0, r1);
+                        unpack_bf16x2(gv.w[k], g0, g1);
                         const float o0 = bf16_round(a[2 * k] * alpha);
                         const float o1 = bf16_round(a[2 * k + 1] * alpha);
-                        r0 = __fmaf_rn(o0, g0, r0);
-                        r1 = __fmaf_rn(o1, g1, r1);
-                        ssq = __fmaf_rn(r0, r0, ssq);
-                        ssq = __fmaf_rn(r1, r1, ssq);
-                        ow[k] = pack_bf16x2(r0, r1);
+                        x[2 * k] = __fmaf_rn(o0, g0, r0);
+                        x[2 * k + 1] = __fmaf_rn(o1, g1, r1);
+                        ob.w[k] = pack_bf16x2(x[2 * k], x[2 * k + 1]);
                     }
-                    st_global_v4(rp, ob);
+                    ob.store(rp);
                     if (emit_q8) {
+                        float u[VW];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
+                        for (int k = 0; k < VW / 2; ++k) {
                             float b0, b1, s0, s1;
-                            unpack_bf16x2(ow[k], b0, b1);          // what the next reader of the residual sees
-                            unpack_bf16x2(mw[k], s0, s1);
+                            unpack_bf16x2(ob.w[k], b0, b1);        // what the next reader of the residual sees
+                            unpack_bf16x2(mv.w[k], s0, s1);
                             u[2 * k] = clamp448(__fmul_rn(__fmul_rn(b0, __fadd_rn(1.0f, s0)), inv_q8));
                             u[2 * k + 1] = clamp448(__fmul_rn(__fmul_rn(b1, __fadd_rn(1.0f, s1)), inv_q8));
                         }
-                        uint2 o8;
-                        o8.x = f32x4_to_e4m3x4(u[0], u[1], u[2], u[3]);
-                        o8.y = f32x4_to_e4m3x4(u[4], u[5], u[6], u[7]);
-                        st_global_v2(p.q8_out + (size_t)m * p.N + n, o8);
+                        uint8_t* q8 = p.q8_out + (size_t)m * p.N + n;
+                        const uint32_t lo = f32x4_to_e4m3x4(u[0], u[1], u[2], u[3]);
+                        if constexpr (VW == 8) st_global_v2(q8, make_uint2(lo, f32x4_to_e4m3x4(u[4], u[5], u[6], u[7])));
+                        else *reinterpret_cast<uint32_t*>(q8) = lo;
                     }
                 }
-                // the G lanes of a token are neighbours (G divides 32): butterfly inside the group, fixed order
+                // the G lanes of a token are neighbours (G divides 32): chains over eight features (of four: the odd lane goes on where its
+                // neighbour ends), then a butterfly over them, in the same order in both forms
 #pragma unroll
-                for (int off = G / 2; off >= 1; off >>= 1) ssq = __fadd_rn(ssq, __shfl_xor_sync(0xffffffffu, ssq, off));
-                if (act && g == 0 && p.stats_out) p.stats_out[tile * p.stat_stride + m] = ssq;
+                for (int j = 0; j < VW; ++j) ssq = __fmaf_rn(x[j], x[j], ssq);
+                if constexpr (VW == 4) {
+                    ssq = __shfl_xor_sync(0xffffffffu, ssq, 1);
+#pragma unroll
+                    for (int j = 0; j < VW; ++j) ssq = __fmaf_rn(x[j], x[j], ssq);      // right on the odd lanes
+                }
+#pragma unroll
+                for (int off = G / 2; off >= 8 / VW; off >>= 1) ssq = __fadd_rn(ssq, __shfl_xor_sync(0xffffffffu, ssq, off));
+                if (act && g == 8 / VW - 1 && p.stats_out) p.stats_out[tile * p.stat_stride + m] = ssq;
             }
         }
     }
