@@ -1333,6 +1333,15 @@ int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const 
     cudaStream_t s = (cudaStream_t)stream;
     bool pdl = flags & 1;
     p.early = pdl ? 1 : 0;
+    if (pdl && splits <= 0 && !(flags & (2 | 0x300))) {
+        const TokPlan pl = pick_tok_nvfp4_rows(M, N, K);
+        if (pl.S) {
+            TokParams t = {};
+            t.M = M; t.N = N; t.sa = p.sa; t.alpha_host = alpha;
+            t.out = p.out; t.bias = p.bias; t.sf_a = p.sf_lane; t.sf_w = p.sf_col;
+            return launch_gemm_tok<64, TOK_PRO_TMA, TOK_EPI_BF16, 0, true>(A, W, t, K, pl, pdl, s);
+        }
+    }
     int pair = 0;
     if (splits <= 1 && !(flags & 2)) {
         pair = ((flags >> 8) & 3) ? 64 + 64 * ((flags >> 8) & 3) : pick_nvfp4_pair(M, N, K);

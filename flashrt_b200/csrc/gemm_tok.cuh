@@ -136,9 +136,10 @@ struct TokParams {
 #endif
 };
 
-// FP4 (BF16 and RoPE finishes, at most 64 tokens): k-blocks of 256 packed e2m1 elements, the scale atoms of both operands behind the
-// operand tiles.  The block-scaled MMA has M = 128 only: with at most 64 tokens its upper 64 lanes read the weight tile behind the
-// 8 KB of tokens and their results are never looked at.
+// FP4 (BF16 and RoPE finishes, m-tiles of 64 tokens): k-blocks of 256 packed e2m1 elements, the scale atoms of both operands behind the
+// operand tiles.  The block-scaled MMA has M = 128 only, and an atom holds the scales of 128 rows: an even m-tile is the lower 64 rows of
+// the operand and the weight tile behind its 8 KB the upper, an odd one the upper 64 rows and the weight tile, in front of it there, the
+// lower.  The results of those lanes are never looked at; every row that an MMA reads lies in its stage.
 template <int BN, bool FP4 = false>
 struct TokCfg {
     static_assert(!FP4 || BN <= 128, "NVFP4: one atom row of column scales");
@@ -278,6 +279,8 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int per = p.per;
     const bool m64 = p.m64 != 0;
     const int A_BYTES = Cfg::a_bytes(m64), STAGE_BYTES = Cfg::stage_bytes(m64);
+    const int odd = FP4 ? (m0 >> 6) & 1 : 0;                        // the upper 64 rows of a group of 128
+    const int A_OFF = odd ? Cfg::W_BYTES : 0, W_OFF = odd ? 0 : A_BYTES, SF_OFF = A_BYTES + Cfg::W_BYTES;   // places in a stage
     // tokens this rank finishes: [tb, te) inside the m-tile
     const int tb = rank * per < Mt ? rank * per : Mt;
     const int te = tb + per < Mt ? tb + per : Mt;
@@ -321,7 +324,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const uint32_t tx = (PRO == TOK_PRO_TMA) ? STAGE_BYTES : Cfg::W_BYTES;
         const uint32_t ring = tc::smem_u32(tiles), full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty);
         auto load_w = [&](int stage, int kb) {
-            const uint32_t dst = ring + stage * STAGE_BYTES + A_BYTES, bar = full_a + 8 * stage;
+            const uint32_t dst = ring + stage * STAGE_BYTES + W_OFF, bar = full_a + 8 * stage;
             if (p.w_kn) {
                 // (K, N) weights: boxes of 128 K-rows x 128 N-bytes, one per 128 output features; the tile is then an
                 // MN-major operand (128-byte rows along N, 8 K-rows per swizzle atom, 16 KB between the chunks)
@@ -337,13 +340,14 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 tc::tma_load_2d(dst, &tmW, bar, kb * 128, n0);
             }
             if constexpr (FP4)
-                tc::bulk_load(dst + Cfg::W_BYTES + Cfg::SF_BYTES, p.sf_w + ((size_t)(n0 / 128) * (p.K >> 6) + (size_t)kb * 4) * 512,
+                tc::bulk_load(ring + stage * STAGE_BYTES + SF_OFF + Cfg::SF_BYTES, p.sf_w + ((size_t)(n0 / 128) * (p.K >> 6) + (size_t)kb * 4) * 512,
                               2048, bar);
         };
         auto load_a = [&](int stage, int kb) {
-            const uint32_t dst = ring + stage * STAGE_BYTES, bar = full_a + 8 * stage;
+            const uint32_t dst = ring + stage * STAGE_BYTES + A_OFF, bar = full_a + 8 * stage;
             tc::tma_load_2d(dst, &tmA, bar, kb * 128, m0);
-            if constexpr (FP4) tc::bulk_load(dst + A_BYTES + Cfg::W_BYTES, p.sf_a + (size_t)kb * 4 * 512, 2048, bar);
+            if constexpr (FP4)
+                tc::bulk_load(ring + stage * STAGE_BYTES + SF_OFF, p.sf_a + ((size_t)(m0 >> 7) * (p.K >> 6) + (size_t)kb * 4) * 512, 2048, bar);
         };
         const int pre = nkb < STG ? nkb : STG;
         if (tc::elect_one()) {
@@ -476,13 +480,13 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         // scales in tensor memory: four columns per K = 64 step; a tile of 64 weight rows may start at row 64 of its atom
         const uint32_t tmem_sfa = tmem_d + BN, tmem_sfw = tmem_sfa + 16;
         const uint32_t sfw_off = FP4 ? (uint32_t)((n0 & 127) >> 5) : 0u;
-        const uint32_t sf0 = tc::smem_u32(tiles) + A_BYTES + Cfg::W_BYTES;
+        const uint32_t sf0 = tc::smem_u32(tiles) + SF_OFF;
         bool failed = false;
         if (PRO == TOK_PRO_NORM) failed = !tc::warp_wait(tc::smem_u32(a_ready), 0, false, deadline, abort_flag);
         const uint32_t full_a = tc::smem_u32(full), empty_a = tc::smem_u32(empty), accum_a = tc::smem_u32(accum_bar);
-        const uint64_t dA0 = tc::make_desc_kmajor_sw128(tc::smem_u32(tiles));
-        const uint64_t dW0 = p.w_kn ? tc::make_desc_mnmajor_sw128(tc::smem_u32(tiles + A_BYTES), 16384)
-                                    : tc::make_desc_kmajor_sw128(tc::smem_u32(tiles + A_BYTES));
+        const uint64_t dA0 = tc::make_desc_kmajor_sw128(tc::smem_u32(tiles + A_OFF - odd * 8192));
+        const uint64_t dW0 = p.w_kn ? tc::make_desc_mnmajor_sw128(tc::smem_u32(tiles + W_OFF), 16384)
+                                    : tc::make_desc_kmajor_sw128(tc::smem_u32(tiles + W_OFF));
         // one K = 32 step: 32 bytes along a K-major row, or 32 rows of 128 bytes of an MN-major tile
         const uint64_t wstep = p.w_kn ? (uint64_t)((32 * 128) >> 4) : 2u;
         int s = 0;
@@ -615,8 +619,9 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     {
         const int quad = warp & 3, chalf = warp >> 2;
         const int qrows = m64 && !FP4 ? 16 : 32;               // accumulator rows per 32-lane quadrant
-        const int row = lane < qrows ? quad * qrows + lane : Mt;   // token inside the m-tile (none on the idle lanes)
-        if (have_acc && quad * qrows < Mt) {
+        const int q0 = (quad - 2 * odd) * qrows;               // first token of the quadrant
+        const int row = lane < qrows ? q0 + lane : Mt;         // token inside the m-tile (none on the idle lanes)
+        if (have_acc && q0 >= 0 && q0 < Mt) {
             const uint32_t trow = tmem_d + ((uint32_t)(quad * 32) << 16);
             const int rq = (row * p.per_magic) >> 16;           // row / per
             const int owner = rq < S ? rq : 0;
@@ -928,7 +933,8 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     auto kern = gemm_tok_kernel<BN, PRO, EPI, ACT, FP4>;
     const uint64_t row_bytes = FP4 ? (uint64_t)K / 2 : (uint64_t)K;
     const int m_tiles = pl.m_tiles;
-    const int mt = (p.M + m_tiles - 1) / m_tiles;             // rows spread evenly over the m-tiles
+    // rows spread evenly over the m-tiles; of NVFP4 operands 64 each, which their scale atoms' 128 hold
+    const int mt = FP4 && m_tiles > 1 ? 64 : (p.M + m_tiles - 1) / m_tiles;
     p.m_rows = mt;
     p.stat_stride = tok_stat_stride(p.M);
     if (p.rows_per_batch <= 0) p.rows_per_batch = p.M;
@@ -1072,6 +1078,19 @@ static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
         }
     }
     return best;
+}
+
+// 65 to 256 rows in a chain: m-tiles of 64, tiles of 64 weight rows, the largest split with a CTA per SM (its k-blocks all in the ring).
+// On CTA pairs a product of N = 1024 is 8 tiles, 16 CTAs, each with the whole of K: loops of 2 x 50 on 768 keys 8.56 -> 7.73 ms, 3 x 50
+// on 400 8.53 -> 8.12, 4 x 20 on 200 7.65 -> 6.95, 4 x 50 on 768 9.11 -> 8.83.  What has more tiles than SMs stays on the pairs (QKV of
+// 200 rows, gate|up).
+static TokPlan pick_tok_nvfp4_rows(int M, int N, int K) {
+    const TokPlan none = {0, 0, 0, 0, 1};
+    const int kbt = K / 256, sms = device_sm_count(), m_tiles = (M + 63) / 64, tiles = (N + 63) / 64 * m_tiles;
+    if ((N & 7) || M <= 64 || M > 256) return none;
+    for (int S = 4; S >= 1; S /= 2)
+        if (kbt % S == 0 && kbt / S <= 8 && tiles * S <= sms) return {64, S, kbt / S, kbt / S, m_tiles};
+    return none;
 }
 
 static int tok_sm_count() {

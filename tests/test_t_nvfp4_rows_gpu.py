@@ -1,0 +1,25 @@
+"""NVFP4 products of 65 to 256 rows in a chain of launches (weights fetched early): m-tiles of 64 rows on the token-major kernel, odd ones
+on the upper half of the operand and of the scale atoms; a last tile of one row, of weight rows that end inside a tile, every split,
+and shapes that stay with the other kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from oracle import oracle as O  # noqa: E402
+from test_h_nvfp4_gpu import _check, _operand  # noqa: E402
+
+
+@pytest.mark.parametrize("M", [65, 100, 128, 129, 193, 256])
+@pytest.mark.parametrize("N,K", [(1024, 2048), (1024, 4096), (72, 256), (1000, 1792), (2560, 1024), (1024, 14336)])
+def test_rows_in_a_chain(M, N, K):
+    from flashrt_b200 import _lib, flash_rt_kernels as fvk
+    from gpu_util import Dev, zeros
+    rng = np.random.default_rng(M + N + K)
+    Ap, Asf = _operand(rng, M, K, 1.0)
+    Wp, Wsf = _operand(rng, N, K, 0.02)
+    bias = O.f32_to_bf16_bits((rng.standard_normal(N) * 0.1).astype(np.float32))
+    d, d_b, d_o = [Dev(Ap), Dev(Asf), Dev(Wp), Dev(Wsf)], Dev(bias), zeros((M, N), np.uint16)
+    _lib.call("frt_b200_gemm_nvfp4_nt", d[0].ptr, d[1].ptr, d[2].ptr, d[3].ptr, d_o.ptr, M, N, K, 1.0, None, d_b.ptr, 0, 1, 0)
+    assert fvk.tensor_core_status() == 0
+    _check(d_o.get(), O.gemm_nvfp4(Ap, Asf, Wp, Wsf, bias=bias, want_f32=True))
