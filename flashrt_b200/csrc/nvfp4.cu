@@ -65,6 +65,44 @@ quantize_nvfp4_kernel(const __nv_bfloat16* in, uint8_t* __restrict__ packed, uin
     }
 }
 
+// The same with four lanes per block of 16, while they all fit the device at once: what bounds a few rows is the chain behind the kernel
+// in front, so a lane has four values, and its place is computed before the wait (a 64-bit division per thread stood behind it).
+template <int FAMILY>
+__global__ void __launch_bounds__(256)
+quantize_nvfp4_lanes_kernel(const __nv_bfloat16* in, uint8_t* __restrict__ packed, uint8_t* __restrict__ sf,
+                            unsigned rows, unsigned D, const float* d_global) {
+    const unsigned nquad = D >> 2;
+    const unsigned idx = blockIdx.x * 256 + threadIdx.x;
+    const unsigned row = idx / nquad, quad = idx - row * nquad;
+    const bool live = row < rows;                     // the four lanes of a block agree
+    const size_t off = (size_t)row * D + quad * 4;
+    uint8_t* sfp = sf + nvfp4::sf_offset(row, quad >> 2, (D + 63) >> 6);
+    pdl_launch_dependents();
+    pdl_wait();
+    uint2 a = make_uint2(0, 0);
+    if (live) a = *reinterpret_cast<const uint2*>(in + off);
+    float v[4], amax = 0.0f;
+    unpack_bf16x2(a.x, v[0], v[1]);
+    unpack_bf16x2(a.y, v[2], v[3]);
+    if (d_global) {
+        const float inv_g = __fdiv_rn(1.0f, *d_global);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(v[i], inv_g);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    float s;
+    const uint32_t sb = nvfp4::block_scale<FAMILY>(amax, s);
+    const float inv = nvfp4::inverse<FAMILY>(s);
+    const uint16_t o = d_global ? nvfp4::pack4<FAMILY>(v, inv)
+                                : nvfp4::pack4_bf16<FAMILY>(v, s, nvfp4::inv_off_ties<FAMILY>(inv, s));
+    if (!live) return;
+    *reinterpret_cast<uint16_t*>(packed + (off >> 1)) = o;
+    if ((quad & 3) == 0) *sfp = (uint8_t)sb;
+}
+
 template <int FAMILY>
 __global__ void __launch_bounds__(256)
 geglu_nvfp4_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ packed, uint8_t* __restrict__ sf,
@@ -110,11 +148,11 @@ geglu_nvfp4_lanes_kernel(const __nv_bfloat16* merged, uint8_t* __restrict__ pack
                          int rows, int H) {
     const int nquad = H >> 2;
     const int katoms = (H + 63) >> 6;
-    pdl_launch_dependents();
-    pdl_wait();
     const int idx = blockIdx.x * 256 + threadIdx.x;
     const int row = idx / nquad, quad = idx - row * nquad;
     const bool live = row < rows;                     // the four lanes of a block agree
+    pdl_launch_dependents();
+    pdl_wait();
     uint2 gv = make_uint2(0, 0), uv = gv;
     if (live) {
         const __nv_bfloat16* g = merged + (size_t)row * 2 * H + quad * 4;
@@ -182,6 +220,13 @@ int frt_b200_quantize_nvfp4(const void* in, void* packed, void* sf, long long ro
     if (family != 0 && family != 1) return FRT_ERR_INVALID;
     if (rows == 0) return FRT_OK;
     const long long work = rows * (D / 16);
+    if (work * 4 <= (long long)device_sm_count() * 2048) {
+        if (family == 0)
+            return launch_1d(quantize_nvfp4_lanes_kernel<0>, work * 4, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+                             (uint8_t*)packed, (uint8_t*)sf, (unsigned)rows, (unsigned)D, d_global_scale);
+        return launch_1d(quantize_nvfp4_lanes_kernel<1>, work * 4, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+                         (uint8_t*)packed, (uint8_t*)sf, (unsigned)rows, (unsigned)D, d_global_scale);
+    }
     if (family == 0)
         return launch_1d(quantize_nvfp4_kernel<0>, work, (cudaStream_t)stream, (const __nv_bfloat16*)in,
                          (uint8_t*)packed, (uint8_t*)sf, rows, D, d_global_scale);

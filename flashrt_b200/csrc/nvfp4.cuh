@@ -136,11 +136,7 @@ __device__ __forceinline__ uint32_t pack8(const float* v, float inv) {
     return cvt8(x);
 }
 // four values -> two bytes
-template <int FAMILY>
-__device__ __forceinline__ uint16_t pack4(const float* v, float inv) {
-    float x[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = e2m1_off_tie<FAMILY>(__fmaf_rn(v[i], inv, 0.0f));
+__device__ __forceinline__ uint16_t cvt4(const float* x) {
     uint16_t w;
     asm("{\n\t.reg .b8 b0, b1;\n\t"
         "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
@@ -150,6 +146,13 @@ __device__ __forceinline__ uint16_t pack4(const float* v, float inv) {
         : "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]));
     return w;
 }
+template <int FAMILY>
+__device__ __forceinline__ uint16_t pack4(const float* v, float inv) {
+    float x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = e2m1_off_tie<FAMILY>(__fmaf_rn(v[i], inv, 0.0f));
+    return cvt4(x);
+}
 // bf16 values of a block with scale s; inv from inv_off_ties
 template <int FAMILY>
 __device__ __forceinline__ uint32_t pack8_bf16(const float* v, float s, float2 inv) {
@@ -158,6 +161,15 @@ __device__ __forceinline__ uint32_t pack8_bf16(const float* v, float s, float2 i
     for (int i = 0; i < 8; ++i)
         x[i] = __fmaf_rn(v[i], FAMILY == 0 ? inv.x : (fabsf(v[i]) < s ? inv.x : inv.y), 0.0f);
     return cvt8(x);
+}
+
+template <int FAMILY>
+__device__ __forceinline__ uint16_t pack4_bf16(const float* v, float s, float2 inv) {
+    float x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        x[i] = __fmaf_rn(v[i], FAMILY == 0 ? inv.x : (fabsf(v[i]) < s ? inv.x : inv.y), 0.0f);
+    return cvt4(x);
 }
 
 }  // namespace nvfp4
