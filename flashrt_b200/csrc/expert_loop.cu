@@ -30,7 +30,7 @@
 // replays are bit-reproducible.  The residual row of token r never leaves the registers of CTA r.
 //
 // Measured (18 blocks x 10 steps, 50 tokens, 768 prefix keys): 10.5 ms per loop; the graph of operator launches took 9.75 ms
-// as 1300 launches and takes 5.03 ms as 912, i.e. a phase costs what a launch costs (barrier 1.1-1.4 us + one L2 round trip for the operand
+// as 1300 launches and takes 4.48 ms as 912, i.e. a phase costs what a launch costs (barrier 1.1-1.4 us + one L2 round trip for the operand
 // 1.5 us + 32 MMAs 2 us + epilogue).
 //
 // Warps: 0 = weight TMA producer, 1 = MMA issuer (one thread), 2-9 = workers (operand loads, softmax, epilogues,
