@@ -398,7 +398,8 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
         const uint32_t xc_slot = ((uint32_t)rows_valid * ((uint32_t)(DV / (int)C) * 2u + 4u) + 15u) & ~15u;
         const uint32_t xc_lse = (uint32_t)rows_valid * (uint32_t)(DV / (int)C) * 2u;
         if constexpr (XC) {
-            // the row's log-sum-exp, once to every split, under the last P.V
+            // the row's log-sum-exp, once to every split, under the last P.V (the aligned barrier wants the warp together again)
+            __syncwarp();
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (alive && row < rows_valid) {
                 uint8_t* recv = smem + Cfg::OFF_RECV(DQ);
