@@ -1333,7 +1333,8 @@ int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const 
     cudaStream_t s = (cudaStream_t)stream;
     bool pdl = flags & 1;
     p.early = pdl ? 1 : 0;
-    if (pdl && splits <= 0 && !(flags & (2 | 0x300))) {
+    // asked for (bit 2), not taken from bit 0: that bit may not change the order of the sums above 64 rows
+    if ((flags & 4) && splits <= 0 && !(flags & (2 | 0x300))) {
         const TokPlan pl = pick_tok_nvfp4_rows(M, N, K);
         if (pl.S) {
             TokParams t = {};
@@ -1386,7 +1387,7 @@ int frt_b200_gemm_nvfp4_nt_rope_split(const void* A, const void* SFA, const void
     p.k_dim = k_dim;
     p.v_dim = v_dim;
     p.head_dim = head_dim;
-    // on CTA pairs where the plain product goes there: the same sums, so the pair of launches gives the same bytes
+    // on CTA pairs where the plain product goes there (without its bit 2): the same sums, so the pair of launches gives the same bytes
     const uintptr_t ptrs = reinterpret_cast<uintptr_t>(rope) | reinterpret_cast<uintptr_t>(Q) |
                            reinterpret_cast<uintptr_t>(Kout) | reinterpret_cast<uintptr_t>(Vout);
     if (splits <= 0 && !(ptrs & 15) && !((q_dim | k_dim | v_dim | head_dim) & 7) && pick_nvfp4_pair(M, p.N, K)) {

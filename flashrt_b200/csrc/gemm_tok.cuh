@@ -1080,7 +1080,7 @@ static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     return best;
 }
 
-// 65 to 256 rows in a chain: m-tiles of 64, tiles of 64 weight rows, the largest split with a CTA per SM (its k-blocks all in the ring).
+// 65 to 256 rows in a chain, where the caller asks for it: m-tiles of 64, tiles of 64 weight rows, the largest split with a CTA per SM (its k-blocks all in the ring).
 // On CTA pairs a product of N = 1024 is 8 tiles, 16 CTAs, each with the whole of K: loops of 2 x 50 on 768 keys 8.56 -> 7.73 ms, 3 x 50
 // on 400 8.53 -> 8.12, 4 x 20 on 200 7.65 -> 6.95, 4 x 50 on 768 9.11 -> 8.83.  What has more tiles than SMs stays on the pairs (QKV of
 // 200 rows, gate|up).

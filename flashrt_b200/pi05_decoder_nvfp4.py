@@ -85,9 +85,10 @@ class Pi05DecoderNvfp4Pipeline(StepIO):
         row = t[step] if layer is None else t[step, layer]
         return row.data_ptr()
 
-    def _gemm(self, a4, a_sf, w: Nvfp4Weight, out, stream, pdl):
+    def _gemm(self, a4, a_sf, w: Nvfp4Weight, out, stream, pdl, chain=True):
         rc = fp4.cutlass_fp4_gemm_variant(0, a4.data_ptr(), a_sf.data_ptr(), w.packed.data_ptr(), w.sf.data_ptr(),
-                                          out.data_ptr(), self.M, w.N, w.K, w.g, 0.0, stream, pdl=pdl)
+                                          out.data_ptr(), self.M, w.N, w.K, w.g, 0.0, stream, pdl=pdl,
+                                          chain=chain)
         if rc != 0:
             raise fvk.KernelError(f"NVFP4 GEMM ({self.M}, {w.N}, {w.K}) failed: status {rc}")
 
@@ -123,7 +124,8 @@ class Pi05DecoderNvfp4Pipeline(StepIO):
                     if rc != 0:
                         raise fvk.KernelError(f"NVFP4 QKV GEMM failed: status {rc}")
                 else:
-                    self._gemm(self.act4, self.act4_sf, w["qkv"], self.qkv, stream, pdl)
+                    # one chunk: the sums of the fused form
+                    self._gemm(self.act4, self.act4_sf, w["qkv"], self.qkv, stream, pdl, chain=B > 1)
                     for b in range(B):
                         self._split_rope(i, b, self.qkv[b * S:], self.q[b * S:], S, stream, pdl and b == 0)
                 self._attention(i, stream, pdl)

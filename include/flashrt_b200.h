@@ -414,15 +414,19 @@ int frt_b200_norm_nvfp4(void* residual, const void* x, const void* gate_in, long
  *   beta is not supported (the decoder path calls with beta = 0).  One kernel for every variant index.
  *   splits: 0 = choose (1: M <= 256 rows on one split of the small-M kernel); flags: bit0 = the weights are settled and may be
  *   read before the kernel in front has ended, bit1 = one-tile-per-CTA kernel for M > 256 (bits 0-1 as frt_b200_gemm_fp8_nt),
+ *   bit2 = a link of a chain of launches: at 65 to 256 rows and splits = 0 tiles of 64 rows with up to four K splits instead of
+ *   CTA pairs where that keeps more SMs busy (another order of the sums; not with bit 1 or bits 8-9),
  *   bits 8-9 = tile columns on CTA pairs (1 = 128, 2 = 192, 3 = 256; 0 = choose).
  *   At most 64 rows: the split chosen for splits = 0, and with it the order of the sums, depends on bit 0 (a chain of launches
- *   wants more and smaller CTAs than one launch).  The same bits with and without early reads: give the split. */
+ *   wants more and smaller CTAs than one launch).  The same bits with and without early reads: give the split.  Above 64 rows
+ *   bit 0 changes no bits. */
 int frt_b200_gemm_nvfp4_nt(const void* A, const void* SFA, const void* W, const void* SFW, void* D, int M, int N,
                            int K, float alpha, const float* d_alpha, const void* bias, int splits, int flags,
                            void* stream);
 /* cutlass_fp4_gemm_variant (csrc/fp4_bindings.cpp:355-370) + qkv_split_rope_kvcache_fp16[_devpos,_vec] fused, the pair
  * called at flash_rt/models/pi05/pipeline_thor.py:366-385:
- *   the NVFP4 form of frt_b200_gemm_fp8_nt_rope_split. */
+ *   the NVFP4 form of frt_b200_gemm_fp8_nt_rope_split.  splits and flag bit 0 as above; bit 2 is not looked at: the sums are those
+ *   of the plain product without it. */
 int frt_b200_gemm_nvfp4_nt_rope_split(const void* A, const void* SFA, const void* W, const void* SFW, int M, int K,
                                       float alpha, const void* rope, void* Q, void* Kout, void* Vout,
                                       const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim, int splits,

@@ -1,6 +1,5 @@
-"""NVFP4 products of 65 to 256 rows in a chain of launches (weights fetched early): m-tiles of 64 rows on the token-major kernel, odd ones
-on the upper half of the operand and of the scale atoms; a last tile of one row, of weight rows that end inside a tile, every split,
-and shapes that stay with the other kernels."""
+"""NVFP4 products of 65 to 256 rows with weights fetched early: a last tile of one row, of weight rows that end inside a tile, short
+and long K.  The quantiser of few rows.  (The form of such products for chains of launches: test_u_nvfp4_chain_flag_gpu.py.)"""
 import numpy as np
 import pytest
 
