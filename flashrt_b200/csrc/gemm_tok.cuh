@@ -1080,16 +1080,27 @@ static TokPlan pick_tok_nvfp4(int M, int N, int K, int want, bool chain) {
     return best;
 }
 
-// 65 to 256 rows in a chain, where the caller asks for it: m-tiles of 64, tiles of 64 weight rows, the largest split with a CTA per SM (its k-blocks all in the ring).
-// On CTA pairs a product of N = 1024 is 8 tiles, 16 CTAs, each with the whole of K: loops of 2 x 50 on 768 keys 8.56 -> 7.73 ms, 3 x 50
-// on 400 8.53 -> 8.12, 4 x 20 on 200 7.65 -> 6.95, 4 x 50 on 768 9.11 -> 8.83.  What has more tiles than SMs stays on the pairs (QKV of
-// 200 rows, gate|up).
+// 65 to 256 rows in a chain, where the caller asks for it: m-tiles of 64, tiles of 64 weight rows, the largest split that pays (its
+// k-blocks all in the ring).  On CTA pairs a product of N = 1024 is 8 tiles, 16 CTAs, each with the whole of K: loops of 2 x 50 on 768
+// keys 8.56 -> 7.73 ms, 3 x 50 on 400 8.53 -> 8.12, 4 x 20 on 200 7.65 -> 6.95, 4 x 50 on 768 9.11 -> 8.83.  What has more tiles than
+// SMs stays on the pairs (QKV of 200 rows, gate|up), and so does what many CTAs cost more than they give.  A sweep of such products
+// behind a norm in a graph (M 65 .. 256, N 512 .. 4736, K 256 .. 8192; us a product with its norm, pairs against this): above three
+// quarters of the SMs a split pays from eight k-blocks on (128 x 1024 x 2048 6.6 / 6.1; 192 x 1536 x 512 4.7 / 5.2), without a split up
+// to two k-blocks do (65 x 4736 x 512 4.94 / 4.84), three and four with fewer CTAs (128 x 2560 x 1024 5.5 / 5.2; 65 x 4736 x 1024
+// 5.6 / 6.0), more never (65 x 4736 x 2048 6.7 / 7.9, 192 x 2560 x 2048 6.9 / 7.7).  Between three quarters and seven eighths with
+// tiles at least two thirds full the product alone is a little slower (150 x 2560 x 1024 5.5 / 5.6) and the loop faster: QKV of
+// 3 x 50 tokens on 400 keys 8.13 / 8.00 ms, 4 x 40 on 300 8.50 / 8.45.
 static TokPlan pick_tok_nvfp4_rows(int M, int N, int K) {
     const TokPlan none = {0, 0, 0, 0, 1};
     const int kbt = K / 256, sms = device_sm_count(), m_tiles = (M + 63) / 64, tiles = (N + 63) / 64 * m_tiles;
     if ((N & 7) || M <= 64 || M > 256) return none;
-    for (int S = 4; S >= 1; S /= 2)
-        if (kbt % S == 0 && kbt / S <= 8 && tiles * S <= sms) return {64, S, kbt / S, kbt / S, m_tiles};
+    for (int S = 4; S >= 1; S /= 2) {
+        if (kbt % S || kbt / S > 8 || tiles * S > sms) continue;
+        const bool crowded = 4 * tiles * S > 3 * sms;
+        const bool full = 8 * tiles * S <= 7 * sms && 3 * M >= 2 * 64 * m_tiles;
+        if (S == 1 ? kbt > (crowded && !full ? 2 : 4) : crowded && kbt < 8) continue;
+        return {64, S, kbt / S, kbt / S, m_tiles};
+    }
     return none;
 }
 

@@ -117,3 +117,19 @@ def test_where_the_chain_form_runs(M, N, K, chain):
     for other in (2, 0x100):                               # a kernel that is asked for stays the one that runs
         assert np.array_equal(_product(d, M, N, K, 0, 1 | other), _product(d, M, N, K, 0, 5 | other))
     assert np.array_equal(_product(d, M, N, K, 1, 1), _product(d, M, N, K, 1, 5))
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 4736, 2048), (65, 4736, 1024), (80, 3584, 1024), (192, 2560, 2048), (65, 2560, 2048),
+                                   (128, 4736, 2048), (192, 2560, 1280)])
+def test_chain_form_stays_off_where_pairs_are_faster(M, N, K):
+    """Unsplit products of many CTAs.  The unsplit form on the token-major kernel and the pairs add in the same order, so the
+    kernel is read from the launch."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from gpu_util import Dev
+    d = [Dev(x) for x in _order_operands(np.random.default_rng(1), M, N, K)]
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        _product(d, M, N, K, 0, 5)
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages() if "gemm" in e.key]
+    assert names and all("pair" in n for n in names), names
