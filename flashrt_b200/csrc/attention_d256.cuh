@@ -434,6 +434,7 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
 #pragma unroll 1
                 for (int c = 0; c < DV; c += 64) {
                     uint32_t va[64];
+                    __syncwarp();                               // the lanes part in the push
                     if (nchunks > 0) {                          // warp-uniform: the loads are warp-collective
                         tc::tmem_ld32(tmem_O + c, va);
                         tc::tmem_ld32(tmem_O + c + 32, va + 32);
@@ -513,8 +514,10 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
                             __stcg(dst, o);
                         }
                     }
+                    __syncwarp();
                 };
                 uint32_t va[64], vb[64];
+                __syncwarp();
                 if (nchunks > 0) {                              // warp-uniform: the loads are warp-collective
                     tc::tmem_ld32(tmem_O + 0, va);
                     tc::tmem_ld32(tmem_O + 32, va + 32);
@@ -554,6 +557,7 @@ __device__ __forceinline__ void attn_d256_body(const CUtensorMap& tmQ, const CUt
 #pragma unroll 1
                 for (int c = 0; c < D; c += 32) {
                     uint32_t v[32];
+                    __syncwarp();                               // the lanes part in the store
                     if (nchunks > 0) {
                         tc::tmem_ld32(tmem_O + c, v);
                         tc::tmem_ld_wait();

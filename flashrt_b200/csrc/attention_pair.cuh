@@ -333,6 +333,7 @@ __device__ __forceinline__ void attn_pair_body(const CUtensorMap& tmQ, const CUt
 #pragma unroll 1
                 for (int c = 0; c < D; c += 32) {
                     uint32_t v[32];
+                    __syncwarp();                               // the lanes part in the store
                     if (nchunks > 0) {
                         tc::tmem_ld32(tmem_O + c, v);
                         tc::tmem_ld_wait();

@@ -406,6 +406,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
 #pragma unroll 1
                 for (int c = 0; c < BN; c += 32) {
                     uint32_t v[32];
+                    __syncwarp();                           // the lanes part in the store
                     if (BN >= 32) tc::tmem_ld32(trow + c, v); else tc::tmem_ld16(trow + c, v);
                     tc::tmem_ld_wait();
                     if (n < p.N) {
@@ -422,6 +423,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__
 #pragma unroll 1
                 for (int c = 0; c < BN; c += 32) {
                     uint32_t v[32];
+                    __syncwarp();                           // the lanes part in the store
                     if (BN >= 32) tc::tmem_ld32(trow + c, v); else tc::tmem_ld16(trow + c, v);
                     tc::tmem_ld_wait();
                     if (m < p.M) {

@@ -178,6 +178,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams& p, uint32_t t_sr
 #pragma unroll 1
     for (int c = 0; c < NC; c += 32) {
         uint32_t v[32];
+        __syncwarp();                                       // the lanes part where they store their own rows
         tc::tmem_ld32(t_src + c, v);
         tc::tmem_ld_wait();
         const int nb = n0 + c;
@@ -238,6 +239,7 @@ __device__ __forceinline__ void epilogue_geglu_rows(const GemmParams& p, uint32_
     if (m_base >= p.M) return;
     const int m = m_base + (threadIdx.x & 31);
     uint32_t g[32], u[32], w[8];
+    __syncwarp();                                           // lanes beyond M skip the stores of the call before
     tc::tmem_ld32(t_gate, g);
     tc::tmem_ld32(t_up, u);
     tc::tmem_ld_wait();
@@ -285,6 +287,7 @@ __device__ __forceinline__ void rope_table_rows(const GemmParams& p, int m, int 
 __device__ __forceinline__ void epilogue_rope_rows(const GemmParams& p, uint32_t t_src, int m, int n0, float alpha, int pos,
                                                    const uint4* tab) {
     uint32_t a[64];
+    __syncwarp();                                           // lanes beyond M skip the stores of the call before
     tc::tmem_ld32(t_src, a);
     tc::tmem_ld32(t_src + 32, a + 32);
     tc::tmem_ld_wait();

@@ -632,6 +632,7 @@ gemm_tok_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll 1
             for (int c = chalf * (BN / 2); c < (chalf + 1) * (BN / 2); c += 32) {
                 uint32_t v[32];
+                __syncwarp();                               // tcgen05.ld is the whole warp's; the lanes part below
                 tc::tmem_ld32(trow + c, v);
                 tc::tmem_ld_wait();
                 if (row < Mt && owner == rank) {            // this rank's own tokens do not leave the SM

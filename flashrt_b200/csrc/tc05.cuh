@@ -374,6 +374,7 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
     return r;
 }
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();                                           // the form is aligned: lanes may come from code that parted them
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t dsmem_map(uint32_t local_smem_addr, uint32_t cta_rank) {

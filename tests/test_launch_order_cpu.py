@@ -70,3 +70,48 @@ def test_shared_memory_limit_of_a_kernel_does_not_follow_the_launch():
     for v in values:                   # no name of a variable: constants and what they make up
         words = set(re.findall(r"[A-Za-z_]\w*", v)) - {"int", "sizeof", "float", "el", "Cfg", "smem_bytes", "ragged_smem_bytes", "true"}
         assert all(w.isupper() for w in words), v
+
+
+def _block(text, at):
+    """The braces that open behind `at`, with what is between them."""
+    start = i = text.index("{", at)
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+        if depth == 0:
+            return text[start:i]
+
+
+LANE_CONDITION = re.compile(r"if \((?:row (?:<|>=) (?:Mt|rows_valid)|m (?:<|>=) p\.M|n < p\.N|store|!lines && m < p\.M)\b")
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and f != "tc05.cuh" and "tmem_ld32(" in source(f)))
+def test_lanes_with_stores_of_their_own_meet_before_the_next_collective_load(name):
+    """tcgen05.ld is an aligned instruction.  A block that loads and then lets some lanes store and others not, and comes round to
+    the load again (a loop, or a function called in one), has a warp barrier in front of the load."""
+    text = source(name)
+    heads = [m.start() for m in re.finditer(r"for \(int c\w* = ", text)]
+    heads += [m.start() for m in re.finditer(r"void epilogue_(?:geglu|rope)_rows\(", text)]
+    for at in heads:
+        body = _block(text, at)
+        load = body.find("tmem_ld")
+        if load < 0 or not LANE_CONDITION.search(body, load) or "for (int c" in body[:load]:
+            continue
+        assert "__syncwarp();" in body[:load], body[:400]
+    for m in re.finditer(r"auto emit = \[&\]", text):      # stores of some lanes between two loads
+        assert re.search(r"__syncwarp\(\);\s*\}$", _block(text, m.start())), name
+
+
+def test_aligned_cluster_barriers_stand_behind_a_warp_or_block_barrier():
+    """barrier.cluster's aligned forms want the warp together: __syncwarp or __syncthreads comes last in front of each, with no
+    branch between."""
+    for name in sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))):
+        text = source(name)
+        for helper in ("cluster_arrive_release", "cluster_wait_acquire"):      # their callers are looked at instead
+            text = re.sub(r"void %s\(\) \{[^}]*\}" % helper, "", text)
+        for m in re.finditer(r"barrier\.cluster\.(?:arrive|wait)[.\w]*aligned|cluster_(?:arrive_release|wait_acquire)\(\);", text):
+            front = text[:m.start()]
+            at = max(front.rfind("__syncwarp();"), front.rfind("__syncthreads();"))
+            between = re.sub(r"if (?:constexpr )?\((?:XC|!XC|EPI == [^()]*)\)", "", front[at:])     # compile-time conditions
+            assert at >= 0 and not re.search(r"\b(?:if|for|while)\b", between), (name, between)
