@@ -998,8 +998,10 @@ static int launch_gemm_tok(const void* A, const void* W, TokParams p, int K, con
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
-    // more CTAs than the device holds: those that wait for a place keep the kernel behind out anyway (4 x 50 tokens, 320 CTAs of the QKV
-    // product: the loop 7.57 ms, let in late 7.64)
+    // more than two CTAs per SM, which no device holds at once: those that wait for a place keep the kernel behind out anyway (4 x 50
+    // tokens, 320 CTAs of the QKV product: the loop 7.57 ms, let in late 7.64).  One or two per SM are let in late also where each
+    // needs an SM to itself: the line between the two has no one side (us in a chain, at once / late: 50 x 49152 x 1024 as 192 CTAs
+    // 18.35 / 18.52, 50 x 24576 x 2048 as 192 19.29 / 19.54, 128 x 14336 x 2048 as 224 17.6 / 17.7, 50 x 8192 x 8192 as 256 22.9 / 22.3)
     p.early = (pdl ? 1 : 0) | ((long long)tiles * m_tiles * pl.S > 2 * device_sm_count() ? 2 : 0);
     cfg.attrs = attr;
     cfg.numAttrs = na;
