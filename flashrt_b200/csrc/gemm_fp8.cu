@@ -1065,6 +1065,13 @@ static int launch_large(int kind, const void* A, const void* W, const GemmParams
 
 using namespace frt;
 
+// RoPE + split finishes: eight features at a time, 16-byte table reads and stores
+static inline int rope_split_status(const void* rope, const void* Q, const void* K, const void* V, int q_dim, int k_dim, int v_dim,
+                                    int head_dim) {
+    if ((head_dim % 8) || (q_dim % head_dim) || (k_dim % head_dim) || (v_dim % 8)) return FRT_ERR_UNSUPPORTED;
+    return ((reinterpret_cast<uintptr_t>(rope) | reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(K) |
+             reinterpret_cast<uintptr_t>(V)) & 15) ? FRT_ERR_INVALID : FRT_OK;
+}
 // flags bits 8-9: tile-width hint of the token-major small-M kernel (1 = 64, 2 = 128, 3 = 256 weight rows)
 static inline int tok_bn_hint(int flags) {
     const int h = (flags >> 8) & 3;
@@ -1226,9 +1233,8 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
                                     int flags, void* stream) {
     if (!A || !W || !rope || !Q || !Kout || !Vout || M < 0 || K <= 0) return FRT_ERR_INVALID;
     if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
-    if ((K % 16) || M > 256 || (head_dim & 1) || (q_dim % head_dim) || (k_dim % head_dim) || (q_dim & 1) ||
-        (k_dim & 1))
-        return FRT_ERR_UNSUPPORTED;
+    if ((K % 16) || M > 256) return FRT_ERR_UNSUPPORTED;
+    if (const int rc = rope_split_status(rope, Q, Kout, Vout, q_dim, k_dim, v_dim, head_dim)) return rc;
     if (M == 0) return FRT_OK;
     GemmParams p = {};
     p.sa = d_scale_a;
@@ -1246,7 +1252,7 @@ int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, 
     p.k_dim = k_dim;
     p.v_dim = v_dim;
     p.head_dim = head_dim;
-    if (tok_eligible(M, p.N, K, flags) && M <= 128 && (head_dim % 8) == 0) {
+    if (tok_eligible(M, p.N, K, flags) && M <= 128) {
         TokParams t = {};
         t.M = M; t.N = p.N; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = 1.0f;
         t.rope = p.rope; t.outQ = p.outQ; t.outK = p.outK; t.outV = p.outV; t.devpos = devpos;
@@ -1274,6 +1280,7 @@ int frt_b200_gemm_fp8_nt_geglu_fp8(const void* A, const void* W, void* out8, int
     if ((K % 16) || (half % 64)) return FRT_ERR_UNSUPPORTED;
     if (M > 256 && ((half % 128) || (reinterpret_cast<uintptr_t>(out8) & 15) || (flags & (16 | 64 | 128))))
         return FRT_ERR_UNSUPPORTED;
+    if (reinterpret_cast<uintptr_t>(out8) & 7) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     GemmParams p = {};
     p.sa = d_scale_a;
@@ -1368,9 +1375,8 @@ int frt_b200_gemm_nvfp4_nt_rope_split(const void* A, const void* SFA, const void
                                       int flags, void* stream) {
     if (!A || !SFA || !W || !SFW || !rope || !Q || !Kout || !Vout || M < 0 || K <= 0) return FRT_ERR_INVALID;
     if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
-    if ((K % 256) || M > 256 || (head_dim & 1) || (q_dim % head_dim) || (k_dim % head_dim) || (q_dim & 1) ||
-        (k_dim & 1))
-        return FRT_ERR_UNSUPPORTED;
+    if ((K % 256) || M > 256) return FRT_ERR_UNSUPPORTED;
+    if (const int rc = rope_split_status(rope, Q, Kout, Vout, q_dim, k_dim, v_dim, head_dim)) return rc;
     if ((reinterpret_cast<uintptr_t>(SFA) & 15) || (reinterpret_cast<uintptr_t>(SFW) & 15)) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     GemmParams p = {};
@@ -1390,9 +1396,7 @@ int frt_b200_gemm_nvfp4_nt_rope_split(const void* A, const void* SFA, const void
     p.v_dim = v_dim;
     p.head_dim = head_dim;
     // on CTA pairs where the plain product goes there (without its bit 2): the same sums, so the pair of launches gives the same bytes
-    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(rope) | reinterpret_cast<uintptr_t>(Q) |
-                           reinterpret_cast<uintptr_t>(Kout) | reinterpret_cast<uintptr_t>(Vout);
-    if (splits <= 0 && !(ptrs & 15) && !((q_dim | k_dim | v_dim | head_dim) & 7) && pick_nvfp4_pair(M, p.N, K)) {
+    if (splits <= 0 && pick_nvfp4_pair(M, p.N, K)) {
         p.early = flags & 1;
         return launch_gemm_pair<128, EPI_P_ROPE, false, true>(A, W, p, K, (cudaStream_t)stream);
     }
@@ -1528,8 +1532,8 @@ int frt_b200_gemm_fp8_nt_rope_split_batched(const void* A, const void* W, int M,
     if (!A || !W || !rope || !Q || !Kout || !Vout || M < 0 || K <= 0 || rows_per_batch < 0) return FRT_ERR_INVALID;
     if (stats_in && (!col_term || n_stat <= 0)) return FRT_ERR_INVALID;
     if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
-    if ((K % 128) || M > 256 || (head_dim % 8) || (q_dim % head_dim) || (k_dim % head_dim) || (v_dim % 8))
-        return FRT_ERR_UNSUPPORTED;
+    if ((K % 128) || M > 256) return FRT_ERR_UNSUPPORTED;
+    if (const int rc = rope_split_status(rope, Q, Kout, Vout, q_dim, k_dim, v_dim, head_dim)) return rc;
     if ((reinterpret_cast<uintptr_t>(col_term) & 15) || (kv_batch_stride & 7)) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     TokParams t = {};
@@ -1570,7 +1574,7 @@ int frt_b200_gemm_fp8_nt_geglu_fp8_rowscale(const void* A, const void* W, void* 
     if (!A || !W || !out8 || !stats_in || !col_term || !d_out_scale || M < 0 || half <= 0 || K <= 0 || n_stat <= 0)
         return FRT_ERR_INVALID;
     if ((K % 128) || M > 256 || (half % 64)) return FRT_ERR_UNSUPPORTED;
-    if (reinterpret_cast<uintptr_t>(col_term) & 15) return FRT_ERR_INVALID;
+    if ((reinterpret_cast<uintptr_t>(col_term) & 15) || (reinterpret_cast<uintptr_t>(out8) & 7)) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     TokParams t = {};
     t.M = M; t.N = 2 * half; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = 1.0f;
@@ -1594,8 +1598,8 @@ int frt_b200_norm_gemm_fp8_nt_rope_split(const void* x, const float* stats_in, i
     if (!x || !stats_in || !style || !W || !rope || !Q || !Kout || !Vout || !d_scale_a || M < 0 || K <= 0 || n_stat <= 0)
         return FRT_ERR_INVALID;
     if (q_dim <= 0 || k_dim <= 0 || v_dim <= 0 || head_dim <= 0) return FRT_ERR_INVALID;
-    if ((K % 128) || M > 128 || (head_dim % 8) || (q_dim % head_dim) || (k_dim % head_dim) || (v_dim % 8))
-        return FRT_ERR_UNSUPPORTED;
+    if ((K % 128) || M > 128) return FRT_ERR_UNSUPPORTED;
+    if (const int rc = rope_split_status(rope, Q, Kout, Vout, q_dim, k_dim, v_dim, head_dim)) return rc;
     if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(style) & 15)) return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     TokParams t = {};
@@ -1619,7 +1623,8 @@ int frt_b200_norm_gemm_fp8_nt_geglu_fp8(const void* x, const float* stats_in, in
         n_stat <= 0)
         return FRT_ERR_INVALID;
     if ((K % 128) || M > 128 || (half % 64)) return FRT_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(style) & 15)) return FRT_ERR_INVALID;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(style) & 15) || (reinterpret_cast<uintptr_t>(out8) & 7))
+        return FRT_ERR_INVALID;
     if (M == 0) return FRT_OK;
     TokParams t = {};
     t.M = M; t.N = 2 * half; t.sa = d_scale_a; t.sb = d_scale_b; t.alpha_host = 1.0f;

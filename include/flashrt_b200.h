@@ -148,14 +148,14 @@ int frt_b200_gemm_fp8_nn(const void* A, const void* B, void* D, int M, int N, in
  *   rope (M, head_dim) = [cos0, sin0, cos1, sin1, ...]; Q -> (M, q_dim); K / V rows -> row (*devpos + m)
  *   of Kout / Vout (devpos NULL: row m).  Byte-identical to frt_b200_gemm_fp8_nt followed by frt_b200_qkv_split_rope when
  *   both are given the same `splits` of 1, 2, 4 or 8; with splits = 0 the two choose on their own (see
- *   frt_b200_gemm_fp8_nn). */
+ *   frt_b200_gemm_fp8_nn).  head_dim % 8 == 0, v_dim % 8 == 0; rope, Q, Kout, Vout 16-byte aligned (all RoPE finishes). */
 int frt_b200_gemm_fp8_nt_rope_split(const void* A, const void* W, int M, int K, const float* d_scale_a,
                                     const float* d_scale_b, const void* rope, void* Q, void* Kout, void* Vout,
                                     const int* devpos, int q_dim, int k_dim, int v_dim, int head_dim, int splits,
                                     int flags, void* stream);
 /* gate|up projection + gate_geglu_merged_fp8 (csrc/bindings.cpp:1037-1044 -> csrc/kernels/activation.cu:249-279):
  *   W (2*half, K), rows [0, half) = gate, [half, 2*half) = up; out8 (M, half) e4m3 with scale *d_out_scale.
- *   half % 64 == 0; M > 256: half % 128 == 0, out8 16-byte aligned.  Byte-identical to frt_b200_gemm_fp8_nt followed by
+ *   half % 64 == 0, out8 8-byte aligned; M > 256: half % 128 == 0, out8 16-byte aligned.  Byte-identical to frt_b200_gemm_fp8_nt followed by
  *   frt_b200_geglu_fp8 when both are given the same `splits` of 1, 2, 4 or 8 (M > 256: when that product is not split).
  *   flags bit 6: SiLU gate (SwiGLU; M <= 128 and K % 128 == 0 only, else -2), byte-identical to frt_b200_geglu_fp8
  *   with its flags bit 1 behind the same GEMM.
