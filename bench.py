@@ -356,9 +356,9 @@ def run_ours(args):
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4),
                          # not measured in this run: dram read + write of one launch from the ncu capture of the
-                         # attention-out projection under profiles/ (2.335 MB, 1.013 x the algorithmic read bytes; the
+                         # attention-out projection under profiles/ (2.334 MB, 1.012 x the algorithmic read bytes; the
                          # result stays in L2), scaled by bytes
-                         "traffic": int(1.013 * (gemm_bytes - gemm_out_bytes)),
+                         "traffic": int(1.012 * (gemm_bytes - gemm_out_bytes)),
                          "traffic_source": "carried over from the ncu capture in profiles/, scaled by bytes",
                          "peak_source": peak_src,
                          "avg_launch_us": round(gemm_us, 3), "algorithmic_bytes_per_launch": int(gemm_bytes)},
@@ -801,6 +801,29 @@ def run_timeline(args):
             cols = (a[:, 0].min(), np.median(a[:, 3]), np.median(a[:, 4]), np.median(a[:, 6]), np.median(a[:, 7]),
                     a[:, 9].max())
         rows.append({"kernel": k, "ctas": int(len(a)), "ns": [float(v) for v in cols]})
+    # block 1 over 75 replays (the mean resolves what a tick of the timer, 0.256 us, does not): us after the last CTA of the launch in
+    # front has ended, median and latest CTA
+    marks = ("starts", "wait returned", "accumulator / P.V", "pushed", "received", "finish done", "ends")
+    sums = np.zeros((5, len(marks), 2))
+    for _ in range(75):
+        with torch.cuda.stream(s):
+            gr.replay()
+        s.synchronize()
+        tt, ta = read(0)
+        stamps = []
+        for i in range(4, 10):                             # FFN-down of block 0, then block 1
+            att = kinds[i] == "attention"
+            a = ta[kinds[:i].count("attention") % 8] if att else tt[(i - kinds[:i].count("attention")) % 8]
+            stamps.append(a[a[:, 0] > 0][:, (0, 1, 7, 8, 10, 11, 12) if att else (0, 3, 4, 5, 6, 7, 9)])
+        for j in range(5):
+            rel = (stamps[j + 1] - stamps[j][:, -1].max()) / 1e3
+            sums[j] += np.stack([np.median(rel, axis=0), rel.max(axis=0)], axis=-1)
+    replays = [{"kernel": kinds[5 + j], "us": {m: [round(float(v), 2) for v in sums[j, c] / 75] for c, m in enumerate(marks)}}
+               for j in range(5)]
+    print("block 1, mean of 75 replays, us after the last CTA of the launch in front (median / latest CTA): " + " | ".join(marks),
+          file=sys.stderr)
+    for r in replays:
+        print(f"{r['kernel']:16s} " + "  ".join(f"{a:6.2f} / {b:5.2f}" for a, b in r["us"].values()), file=sys.stderr)
     t0 = rows[0]["ns"][0]
     for r in rows:
         r["us"] = [round((v - t0) / 1e3, 2) for v in r.pop("ns")]
@@ -847,7 +870,7 @@ def run_timeline(args):
             splits.append({"split": z, "us": us})
             print(f"  split {z!s:8s} " + "  ".join(f"{v:6.2f}" for v in us), file=sys.stderr)
     print(json.dumps({"metric": "operator-graph phase timeline (diagnostic)", "unit": "us", "rows": rows,
-                      "block_us": rows[-1]["us"][-1] - rows[4]["us"][-1], "attention_splits": splits}), flush=True)
+                      "block_us": rows[-1]["us"][-1] - rows[4]["us"][-1], "attention_splits": splits, "block_1_replays": replays}), flush=True)
 
 
 # ---------------------------------------------------------------------------------------------------------------

@@ -1506,7 +1506,7 @@ int frt_b200_gemm_fp8_nt_gate_residual_q8(const void* A, const void* W, int M, i
     if (pl.BN == 128)
         return launch_gemm_tok<128, TOK_PRO_TMA, TOK_EPI_RESID>(A, W, t, K, pl, flags & 1, (cudaStream_t)stream);
     const int rank_tokens = ((M + mts - 1) / mts + pl.S - 1) / pl.S;
-    if (rank_tokens <= 8)                                  // two warps' items of eight features at most
+    if (rank_tokens <= 8)                                  // two warps' items of eight features at most (see ACT)
         return launch_gemm_tok<64, TOK_PRO_TMA, TOK_EPI_RESID, 1>(A, W, t, K, pl, flags & 1, (cudaStream_t)stream);
     return launch_gemm_tok<64, TOK_PRO_TMA, TOK_EPI_RESID>(A, W, t, K, pl, flags & 1, (cudaStream_t)stream);
 }

@@ -37,8 +37,8 @@
 // from the beginning.  A CTA that starts costs the one beside it: the softmax of the attention took 1.3 us instead of 0.75 when the
 // attention-out CTAs started under it.  gate|up lets it in when its own wait has returned, QKV and the gated residual with the
 // accumulator, the plain result (whose dependents are small) behind the push: all times and products of the loops tried.  With the
-// attention's (behind its softmax) and the carve-outs that let CTAs share an SM: loop of 50 tokens on 768 keys 4.82 -> 4.62 ms,
-// NVFP4 5.95 -> 5.82, guided 5.98 -> 5.93.
+// attention's (behind its softmax) and the carve-outs that let CTAs share an SM: loop of 50 tokens on 768 keys 4.82 -> 4.66 ms,
+// NVFP4 5.95 -> 5.80, guided 5.98 -> 5.91.
 //
 // Warps: 0 (lane 0) TMA producer, 1 (lane 0) MMA issuer, 2 TMEM owner; all 8 warps stage and finish the tile.
 // Every wait is bounded by the kernel deadline; on expiry the status word is set, the work is skipped and every
@@ -136,7 +136,7 @@ struct TokParams {
 #endif
 };
 
-// FP4 (BF16 and RoPE finishes, m-tiles of 64 tokens): k-blocks of 256 packed e2m1 elements, the scale atoms of both operands behind the
+// FP4 (BF16 finish, and RoPE for one m-tile; m-tiles of 64 tokens): k-blocks of 256 packed e2m1 elements, the scale atoms of both operands behind the
 // operand tiles.  The block-scaled MMA has M = 128 only, and an atom holds the scales of 128 rows: an even m-tile is the lower 64 rows of
 // the operand and the weight tile behind its 8 KB the upper, an odd one the upper 64 rows and the weight tile, in front of it there, the
 // lower.  The results of those lanes are never looked at; every row that an MMA reads lies in its stage.
@@ -234,7 +234,7 @@ struct alignas(2 * VW) TokVec {
 // ACT, gated residual: 1 = items of four features instead of eight.  A rank of eight splits finishes few tokens (7 of 50), whose items
 // of eight are the work of two warps with six idle, and the finish takes as long as an item's code: attention-out 0.75 -> 0.5 us from
 // the last slot to the result, the loop of 50 tokens on 768 keys 4.66 -> 4.60 ms; with 25 tokens of a rank it is two rounds instead of
-// one (4 x 50 tokens 7.54 -> 7.59).
+// one (4 x 50 tokens 7.54 -> 7.59).  The line is at eight tokens; nine to sixteen would be one round too and were not timed.
 // ACT, GeGLU: the gate activation, 0 exact GELU(tanh), 1 SiLU, 2 GELU through the hardware tanh.  A
 // template argument, not a field of the parameters: selected at run time inside the unrolled finish the choice cost
 // 0.55 us per gate|up launch of the action-expert loop (0.10 ms per loop), a third of that epilogue's arithmetic.

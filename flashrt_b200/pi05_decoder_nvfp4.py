@@ -70,9 +70,9 @@ class Pi05DecoderNvfp4Pipeline(StepIO):
         self.hid4, self.hid4_sf = z(M, DEC_H // 2, dtype=torch.uint8), sfb(DEC_H)
         self.ones = torch.ones(DEC_D, dtype=BF16, device=dev)
         self.attn_splits = fe.attn_splits
-        # eight splits at every batch size.  Chosen by size (flag 16, as in the FP8 loop) 4 x 50 tokens take 9.03 instead of 9.18 ms, but
-        # the sums are then split differently at batch 4 and batch 1, and a batch no longer equals its single runs within the
-        # bound that NVFP4's own steps allow (largest difference 2.9e-2, 2 % of the actions' RMS are 2.4e-2)
+        # eight splits at every batch size.  Chosen by size (flag 16, as in the FP8 loop) 4 x 50 tokens on 768 keys take 8.34 instead of
+        # 8.60 ms, but the sums are then split differently at batch 4 and batch 1, and a batch no longer equals its single runs within
+        # the bound that NVFP4's own steps allow (largest difference 3.0e-2, 2 % of the actions' RMS are 2.4e-2; with eight splits 0)
         self.attn_flags = 0
         self.o_accum = z(self.attn_splits, B, S, DEC_NH, DEC_HD, dtype=torch.float32)
         self.lse_accum = z(self.attn_splits, B, DEC_NH, S, dtype=torch.float32)
